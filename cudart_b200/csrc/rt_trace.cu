@@ -995,37 +995,29 @@ __device__ __forceinline__ void trace_warp_coop_clusters(const uint32_t r, const
   }
 }
 
-// A float as an unsigned key of the same order (for warp minimum reductions).
-__device__ __forceinline__ uint32_t order_key(float f) {
-  const uint32_t u = __float_as_uint(f);
-  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-// Compare-exchange of packet slots on a warp-uniform key, the lane's own entry distance and the reference riding along.
-__device__ __forceinline__ void cswap_packet(uint32_t (&key)[4], float (&t)[4], uint32_t (&r)[4], int a, int b) {
-  if (key[b] < key[a]) {
-    const uint32_t kk = key[a]; key[a] = key[b]; key[b] = kk;
-    const float tt = t[a]; t[a] = t[b]; t[b] = tt;
-    const uint32_t rr = r[a]; r[a] = r[b]; r[b] = rr;
-  }
-}
-
+constexpr uint32_t kPacketMiss = 0x7f800000u;  // +inf: no lane enters the slot
 // Packet walk of the cluster tree: the 32 lanes of a warp trace rays of one
 // mesh along one node sequence. Every lane tests the same record (one load,
 // shared by the warp) against its own ray; a slot is entered when some lane's
 // ray enters it within that lane's reach, slots in order of the warp's
-// smallest entry distance, and a stacked slot is skipped once no lane can
-// still find a closer hit in it (each lane keeps its own entry distances).
-// At a cluster the lanes whose ray enters it test its triangles. Lanes whose
-// ray is idle (no ray, or tmax <= 0) ride along without tests. For coherent
+// smallest entry distance, and a stacked slot is skipped once that distance is
+// out of every lane's reach. At a cluster every lane tests its triangles.
+// Lanes whose ray is idle (no ray, or tmax <= 0) reach nothing. For coherent
 // rays (pixel tiles) the warp stays converged where per-lane walks diverge.
-// min_lanes > 0: once fewer lanes than that want the node the packet is at,
+// The stack holds what is the same for the warp -- a reference and the
+// smallest entry distance -- in shared memory (`stack`, kStack entries).
+// kAlone (min_lanes > 0): once fewer lanes than that enter a record's slots,
 // the warp leaves the packet walk and every lane walks on alone from its own
-// copy of the stack (which already holds its own entry distances).
+// copy of the stack.
 // kBounce: also write each ray's bounce (A.b_*); a separate instantiation, since the bounce code alone (taken or
 // not) costs the walk about 3% in a kernel that does not write bounces.
-template <bool kCount, bool kBounce = false>
+// Bound by issue (71% of the slots). With per-lane entry distances stacked in local memory, a five-exchange sort of
+// (key, distance, reference) and a minimum and maximum per plane pair it took 0.91 ms for 1080p camera rays of the
+// 2^20-triangle soup and 3.86 ms for 16.6M of the instanced scene; the warp-wide stack and the sort on packed keys
+// 0.90 and 3.75 ms, the planes read by sign 0.85 and 3.75 ms.
+template <bool kCount, bool kBounce, bool kAlone>
 __device__ __forceinline__ void trace_warp_packet_clusters(const uint32_t r, const bool valid, const TraceArgs& A, const ClusterArgs& C,
-                                                           const uint32_t min_lanes) {
+                                                           const uint32_t min_lanes, uint2* stack) {
   float4 o = make_float4(0.f, 0.f, 0.f, 0.f), d = make_float4(0.f, 0.f, 1.f, 0.f);
   float tmax0 = -1.0f;
   if (valid) {
@@ -1049,111 +1041,176 @@ __device__ __forceinline__ void trace_warp_packet_clusters(const uint32_t r, con
     const float zu = o.w * 0.0f, zv = d.w * 0.0f;
     const float4* tris = A.tris + 3 * (size_t)C.F;
     const float4* recs = C.crec + 8 * (size_t)C.F;
-    uint32_t st_ref[kStack];
-    float st_t[kStack];
-    int sp = 0;
+    const uint32_t ox = ix < 0.0f ? 48u : 0u, oy = iy < 0.0f ? 48u : 0u, oz = iz < 0.0f ? 48u : 0u;
+    float reach = live ? bt * kCullSlack : -1.0f;  // entry distances this lane can still use (never negative)
+    int sp = 0;                                    // the same for every lane, as ref is
     uint32_t steps = 0;
-    const uint32_t kMiss = order_key(INFINITY);
-    float cur_t = live ? 0.0f : INFINITY;  // this lane's entry distance of the node at hand
-    auto push = [&](uint32_t sref, float st) {
-      if (sp < kStack) {
-        st_ref[sp] = sref;
-        st_t[sp] = st;
-        ++sp;
-      } else if (A.err) {
-        atomicOr(A.err, (uint32_t)RT_DEVERR_STACK_OVERFLOW);
-      }
-    };
+    bool alone = false;  // this warp left the packet walk
+    float cur_t = 0.0f;  // counters only: the warp's entry distance of the node at hand
+    uint32_t l_ref[kAlone ? kStack : 1];
+    float l_t[kAlone ? kStack : 1];
     auto test_cluster = [&]() {
       const uint32_t p0 = ref & kClusterFirstMask, p1 = p0 + ((ref >> 28) & 7u) + 1u;
       for (uint32_t pos = p0; pos < p1; ++pos) {
         const float4 v0 = ldg4(tris + 3 * (size_t)pos);
         const float4 e1 = ldg4(tris + 3 * (size_t)pos + 1);
         const float4 e2 = ldg4(tris + 3 * (size_t)pos + 2);
-        if (kCount) ++tests;
         float th, u, v;
         if (!mt_test(o, d, zu, zv, v0, e1, e2, th, u, v)) continue;
         if (th < bt || (best >= 0 && th == bt && (int32_t)pos < best)) {
           best = (int32_t)pos; bt = th; bu = u; bv = v;
         }
       }
+      if (live) reach = bt * kCullSlack;
+      if (kCount && live && cur_t <= reach) tests += p1 - p0;
     };
-    bool alone = false;  // this warp left the packet walk
     for (;;) {
       if (!cluster_ref_ok(ref, C.n, steps)) {
         if (live && A.err) atomicOr(A.err, (uint32_t)RT_DEVERR_ACCEL_MISSING);
         break;
       }
-      const bool want = live && cur_t <= bt * kCullSlack;
-      if (min_lanes && (uint32_t)__popc(__ballot_sync(0xffffffffu, want)) < min_lanes) {
-        if (want) push(ref, cur_t);
-        alone = true;
-        break;
-      }
-      bool next = false;
       if (!(ref & kClusterLeaf)) {
         float t[4];
         uint32_t k[4], key[4];
-        cluster_slots(recs + 8 * (size_t)ref, oi, ix, iy, iz, bt, t, k);
-        if (kCount && want) visits += 4;
+        {
+          // each lane reads the planes its ray enters through and the ones it leaves through by the signs of its
+          // direction (the warp's lanes mostly agree), instead of a minimum and a maximum per pair of planes
+          const char* rb = (const char*)(recs + 8 * (size_t)ref);
+          const float4 nx = ldg4((const float4*)(rb + ox)), fx = ldg4((const float4*)(rb + 48 - ox));
+          const float4 ny = ldg4((const float4*)(rb + 16 + oy)), fy = ldg4((const float4*)(rb + 64 - oy));
+          const float4 nz = ldg4((const float4*)(rb + 32 + oz)), fz = ldg4((const float4*)(rb + 80 - oz));
+          const uint4 wr = ldg4((const uint4*)(rb + 96));
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const float tn = max3f(__fmaf_rn(f4c(nx, q), ix, -oi.x), __fmaf_rn(f4c(ny, q), iy, -oi.y), __fmaf_rn(f4c(nz, q), iz, -oi.z));
+            const float tf = fminf(min3f(__fmaf_rn(f4c(fx, q), ix, -oi.x), __fmaf_rn(f4c(fy, q), iy, -oi.y),
+                                         __fmaf_rn(f4c(fz, q), iz, -oi.z)), reach);
+            t[q] = (tn <= tf && tf >= 0.0f) ? tn : INFINITY;  // an unused slot's tn is NaN
+            k[q] = u4c(wr, q);
+          }
+        }
+        if (kCount && live && cur_t <= reach) visits += 4;
+        // the warp's smallest entry distance of each slot (not below 0), the slot number in its two lowest bits: rounded
+        // down by at most three units in the last place, so a stacked slot is never skipped too early
+        bool mine = false;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          if (!want) t[q] = INFINITY;
-          key[q] = __reduce_min_sync(0xffffffffu, order_key(t[q]));
+          const bool in = t[q] != INFINITY;
+          mine |= in;
+          key[q] = (__reduce_min_sync(0xffffffffu, in ? __float_as_uint(fmaxf(t[q], 0.0f)) : kPacketMiss) & ~3u) | (uint32_t)q;
         }
-        cswap_packet(key, t, k, 0, 1);
-        cswap_packet(key, t, k, 2, 3);
-        cswap_packet(key, t, k, 0, 2);
-        cswap_packet(key, t, k, 1, 3);
-        cswap_packet(key, t, k, 1, 2);
-        if (key[0] != kMiss) {
+        if (kAlone) {
+          const uint32_t m = __ballot_sync(0xffffffffu, mine);
+          if (m && (uint32_t)__popc(m) < min_lanes) {
+            // every lane takes the warp's stack and its own slots of this record, nearest on top
+            for (int i = 0; i < sp; ++i) {
+              l_ref[i] = stack[i].x;
+              l_t[i] = __uint_as_float(stack[i].y);
+            }
+            cswap_tr(t, k, 0, 1);
+            cswap_tr(t, k, 2, 3);
+            cswap_tr(t, k, 0, 2);
+            cswap_tr(t, k, 1, 3);
+            cswap_tr(t, k, 1, 2);
 #pragma unroll
-          for (int q = 3; q >= 1; --q)
-            if (key[q] != kMiss) push(k[q], t[q]);
-          ref = k[0];
-          cur_t = t[0];
-          next = true;
+            for (int q = 3; q >= 0; --q) {
+              if (live && t[q] != INFINITY) {
+                if (sp < kStack) {
+                  l_ref[sp] = k[q];
+                  l_t[sp] = t[q];
+                  ++sp;
+                } else if (A.err) {
+                  atomicOr(A.err, (uint32_t)RT_DEVERR_STACK_OVERFLOW);
+                }
+              }
+            }
+            alone = true;
+            break;
+          }
         }
-      } else if (want) {
+        auto order = [&](int a, int b) {
+          const uint32_t lo = min(key[a], key[b]);
+          key[b] = max(key[a], key[b]);
+          key[a] = lo;
+        };
+        order(0, 1);
+        order(2, 3);
+        order(0, 2);
+        order(1, 3);
+        order(1, 2);
+        auto slot_ref = [&](uint32_t kk) {
+          const uint32_t lo = (kk & 1u) ? k[1] : k[0], hi = (kk & 1u) ? k[3] : k[2];
+          return (kk & 2u) ? hi : lo;
+        };
+        if (key[0] < kPacketMiss) {
+#pragma unroll
+          for (int q = 3; q >= 1; --q) {
+            if (key[q] < kPacketMiss) {
+              if (sp < kStack) {
+                stack[sp] = make_uint2(slot_ref(key[q]), key[q]);
+                ++sp;
+              } else if (A.err) {
+                atomicOr(A.err, (uint32_t)RT_DEVERR_STACK_OVERFLOW);
+              }
+            }
+          }
+          ref = slot_ref(key[0]);
+          if (kCount) cur_t = __uint_as_float(key[0]);
+          __syncwarp();
+          continue;
+        }
+      } else {
         test_cluster();
       }
-      if (next) continue;
       // the nearest stacked slot some lane can still use
       bool more = false;
       while (sp > 0) {
-        --sp;
-        if (__any_sync(0xffffffffu, live && st_t[sp] <= bt * kCullSlack)) {
-          ref = st_ref[sp];
-          cur_t = st_t[sp];
+        const uint2 top = stack[--sp];
+        if (__any_sync(0xffffffffu, __uint_as_float(top.y & ~3u) <= reach)) {
+          ref = top.x;
+          if (kCount) cur_t = __uint_as_float(top.y & ~3u);
           more = true;
           break;
         }
       }
       if (!more) break;
     }
-    if (alone && live) {  // every lane on its own, from its stack
-      bool walking = pop_within(st_ref, st_t, sp, bt, ref);
-      while (walking) {
-        if (!cluster_ref_ok(ref, C.n, steps)) {
-          if (A.err) atomicOr(A.err, (uint32_t)RT_DEVERR_ACCEL_MISSING);
-          break;
-        }
-        if (!(ref & kClusterLeaf)) {
-          float t[4];
-          uint32_t k[4];
-          cluster_test(recs + 8 * (size_t)ref, oi, ix, iy, iz, bt, t, k);
-          if (kCount) visits += 4;
-          if (t[0] != INFINITY) {
-#pragma unroll
-            for (int q = 3; q >= 1; --q)
-              if (t[q] != INFINITY) push(k[q], t[q]);
-            ref = k[0];
-            continue;
+    __syncwarp();  // the next packet of the warp writes the stack again
+    if constexpr (kAlone) {
+      if (alone && live) {  // every lane on its own
+        cur_t = 0.0f;
+        bool walking = pop_within(l_ref, l_t, sp, bt, ref);
+        while (walking) {
+          if (!cluster_ref_ok(ref, C.n, steps)) {
+            if (A.err) atomicOr(A.err, (uint32_t)RT_DEVERR_ACCEL_MISSING);
+            break;
           }
-        } else {
-          test_cluster();
+          if (!(ref & kClusterLeaf)) {
+            float t[4];
+            uint32_t k[4];
+            cluster_test(recs + 8 * (size_t)ref, oi, ix, iy, iz, bt, t, k);
+            if (kCount) visits += 4;
+            if (t[0] != INFINITY) {
+#pragma unroll
+              for (int q = 3; q >= 1; --q) {
+                if (t[q] != INFINITY) {
+                  if (sp < kStack) {
+                    l_ref[sp] = k[q];
+                    l_t[sp] = t[q];
+                    ++sp;
+                  } else if (A.err) {
+                    atomicOr(A.err, (uint32_t)RT_DEVERR_STACK_OVERFLOW);
+                  }
+                }
+              }
+              ref = k[0];
+              continue;
+            }
+          } else {
+            test_cluster();
+          }
+          walking = pop_within(l_ref, l_t, sp, bt, ref);
         }
-        walking = pop_within(st_ref, st_t, sp, bt, ref);
       }
     }
   }
@@ -1569,9 +1626,10 @@ __global__ __launch_bounds__(128) void k_trace_clusters_coop(TraceArgs A, Cluste
   }
 }
 
-template <bool kCount>
+template <bool kCount, bool kAlone>
 __global__ __launch_bounds__(128) void k_trace_clusters_packet(TraceArgs A, ClusterArgs C, SlotMap M, uint32_t* counter,
                                                                 uint32_t min_lanes) {
+  __shared__ uint2 s_stack[4][kStack];
   const uint32_t lane = lane_id();
   C.F = 0;
   for (;;) {
@@ -1582,7 +1640,7 @@ __global__ __launch_bounds__(128) void k_trace_clusters_packet(TraceArgs A, Clus
     uint32_t r = 0;
     const uint32_t s = base + lane;
     const bool valid = s < M.slots && M.ray_of(s, r);
-    trace_warp_packet_clusters<kCount>(r, valid, A, C, min_lanes);
+    trace_warp_packet_clusters<kCount, false, kAlone>(r, valid, A, C, min_lanes, s_stack[threadIdx.x >> 5]);
   }
 }
 
@@ -1655,9 +1713,10 @@ __global__ __launch_bounds__(128, 8) void k_batch_trace_clusters_refill(TraceArg
 
 // Packet walks over batched rays: a warp whose valid rays all belong to one mesh walks it as a packet; a warp
 // spanning meshes falls back to per-lane walks.
-template <bool kCount, bool kBounce>
-__global__ __launch_bounds__(128) void k_batch_trace_clusters_packet(TraceArgs A, BatchTraceArgs B, uint32_t* counter,
+template <bool kCount, bool kBounce, bool kAlone>
+__global__ __launch_bounds__(128, 8) void k_batch_trace_clusters_packet(TraceArgs A, BatchTraceArgs B, uint32_t* counter,
                                                                       uint32_t min_lanes) {
+  __shared__ uint2 s_stack[4][kStack];
   const uint32_t lane = lane_id();
   for (;;) {
     uint32_t base = 0;
@@ -1679,7 +1738,7 @@ __global__ __launch_bounds__(128) void k_batch_trace_clusters_packet(TraceArgs A
       P.hdr = (const uint32_t*)__shfl_sync(0xffffffffu, (unsigned long long)C.hdr, 0);
       P.F = F0;
       P.n = __shfl_sync(0xffffffffu, C.n, 0);
-      trace_warp_packet_clusters<kCount, kBounce>(r, valid, A, P, min_lanes);
+      trace_warp_packet_clusters<kCount, kBounce, kAlone>(r, valid, A, P, min_lanes, s_stack[threadIdx.x >> 5]);
     } else if (valid) {
       trace_ray_clusters<kCount, false, kBounce>(r, A, C);
     }
@@ -1965,8 +2024,10 @@ rt_status launch_clusters(const rt_trace_desc* d, const TraceArgs& A, cudaStream
     const uint32_t blocks = (uint32_t)hmin<uint64_t>((uint64_t)sms() * (d->persistent_blocks_per_sm ? d->persistent_blocks_per_sm : 8u),
                                                      ((uint64_t)M.slots + 127) / 128);
     if (d->schedule & RT_TRACE_PACKET) {
-      if (count) k_trace_clusters_packet<true><<<blocks, 128, 0, st>>>(A, C, M, d->work_counter, d->lane_threshold);
-      else k_trace_clusters_packet<false><<<blocks, 128, 0, st>>>(A, C, M, d->work_counter, d->lane_threshold);
+#define RT_LAUNCH_CK(CNT, ALN) k_trace_clusters_packet<CNT, ALN><<<blocks, 128, 0, st>>>(A, C, M, d->work_counter, d->lane_threshold)
+      if (count) { if (d->lane_threshold) RT_LAUNCH_CK(true, true); else RT_LAUNCH_CK(true, false); }
+      else { if (d->lane_threshold) RT_LAUNCH_CK(false, true); else RT_LAUNCH_CK(false, false); }
+#undef RT_LAUNCH_CK
     } else if (d->schedule & RT_TRACE_REFILL) {
       if (count) k_trace_clusters_refill<true><<<blocks, 128, 0, st>>>(A, C, M, d->work_counter, d->lane_threshold);
       else k_trace_clusters_refill<false><<<blocks, 128, 0, st>>>(A, C, M, d->work_counter, d->lane_threshold);
@@ -2305,9 +2366,11 @@ rt_status batch_launch_clusters(const rt_batch_trace_desc* d, const TraceArgs& A
     const uint32_t per_sm = d->persistent_blocks_per_sm ? d->persistent_blocks_per_sm : 8u;
     const uint32_t blocks = (uint32_t)hmin<uint64_t>((uint64_t)sms() * per_sm, ((uint64_t)d->ray_count + 127) / 128);
     if (d->schedule & RT_TRACE_PACKET) {
-#define RT_LAUNCH_BCK(CNT, BNC) k_batch_trace_clusters_packet<CNT, BNC><<<blocks, 128, 0, st>>>(A, B, d->work_counter, d->lane_threshold)
-      if (A.b_orig) { if (count) RT_LAUNCH_BCK(true, true); else RT_LAUNCH_BCK(false, true); }
-      else { if (count) RT_LAUNCH_BCK(true, false); else RT_LAUNCH_BCK(false, false); }
+#define RT_LAUNCH_BCK(CNT, BNC)                                                                                           \
+  if (d->lane_threshold) k_batch_trace_clusters_packet<CNT, BNC, true><<<blocks, 128, 0, st>>>(A, B, d->work_counter, d->lane_threshold); \
+  else k_batch_trace_clusters_packet<CNT, BNC, false><<<blocks, 128, 0, st>>>(A, B, d->work_counter, 0u)
+      if (A.b_orig) { if (count) { RT_LAUNCH_BCK(true, true); } else { RT_LAUNCH_BCK(false, true); } }
+      else { if (count) { RT_LAUNCH_BCK(true, false); } else { RT_LAUNCH_BCK(false, false); } }
 #undef RT_LAUNCH_BCK
     } else if (d->schedule & RT_TRACE_REFILL) {
       if (count) k_batch_trace_clusters_refill<true><<<blocks, 128, 0, st>>>(A, B, d->work_counter, d->lane_threshold);
