@@ -425,14 +425,14 @@ constexpr int kCoopWarps = 4;  // 128-thread CTAs
 // ray of the item's owner (fetched by shuffles) and merges its best hit into
 // the owner's slot with a 64-bit shared-memory atomicMin on (t bits, position),
 // the same (t, position) rule as the other schedules. The (u, v) of the
-// current best are written by the lane whose key is the minimum right after
-// its merge. key0 is this lane's best so far (t bits, position); on return
-// s_key[lane] / s_uv[lane] hold the merged best of this lane's ray.
+// current best, and its t (a -0 keeps its sign, which the key drops), are
+// written by the lane whose key is the minimum right after its merge. key0 is this lane's best so far (t bits, position); on return
+// s_key[lane] / s_uvt[lane] hold the merged best of this lane's ray.
 template <uint32_t kGroup>
 __device__ __forceinline__ void coop_items(const uint32_t lane, const uint32_t mask, const uint32_t first, const uint32_t cnt,
                                            const uint32_t F, const float4& o, const float4& d, const float zu, const float zv,
-                                           const float4* __restrict__ tris, const unsigned long long key0, const float bu,
-                                           const float bv, unsigned long long* s_key, float2* s_uv) {
+                                           const float4* __restrict__ tris, const unsigned long long key0, const float bt,
+                                           const float bu, const float bv, unsigned long long* s_key, float4* s_uvt) {
   const uint32_t my_items = __popc(mask);
   uint32_t incl = my_items;
 #pragma unroll
@@ -443,12 +443,12 @@ __device__ __forceinline__ void coop_items(const uint32_t lane, const uint32_t m
   const uint32_t excl = incl - my_items;
   const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
   s_key[lane] = key0;
-  s_uv[lane] = make_float2(bu, bv);
+  s_uvt[lane] = make_float4(bu, bv, bt, 0.0f);
   __syncwarp();
   for (uint32_t base = 0; base < total; base += 32) {
     const uint32_t item = base + lane;
     unsigned long long cand = ~0ull;
-    float cu = 0.f, cv = 0.f;
+    float cu = 0.f, cv = 0.f, ct = 0.f;
     // owner: last lane whose exclusive offset is <= item
     uint32_t lo = 0, hi = 31;
 #pragma unroll
@@ -474,7 +474,7 @@ __device__ __forceinline__ void coop_items(const uint32_t lane, const uint32_t m
       const uint32_t kend = min(ocnt, g * kGroup + kGroup);
       const unsigned long long cur = s_key[owner];
       unsigned long long mine = ~0ull;
-      float mu = 0.f, mv = 0.f;
+      float mu = 0.f, mv = 0.f, mt = 0.f;
       for (uint32_t k = g * kGroup; k < kend; ++k) {
         const uint32_t pos = ofirst + k;
         const float4 v0 = ldg4(otris + 3 * (size_t)pos);
@@ -482,23 +482,23 @@ __device__ __forceinline__ void coop_items(const uint32_t lane, const uint32_t m
         const float4 e2 = ldg4(otris + 3 * (size_t)pos + 2);
         float t, u, v;
         if (!mt_test(oo, od, ozu, ozv, v0, e1, e2, t, u, v)) continue;
-        const unsigned long long key = ((unsigned long long)__float_as_uint(t) << 32) | pos;
-        if (key < mine) { mine = key; mu = u; mv = v; }
+        const unsigned long long key = ((unsigned long long)__float_as_uint(t + 0.0f) << 32) | pos;  // -0 ties with +0
+        if (key < mine) { mine = key; mu = u; mv = v; mt = t; }
       }
       if (mine < cur) atomicMin(s_key + owner, mine);
       cand = mine;
-      cu = mu; cv = mv;
+      cu = mu; cv = mv; ct = mt;
     }
     __syncwarp();
-    // (u, v) of the owner's minimum, written by the one lane holding that key
-    if (item < total && cand != ~0ull && s_key[owner] == cand) s_uv[owner] = make_float2(cu, cv);
+    // (u, v, t) of the owner's minimum, written by the one lane holding that key
+    if (item < total && cand != ~0ull && s_key[owner] == cand) s_uvt[owner] = make_float4(cu, cv, ct, 0.0f);
     __syncwarp();
   }
 }
 
 template <bool kCount, bool kSeed = false, bool kWide = false>
 __device__ __forceinline__ void trace_warp_coop(const uint32_t r, const bool valid, const TraceArgs& A, const AccelArgs& C,
-                                                unsigned long long* s_key, float2* s_uv, const SeedArgs& S = SeedArgs{}) {
+                                                unsigned long long* s_key, float4* s_uvt, const SeedArgs& S = SeedArgs{}) {
   const uint32_t lane = lane_id();
   float4 o = make_float4(0.f, 0.f, 0.f, 0.f), d = make_float4(0.f, 0.f, 1.f, 0.f);
   float tmax0 = -1.0f;
@@ -632,16 +632,15 @@ __device__ __forceinline__ void trace_warp_coop(const uint32_t r, const bool val
     // 3. spread the warp's (ray, group) items over the lanes
     // (t bits, position) of the best hit so far; with no hit yet, (tmax bits, 0),
     // which no accepted hit equals (t < tmax is required)
-    const unsigned long long key0 = ((unsigned long long)__float_as_uint(bt) << 32) | (uint32_t)(best >= 0 ? best : 0);
-    coop_items<8>(lane, mask, first, cnt, C.F, o, d, zu, zv, A.tris, key0, bu, bv, s_key, s_uv);
+    const unsigned long long key0 = ((unsigned long long)__float_as_uint(bt + 0.0f) << 32) | (uint32_t)(best >= 0 ? best : 0);
+    coop_items<8>(lane, mask, first, cnt, C.F, o, d, zu, zv, A.tris, key0, bt, bu, bv, s_key, s_uvt);
     // 4. read back the merged best and move on
     if (has_leaf) {
       const unsigned long long k = s_key[lane];
       if (k < key0) {
-        bt = __uint_as_float((uint32_t)(k >> 32));
         best = (int32_t)(k & 0xFFFFFFFFu);
-        const float2 uv = s_uv[lane];
-        bu = uv.x; bv = uv.y;
+        const float4 uvt = s_uvt[lane];
+        bu = uvt.x; bv = uvt.y; bt = uvt.z;
         best_phase = phase;
       }
       // groups beyond the first 32 (leaves of more than 256 triangles): this lane alone
@@ -906,7 +905,7 @@ __device__ __forceinline__ void trace_ray_clusters(const uint32_t r, const Trace
 // lane) are tested by the whole warp (coop_items), and every lane moves on.
 template <bool kCount>
 __device__ __forceinline__ void trace_warp_coop_clusters(const uint32_t r, const bool valid, const TraceArgs& A, const ClusterArgs& C,
-                                                         unsigned long long* s_key, float2* s_uv) {
+                                                         unsigned long long* s_key, float4* s_uvt) {
   const uint32_t lane = lane_id();
   float4 o = make_float4(0.f, 0.f, 0.f, 0.f), d = make_float4(0.f, 0.f, 1.f, 0.f);
   float tmax0 = -1.0f;
@@ -972,16 +971,15 @@ __device__ __forceinline__ void trace_warp_coop_clusters(const uint32_t r, const
     }
     if (kCount) tests += cnt;
     // 2. the warp's clusters, spread over the lanes
-    const unsigned long long key0 = ((unsigned long long)__float_as_uint(bt) << 32) | (uint32_t)(best >= 0 ? best : 0);
-    coop_items<kClusterLeafMax>(lane, mask, first, cnt, C.F, o, d, zu, zv, A.tris, key0, bu, bv, s_key, s_uv);
+    const unsigned long long key0 = ((unsigned long long)__float_as_uint(bt + 0.0f) << 32) | (uint32_t)(best >= 0 ? best : 0);
+    coop_items<kClusterLeafMax>(lane, mask, first, cnt, C.F, o, d, zu, zv, A.tris, key0, bt, bu, bv, s_key, s_uvt);
     // 3. read back the merged best and move on
     if (mask) {
       const unsigned long long key = s_key[lane];
       if (key < key0) {
-        bt = __uint_as_float((uint32_t)(key >> 32));
         best = (int32_t)(key & 0xFFFFFFFFu);
-        const float2 uv = s_uv[lane];
-        bu = uv.x; bv = uv.y;
+        const float4 uvt = s_uvt[lane];
+        bu = uvt.x; bv = uvt.y; bt = uvt.z;
       }
       if (!pop_within(st_ref, st_t, sp, bt, ref)) alive = false;
     }
@@ -1434,22 +1432,22 @@ __global__ __launch_bounds__(128) void k_trace_accel(TraceArgs A, AccelArgs C, S
 }
 
 template <bool kCount, bool kSeed, bool kWide>
-__global__ __launch_bounds__(128, kSeed ? 6 : 0) void k_trace_coop(TraceArgs A, AccelArgs C, SlotMap M, SeedArgs S) {
+__global__ __launch_bounds__(128, kSeed ? 6 : (kCount ? 0 : 7)) void k_trace_coop(TraceArgs A, AccelArgs C, SlotMap M, SeedArgs S) {
   __shared__ unsigned long long s_key[kCoopWarps][32];
-  __shared__ float2 s_uv[kCoopWarps][32];
+  __shared__ float4 s_uvt[kCoopWarps][32];
   const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
   uint32_t r = 0;
   const bool valid = s < M.slots && M.ray_of(s, r);
   const uint32_t w = threadIdx.x >> 5;
   C.F = C.G = 0;
-  trace_warp_coop<kCount, kSeed, kWide>(r, valid, A, C, s_key[w], s_uv[w], S);
+  trace_warp_coop<kCount, kSeed, kWide>(r, valid, A, C, s_key[w], s_uvt[w], S);
 }
 
 template <bool kCount, bool kSeed, bool kWide>
 __global__ __launch_bounds__(128, kSeed ? 6 : (kCount ? 0 : 7)) void k_trace_coop_persistent(TraceArgs A, AccelArgs C, SlotMap M, uint32_t* counter,
                                                                           SeedArgs S) {
   __shared__ unsigned long long s_key[kCoopWarps][32];
-  __shared__ float2 s_uv[kCoopWarps][32];
+  __shared__ float4 s_uvt[kCoopWarps][32];
   __shared__ uint32_t s_rec[kMaxStaged];
   extern __shared__ float4 s_tree[];
   C.F = C.G = 0;
@@ -1463,7 +1461,7 @@ __global__ __launch_bounds__(128, kSeed ? 6 : (kCount ? 0 : 7)) void k_trace_coo
     uint32_t r = 0;
     const uint32_t s = base + lane;
     const bool valid = s < M.slots && M.ray_of(s, r);
-    trace_warp_coop<kCount, kSeed, kWide>(r, valid, A, C, s_key[w], s_uv[w], S);
+    trace_warp_coop<kCount, kSeed, kWide>(r, valid, A, C, s_key[w], s_uvt[w], S);
   }
 }
 
@@ -1553,7 +1551,7 @@ template <bool kCount, bool kSeed, bool kWide>
 __global__ __launch_bounds__(128, kSeed ? 6 : (kCount ? 0 : 7)) void k_batch_trace_coop(TraceArgs A, BatchTraceArgs B, SeedArgs S,
                                                                                       uint32_t* counter) {
   __shared__ unsigned long long s_key[kCoopWarps][32];
-  __shared__ float2 s_uv[kCoopWarps][32];
+  __shared__ float4 s_uvt[kCoopWarps][32];
   const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
   for (;;) {
     uint32_t base = 0;
@@ -1568,7 +1566,7 @@ __global__ __launch_bounds__(128, kSeed ? 6 : (kCount ? 0 : 7)) void k_batch_tra
     C.hdr = B.acc.hdr; C.tnodes = B.acc.tnodes; C.leaves = B.acc.leaves; C.groups = B.acc.groups; C.wide = B.acc.wide;
     SeedArgs Sm = S;
     if (valid) batch_ray_args<kSeed>(r, A, B, S, Am, C, Sm);  // idle lanes keep mesh 0's header and zero offsets
-    trace_warp_coop<kCount, kSeed, kWide>(r, valid, Am, C, s_key[w], s_uv[w], Sm);
+    trace_warp_coop<kCount, kSeed, kWide>(r, valid, Am, C, s_key[w], s_uvt[w], Sm);
   }
 }
 
@@ -1611,7 +1609,7 @@ __global__ __launch_bounds__(128) void k_trace_clusters_persistent(TraceArgs A, 
 template <bool kCount>
 __global__ __launch_bounds__(128) void k_trace_clusters_coop(TraceArgs A, ClusterArgs C, SlotMap M, uint32_t* counter) {
   __shared__ unsigned long long s_key[kCoopWarps][32];
-  __shared__ float2 s_uv[kCoopWarps][32];
+  __shared__ float4 s_uvt[kCoopWarps][32];
   const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
   C.F = 0;
   for (;;) {
@@ -1622,7 +1620,7 @@ __global__ __launch_bounds__(128) void k_trace_clusters_coop(TraceArgs A, Cluste
     uint32_t r = 0;
     const uint32_t s = base + lane;
     const bool valid = s < M.slots && M.ray_of(s, r);
-    trace_warp_coop_clusters<kCount>(r, valid, A, C, s_key[w], s_uv[w]);
+    trace_warp_coop_clusters<kCount>(r, valid, A, C, s_key[w], s_uvt[w]);
   }
 }
 
@@ -1748,7 +1746,7 @@ __global__ __launch_bounds__(128, 8) void k_batch_trace_clusters_packet(TraceArg
 template <bool kCount>
 __global__ __launch_bounds__(128) void k_batch_trace_clusters_coop(TraceArgs A, BatchTraceArgs B, uint32_t* counter) {
   __shared__ unsigned long long s_key[kCoopWarps][32];
-  __shared__ float2 s_uv[kCoopWarps][32];
+  __shared__ float4 s_uvt[kCoopWarps][32];
   const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
   for (;;) {
     uint32_t base = 0;
@@ -1762,7 +1760,7 @@ __global__ __launch_bounds__(128) void k_batch_trace_clusters_coop(TraceArgs A, 
     C.crec = B.acc.crec;
     C.hdr = B.acc.hdr;
     if (valid) batch_cluster_args(r, B, C);
-    trace_warp_coop_clusters<kCount>(r, valid, A, C, s_key[w], s_uv[w]);
+    trace_warp_coop_clusters<kCount>(r, valid, A, C, s_key[w], s_uvt[w]);
   }
 }
 
@@ -2052,6 +2050,13 @@ rt_status launch_clusters(const rt_trace_desc* d, const TraceArgs& A, cudaStream
   return RT_OK;
 }
 
+// A call that asks for no schedule (and no counters) gets the warp-cooperative walk of the 4-wide records too: node
+// trees stop at leaves of up to 223 triangles, and a lane alone with such a leaf keeps 31 others waiting. Camera
+// rays and bounces together, per-lane walk -> this one: 128 x 128 terrain at 512 x 512 0.82 -> 0.32 ms, 2^14-triangle
+// soup at 400 x 300 0.78 -> 0.56 ms, 2^17 at 1000 x 700 3.15 -> 1.95 ms, 2^20 at 1920 x 1080 7.32 -> 5.51 ms (there
+// its camera rays alone lose, 2.29 -> 2.58 ms: neighbouring rays read the same leaves together).
+bool no_schedule(const rt_trace_desc* d) { return d->schedule == 0 && !d->work_counter && !d->ray_visits && !d->ray_tests; }
+
 // Blob traversal launch for every schedule of rt_trace_desc.
 template <bool kSeed, bool kWide>
 rt_status launch_accel_w(const rt_trace_desc* d, const TraceArgs& A, const SeedArgs& S, cudaStream_t st) {
@@ -2073,7 +2078,7 @@ rt_status launch_accel_w(const rt_trace_desc* d, const TraceArgs& A, const SeedA
   const uint32_t pblocks = (uint32_t)sms() * (d->persistent_blocks_per_sm ? d->persistent_blocks_per_sm : 8u);
   const uint32_t sblocks = (M.slots + 127) / 128;
   if (d->work_counter && cudaMemsetAsync(d->work_counter, 0, 4, st) != cudaSuccess) return RT_ERR_CUDA;
-  if (d->schedule & RT_TRACE_COOP) {
+  if ((d->schedule & RT_TRACE_COOP) || (!kSeed && no_schedule(d))) {
     if (d->work_counter) {
       if (count) k_trace_coop_persistent<true, kSeed, kWide><<<pblocks, 128, stage_smem, st>>>(A, C, M, d->work_counter, S);
       else k_trace_coop_persistent<false, kSeed, kWide><<<pblocks, 128, stage_smem, st>>>(A, C, M, d->work_counter, S);
@@ -2101,7 +2106,7 @@ rt_status launch_accel_w(const rt_trace_desc* d, const TraceArgs& A, const SeedA
 template <bool kSeed>
 rt_status launch_accel(const rt_trace_desc* d, const TraceArgs& A, const SeedArgs& S, cudaStream_t st) {
   if (d->schedule & RT_TRACE_CLUSTERS) return kSeed ? RT_ERR_UNSUPPORTED : launch_clusters(d, A, st);
-  if (d->schedule & RT_TRACE_WIDE) return launch_accel_w<kSeed, true>(d, A, S, st);
+  if ((d->schedule & RT_TRACE_WIDE) || (!kSeed && no_schedule(d))) return launch_accel_w<kSeed, true>(d, A, S, st);
   return launch_accel_w<kSeed, false>(d, A, S, st);
 }
 
