@@ -7,12 +7,12 @@
 // real_depth full passes for the boxes. Here everything stays on the device,
 // with no host round trip:
 //
-//   k_boxes_morton   per face: box (4-wide min/max of the 3 vertices), index,
+//   k_boxes_morton   per face: box (4-wide min/max of the 3 vertices),
 //                    Morton code (reference 11/11/10 layout or 10/10/10)
 //   radix sort       (code, index) pairs, stable (rt_sort.cu)
-//   k_levels         split level of each adjacent code pair (clz of the xor)
-//   radix pass       stable partition of split positions by level, which is
-//                    the per-level ascending split list the recursion walks
+//   level sort       split positions by split level (clz of the xor of adjacent
+//                    codes, computed as the pass reads them): the per-level
+//                    ascending split lists the recursion walks
 //   k_topo_morton    one CTA: the Morton levels of the tree, level by level,
 //                    with the reference's split-pointer semantics (see below);
 //                    leaf counts, pre-order ranks and node ids
@@ -131,17 +131,9 @@ __global__ __launch_bounds__(256) void k_hitbox(const float4* __restrict__ v, ui
 // ----------------------------------------------------------------------------
 // kernels/CUDA_calcMeshBoxes.cu:30-58 (boxes, iota) fused with
 // kernels/CUDA_buildMeshTreeLBVH.cu:115-173 (Morton code of the box centre).
-// code_counts (optional, 4 x 256 zeroed words): the digit counts of the codes for the four 8-bit passes of their
-// sort, so that the sort need not read the codes once more to count them.
 __global__ __launch_bounds__(256) void k_boxes_morton(const float4* __restrict__ verts, const uint4* __restrict__ faces, uint32_t n,
                                                      const float4* __restrict__ hit, int layout, float4* __restrict__ boxes,
-                                                     uint32_t* __restrict__ codes, uint32_t* __restrict__ idx,
-                                                     uint32_t* __restrict__ code_counts) {
-  __shared__ uint32_t s_cc[4 * 256];
-  if (code_counts) {
-    for (int i = threadIdx.x; i < 4 * 256; i += blockDim.x) s_cc[i] = 0;
-    __syncthreads();
-  }
+                                                     uint32_t* __restrict__ codes, uint32_t* __restrict__ idx) {
   const float4 hmin = codes ? hit[0] : make_float4(0.f, 0.f, 0.f, 0.f);
   const float4 hmax = codes ? hit[1] : make_float4(1.f, 1.f, 1.f, 1.f);
   const float lx = hmax.x - hmin.x, ly = hmax.y - hmin.y, lz = hmax.z - hmin.z;
@@ -159,12 +151,7 @@ __global__ __launch_bounds__(256) void k_boxes_morton(const float4* __restrict__
       const uint32_t qx = f2u_sat((cx - hmin.x) * sx);
       const uint32_t qy = f2u_sat((cy - hmin.y) * sy);
       const uint32_t qz = f2u_sat((cz - hmin.z) * sz);
-      const uint32_t code = spread_code(qx, qy, qz, layout);
-      codes[k] = code;
-      if (code_counts) {
-#pragma unroll
-        for (int p = 0; p < 4; ++p) atomicAdd(&s_cc[p * 256 + ((code >> (8 * p)) & 255u)], 1u);
-      }
+      codes[k] = spread_code(qx, qy, qz, layout);
     }
   };
   // two faces per iteration: their face and vertex loads are in flight together
@@ -179,32 +166,6 @@ __global__ __launch_bounds__(256) void k_boxes_morton(const float4* __restrict__
     face(k, v0, v1, v2);
     if (two) face(k2, w0, w1, w2);
   }
-  if (code_counts) {
-    __syncthreads();
-    for (int i = threadIdx.x; i < 4 * 256; i += blockDim.x)
-      if (s_cc[i]) atomicAdd(code_counts + i, s_cc[i]);
-  }
-}
-
-// ----------------------------------------------------------------------------
-// split levels: key = clz(code[i] ^ code[i+1]) (32 when equal), value = i + 1
-// (kernels/CUDA_buildMeshTreeLBVH.cu:175-233)
-// ----------------------------------------------------------------------------
-// lev_counts (256 zeroed words): how many pairs have each level, the digit counts of the level sort's one pass.
-__global__ __launch_bounds__(256) void k_levels(const uint32_t* __restrict__ codes, uint32_t n, uint32_t* __restrict__ lev,
-                                               uint32_t* __restrict__ pos, uint32_t* __restrict__ lev_counts) {
-  __shared__ uint32_t s_lc[33];
-  if (threadIdx.x < 33) s_lc[threadIdx.x] = 0;
-  __syncthreads();
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i + 1 < n; i += gridDim.x * blockDim.x) {
-    uint32_t d = __ldg(codes + i) ^ __ldg(codes + i + 1);
-    const uint32_t l = d ? (uint32_t)__clz(d) : 32u;
-    lev[i] = l;
-    pos[i] = i + 1;
-    atomicAdd(&s_lc[l], 1u);
-  }
-  __syncthreads();
-  if (threadIdx.x < 33 && s_lc[threadIdx.x]) atomicAdd(lev_counts + threadIdx.x, s_lc[threadIdx.x]);
 }
 
 // ----------------------------------------------------------------------------
@@ -631,7 +592,6 @@ struct BuildLayout {
   float4* hit;
   float4* partial;
   uint32_t* codes;
-  uint32_t* lev;
   uint32_t* C;
   uint32_t* lev_count;
   void* sort_scratch;
@@ -646,7 +606,7 @@ struct BuildLayout {
   uint32_t* err;
   uint32_t* leaf_lambda;
   uint4* faces_tmp;
-  uint32_t* counts;  // [5 x 256]: the code sort's digit counts (4 passes), then the level sort's (1 pass)
+  uint32_t* hit_done;  // the hit box's block counter
   ClusterTemps ct;   // cluster tree build (RT_ACCEL_CLUSTERS only)
 };
 
@@ -674,10 +634,9 @@ size_t carve_build(Carve& c, BuildLayout& L, uint32_t n, uint32_t D, bool need_c
   L.hit = c.take<float4>(2);
   L.partial = c.take<float4>(2 * kHitParts);
   L.codes = need_codes ? c.take<uint32_t>(n) : nullptr;
-  L.lev = c.take<uint32_t>(n);
   L.C = c.take<uint32_t>(n);
   L.lev_count = c.take<uint32_t>(256);
-  L.sort_bytes = radix_scratch_bytes(n);
+  L.sort_bytes = hmax<size_t>(radix_scratch_bytes(n), segment_sort_scratch_bytes(n, 1));
   L.sort_scratch = c.take<char>(L.sort_bytes);
   uint32_t** bfs[] = {&L.ra, &L.rb, &L.parent, &L.info, &L.child, &L.leaves, &L.mleaves, &L.rank, &L.lambda, &L.ord, &L.id};
   for (auto p : bfs) *p = c.take<uint32_t>(L.cap_m);
@@ -690,7 +649,7 @@ size_t carve_build(Carve& c, BuildLayout& L, uint32_t n, uint32_t D, bool need_c
   L.err = c.take<uint32_t>(4);
   L.leaf_lambda = c.take<uint32_t>(L.max_nodes);
   L.faces_tmp = need_faces_tmp ? c.take<uint4>(n) : nullptr;
-  L.counts = c.take<uint32_t>(5 * 256 + 1);  // digit counts of the code and level sorts, then the hit box's block counter
+  L.hit_done = c.take<uint32_t>(1);
   L.ct = ClusterTemps{};
   if (clusters) carve_cluster_temps(c, L.ct, n, 1);
   return c.off + 256;
@@ -809,40 +768,33 @@ extern "C" rt_status rt_lbvh_build(const rt_build_desc* d, rt_stream stream_) {
   uint32_t* codes = d->codes ? d->codes : L.codes;
   const int sms = sm_count();
 
-  // 1. hit box (the sorts' digit counts and the hit box's block counter start at zero)
-  if (cudaMemsetAsync(L.counts, 0, (5 * 256 + 1) * 4, st) != cudaSuccess) return RT_ERR_CUDA;
+  // 1. hit box
   if (d->hitbox) {
     float4 mn = make_float4(d->hitbox[0], d->hitbox[1], d->hitbox[2], d->hitbox[3]);
     float4 mx = make_float4(d->hitbox[4], d->hitbox[5], d->hitbox[6], d->hitbox[7]);
     k_set_hitbox<<<1, 1, 0, st>>>(L.hit, mn, mx);
     note_launch();
   } else {
-    k_hitbox<<<kHitParts, 256, 0, st>>>((const float4*)d->vertices, d->vertex_count, L.partial, L.counts + 5 * 256, L.hit);
+    if (cudaMemsetAsync(L.hit_done, 0, 4, st) != cudaSuccess) return RT_ERR_CUDA;
+    k_hitbox<<<kHitParts, 256, 0, st>>>((const float4*)d->vertices, d->vertex_count, L.partial, L.hit_done, L.hit);
     note_launch();
   }
   RT_CHECK_LAUNCH();
-  // 2. boxes, indices, codes (and the digit counts of both sorts, counted by the kernels that make the keys)
+  // 2. boxes, codes
   {
     uint32_t blocks = (uint32_t)hmin<uint64_t>((n + 255) / 256, (uint64_t)sms * 16);
     k_boxes_morton<<<blocks, 256, 0, st>>>((const float4*)d->vertices, (const uint4*)d->faces_in, n, L.hit, (int)q.morton_bits,
-                                           (float4*)d->boxes, codes, d->indices, L.counts);
+                                           (float4*)d->boxes, codes, nullptr);
     note_launch();
     RT_CHECK_LAUNCH();
   }
-  // 3. sort (code, index); the build's error word starts here, so that the sorts' bounded waits report into it
+  // 3. sort (code, index)
   if (cudaMemsetAsync(L.err, 0, 16, st) != cudaSuccess) return RT_ERR_CUDA;
-  rt_status s = radix_sort_pairs(codes, d->indices, n, 0, 32, 0, L.sort_scratch, L.sort_bytes, st, nullptr, L.err, L.counts);
+  rt_status s = radix_sort_pairs(codes, d->indices, n, 0, 32, 1, L.sort_scratch, L.sort_bytes, st);
   if (s != RT_OK) return s;
   // 4. per-level split lists
-  if (cudaMemsetAsync(L.lev_count, 0, 256 * 4, st) != cudaSuccess) return RT_ERR_CUDA;
-  if (n > 1) {
-    uint32_t blocks = (uint32_t)hmin<uint64_t>((n + 255) / 256, (uint64_t)sms * 16);
-    k_levels<<<blocks, 256, 0, st>>>(codes, n, L.lev, L.C, L.counts + 4 * 256);
-    note_launch();
-    RT_CHECK_LAUNCH();
-    s = radix_sort_pairs(L.lev, L.C, n - 1, 0, 8, 0, L.sort_scratch, L.sort_bytes, st, L.lev_count, L.err, L.counts + 4 * 256);
-    if (s != RT_OK) return s;
-  }
+  s = sort_split_levels(codes, n, L.C, L.lev_count, 256, L.sort_scratch, L.sort_bytes, st);
+  if (s != RT_OK) return s;
   // 5. Morton top tree
   {
     TopoArgs A;
@@ -906,7 +858,7 @@ extern "C" rt_status rt_mesh_boxes(const float* vertices, const uint32_t* faces,
   if (rt_device_check() != RT_OK) return RT_ERR_NO_DEVICE;
   uint32_t blocks = (uint32_t)hmin<uint64_t>((n + 255) / 256, (uint64_t)sm_count() * 16);
   k_boxes_morton<<<blocks, 256, 0, (cudaStream_t)st>>>((const float4*)vertices, (const uint4*)faces, n, nullptr, 32, (float4*)boxes,
-                                                      nullptr, indices, nullptr);
+                                                      nullptr, indices);
     note_launch();
   RT_CHECK_LAUNCH();
   return RT_OK;
@@ -957,11 +909,8 @@ struct BatchArgs {
   float4* hitpart;        // [2 M kHitSplit]: the hit box shares of k_batch_hitbox
   uint32_t* hitdone;      // [M]: finished shares per mesh
   uint32_t* idx;          // [N] global face index in sorted order
-  uint32_t* codes_raw;    // [N] codes before sorting
-  uint32_t* mkey;         // [N] mesh id per position
-  uint32_t* lev;          // [N] (mesh, level) keys
   uint32_t* C;            // [N] split positions
-  uint32_t* hist;         // [M * 64 + 1]
+  uint32_t* hist;         // [M * 64]: split positions per mesh and level
   uint32_t *ra, *rb, *parent, *info, *child, *leaves, *mleaves, *rank, *lambda, *ord, *id;  // [2N + 3M]
   uint32_t* ml_lambda;
   uint4* ml_rec;
@@ -972,9 +921,7 @@ struct BatchArgs {
   uint32_t* hdr;          // [16 M]
   uint32_t* leaf_base;    // [M + 1]
   uint32_t* err;          // [4]
-  uint32_t* counts;       // [9 x 256 + 64]: digit counts of the code sort (4 passes), the mesh sort (2), the level
-                          // sort (3), then the count of finished topology CTAs
-
+  uint32_t* topo_done;    // finished topology CTAs
   // traversal blob
   uint32_t* acc_hdr;      // [64 M]
   float4* tnodes;         // [4 N]
@@ -995,10 +942,6 @@ __global__ __launch_bounds__(512) void k_batch_hitbox(BatchArgs B) {
   const uint32_t v0 = min(w1, w0 + part * share), v1 = min(w1, v0 + share);
   if (part == 0 && threadIdx.x == 0) {
     B.acc_hdr[64 * (size_t)m + kHdrClusterValid] = 0;  // set again by the cluster build, if any
-    // the mesh sort's digit counts: mesh m holds foff[m + 1] - foff[m] keys of value m
-    const uint32_t faces = B.foff[m + 1] - B.foff[m];
-    atomicAdd(B.counts + 4 * 256 + (m & 255u), faces);
-    atomicAdd(B.counts + 5 * 256 + ((m >> 8) & 255u), faces);
   }
   float4 mn[4], mx[4];
 #pragma unroll
@@ -1053,9 +996,6 @@ __global__ __launch_bounds__(512) void k_batch_hitbox(BatchArgs B) {
 }
 
 __global__ __launch_bounds__(256) void k_batch_boxes_morton(BatchArgs B) {
-  __shared__ uint32_t s_cc[4 * 256];  // the code sort's digit counts of this block's faces
-  for (int i = threadIdx.x; i < 4 * 256; i += blockDim.x) s_cc[i] = 0;
-  __syncthreads();
   const int layout = (int)B.q.morton_bits;
   for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < B.N; k += gridDim.x * blockDim.x) {
     const uint32_t m = find_seg(B.foff, B.M, k);
@@ -1070,58 +1010,9 @@ __global__ __launch_bounds__(256) void k_batch_boxes_morton(BatchArgs B) {
     const float4 mx = f4max(f4max(v0, v1), v2);
     B.boxes[2 * (size_t)k] = mn;
     B.boxes[2 * (size_t)k + 1] = mx;
-    B.idx[k] = k;
     const float cx = 0.5f * (mn.x + mx.x), cy = 0.5f * (mn.y + mx.y), cz = 0.5f * (mn.z + mx.z);
-    const uint32_t code = spread_code(f2u_sat((cx - hmin.x) * sx), f2u_sat((cy - hmin.y) * sy), f2u_sat((cz - hmin.z) * sz), layout);
-    B.codes[k] = code;
-    B.codes_raw[k] = code;
-#pragma unroll
-    for (int p = 0; p < 4; ++p) atomicAdd(&s_cc[p * 256 + ((code >> (8 * p)) & 255u)], 1u);
+    B.codes[k] = spread_code(f2u_sat((cx - hmin.x) * sx), f2u_sat((cy - hmin.y) * sy), f2u_sat((cz - hmin.z) * sz), layout);
   }
-  __syncthreads();
-  for (int i = threadIdx.x; i < 4 * 256; i += blockDim.x)
-    if (s_cc[i]) atomicAdd(B.counts + i, s_cc[i]);
-}
-
-// After the (mesh, code) order is complete: the code of each position, and per pair (i, i + 1) the split level
-// key (mesh * 64 + level; 32 = no split, also across meshes), its (mesh, level) count and the level sort's digit
-// counts (up to three 8-bit passes).
-__global__ __launch_bounds__(256) void k_batch_levels(BatchArgs B) {
-  __shared__ uint32_t s_lc[3 * 256];
-  for (int i = threadIdx.x; i < 3 * 256; i += blockDim.x) s_lc[i] = 0;
-  __syncthreads();
-  // whole warps step together, so that equal keys of a warp are counted with one atomic (the keys of a mesh
-  // crowd onto a few levels: one atomic per position would queue on those few counters)
-  const uint32_t lane = threadIdx.x & 31u;
-  for (uint32_t base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < B.N; base += gridDim.x * blockDim.x) {
-    const uint32_t i = base + lane;
-    uint32_t key = ~0u;
-    if (i < B.N) {
-      const uint32_t c0 = B.codes_raw[B.idx[i]];
-      B.codes[i] = c0;
-      if (i + 1 < B.N) {
-        const uint32_t m = B.mkey[i];
-        uint32_t lev = 32;
-        if (B.mkey[i + 1] == m) {
-          const uint32_t d = c0 ^ B.codes_raw[B.idx[i + 1]];
-          if (d) lev = (uint32_t)__clz(d);
-        }
-        key = m * 64 + lev;
-        B.lev[i] = key;
-        B.C[i] = i + 1;
-      }
-    }
-    const uint32_t peers = __match_any_sync(0xffffffffu, key);
-    if (key != ~0u && lane == (uint32_t)(__ffs(peers) - 1)) {
-      const uint32_t cnt = (uint32_t)__popc(peers);
-      atomicAdd(B.hist + key, cnt);
-#pragma unroll
-      for (int p = 0; p < 3; ++p) atomicAdd(&s_lc[p * 256 + ((key >> (8 * p)) & 255u)], cnt);
-    }
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < 3 * 256; i += blockDim.x)
-    if (s_lc[i]) atomicAdd(B.counts + 6 * 256 + i, s_lc[i]);
 }
 
 __global__ __launch_bounds__(kTopoThreads) void k_batch_topo(BatchArgs B) {
@@ -1135,8 +1026,7 @@ __global__ __launch_bounds__(kTopoThreads) void k_batch_topo(BatchArgs B) {
   A.leaves = B.leaves + bb; A.mleaves = B.mleaves + bb; A.rank = B.rank + bb; A.lambda = B.lambda + bb; A.ord = B.ord + bb;
   A.id = B.id + bb; A.ml_lambda = B.ml_lambda + bb; A.ml_rec = B.ml_rec + bb; A.ml_rank = B.ml_rank + bb;
   A.parent_id = B.parent_id + nb; A.nodes = B.nodes + 8 * (size_t)nb; A.max_nodes = 2 * n - 1; A.hdr = B.hdr + 16 * m;
-  // the pairs of the meshes before m are their F positions (every position but the last of all has one pair),
-  // so this mesh's level lists start at F in the level order
+  // the meshes before m hold F positions, so this mesh's level lists start at F
   A.level_hist = B.hist + 64 * m; A.level_base = F; A.pos_base = F;
   topo_morton(A);
   // the CTA that finishes last (every other mesh's header is written) makes the leaf-order bases per mesh (an
@@ -1146,7 +1036,7 @@ __global__ __launch_bounds__(kTopoThreads) void k_batch_topo(BatchArgs B) {
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
-    s_last = atomicAdd(B.counts + 9 * 256, 1u) == B.M - 1 ? 1u : 0u;
+    s_last = atomicAdd(B.topo_done, 1u) == B.M - 1 ? 1u : 0u;
   }
   __syncthreads();
   if (!s_last) return;
@@ -1247,16 +1137,15 @@ __global__ __launch_bounds__(256) void k_batch_records(BatchArgs B) {
   }
 }
 
+size_t batch_sort_bytes(uint32_t N, uint32_t M) { return hmax<size_t>(radix_scratch_bytes(N), segment_sort_scratch_bytes(N, M)); }
+
 size_t carve_batch(Carve& c, BatchArgs& B, uint32_t M, uint32_t N, bool clusters) {
   B.hits = c.take<float4>(2 * (size_t)M);
   B.hitpart = c.take<float4>(2 * (size_t)M * kHitSplit);
   B.hitdone = c.take<uint32_t>(M);
   B.idx = c.take<uint32_t>(N);
-  B.codes_raw = c.take<uint32_t>(N);
-  B.mkey = c.take<uint32_t>(N);
-  B.lev = c.take<uint32_t>(N);
   B.C = c.take<uint32_t>(N);
-  B.hist = c.take<uint32_t>((size_t)M * 64 + 1);
+  B.hist = c.take<uint32_t>((size_t)M * 64);
   const size_t bfs = 2 * (size_t)N + 3 * (size_t)M + 4;
   uint32_t** arrs[] = {&B.ra, &B.rb, &B.parent, &B.info, &B.child, &B.leaves, &B.mleaves, &B.rank, &B.lambda, &B.ord, &B.id};
   for (auto a : arrs) *a = c.take<uint32_t>(bfs);
@@ -1270,10 +1159,10 @@ size_t carve_batch(Carve& c, BatchArgs& B, uint32_t M, uint32_t N, bool clusters
   B.hdr = c.take<uint32_t>(16 * (size_t)M);
   B.leaf_base = c.take<uint32_t>((size_t)M + 1);
   B.err = c.take<uint32_t>(4);
-  B.counts = c.take<uint32_t>(9 * 256 + 64);
+  B.topo_done = c.take<uint32_t>(1);
   B.ct = ClusterTemps{};
   if (clusters) carve_cluster_temps(c, B.ct, N, M);
-  const size_t sort_bytes = radix_scratch_bytes(N);
+  const size_t sort_bytes = batch_sort_bytes(N, M);
   c.take<char>(sort_bytes);
   return c.off + 256;
 }
@@ -1318,7 +1207,7 @@ extern "C" rt_status rt_batch_build(const rt_batch_build_desc* d, rt_stream stre
   carve_batch(c, B, M, N, clusters);
   if (!d->scratch || !c.ok()) return RT_ERR_SCRATCH_TOO_SMALL;
   // the sort scratch is the last region
-  const size_t sort_bytes = radix_scratch_bytes(N);
+  const size_t sort_bytes = batch_sort_bytes(N, M);
   void* sort_scratch = (char*)d->scratch + (c.off - sort_bytes - 0);
   {
     Carve a(d->accel, d->accel_bytes);
@@ -1332,35 +1221,19 @@ extern "C" rt_status rt_batch_build(const rt_batch_build_desc* d, rt_stream stre
   cudaStream_t st = (cudaStream_t)stream_;
   const int sms = sm_count();
   const uint32_t fblocks = (uint32_t)hmin<uint64_t>((N + 255) / 256, (uint64_t)sms * 16);
-  // the error word and every sort's digit counts (counted by the kernels that make the keys) start at zero
   if (cudaMemsetAsync(B.err, 0, 16, st) != cudaSuccess) return RT_ERR_CUDA;
-  if (cudaMemsetAsync(B.counts, 0, (9 * 256 + 64) * 4, st) != cudaSuccess) return RT_ERR_CUDA;
-  if (cudaMemsetAsync(B.hist, 0, ((size_t)M * 64 + 1) * 4, st) != cudaSuccess) return RT_ERR_CUDA;
+  if (cudaMemsetAsync(B.topo_done, 0, 4, st) != cudaSuccess) return RT_ERR_CUDA;
+  if (cudaMemsetAsync(B.hist, 0, (size_t)M * 64 * 4, st) != cudaSuccess) return RT_ERR_CUDA;
   if (cudaMemsetAsync(B.hitdone, 0, (size_t)M * 4, st) != cudaSuccess) return RT_ERR_CUDA;
   k_batch_hitbox<<<M * kHitSplit, 512, 0, st>>>(B);
   k_batch_boxes_morton<<<fblocks, 256, 0, st>>>(B);
   note_launch(2);
   RT_CHECK_LAUNCH();
-  // Morton order of all faces; its last pass also writes each position's mesh (the key of the next sort)
-  rt_status s = radix_sort_pairs(B.codes, B.idx, N, 0, 32, 0, sort_scratch, sort_bytes, st, nullptr, B.err, B.counts, B.foff, M,
-                                 B.mkey);
+  // every mesh's faces in Morton order (a mesh is a segment of the sort), then its split positions in level order
+  rt_status s = radix_sort_pairs(B.codes, B.idx, N, 0, 32, 1, sort_scratch, sort_bytes, st, B.foff, M);
   if (s != RT_OK) return s;
-  // key widths in whole 8-bit digits: mesh ids < M, level keys < 64 (M - 1) + 33
-  auto digit_bits = [](uint64_t maxval) -> uint32_t {
-    uint32_t b = 1;
-    while (b < 64 && (1ull << b) <= maxval) ++b;
-    return b > 24 ? 32u : (b + 7) / 8 * 8;
-  };
-  s = radix_sort_pairs(B.mkey, B.idx, N, 0, digit_bits(M - 1), 0, sort_scratch, sort_bytes, st, nullptr, B.err, B.counts + 4 * 256);
+  s = sort_split_levels(B.codes, N, B.C, B.hist, 64, sort_scratch, sort_bytes, st, B.foff, M);
   if (s != RT_OK) return s;
-  k_batch_levels<<<fblocks, 256, 0, st>>>(B);
-  note_launch();
-  RT_CHECK_LAUNCH();
-  if (N > 1) {
-    s = radix_sort_pairs(B.lev, B.C, N - 1, 0, digit_bits(64ull * (M - 1) + 32), 0, sort_scratch, sort_bytes, st, nullptr, B.err,
-                         B.counts + 6 * 256);
-    if (s != RT_OK) return s;
-  }
   k_batch_topo<<<M, kTopoThreads, 0, st>>>(B);
   note_launch();
   RT_CHECK_LAUNCH();

@@ -55,6 +55,8 @@ struct NvtxRange {
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 template <typename T>
 inline T hmin(T a, T b) { return a < b ? a : b; }
+template <typename T>
+inline T hmax(T a, T b) { return a > b ? a : b; }
 
 // Bump allocator over a caller-provided scratch buffer.
 struct Carve {
@@ -122,25 +124,29 @@ void note_launch(uint32_t kernels = 1);
 void excl_scan(uint32_t* v, uint32_t n, uint32_t* sums, uint32_t* total, cudaStream_t st);
 
 // Radix sort internals shared by the build (rt_sort.cu).
-// Scratch bytes of an n-key sort (n > 4096 keys; n <= 4096 needs none): the other key and value buffers, and
-// per digit pass (at most 4) one status word per (4096-key tile, digit), a tile counter and 256 digit counts;
-// each region starts on a 256-byte boundary, plus 256 bytes of slack. radix_scratch_bytes() returns this.
+// Scratch bytes of an n-key sort (n > 4096 keys; n <= 4096 needs none): the other key and value buffers and at most a
+// byte per key (and 5 KB) of digit counts; each region starts on a 256-byte boundary, plus 256 bytes of slack.
+// radix_scratch_bytes() returns this.
 constexpr size_t radix_scratch_bytes_of(uint32_t n) {
   const size_t tiles = ((size_t)n + 4095) / 4096;
   const size_t a = ((size_t)n * 4 + 255) / 256 * 256;
   return 2 * a + 4 * (4 * tiles * 256 + 4 * 64 + 4 * 256) + 256;
 }
 size_t radix_scratch_bytes(uint32_t n);
-// Stable sort of (key, value) pairs by bits [begin_bit, end_bit) of the key; digit_totals_out (device, 256 words,
-// optional) receives the digit counts of the last pass; err (device, optional) receives RT_DEVERR_WAIT_TIMEOUT
-// if a bounded wait between tiles ran out. digit_counts_in (device, optional): the digit counts of every pass
-// (pass p's 256 counts at p * 256, digit p = bits [begin_bit + 8p, begin_bit + 8p + 8)), counted by the keys'
-// producer; the sort then reads the keys once less. seg_off / seg_count / seg_out (optional, with values):
-// the last pass also writes seg_out[position] = the segment of the value placed there (the largest m < seg_count
-// with seg_off[m] <= value).
+// Scratch of a sort in M segments, any n (radix_scratch_bytes covers M = 1 with more than 4096 keys).
+size_t segment_sort_scratch_bytes(uint32_t n, uint32_t M);
+// Stable sort of (key, value) pairs by bits [begin_bit, end_bit) of the key; init_vals: the values are the keys' input
+// positions. With M > 1 segments (seg_off: DEVICE, M + 1 ascending offsets from 0 to n) each segment is sorted by itself.
 rt_status radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_t begin_bit, uint32_t end_bit, int init_vals,
-                           void* scratch, size_t scratch_bytes, cudaStream_t stream, uint32_t* digit_totals_out,
-                           uint32_t* err = nullptr, const uint32_t* digit_counts_in = nullptr, const uint32_t* seg_off = nullptr,
-                           uint32_t seg_count = 0, uint32_t* seg_out = nullptr);
+                           void* scratch, size_t scratch_bytes, cudaStream_t stream, const uint32_t* seg_off = nullptr, uint32_t M = 1);
+// The split positions of sorted Morton codes in level order, per segment: position i + 1 at level clz(code[i] ^ code[i + 1]),
+// ascending inside a level; positions without a split (equal codes, and a segment's last) at level 32, after the others.
+// splits: n words, a segment's in its own places; level_counts[m * count_stride + l]: positions of level l (l < 64 and
+// below count_stride) of a segment that is not empty.
+rt_status sort_split_levels(const uint32_t* codes, uint32_t n, uint32_t* splits, uint32_t* level_counts, uint32_t count_stride,
+                            void* scratch, size_t scratch_bytes, cudaStream_t stream, const uint32_t* seg_off = nullptr,
+                            uint32_t M = 1);
+// First chunk of segment m, whose keys start at F, in a sort with chunks of per_chunk keys (chunks never span segments).
+__host__ __device__ __forceinline__ uint32_t sort_chunk_base(uint32_t F, uint32_t m, uint32_t per_chunk) { return F / per_chunk + m; }
 
 }  // namespace rt

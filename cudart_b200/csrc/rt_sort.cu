@@ -5,26 +5,25 @@
 // CUDA_bitonicSort*, CUDA_bubbleSort512; kernels/CUDA_radixSortGeneral.cu:397-482
 // etc.), which serialises its shared histogram 256 ways and ranks keys with
 // warp-synchronous code that is undefined on Volta and later. Here:
-//   * one histogram launch reads the keys once and counts the digits of every
-//     pass (so each pass knows where every digit's run starts);
-//   * per pass, one launch over tiles of 4096 keys (512 threads x 8 keys).
-//     A CTA takes the next tile index from a counter, ranks its keys stably
-//     (the lanes of equal digit found by one ballot per digit bit, plus
-//     per-warp counters), publishes its per-digit counts, and finds how many
-//     keys of each digit the earlier tiles hold by reading
-//     their published counts backwards until it meets a tile that already
-//     published its inclusive prefix (decoupled look-back, after Merrill and
-//     Adinets, "Onesweep: a faster least significant digit radix sort for
-//     GPUs", 2022). It then publishes its own inclusive prefix, stages the
-//     tile in shared memory in sorted order and writes it out so that
-//     consecutive threads write consecutive addresses of each digit run.
-//     Traffic per pass: keys (and values) read once and written once.
-//   * n <= 4096: a single CTA does every pass in shared memory (one launch).
-// The look-back waits only on tiles whose index was taken earlier, by CTAs that
-// were already running and publish their counts before they wait on anything,
-// so every wait ends; each is still bounded (an iteration limit, after which
-// RT_DEVERR_WAIT_TIMEOUT is OR-ed into the caller's error word and the CTA goes
-// on with what it has).
+//   * the keys are cut into chunks of whole tiles, about two chunks per SM; a
+//     pass is two launches. k_sort_count reads its chunk's keys and writes the
+//     chunk's 256 digit counts (and adds them to a sum per 16 chunks);
+//     k_sort_scatter adds up the counts before its chunk, then takes the
+//     chunk's tiles one after another: ranks the keys stably (the lanes of
+//     equal digit, plus per-warp counters),
+//     stages the tile in shared memory in sorted order and writes it out so
+//     that consecutive threads write consecutive addresses of each digit run,
+//     while the next tile's keys are on their way. No CTA waits for another.
+//   * segments (the meshes of a batched build) are sorted side by side: every
+//     chunk belongs to one segment, and counts are added up inside it, so the
+//     segment number is never a sort key.
+//   * n <= 4096, one segment: a single CTA does every pass in shared memory
+//     (one launch).
+// Traffic per pass: keys (and values) read once and written once, and the keys
+// once more for the counts (from L2 when the keys fit there). One launch per
+// pass with a decoupled look-back over the earlier tiles' counts (which this
+// replaces) moved 4 bytes per pair less, but a pass over 2^24 pairs took
+// 166 us of which the look-back's L2 round trips were most.
 #include "rt_common.cuh"
 
 namespace rt {
@@ -37,31 +36,19 @@ constexpr int kItems = 16;
 constexpr int kTile = kThreads * kItems;  // 4096
 constexpr int kRadix = 256;
 
-// onesweep passes
-constexpr int kOsThreads = 512;
-constexpr int kOsWarps = kOsThreads / 32;
-constexpr int kOsItems = 8;
-constexpr int kOsTile = kOsThreads * kOsItems;  // 4096
-static_assert(kOsTile == kTile, "both sorts use 4096-key tiles");
-constexpr uint32_t kFlagAggregate = 1u << 30;  // the tile's own count of the digit is published
-constexpr uint32_t kFlagPrefix = 2u << 30;     // the count of all keys of the digit up to and including the tile
-constexpr uint32_t kCountMask = (1u << 30) - 1u;
-constexpr uint32_t kSpinLimit = 1u << 22;      // look-back reads of one status word before giving up (seconds)
+// chunked passes
+constexpr int kScThreads = 512;
+constexpr int kScWarps = kScThreads / 32;
+constexpr int kCountThreads = 1024;
+constexpr int kMaskRows = 3;  // of every four rows of a warp, those ranked by masks in shared memory (the fourth by ballots)
+constexpr int kGroup = 16;  // chunks whose counts are also kept as one sum
 constexpr int kMaxPasses = 4;
+constexpr uint32_t kMaxKeys = (1u << 30) - 1u;
 
 __device__ __forceinline__ uint32_t lanemask_lt() {
   uint32_t m;
   asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
   return m;
-}
-
-__device__ __forceinline__ uint32_t ld_relaxed(const uint32_t* p) {
-  uint32_t v;
-  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ void st_relaxed(uint32_t* p, uint32_t v) {
-  asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
 // Block-wide exclusive scan of one value per thread (NT threads).
@@ -93,34 +80,6 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* s_warp
   return warp_prefix + x - v;
 }
 
-// Digit counts of every pass in one read of the keys: counts[p * 256 + d] = keys whose digit p is d.
-__global__ __launch_bounds__(256) void k_sort_hist(const uint32_t* __restrict__ keys, uint32_t n, uint32_t begin_bit, uint32_t passes,
-                                                   uint32_t* __restrict__ counts) {
-  __shared__ uint32_t h[kMaxPasses][kRadix];
-  for (int i = threadIdx.x; i < kMaxPasses * kRadix; i += 256) (&h[0][0])[i] = 0;
-  __syncthreads();
-  const uint32_t n4 = n >> 2;
-  const uint4* k4 = reinterpret_cast<const uint4*>(keys);
-  const bool vec = ((uintptr_t)keys & 15u) == 0;
-  auto count = [&](uint32_t k) {
-    for (uint32_t p = 0; p < passes; ++p) atomicAdd(&h[p][(k >> (begin_bit + 8 * p)) & 255u], 1u);
-  };
-  if (vec) {
-    for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < n4; i += gridDim.x * 256) {
-      const uint4 k = __ldg(k4 + i);
-      count(k.x); count(k.y); count(k.z); count(k.w);
-    }
-    for (uint32_t i = 4 * n4 + blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) count(__ldg(keys + i));
-  } else {
-    for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) count(__ldg(keys + i));
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < (int)passes * kRadix; i += 256) {
-    const uint32_t c = (&h[0][0])[i];
-    if (c) atomicAdd(counts + i, c);
-  }
-}
-
 // The lanes of the warp whose 9-bit digit equals this lane's (digits 0..255, 256 for a lane without a key): one
 // ballot per bit, each lane keeping the lanes that agree with it on that bit -- the mask __match_any_sync gives.
 __device__ __forceinline__ uint32_t match_digit(uint32_t d) {
@@ -134,144 +93,291 @@ __device__ __forceinline__ uint32_t match_digit(uint32_t d) {
   return m;
 }
 
-// Optional epilogue of a pass: out[position] = the segment of the value written there (largest m with
-// off[m] <= value, m < count), for a caller that needs each sorted value's segment next.
-struct SegOut {
-  const uint32_t* off;
-  uint32_t count;
-  uint32_t* out;
+// One pass over chunked keys. kMode 0: keys_in are the keys; 1: the key of position i is the split level of the sorted
+// Morton codes in keys_in, clz(code[i] ^ code[i + 1]) (32 for equal codes and for a segment's last position).
+struct PassArgs {
+  const uint32_t* keys_in;
+  const uint32_t* vals_in;  // null: value i is val_base + i
+  uint32_t* keys_out;       // null: the sorted keys are not needed
+  uint32_t* vals_out;
+  uint32_t n, shift, val_base;
+  uint32_t per_chunk;        // keys of a whole chunk
+  const uint32_t* seg_off;   // null: one segment, 0 .. n
+  const uint32_t* chunk_seg; // segment of each chunk (~0: no chunk); with seg_off
+  uint32_t* rows;            // [chunks][256]
+  uint32_t* groups;          // [chunks / kGroup + 1][256], zero before the pass
+  uint32_t* totals;          // optional: [segments][totals_stride] digit counts
+  uint32_t totals_stride;
 };
-__device__ __forceinline__ uint32_t find_seg(const uint32_t* __restrict__ off, uint32_t M, uint32_t x) {
-  uint32_t lo = 0, hi = M - 1;
-  while (lo < hi) {
-    const uint32_t mid = (lo + hi + 1) >> 1;
-    if (__ldg(off + mid) <= x) lo = mid; else hi = mid - 1;
+struct Chunk {
+  uint32_t seg_begin, seg_end;    // keys of the segment
+  uint32_t first_chunk, n_chunks; // its chunks
+  uint32_t begin, end;            // keys of this chunk
+  uint32_t seg;
+};
+__device__ __forceinline__ bool chunk_of(const PassArgs& P, uint32_t c, Chunk& C) {
+  if (!P.seg_off) {
+    C.seg = 0; C.seg_begin = 0; C.seg_end = P.n; C.first_chunk = 0;
+  } else {
+    C.seg = __ldg(P.chunk_seg + c);
+    if (C.seg == ~0u) return false;
+    C.seg_begin = __ldg(P.seg_off + C.seg);
+    C.seg_end = __ldg(P.seg_off + C.seg + 1);
+    C.first_chunk = sort_chunk_base(C.seg_begin, C.seg, P.per_chunk);
   }
-  return lo;
+  C.n_chunks = (C.seg_end - C.seg_begin + P.per_chunk - 1) / P.per_chunk;
+  C.begin = C.seg_begin + (c - C.first_chunk) * P.per_chunk;
+  C.end = C.seg_end - C.begin <= P.per_chunk ? C.seg_end : C.begin + P.per_chunk;
+  return true;
+}
+template <int kMode>
+__device__ __forceinline__ uint32_t load_key(const PassArgs& P, const Chunk& C, uint32_t i) {
+  const uint32_t k = __ldg(P.keys_in + i);
+  if (kMode == 0) return k;
+  if (i + 1 >= C.seg_end) return 32u;
+  const uint32_t x = k ^ __ldg(P.keys_in + i + 1);
+  return x ? (uint32_t)__clz(x) : 32u;
 }
 
-// One digit pass. status[tile * 256 + d] holds a flag (bits 30-31) and a count (bits 0-29); all zero at the start.
-// vals_in == nullptr with kVals: the values are the keys' input positions (first pass of an index sort).
-template <bool kVals>
-__global__ __launch_bounds__(kOsThreads, 3) void k_onesweep(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
-                                                            uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, uint32_t n,
-                                                            uint32_t shift, const uint32_t* __restrict__ digit_counts,
-                                                            uint32_t* __restrict__ status, uint32_t* __restrict__ tile_counter,
-                                                            uint32_t* __restrict__ digit_totals_out, uint32_t* __restrict__ err,
-                                                            SegOut seg) {
-  __shared__ uint32_t s_keys[kOsTile];
-  __shared__ uint32_t s_vals[kVals ? kOsTile : 1];
-  __shared__ uint16_t s_cnt[kOsWarps][kRadix];  // per warp and digit: count, then the warp's offset in the tile's run (<= 4096)
-  __shared__ uint32_t s_tile_start[kRadix];
-  __shared__ uint32_t s_glob[kRadix];
-  __shared__ uint32_t s_warp[kOsWarps];
-  __shared__ uint32_t s_tile;
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tid = threadIdx.x;
-  if (tid == 0) s_tile = atomicAdd(tile_counter, 1u);
-  for (int i = tid; i < kOsWarps * kRadix; i += kOsThreads) (&s_cnt[0][0])[i] = 0;
+// Digit counts of one chunk. Sixteen counters per digit, picked by lane, keep equal digits of a warp apart (Morton
+// codes and split levels come in long runs of equal digits).
+template <int kBits, int kMode>
+__global__ __launch_bounds__(kCountThreads) void k_sort_count(PassArgs P) {
+  constexpr uint32_t D = 1u << kBits;
+  __shared__ uint32_t h[D * 16];
+  Chunk C;
+  if (!chunk_of(P, blockIdx.x, C)) return;
+  for (uint32_t i = threadIdx.x; i < D * 16; i += kCountThreads) h[i] = 0;
   __syncthreads();
-  const uint32_t tile = s_tile;
-  const size_t base = (size_t)tile * kOsTile;
+  const uint32_t copy = threadIdx.x & 15u;
+  for (uint32_t base = C.begin + threadIdx.x; base < C.end; base += 8 * kCountThreads) {
+    uint32_t k[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const uint32_t i = base + q * kCountThreads;  // below 2^31: positions are below 2^30
+      k[q] = i < C.end ? load_key<kMode>(P, C, i) : 0u;
+    }
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (base + q * kCountThreads < C.end) atomicAdd(&h[((k[q] >> P.shift) & (D - 1u)) * 16u + copy], 1u);
+  }
+  __syncthreads();
+  const uint32_t d = threadIdx.x;
+  if (d < kRadix) {
+    uint32_t sum = 0;
+    if (d < D) {
+#pragma unroll
+      for (uint32_t q = 0; q < 16; ++q) sum += h[d * 16u + ((q + d) & 15u)];
+    }
+    P.rows[(size_t)blockIdx.x * kRadix + d] = sum;
+    if (sum) atomicAdd(P.groups + (size_t)(blockIdx.x / kGroup) * kRadix + d, sum);
+  }
+}
 
-  // stable ranks inside the tile: warp w owns keys [w * 256, w * 256 + 256), 32 consecutive keys per round
-  uint32_t key[kOsItems], val[kOsItems], rank[kOsItems];
+// Sum of the 256-word rows [from, to) at one digit, eight loads in flight; `upto` (from <= upto): the part below it.
+__device__ __forceinline__ void sum_rows(const uint32_t* __restrict__ rows, uint32_t d, uint32_t from, uint32_t to, uint32_t upto,
+                                         uint32_t& all, uint32_t& part) {
+  for (uint32_t x = from; x < to; x += 8) {
+    uint32_t v[8];
+#pragma unroll
+    for (uint32_t q = 0; q < 8; ++q) v[q] = x + q < to ? __ldg(rows + (size_t)(x + q) * kRadix + d) : 0u;
+#pragma unroll
+    for (uint32_t q = 0; q < 8; ++q) {
+      all += v[q];
+      if (x + q < upto) part += v[q];
+    }
+  }
+}
+
+// The tiles of one chunk, in order. What bounds it: the shared-memory pipe (ranking, and the move of the tile into
+// sorted order: about 30 wavefronts per 32 keys) beside the integer pipe, at two CTAs per SM. 2^24 pairs, whole
+// sort: ballots alone 561 us (60% of the integer pipe), masks alone 463 (equal digits everywhere: 523), three rows of
+// masks to one of ballots 461 (467); __match_any_sync 750; the look-back sort that this replaced 694.
+template <bool kVals, int kItems, int kBits, int kMode>
+__global__ __launch_bounds__(kScThreads, kItems == 16 ? 2 : 3) void k_sort_scatter(PassArgs P) {
+  constexpr uint32_t T = kScThreads * kItems, D = 1u << kBits;
+  extern __shared__ uint32_t s_dyn[];
+  uint32_t* s_keys = s_dyn;
+  uint32_t* s_vals = s_dyn + T;                  // kVals only
+  uint32_t* s_mask = s_dyn + T * (kVals ? 2 : 1) + (threadIdx.x >> 5) * D;  // the warp's masks
+  __shared__ __align__(16) uint16_t s_cnt[kScWarps][kRadix];  // per warp and digit: count, then the place of its first key in the tile
+  __shared__ uint32_t s_out[kRadix];             // where the tile's run of a digit goes, less where it starts in the tile
+  __shared__ uint32_t s_half[2 * kRadix];
+  __shared__ uint32_t s_scan[8];
+  Chunk C;
+  if (!chunk_of(P, blockIdx.x, C)) return;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t lt = lanemask_lt();
-#pragma unroll
-  for (int r = 0; r < kOsItems; ++r) {
-    const size_t idx = base + (size_t)warp * (kOsItems * 32) + r * 32 + lane;
-    const bool valid = idx < n;
-    key[r] = valid ? __ldg(keys_in + idx) : 0u;
-    if (kVals) val[r] = valid ? (vals_in ? __ldg(vals_in + idx) : (uint32_t)idx) : 0u;
-    const uint32_t d = valid ? ((key[r] >> shift) & 255u) : (uint32_t)kRadix;
-    const uint32_t peers = match_digit(d);
-    uint32_t pre = 0;
-    if (d < (uint32_t)kRadix) pre = s_cnt[warp][d];
-    rank[r] = pre + __popc(peers & lt);
-    __syncwarp();
-    if (d < (uint32_t)kRadix && (peers & lt) == 0) s_cnt[warp][d] = (uint16_t)(pre + __popc(peers));
-    __syncwarp();
-  }
-  __syncthreads();
+  const uint32_t lane0 = (uint32_t)warp * (kItems * 32) + lane;  // the warp's keys of a tile: kItems rows of 32
 
-  // per digit (threads 0..255): warp offsets inside the tile's digit run, the tile's count, published at once
-  uint32_t tile_count = 0;
-  if (tid < kRadix) {
-    uint32_t run = 0;
+  uint32_t key[kItems];
+  auto load_tile = [&](uint32_t base) {
 #pragma unroll
-    for (int w = 0; w < kOsWarps; ++w) {
-      const uint32_t c = s_cnt[w][tid];
-      s_cnt[w][tid] = (uint16_t)run;
-      run += c;
+    for (int r = 0; r < kItems; ++r) {
+      const uint32_t i = base + lane0 + r * 32;
+      key[r] = i < C.end ? load_key<kMode>(P, C, i) : 0u;
     }
-    tile_count = run;
-    st_relaxed(status + (size_t)tile * kRadix + tid, (tile == 0 ? kFlagPrefix : kFlagAggregate) | run);
-  }
-  uint32_t total;
-  const uint32_t start = block_excl_scan<kOsThreads>(tile_count, s_warp, total);
-  const uint32_t dc = tid < kRadix ? digit_counts[tid] : 0u;
-  const uint32_t dbase = block_excl_scan<kOsThreads>(dc, s_warp, total);
-  if (tid < kRadix) {
-    s_tile_start[tid] = start;
-    // keys of this digit in the tiles before this one: the look-back reads four earlier tiles' words at a time
-    // (independent loads, one round trip) and walks them nearest first; a word not yet published is read again
-    uint32_t excl = 0, spins = 0;
-    for (int64_t j = (int64_t)tile - 1; j >= 0;) {
-      uint32_t w4[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) w4[q] = (j - q >= 0) ? ld_relaxed(status + (size_t)(j - q) * kRadix + tid) : kFlagPrefix;
-      bool done = false;
-      int q = 0;
-      for (; q < 4; ++q) {
-        const uint32_t flag = w4[q] & ~kCountMask;
-        if (flag == 0u) break;  // tile j - q has published nothing yet
-        excl += w4[q] & kCountMask;
-        if (flag == kFlagPrefix) { done = true; break; }
-      }
-      if (done) break;
-      j -= q;
-      if (q == 0 && ++spins > kSpinLimit) {
-        if (err) atomicOr(err, (uint32_t)RT_DEVERR_WAIT_TIMEOUT);
-        break;
+  };
+  load_tile(C.begin);
+
+  // where this chunk's keys of each digit start: the segment's keys of smaller digits, then the digit's keys in
+  // earlier chunks. Threads 0 .. 255 add up whole groups, threads 256 .. 511 the rows beside them.
+  uint32_t next = 0;  // thread d < 256: where the next tile's keys of digit d go
+  {
+    const uint32_t c = blockIdx.x, cs = C.first_chunk, ce = cs + C.n_chunks, d = tid & 255u;
+    const uint32_t g0 = (cs + kGroup - 1) / kGroup, g1 = max(g0, ce / kGroup);  // whole groups of the segment
+    uint32_t all = 0, part = 0;
+    if (d < D) {
+      if (tid < kRadix) {
+        sum_rows(P.groups, d, g0, g1, c / kGroup, all, part);
+      } else {
+        const uint32_t h1 = min(ce, g0 * kGroup), t0 = max(h1, g1 * kGroup);
+        sum_rows(P.rows, d, cs, h1, c, all, part);
+        sum_rows(P.rows, d, t0, ce, c, all, part);
+        const uint32_t own = c / kGroup;
+        uint32_t unused = 0;
+        if (own >= g0 && own < g1) sum_rows(P.rows, d, own * kGroup, c, c, unused, part);  // earlier chunks of its own group
       }
     }
-    if (tile > 0) st_relaxed(status + (size_t)tile * kRadix + tid, kFlagPrefix | (excl + tile_count));
-    s_glob[tid] = dbase + excl;
-    if (digit_totals_out && tile == 0) digit_totals_out[tid] = dc;
-  }
-  __syncthreads();
-
+    if (tid >= kRadix) { s_half[d] = all; s_half[kRadix + d] = part; }
+    __syncthreads();
+    uint32_t x = 0;
+    if (tid < kRadix) {
+      all += s_half[d];
+      part += s_half[kRadix + d];
+      x = all;
 #pragma unroll
-  for (int r = 0; r < kOsItems; ++r) {
-    const size_t idx = base + (size_t)warp * (kOsItems * 32) + r * 32 + lane;
-    if (idx < n) {
-      const uint32_t d = (key[r] >> shift) & 255u;
-      const uint32_t pos = s_tile_start[d] + s_cnt[warp][d] + rank[r];
-      s_keys[pos] = key[r];
-      if (kVals) s_vals[pos] = val[r];
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
+      if (lane == 31) s_scan[warp] = x;
+    }
+    __syncthreads();
+    if (tid < kRadix) {
+      uint32_t before = 0;
+      for (int w = 0; w < warp; ++w) before += s_scan[w];
+      next = C.seg_begin + before + x - all + part;
+      if (P.totals && c == cs && d < P.totals_stride) P.totals[(size_t)C.seg * P.totals_stride + d] = all;
     }
   }
-  __syncthreads();
-  const uint32_t tile_n = (uint32_t)min((size_t)kOsTile, (size_t)n - base);
-  for (uint32_t i = tid; i < tile_n; i += kOsThreads) {
-    const uint32_t k = s_keys[i];
-    const uint32_t d = (k >> shift) & 255u;
-    const size_t out = (size_t)s_glob[d] + (i - s_tile_start[d]);
-    keys_out[out] = k;
+
+  for (uint32_t q = lane; q < D; q += 32) s_mask[q] = 0;
+  for (uint32_t base = C.begin; base < C.end; base += T) {
+    const uint32_t tile_n = min(T, C.end - base);
+    // stable ranks inside the tile, the warp's counters in its own row of s_cnt. The lanes of equal digit come from a
+    // mask per digit in shared memory that every lane sets its bit in (and the first of them clears), or from one
+    // ballot per digit bit: masks load the shared-memory pipe, ballots the integer pipe, so a warp uses both.
+    *reinterpret_cast<uint4*>(&s_cnt[warp][8 * lane]) = make_uint4(0, 0, 0, 0);
+    __syncwarp();
+    uint32_t rank[kItems / 2] = {};  // two 16-bit ranks per word
+#pragma unroll
+    for (int r = 0; r < kItems; ++r) {
+      if ((uint32_t)warp * (kItems * 32) + r * 32 >= tile_n) continue;  // a row without keys (the same for the warp)
+      const bool valid = lane0 + r * 32 < tile_n;
+      const uint32_t d = (key[r] >> P.shift) & (D - 1u);
+      uint32_t peers;
+      const bool by_mask = r % 4 < kMaskRows;
+      if (by_mask) {
+        if (valid) atomicOr(&s_mask[d], 1u << lane);
+        __syncwarp();
+        peers = s_mask[d];
+      } else {
+        peers = __ballot_sync(0xffffffffu, valid);
+#pragma unroll
+        for (int b = 0; b < kBits; ++b) {
+          const bool bit = (d >> b) & 1u;
+          const uint32_t v = __ballot_sync(0xffffffffu, bit);
+          peers &= bit ? v : ~v;
+        }
+      }
+      const uint32_t pre = s_cnt[warp][d];
+      rank[r / 2] |= (pre + __popc(peers & lt)) << (16 * (r & 1));
+      __syncwarp();
+      if (valid && (peers & lt) == 0) {
+        s_cnt[warp][d] = (uint16_t)(pre + __popc(peers));
+        if (by_mask) s_mask[d] = 0;
+      }
+      __syncwarp();
+    }
+    uint32_t val[kVals ? kItems : 1];
     if (kVals) {
-      vals_out[out] = s_vals[i];
-      if (seg.out) seg.out[out] = find_seg(seg.off, seg.count, s_vals[i]);
+#pragma unroll
+      for (int r = 0; r < kItems; ++r) {
+        const uint32_t i = base + lane0 + r * 32;
+        val[r] = P.vals_in ? (i < C.end ? __ldg(P.vals_in + i) : 0u) : P.val_base + i;
+      }
+    }
+    __syncthreads();
+    // threads 0 .. 255, one digit each: the tile's run of the digit and where each warp's keys start in it
+    uint32_t x = 0, tile_count = 0;
+    if (tid < kRadix) {
+#pragma unroll
+      for (int w = 0; w < kScWarps; ++w) tile_count += s_cnt[w][tid];
+      x = tile_count;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
+      if (lane == 31) s_scan[warp] = x;
+    }
+    __syncthreads();
+    if (tid < kRadix) {
+      uint32_t start = x - tile_count;
+      for (int w = 0; w < warp; ++w) start += s_scan[w];
+      s_out[tid] = next - start;
+      next += tile_count;
+#pragma unroll
+      for (int w = 0; w < kScWarps; ++w) {
+        const uint32_t c = s_cnt[w][tid];
+        s_cnt[w][tid] = (uint16_t)start;
+        start += c;
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kItems; ++r) {
+      if (lane0 + r * 32 < tile_n) {
+        const uint32_t pos = s_cnt[warp][(key[r] >> P.shift) & (D - 1u)] + ((rank[r / 2] >> (16 * (r & 1))) & 0xffffu);
+        s_keys[pos] = key[r];
+        if (kVals) s_vals[pos] = val[r];
+      }
+    }
+    if (base + T < C.end) load_tile(base + T);  // on its way while this tile is written out
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kItems; ++r) {
+      const uint32_t i = tid + r * kScThreads;
+      if (i < tile_n) {
+        const uint32_t k = s_keys[i];
+        const uint32_t out = s_out[(k >> P.shift) & (D - 1u)] + i;
+        if (P.keys_out) P.keys_out[out] = k;
+        if (kVals) P.vals_out[out] = s_vals[i];
+      }
     }
   }
+}
+
+// The segment of every chunk (~0 for a gap of the chunk numbering).
+__global__ __launch_bounds__(256) void k_chunk_segs(const uint32_t* __restrict__ off, uint32_t M, uint32_t per_chunk, uint32_t chunks,
+                                                    uint32_t* __restrict__ chunk_seg) {
+  const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= chunks) return;
+  uint32_t lo = 0, hi = M - 1;  // largest m with sort_chunk_base(off[m], m) <= c
+  while (lo < hi) {
+    const uint32_t mid = (lo + hi + 1) >> 1;
+    if (sort_chunk_base(__ldg(off + mid), mid, per_chunk) <= c) lo = mid; else hi = mid - 1;
+  }
+  const uint32_t F = __ldg(off + lo), j = c - sort_chunk_base(F, lo, per_chunk);
+  chunk_seg[c] = (uint64_t)j * per_chunk < __ldg(off + lo + 1) - F ? lo : ~0u;
 }
 
 // n <= kTile: every pass in shared memory, one CTA. Dynamic shared memory:
 // 2 x kTile keys (+ 2 x kTile values).
 template <bool kVals>
 __global__ __launch_bounds__(kThreads) void k_radix_small(uint32_t* __restrict__ keys, uint32_t* __restrict__ vals, uint32_t n,
-                                                         uint32_t begin_bit, uint32_t passes, int init_vals,
-                                                         uint32_t* __restrict__ digit_totals_out, SegOut seg) {
+                                                         uint32_t begin_bit, uint32_t passes, int init_vals) {
   extern __shared__ uint32_t dyn[];
   uint32_t* kbuf[2] = {dyn, dyn + kTile};
   uint32_t* vbuf[2] = {dyn + 2 * kTile, dyn + 3 * kTile};
@@ -310,7 +416,6 @@ __global__ __launch_bounds__(kThreads) void k_radix_small(uint32_t* __restrict__
       s_cnt[w][threadIdx.x] = run;
       run += c;
     }
-    if (digit_totals_out && p + 1 == passes) digit_totals_out[threadIdx.x] = run;
     uint32_t total;
     s_tile_start[threadIdx.x] = block_excl_scan<kThreads>(run, s_warp, total);
     __syncthreads();
@@ -330,10 +435,7 @@ __global__ __launch_bounds__(kThreads) void k_radix_small(uint32_t* __restrict__
   }
   for (uint32_t i = threadIdx.x; i < n; i += kThreads) {
     keys[i] = kbuf[cur][i];
-    if (kVals) {
-      vals[i] = vbuf[cur][i];
-      if (seg.out) seg.out[i] = find_seg(seg.off, seg.count, vbuf[cur][i]);
-    }
+    if (kVals) vals[i] = vbuf[cur][i];
   }
 }
 
@@ -353,22 +455,69 @@ bool small_smem_ready() {
   });
 }
 
-// Scratch regions of an n-key sort (n > one tile), in carve order: the other key and value buffers, then one
-// zero-initialised block of every pass's tile status words, tile counters and digit counts.
-struct SortLayout {
-  uint32_t *kalt, *valt, *status, *counters, *counts;
-  size_t zero_bytes;
+// Tiles and chunks of an n-key sort with M segments. Tiles of 2048, 4096 or 8192 keys (4, 8 or 16 per thread): the
+// smallest that leaves every SM's two (three for 4096) resident CTAs at most one tile each, so that small sorts
+// spread over the chip and large ones have long digit runs; chunks of as many whole tiles as give two CTAs per SM.
+// 2^24 pairs: 8192-key tiles take 461 us, 6144 about 480, 4096 (three CTAs per SM) 610.
+struct SortPlan {
+  uint32_t items, per_chunk, chunks;
 };
-SortLayout carve_sort(Carve& c, uint32_t n) {
+SortPlan sort_plan(uint32_t n, uint32_t M) {
+  constexpr uint32_t kSms = 148;
+  SortPlan P;
+    P.items = n <= 2 * kSms * kScThreads * 4 ? 4 : (n <= 3 * kSms * kScThreads * 8 ? 8 : 16);
+  const uint32_t T = kScThreads * P.items, tiles = (uint32_t)(((uint64_t)n + T - 1) / T);
+  const uint32_t per = P.items == 16 ? (tiles + 2 * kSms - 1) / (2 * kSms) : 1;
+  P.per_chunk = per * T;
+  P.chunks = M > 1 ? n / P.per_chunk + M : (tiles + per - 1) / per;
+  return P;
+}
+// Scratch regions, in carve order: the other key and value buffers, the chunks' digit counts, the groups' (zeroed, one
+// set per pass), and with segments the chunks' segments.
+struct SortLayout {
+  uint32_t *kalt, *valt, *rows, *groups, *chunk_seg;
+  size_t group_words;  // of one pass
+};
+SortLayout carve_sort(Carve& c, uint32_t n, uint32_t M, const SortPlan& P) {
   SortLayout L;
-  const size_t tiles = (n + kOsTile - 1) / kOsTile;
   L.kalt = c.take<uint32_t>(n);
   L.valt = c.take<uint32_t>(n);
-  L.status = c.take<uint32_t>((size_t)kMaxPasses * tiles * kRadix + (size_t)kMaxPasses * 64 + (size_t)kMaxPasses * kRadix);
-  L.counters = L.status ? L.status + (size_t)kMaxPasses * tiles * kRadix : nullptr;  // one word per pass, 256 B apart
-  L.counts = L.counters ? L.counters + (size_t)kMaxPasses * 64 : nullptr;
-  L.zero_bytes = ((size_t)kMaxPasses * tiles * kRadix + (size_t)kMaxPasses * 64 + (size_t)kMaxPasses * kRadix) * 4;
+  L.rows = c.take<uint32_t>((size_t)P.chunks * kRadix);
+  L.group_words = ((size_t)P.chunks / kGroup + 1) * kRadix;
+  L.groups = c.take<uint32_t>(kMaxPasses * L.group_words);
+  L.chunk_seg = M > 1 ? c.take<uint32_t>(P.chunks) : nullptr;
   return L;
+}
+
+template <bool kVals, int kItems, int kBits, int kMode>
+rt_status launch_pass_of(const PassArgs& P, uint32_t chunks, cudaStream_t st) {
+  constexpr size_t smem = (size_t)kScThreads * kItems * 4 * (kVals ? 2 : 1) + (size_t)kScWarps * (1u << kBits) * 4;
+  if (smem + 12 * 1024 > 48 * 1024) {  // above what a launch may use unasked, with the static arrays
+    static PerDeviceOnce once;
+    if (!once.run([] {
+          return cudaFuncSetAttribute(k_sort_scatter<kVals, kItems, kBits, kMode>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)smem) == cudaSuccess;
+        }))
+      return RT_ERR_CUDA;
+  }
+  k_sort_count<kBits, kMode><<<chunks, kCountThreads, 0, st>>>(P);
+  k_sort_scatter<kVals, kItems, kBits, kMode><<<chunks, kScThreads, smem, st>>>(P);
+  note_launch(2);
+  RT_CHECK_LAUNCH();
+  return RT_OK;
+}
+template <bool kVals, int kBits, int kMode>
+rt_status launch_pass(const PassArgs& P, const SortPlan& S, cudaStream_t st) {
+  if (S.items == 4) return launch_pass_of<kVals, 4, kBits, kMode>(P, S.chunks, st);
+  if (S.items == 8) return launch_pass_of<kVals, 8, kBits, kMode>(P, S.chunks, st);
+  return launch_pass_of<kVals, 16, kBits, kMode>(P, S.chunks, st);
+}
+
+rt_status make_chunk_segs(const SortLayout& L, const SortPlan& S, const uint32_t* seg_off, uint32_t M, cudaStream_t st) {
+  k_chunk_segs<<<(S.chunks + 255) / 256, 256, 0, st>>>(seg_off, M, S.per_chunk, S.chunks, L.chunk_seg);
+  note_launch();
+  RT_CHECK_LAUNCH();
+  return RT_OK;
 }
 
 }  // namespace
@@ -378,56 +527,46 @@ size_t radix_scratch_bytes(uint32_t n) {
   return radix_scratch_bytes_of(n);
 }
 
+size_t segment_sort_scratch_bytes(uint32_t n, uint32_t M) {
+  Carve c(nullptr, 0);
+  carve_sort(c, n, M, sort_plan(n, M));
+  return c.off + 256;
+}
+
 rt_status radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_t begin_bit, uint32_t end_bit, int init_vals,
-                           void* scratch, size_t scratch_bytes, cudaStream_t stream, uint32_t* digit_totals_out, uint32_t* err,
-                           const uint32_t* digit_counts_in, const uint32_t* seg_off, uint32_t seg_count, uint32_t* seg_out) {
+                           void* scratch, size_t scratch_bytes, cudaStream_t stream, const uint32_t* seg_off, uint32_t M) {
   if (n == 0) return RT_OK;
   if (end_bit <= begin_bit || end_bit > 32) return RT_ERR_INVALID_ARGUMENT;
-  if (n > kCountMask) return RT_ERR_INVALID_ARGUMENT;
+  if (n > kMaxKeys) return RT_ERR_INVALID_ARGUMENT;
   const uint32_t passes = (end_bit - begin_bit + 7) / 8;
-  if (n <= (uint32_t)kTile) {
+  if (M <= 1 && n <= (uint32_t)kTile) {
     if (!small_smem_ready()) return RT_ERR_CUDA;
-    if (vals)
-      k_radix_small<true><<<1, kThreads, kSmallSmem, stream>>>(keys, vals, n, begin_bit, passes, init_vals, digit_totals_out,
-                                                               SegOut{seg_off, seg_count, (seg_off && seg_count) ? seg_out : nullptr});
-    else
-      k_radix_small<false><<<1, kThreads, kSmallSmem, stream>>>(keys, nullptr, n, begin_bit, passes, 0, digit_totals_out, SegOut{});
+    if (vals) k_radix_small<true><<<1, kThreads, kSmallSmem, stream>>>(keys, vals, n, begin_bit, passes, init_vals);
+    else k_radix_small<false><<<1, kThreads, kSmallSmem, stream>>>(keys, nullptr, n, begin_bit, passes, 0);
     note_launch();
     RT_CHECK_LAUNCH();
     return RT_OK;
   }
-  if (!scratch || scratch_bytes < radix_scratch_bytes(n)) return RT_ERR_SCRATCH_TOO_SMALL;
-  const uint32_t tiles = (n + kOsTile - 1) / kOsTile;
+  if (!scratch) return RT_ERR_SCRATCH_TOO_SMALL;
+  const SortPlan S = sort_plan(n, M);
   Carve c(scratch, scratch_bytes);
-  const SortLayout L = carve_sort(c, n);
+  const SortLayout L = carve_sort(c, n, M, S);
   if (!c.ok()) return RT_ERR_SCRATCH_TOO_SMALL;
-  if (cudaMemsetAsync(L.status, 0, L.zero_bytes, stream) != cudaSuccess) return RT_ERR_CUDA;
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
-    sms = 148;
-  const uint32_t* counts = digit_counts_in;
-  if (!counts) {  // one read of the keys for every pass's digit counts, unless the keys' producer counted them
-    const uint32_t hist_blocks = (uint32_t)hmin<size_t>((n / 4 + 255) / 256, (size_t)sms * 4);
-    k_sort_hist<<<hist_blocks ? hist_blocks : 1, 256, 0, stream>>>(keys, n, begin_bit, passes, L.counts);
-    note_launch();
-    RT_CHECK_LAUNCH();
-    counts = L.counts;
+  if (cudaMemsetAsync(L.groups, 0, passes * L.group_words * 4, stream) != cudaSuccess) return RT_ERR_CUDA;
+  if (M > 1) {
+    const rt_status s = make_chunk_segs(L, S, seg_off, M, stream);
+    if (s != RT_OK) return s;
   }
   uint32_t *ks = keys, *vs = vals, *kd = L.kalt, *vd = L.valt;
   for (uint32_t p = 0; p < passes; ++p) {
-    const uint32_t shift = begin_bit + 8 * p;
-    uint32_t* st = L.status + (size_t)p * tiles * kRadix;
-    uint32_t* ctr = L.counters + (size_t)p * 64;
-    const uint32_t* dc = counts + (size_t)p * kRadix;
-    uint32_t* dto = p + 1 == passes ? digit_totals_out : nullptr;
-    const SegOut seg{seg_off, seg_count, (p + 1 == passes && seg_off && seg_count) ? seg_out : nullptr};
-    if (vals)
-      k_onesweep<true><<<tiles, kOsThreads, 0, stream>>>(ks, (p == 0 && init_vals) ? nullptr : vs, kd, vd, n, shift, dc, st, ctr, dto, err,
-                                                          seg);
-    else
-      k_onesweep<false><<<tiles, kOsThreads, 0, stream>>>(ks, nullptr, kd, nullptr, n, shift, dc, st, ctr, dto, err, SegOut{});
-    note_launch();
-    RT_CHECK_LAUNCH();
+    PassArgs P = {};
+    P.keys_in = ks; P.keys_out = kd;
+    P.vals_in = (p == 0 && init_vals) ? nullptr : vs; P.vals_out = vd;
+    P.n = n; P.shift = begin_bit + 8 * p; P.per_chunk = S.per_chunk;
+    if (M > 1) { P.seg_off = seg_off; P.chunk_seg = L.chunk_seg; }
+    P.rows = L.rows; P.groups = L.groups + p * L.group_words;
+    const rt_status s = vals ? launch_pass<true, 8, 0>(P, S, stream) : launch_pass<false, 8, 0>(P, S, stream);
+    if (s != RT_OK) return s;
     uint32_t* t;
     t = ks; ks = kd; kd = t;
     t = vs; vs = vd; vd = t;
@@ -437,6 +576,27 @@ rt_status radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_t 
     if (vals && cudaMemcpyAsync(vals, vs, (size_t)n * 4, cudaMemcpyDeviceToDevice, stream) != cudaSuccess) return RT_ERR_CUDA;
   }
   return RT_OK;
+}
+
+rt_status sort_split_levels(const uint32_t* codes, uint32_t n, uint32_t* splits, uint32_t* level_counts, uint32_t count_stride,
+                            void* scratch, size_t scratch_bytes, cudaStream_t stream, const uint32_t* seg_off, uint32_t M) {
+  if (n == 0) return RT_OK;
+  if (!scratch || n > kMaxKeys) return RT_ERR_INVALID_ARGUMENT;
+  const SortPlan S = sort_plan(n, M);
+  Carve c(scratch, scratch_bytes);
+  const SortLayout L = carve_sort(c, n, M, S);
+  if (!c.ok()) return RT_ERR_SCRATCH_TOO_SMALL;
+  if (cudaMemsetAsync(L.groups, 0, L.group_words * 4, stream) != cudaSuccess) return RT_ERR_CUDA;
+  if (M > 1) {
+    const rt_status s = make_chunk_segs(L, S, seg_off, M, stream);
+    if (s != RT_OK) return s;
+  }
+  PassArgs P = {};
+  P.keys_in = codes; P.vals_out = splits; P.val_base = 1;
+  P.n = n; P.per_chunk = S.per_chunk;
+  if (M > 1) { P.seg_off = seg_off; P.chunk_seg = L.chunk_seg; }
+  P.rows = L.rows; P.groups = L.groups; P.totals = level_counts; P.totals_stride = count_stride;
+  return launch_pass<true, 6, 1>(P, S, stream);
 }
 
 }  // namespace rt
@@ -466,13 +626,12 @@ extern "C" rt_status rt_radix_sort_pairs(uint32_t* keys, uint32_t* values, uint3
     RT_CHECK_LAUNCH();
     return RT_OK;
   }
-  return radix_sort_pairs(keys, values, n, 0, bits_of(bit_depth), init_values, scratch, scratch_bytes, (cudaStream_t)stream, nullptr,
-                          nullptr);
+  return radix_sort_pairs(keys, values, n, 0, bits_of(bit_depth), init_values, scratch, scratch_bytes, (cudaStream_t)stream);
 }
 
 extern "C" rt_status rt_radix_sort_keys(uint32_t* keys, uint32_t n, uint32_t bit_depth, void* scratch, size_t scratch_bytes, rt_stream stream) {
   if (n && !keys) return RT_ERR_INVALID_ARGUMENT;
   if (n > (uint32_t)kTile && (!scratch || scratch_bytes < radix_scratch_bytes(n))) return RT_ERR_SCRATCH_TOO_SMALL;
   if (rt_device_check() != RT_OK) return RT_ERR_NO_DEVICE;
-  return radix_sort_pairs(keys, nullptr, n, 0, bits_of(bit_depth), 0, scratch, scratch_bytes, (cudaStream_t)stream, nullptr, nullptr);
+  return radix_sort_pairs(keys, nullptr, n, 0, bits_of(bit_depth), 0, scratch, scratch_bytes, (cudaStream_t)stream);
 }

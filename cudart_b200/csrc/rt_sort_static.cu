@@ -73,5 +73,5 @@ extern "C" rt_status rt_radix_sort_pairs_static(uint32_t* keys, uint32_t* values
     if (init_values && cudaMemsetAsync(values, 0, 4, (cudaStream_t)stream) != cudaSuccess) return RT_ERR_CUDA;
     return RT_OK;
   }
-  return rt::radix_sort_pairs(keys, values, n, 0, 8 * bytes, init_values, scratch, kScratchBytes, (cudaStream_t)stream, nullptr);
+  return rt::radix_sort_pairs(keys, values, n, 0, 8 * bytes, init_values, scratch, kScratchBytes, (cudaStream_t)stream);
 }

@@ -2191,7 +2191,7 @@ extern "C" rt_status rt_ray_order(const float* orig, const float* dir, const flo
   k_ray_keys<<<blocks, 256, 0, st>>>((const float4*)orig, (const float4*)dir, tmax, count, lo, sc, keys, order);
   note_launch();
   RT_CHECK_LAUNCH();
-  return radix_sort_pairs(keys, order, count, 0, 24, 0, sort_scratch, radix_scratch_bytes(count), st, nullptr);
+  return radix_sort_pairs(keys, order, count, 0, 24, 0, sort_scratch, radix_scratch_bytes(count), st);
 }
 
 extern "C" rt_status rt_batch_ray_order_scratch_bytes(uint32_t count, size_t* bytes) { return rt_ray_order_scratch_bytes(count, bytes); }
@@ -2222,7 +2222,7 @@ extern "C" rt_status rt_batch_ray_order(const float* orig, const float* dir, con
                                            keys, order);
   note_launch();
   RT_CHECK_LAUNCH();
-  return radix_sort_pairs(keys, order, count, 0, (key_bits + 7) / 8 * 8, 0, sort_scratch, radix_scratch_bytes(count), st, nullptr);
+  return radix_sort_pairs(keys, order, count, 0, (key_bits + 7) / 8 * 8, 0, sort_scratch, radix_scratch_bytes(count), st);
 }
 
 extern "C" rt_status rt_image_tile_order(uint32_t images, uint32_t width, uint32_t height, uint32_t* order, rt_stream stream) {
