@@ -47,7 +47,7 @@ RASTER_EXPORTS = ("rt_camera_view_dir", "rt_raster_matrix", "rt_raster_scratch_b
 PROPOSE_EXPORTS = (
     "rt_propose_abi_version", "rt_gemm_bf16", "rt_gemm_argmax_bf16", "rt_ray_features", "rt_softmax_xent", "rt_transpose_bf16",
     "rt_colsum_bf16", "rt_adam_step", "rt_subtree_slots", "rt_hit_labels", "rt_trace_closest_seeded", "rt_transpose_bf16_grouped",
-    "rt_colsum_bf16_grouped", "rt_gather_batch", "rt_batch_subtree_slots", "rt_batch_hit_labels", "rt_batch_trace_seeded",
+    "rt_gemm_bf16_multi", "rt_colsum_bf16_multi", "rt_adam_step_multi", "rt_colsum_bf16_grouped", "rt_gather_batch", "rt_batch_subtree_slots", "rt_batch_hit_labels", "rt_batch_trace_seeded",
     "rt_group_select", "rt_mlp_propose", "rt_gemm_xent_bf16", "rt_tc_wait_selftest",
 )
 
@@ -144,6 +144,10 @@ class GemmArgmaxDesc(C.Structure):
 class FeatureDesc(C.Structure):
     _fields_ = [("orig", _P), ("dir", _P), ("count", _U32), ("box_lo", C.c_float * 3), ("box_hi", C.c_float * 3), ("out", _P),
                 ("ld_out", _U32), ("out_t", _P), ("ld_out_t", _U32), ("group_rows", _U32)]
+
+
+class ColsumDesc(C.Structure):
+    _fields_ = [("in_", _P), ("out", _P), ("groups", _U32), ("rows", _U32), ("cols", _U32), ("ld", _U32)]
 
 
 class AdamDesc(C.Structure):
@@ -246,6 +250,9 @@ def lib():
         L.rt_transpose_bf16.argtypes = [_P, _U32, _U32, _U32, _P, _U32, _P]
         L.rt_colsum_bf16.argtypes = [_P, _U32, _U32, _U32, _P, _P]
         L.rt_adam_step.argtypes = [C.POINTER(AdamDesc), _P]
+        L.rt_gemm_bf16_multi.argtypes = [C.POINTER(GemmDesc), _U32, _P]
+        L.rt_colsum_bf16_multi.argtypes = [C.POINTER(ColsumDesc), _U32, _P]
+        L.rt_adam_step_multi.argtypes = [C.POINTER(AdamDesc), _U32, _P]
         L.rt_subtree_slots.argtypes = [C.POINTER(SlotDesc), _P]
         L.rt_hit_labels.argtypes = [_P, _U32, _P, _P, _P]
         L.rt_trace_closest_seeded.argtypes = [C.POINTER(TraceDesc), C.POINTER(SeedDesc), _P]

@@ -31,6 +31,7 @@ using namespace tc;
 
 constexpr uint32_t kBM = 128, kBK = 64, kStages = 4;
 constexpr uint32_t kTileA = kBM * kBK * 2;  // 16 KB per A stage
+constexpr uint32_t kMulti = RT_MULTI_MAX;   // products, sums or tensors of one launch
 
 // Four bf16 values as one 8-byte word, the first at the lowest address (an 8-byte store writes them in order).
 __device__ __forceinline__ uint2 pack_bf16x4(__nv_bfloat16 a, __nv_bfloat16 b, __nv_bfloat16 c, __nv_bfloat16 d) {
@@ -134,9 +135,9 @@ __device__ __forceinline__ void epilogue16(const GemmEpi& E, uint32_t g, uint32_
 // short-K GEMM leaves room for more CTAs per SM), warp 1 lane 0 issues the
 // MMAs, then all four warps drain TMEM.
 // ----------------------------------------------------------------------------
-__global__ void __launch_bounds__(128, 1)
-    k_gemm_tc(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb, GemmEpi E, uint32_t bn,
-              uint32_t tmem_cols, uint32_t num_k, uint32_t stages, uint32_t* err) {
+__device__ __forceinline__ void gemm_tile(const CUtensorMap& ta, const CUtensorMap& tb, const GemmEpi& E, uint32_t bn,
+                                          uint32_t tmem_cols, uint32_t num_k, uint32_t stages, uint32_t* err, uint32_t bx, uint32_t by,
+                                          uint32_t g) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const uint32_t tile_b = bn * 128u;
@@ -166,8 +167,7 @@ __global__ void __launch_bounds__(128, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  const uint32_t g = blockIdx.z;
-  const int32_t m0 = (int32_t)(g * E.gm + blockIdx.y * kBM), n0 = (int32_t)(blockIdx.x * bn);
+  const int32_t m0 = (int32_t)(g * E.gm + by * kBM), n0 = (int32_t)(bx * bn);
 
   if (warp == 0 && lane == 0) {
     const int32_t b0 = (int32_t)(g * E.gn) + n0;
@@ -212,6 +212,33 @@ __global__ void __launch_bounds__(128, 1)
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, tmem_cols);
+}
+__global__ void __launch_bounds__(128, 1)
+    k_gemm_tc(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb, GemmEpi E, uint32_t bn,
+              uint32_t tmem_cols, uint32_t num_k, uint32_t stages, uint32_t* err) {
+  gemm_tile(ta, tb, E, bn, tmem_cols, num_k, stages, err, blockIdx.x, blockIdx.y, blockIdx.z);
+}
+
+// Several independent products, their tiles side by side in one grid. A tile's MMAs are a chain (about 98 ns per
+// 16-deep step whatever its width, since each adds to the sum before), so the four weight gradients of a step with
+// K = 8192 took 51 us each one after another, 33 of 148 SMs at the most; together they take 51.
+struct GemmProblem {
+  CUtensorMap ta, tb;
+  GemmEpi E;
+  uint32_t bn, tmem_cols, num_k, stages, nx, ny, first;  // tiles nx x ny per group, from block `first`
+  uint32_t* err;
+};
+struct GemmBatch {
+  GemmProblem p[kMulti];
+  uint32_t count;
+};
+static_assert(sizeof(GemmBatch) <= 4096, "kernel parameters");
+__global__ void __launch_bounds__(128, 1) k_gemm_multi_tc(const __grid_constant__ GemmBatch B) {
+  uint32_t i = 0;
+  while (i + 1 < B.count && blockIdx.x >= B.p[i + 1].first) ++i;
+  const GemmProblem& P = B.p[i];
+  const uint32_t t = blockIdx.x - P.first;
+  gemm_tile(P.ta, P.tb, P.E, P.bn, P.tmem_cols, P.num_k, P.stages, P.err, t % P.nx, t / P.nx % P.ny, t / (P.nx * P.ny));
 }
 
 // ----------------------------------------------------------------------------
@@ -544,7 +571,12 @@ __global__ void __launch_bounds__(kXentThreads, 1)
           // every partial has been read above: slot 0 now carries the merged row
           s_x[trow] = make_float4(mx, sum, 0.0f, 0.0f);
           mbar_arrive(xch_b);
-          if (valid && X.loss_sum) atomicAdd(X.loss_sum, (logf(sum) + mx - xl) * X.scale);
+          if (X.loss_sum) {  // one addition per warp: 8192 rows added one by one were off by 1.6e-6
+            float l = valid ? (logf(sum) + mx - xl) * X.scale : 0.0f;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+            if (lane == 0) atomicAdd(X.loss_sum, l);
+          }
         }
         inv = 1.0f / sum;
       }
@@ -728,24 +760,39 @@ __global__ __launch_bounds__(256) void k_transpose_bf16(const __nv_bfloat16* __r
 // order: block (32, 8) per 32 columns of one group (blockIdx.y); thread y sums
 // rows y, y + 8, ... and the eight partial sums are added in order y = 0..7.
 // The same sums with two columns per thread (4-byte loads, whole 128-byte
-// rows per warp) and four rows in flight; each column's summation order is
+// rows per warp) and 32 rows in flight; each column's summation order is
 // unchanged (row y, y + 8, ... per thread, then the eight partials in order),
-// so the results are the same bits. Needs even cols and ld.
-__global__ __launch_bounds__(256) void k_colsum2_bf16(const __nv_bfloat16* __restrict__ in, uint32_t rows, uint32_t cols, uint32_t ld,
-                                                      float* __restrict__ out) {
+// so the results are the same bits. Needs even cols and ld. Several inputs can
+// share a launch, their column blocks side by side. Bound by latency (256
+// threads per 64 columns): four rows in flight took 85 us for 8192 rows, once
+// for each of a step's four inputs; the four together now take 61.
+struct ColsumProblem {
+  const __nv_bfloat16* in;
+  float* out;
+  uint32_t rows, cols, ld, nx, first;  // nx column blocks per group, from block `first`
+};
+struct ColsumBatch {
+  ColsumProblem p[kMulti];
+  uint32_t count;
+};
+__global__ __launch_bounds__(256) void k_colsum2_bf16(const __grid_constant__ ColsumBatch B) {
+  constexpr int kAhead = 32;
   __shared__ float2 part[8][33];
-  const uint32_t c = (blockIdx.x * 32 + threadIdx.x) * 2, g = blockIdx.y;
-  const __nv_bfloat162* p = (const __nv_bfloat162*)(in + (size_t)g * rows * ld + c);
-  const uint32_t ld2 = ld / 2;
+  uint32_t i = 0;
+  while (i + 1 < B.count && blockIdx.x >= B.p[i + 1].first) ++i;
+  const uint32_t rows = B.p[i].rows, cols = B.p[i].cols, ld2 = B.p[i].ld / 2;
+  float* out = B.p[i].out;
+  const uint32_t t = blockIdx.x - B.p[i].first, c = (t % B.p[i].nx * 32 + threadIdx.x) * 2, g = t / B.p[i].nx;
+  const __nv_bfloat162* p = (const __nv_bfloat162*)(B.p[i].in + (size_t)g * rows * B.p[i].ld + c);
   float s0 = 0.0f, s1 = 0.0f;
   if (c < cols) {
     uint32_t r = threadIdx.y;
-    for (; r + 24 < rows; r += 32) {
-      __nv_bfloat162 h[4];
+    for (; r + 8 * (kAhead - 1) < rows; r += 8 * kAhead) {
+      __nv_bfloat162 h[kAhead];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) h[k] = p[(size_t)(r + 8 * k) * ld2];
+      for (int k = 0; k < kAhead; ++k) h[k] = p[(size_t)(r + 8 * k) * ld2];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
+      for (int k = 0; k < kAhead; ++k) {
         s0 += __low2float(h[k]);
         s1 += __high2float(h[k]);
       }
@@ -877,12 +924,27 @@ __global__ __launch_bounds__(256) void k_adam(float* __restrict__ p, const float
 // and stores; rows, cols, the BF16 leading dimensions and the group rows are
 // multiples of 4 and the FP32 arrays 16-byte aligned): 256 threads per 32 x 32
 // tile, the transposed BF16 copy through shared memory, 4 rows per 8-byte store.
-__global__ __launch_bounds__(256) void k_adam_t4(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
-                                                 float* __restrict__ v, uint32_t rows, uint32_t cols, float lr, float b1, float b2,
-                                                 float eps, float c1, float c2, __nv_bfloat16* __restrict__ out16, uint32_t ld16,
-                                                 __nv_bfloat16* __restrict__ out16t, uint32_t ld16t, uint32_t group_rows) {
-  __shared__ __nv_bfloat16 tile[32][40];
-  const uint32_t c0 = blockIdx.x * 32, r0 = blockIdx.y * 32, t = threadIdx.x;
+struct AdamProblem {
+  float* p;
+  const float* g;
+  float* m;
+  float* v;
+  uint32_t rows, cols;
+  float lr, b1, b2, eps, c1, c2;
+  __nv_bfloat16* out16;
+  __nv_bfloat16* out16t;  // null: no BF16 copies (a bias)
+  uint32_t ld16, ld16t, group_rows, nx, first;  // nx tiles (or blocks of 256 words) per row of tiles, from block `first`
+};
+struct AdamBatch {
+  AdamProblem p[kMulti];
+  uint32_t count;
+};
+__device__ __forceinline__ void adam_tile4(__nv_bfloat16 (&tile)[32][40], uint32_t bx, uint32_t by, float* __restrict__ p,
+                                           const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v, uint32_t rows,
+                                           uint32_t cols, float lr, float b1, float b2, float eps, float c1, float c2,
+                                           __nv_bfloat16* __restrict__ out16, uint32_t ld16, __nv_bfloat16* __restrict__ out16t,
+                                           uint32_t ld16t, uint32_t group_rows) {
+  const uint32_t c0 = bx * 32, r0 = by * 32, t = threadIdx.x;
   {
     const uint32_t lr_ = t >> 3, lc = (t & 7u) * 4u, r = r0 + lr_, c = c0 + lc;
     if (r < rows && c < cols) {
@@ -920,6 +982,23 @@ __global__ __launch_bounds__(256) void k_adam_t4(float* __restrict__ p, const fl
       const uint32_t q = r / group_rows;
       *(uint2*)(out16t + ((size_t)q * cols + c) * ld16t + (r - q * group_rows)) = pack_bf16x4(h[0], h[1], h[2], h[3]);
     }
+  }
+}
+
+// Every tensor of a network in one launch: matrices in 32 x 32 tiles, biases in blocks of 256 (a step's eight tensors took
+// eight launches of 3 to 5 us).
+__global__ __launch_bounds__(256) void k_adam_multi(const __grid_constant__ AdamBatch B) {
+  __shared__ __nv_bfloat16 tile[32][40];
+  uint32_t i = 0;
+  while (i + 1 < B.count && blockIdx.x >= B.p[i + 1].first) ++i;
+  const AdamProblem& P = B.p[i];
+  const uint32_t t = blockIdx.x - P.first;
+  if (P.out16t) {
+    adam_tile4(tile, t % P.nx, t / P.nx, P.p, P.g, P.m, P.v, P.rows, P.cols, P.lr, P.b1, P.b2, P.eps, P.c1, P.c2, P.out16, P.ld16,
+               P.out16t, P.ld16t, P.group_rows);
+  } else {
+    const size_t k = (size_t)t * 256 + threadIdx.x;
+    if (k < (size_t)P.rows * P.cols) adam_update(P.p, P.g, P.m, P.v, k, P.lr, P.b1, P.b2, P.eps, P.c1, P.c2);
   }
 }
 
@@ -1445,8 +1524,9 @@ extern "C" rt_status rt_tc_wait_selftest(uint32_t limit_us, uint32_t* error_word
 
 extern "C" uint32_t rt_propose_abi_version(void) { return RT_PROPOSE_ABI_VERSION; }
 
-extern "C" rt_status rt_gemm_bf16(const rt_gemm_desc* d, rt_stream stream) {
-  if (!d || !d->a || !d->b) return RT_ERR_INVALID_ARGUMENT;
+// One product's checks, and its part of a launch.
+static rt_status gemm_check(const rt_gemm_desc* d) {
+  if (!d->a || !d->b) return RT_ERR_INVALID_ARGUMENT;
   if (d->m == 0 || d->n == 0 || d->k == 0) return RT_ERR_INVALID_ARGUMENT;
   if (d->m % kBM || d->k % kBK || d->n % 16) return RT_ERR_INVALID_ARGUMENT;
   if (d->lda < d->k || d->ldb < d->k || d->lda % 8 || d->ldb % 8) return RT_ERR_INVALID_ARGUMENT;
@@ -1457,11 +1537,13 @@ extern "C" rt_status rt_gemm_bf16(const rt_gemm_desc* d, rt_stream stream) {
   if (d->ct_bf16 && d->ldct < d->m) return RT_ERR_INVALID_ARGUMENT;
   const uint32_t G = d->groups ? d->groups : 1u;
   if (G > 65535u || (uint64_t)G * d->m > 0x7FFFFFFFull || (uint64_t)G * d->n > 0x7FFFFFFFull) return RT_ERR_INVALID_ARGUMENT;
-  if (rt_device_check() != RT_OK) return RT_ERR_NO_DEVICE;
+  return RT_OK;
+}
+static rt_status gemm_problem(const rt_gemm_desc* d, GemmProblem& P) {
+  const uint32_t G = d->groups ? d->groups : 1u;
   const uint32_t bn = pick_bn(d->n);
-  CUtensorMap ta, tb;
-  if (!make_map(&ta, d->a, d->k, G * d->m, d->lda, kBM) || !make_map(&tb, d->b, d->k, G * d->n, d->ldb, bn)) return RT_ERR_UNSUPPORTED;
-  GemmEpi E;
+  if (!make_map(&P.ta, d->a, d->k, G * d->m, d->lda, kBM) || !make_map(&P.tb, d->b, d->k, G * d->n, d->ldb, bn)) return RT_ERR_UNSUPPORTED;
+  GemmEpi& E = P.E;
   E.alpha = d->alpha; E.bias = d->bias; E.relu = d->relu; E.mask = (const __nv_bfloat16*)d->mask; E.ldmask = d->ldmask;
   E.c32 = d->c_f32; E.ldc32 = d->ldc_f32; E.c16 = (__nv_bfloat16*)d->c_bf16; E.ldc16 = d->ldc_bf16;
   E.ct16 = (__nv_bfloat16*)d->ct_bf16; E.ldct = d->ldct;
@@ -1469,12 +1551,53 @@ extern "C" rt_status rt_gemm_bf16(const rt_gemm_desc* d, rt_stream stream) {
   E.c32_v8 = (d->c_f32 && d->ldc_f32 % 8 == 0 && ((uintptr_t)d->c_f32 & 31u) == 0) ? 1u : 0u;
   E.c16_v8 = (d->c_bf16 && d->ldc_bf16 % 16 == 0 && ((uintptr_t)d->c_bf16 & 31u) == 0) ? 1u : 0u;
   const uint32_t num_k = d->k / kBK, stages = num_k < kStages ? num_k : kStages;
-  const size_t smem = gemm_smem(bn, stages);
+  P.bn = bn; P.tmem_cols = pow2_cols(bn); P.num_k = num_k; P.stages = stages;
+  P.nx = d->n / bn; P.ny = d->m / kBM; P.err = d->error_word;
+  return RT_OK;
+}
+
+extern "C" rt_status rt_gemm_bf16(const rt_gemm_desc* d, rt_stream stream) {
+  if (!d) return RT_ERR_INVALID_ARGUMENT;
+  rt_status s = gemm_check(d);
+  if (s != RT_OK) return s;
+  if (rt_device_check() != RT_OK) return RT_ERR_NO_DEVICE;
+  GemmProblem P;
+  if ((s = gemm_problem(d, P)) != RT_OK) return s;
   static PerDeviceOnce once;
   if (!once.run([] { return cudaFuncSetAttribute(k_gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem(256)) == cudaSuccess; }))
     return RT_ERR_CUDA;
-  dim3 grid(d->n / bn, d->m / kBM, G);
-  k_gemm_tc<<<grid, 128, smem, (cudaStream_t)stream>>>(ta, tb, E, bn, pow2_cols(bn), num_k, stages, d->error_word);
+  k_gemm_tc<<<dim3(P.nx, P.ny, d->groups ? d->groups : 1u), 128, gemm_smem(P.bn, P.stages), (cudaStream_t)stream>>>(
+      P.ta, P.tb, P.E, P.bn, P.tmem_cols, P.num_k, P.stages, P.err);
+  note_launch();
+  RT_CHECK_LAUNCH();
+  return RT_OK;
+}
+
+extern "C" rt_status rt_gemm_bf16_multi(const rt_gemm_desc* d, uint32_t count, rt_stream stream) {
+  if (!d || count == 0 || count > kMulti) return RT_ERR_INVALID_ARGUMENT;
+  for (uint32_t i = 0; i < count; ++i) {
+    const rt_status s = gemm_check(d + i);
+    if (s != RT_OK) return s;
+  }
+  if (rt_device_check() != RT_OK) return RT_ERR_NO_DEVICE;
+  GemmBatch B;
+  B.count = count;
+  uint64_t blocks = 0;
+  size_t smem = 0;
+  for (uint32_t i = 0; i < count; ++i) {
+    const rt_status s = gemm_problem(d + i, B.p[i]);
+    if (s != RT_OK) return s;
+    B.p[i].first = (uint32_t)blocks;
+    blocks += (uint64_t)B.p[i].nx * B.p[i].ny * (d[i].groups ? d[i].groups : 1u);
+    if (blocks > 0x7FFFFFFFull) return RT_ERR_INVALID_ARGUMENT;
+    smem = hmax<size_t>(smem, gemm_smem(B.p[i].bn, B.p[i].stages));
+  }
+  static PerDeviceOnce once;
+  if (!once.run([] {
+        return cudaFuncSetAttribute(k_gemm_multi_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem(256)) == cudaSuccess;
+      }))
+    return RT_ERR_CUDA;
+  k_gemm_multi_tc<<<(uint32_t)blocks, 128, smem, (cudaStream_t)stream>>>(B);
   note_launch();
   RT_CHECK_LAUNCH();
   return RT_OK;
@@ -1623,18 +1746,42 @@ extern "C" rt_status rt_transpose_bf16(const void* in, uint32_t rows, uint32_t c
   return rt_transpose_bf16_grouped(in, 1, rows, cols, ld_in, out, ld_out, stream);
 }
 
+static bool colsum_by_two(const rt_colsum_desc* d) {
+  return d->cols % 2 == 0 && d->ld % 2 == 0 && ((uintptr_t)d->in & 3u) == 0 && ((uintptr_t)d->out & 7u) == 0;
+}
+extern "C" rt_status rt_colsum_bf16_multi(const rt_colsum_desc* d, uint32_t count, rt_stream stream) {
+  if (!d || count == 0 || count > kMulti) return RT_ERR_INVALID_ARGUMENT;
+  for (uint32_t i = 0; i < count; ++i)
+    if (!d[i].in || !d[i].out || d[i].ld < d[i].cols || d[i].groups == 0 || d[i].groups > 65535u) return RT_ERR_INVALID_ARGUMENT;
+  if (rt_device_check() != RT_OK) return RT_ERR_NO_DEVICE;
+  ColsumBatch B = {};
+  uint64_t blocks = 0;
+  for (uint32_t i = 0; i < count; ++i) {
+    if (d[i].cols == 0) continue;
+    if (!colsum_by_two(d + i)) {
+      k_colsum_bf16<<<dim3((d[i].cols + 31) / 32, d[i].groups), dim3(32, 8), 0, (cudaStream_t)stream>>>(
+          (const __nv_bfloat16*)d[i].in, d[i].rows, d[i].cols, d[i].ld, d[i].out);
+      note_launch();
+      RT_CHECK_LAUNCH();
+      continue;
+    }
+    ColsumProblem& P = B.p[B.count++];
+    P.in = (const __nv_bfloat16*)d[i].in; P.out = d[i].out; P.rows = d[i].rows; P.cols = d[i].cols; P.ld = d[i].ld;
+    P.nx = (d[i].cols + 63) / 64; P.first = (uint32_t)blocks;
+    blocks += (uint64_t)P.nx * d[i].groups;
+    if (blocks > 0x7FFFFFFFull) return RT_ERR_INVALID_ARGUMENT;
+  }
+  if (B.count) {
+    k_colsum2_bf16<<<(uint32_t)blocks, dim3(32, 8), 0, (cudaStream_t)stream>>>(B);
+    note_launch();
+    RT_CHECK_LAUNCH();
+  }
+  return RT_OK;
+}
 extern "C" rt_status rt_colsum_bf16_grouped(const void* in, uint32_t groups, uint32_t rows, uint32_t cols, uint32_t ld, float* out,
                                             rt_stream stream) {
-  if (!in || !out || ld < cols || groups == 0 || groups > 65535u) return RT_ERR_INVALID_ARGUMENT;
-  if (rt_device_check() != RT_OK) return RT_ERR_NO_DEVICE;
-  if (cols == 0) return RT_OK;
-  if (cols % 2 == 0 && ld % 2 == 0 && ((uintptr_t)in & 3u) == 0 && ((uintptr_t)out & 7u) == 0)
-    k_colsum2_bf16<<<dim3((cols + 63) / 64, groups), dim3(32, 8), 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)in, rows, cols, ld, out);
-  else
-    k_colsum_bf16<<<dim3((cols + 31) / 32, groups), dim3(32, 8), 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)in, rows, cols, ld, out);
-  note_launch();
-  RT_CHECK_LAUNCH();
-  return RT_OK;
+  const rt_colsum_desc d = {in, out, groups, rows, cols, ld};
+  return rt_colsum_bf16_multi(&d, 1, stream);
 }
 
 extern "C" rt_status rt_colsum_bf16(const void* in, uint32_t rows, uint32_t cols, uint32_t ld, float* out, rt_stream stream) {
@@ -1667,33 +1814,55 @@ extern "C" rt_status rt_group_select(const int32_t* labels, uint32_t groups, uin
   return RT_OK;
 }
 
-extern "C" rt_status rt_adam_step(const rt_adam_desc* d, rt_stream stream) {
-  if (!d || !d->param || !d->grad || !d->m || !d->v || d->step == 0) return RT_ERR_INVALID_ARGUMENT;
-  const uint32_t G = d->groups ? d->groups : 1u;
-  if (d->rows % G) return RT_ERR_INVALID_ARGUMENT;
-  if (rt_device_check() != RT_OK) return RT_ERR_NO_DEVICE;
-  const size_t total = (size_t)d->rows * d->cols;
-  if (total == 0) return RT_OK;
-  const float c1 = 1.0f / (1.0f - powf(d->beta1, (float)d->step));
-  const float c2 = 1.0f / (1.0f - powf(d->beta2, (float)d->step));
-  const uint32_t gr = G > 1 ? d->rows / G : (d->rows ? d->rows : 1u);
-  const bool by4 = d->rows % 4 == 0 && d->cols % 4 == 0 && gr % 4 == 0 && d->ld_bf16_t % 4 == 0 && (!d->out_bf16 || d->ld_bf16 % 4 == 0) &&
-                   aligned16(d->param) && aligned16(d->grad) && aligned16(d->m) && aligned16(d->v) &&
-                   ((uintptr_t)d->out_bf16 & 7u) == 0 && ((uintptr_t)d->out_bf16_t & 7u) == 0;
-  if (d->out_bf16_t && by4) {
-    k_adam_t4<<<dim3((d->cols + 31) / 32, (d->rows + 31) / 32), 256, 0, (cudaStream_t)stream>>>(
-        d->param, d->grad, d->m, d->v, d->rows, d->cols, d->lr, d->beta1, d->beta2, d->eps, c1, c2, (__nv_bfloat16*)d->out_bf16,
-        d->ld_bf16, (__nv_bfloat16*)d->out_bf16_t, d->ld_bf16_t, gr);
-  } else if (d->out_bf16_t) {
-    k_adam_t<<<dim3((d->cols + 31) / 32, (d->rows + 31) / 32), dim3(32, 8), 0, (cudaStream_t)stream>>>(
-        d->param, d->grad, d->m, d->v, d->rows, d->cols, d->lr, d->beta1, d->beta2, d->eps, c1, c2, (__nv_bfloat16*)d->out_bf16,
-        d->ld_bf16, (__nv_bfloat16*)d->out_bf16_t, d->ld_bf16_t, gr);
-  } else {
-    const uint32_t blocks = (uint32_t)hmin<size_t>((total + 255) / 256, (size_t)num_sms() * 8);
-    k_adam<<<blocks, 256, 0, (cudaStream_t)stream>>>(d->param, d->grad, d->m, d->v, d->rows, d->cols, d->lr, d->beta1, d->beta2, d->eps,
-                                                      c1, c2, (__nv_bfloat16*)d->out_bf16, d->ld_bf16, nullptr, 0, gr);
+extern "C" rt_status rt_adam_step_multi(const rt_adam_desc* descs, uint32_t count, rt_stream stream) {
+  if (!descs || count == 0 || count > kMulti) return RT_ERR_INVALID_ARGUMENT;
+  for (uint32_t i = 0; i < count; ++i) {
+    const rt_adam_desc* d = descs + i;
+    if (!d->param || !d->grad || !d->m || !d->v || d->step == 0 || d->rows % (d->groups ? d->groups : 1u)) return RT_ERR_INVALID_ARGUMENT;
   }
-  note_launch();
-  RT_CHECK_LAUNCH();
+  if (rt_device_check() != RT_OK) return RT_ERR_NO_DEVICE;
+  AdamBatch B = {};
+  uint64_t nblocks = 0;
+  for (uint32_t i = 0; i < count; ++i) {
+    const rt_adam_desc* d = descs + i;
+    const uint32_t G = d->groups ? d->groups : 1u;
+    const size_t total = (size_t)d->rows * d->cols;
+    if (total == 0) continue;
+    const float c1 = 1.0f / (1.0f - powf(d->beta1, (float)d->step));
+    const float c2 = 1.0f / (1.0f - powf(d->beta2, (float)d->step));
+    const uint32_t gr = G > 1 ? d->rows / G : (d->rows ? d->rows : 1u);
+    const bool by4 = d->rows % 4 == 0 && d->cols % 4 == 0 && gr % 4 == 0 && d->ld_bf16_t % 4 == 0 &&
+                     (!d->out_bf16 || d->ld_bf16 % 4 == 0) && aligned16(d->param) && aligned16(d->grad) && aligned16(d->m) &&
+                     aligned16(d->v) && ((uintptr_t)d->out_bf16 & 7u) == 0 && ((uintptr_t)d->out_bf16_t & 7u) == 0;
+    const uint64_t tiles = (uint64_t)((d->cols + 31) / 32) * ((d->rows + 31) / 32);
+    if ((d->out_bf16_t && by4) || (!d->out_bf16_t && !d->out_bf16)) {
+      AdamProblem& P = B.p[B.count++];
+      P.p = d->param; P.g = d->grad; P.m = d->m; P.v = d->v; P.rows = d->rows; P.cols = d->cols;
+      P.lr = d->lr; P.b1 = d->beta1; P.b2 = d->beta2; P.eps = d->eps; P.c1 = c1; P.c2 = c2;
+      P.out16 = (__nv_bfloat16*)d->out_bf16; P.out16t = (__nv_bfloat16*)d->out_bf16_t; P.ld16 = d->ld_bf16; P.ld16t = d->ld_bf16_t;
+      P.group_rows = gr; P.first = (uint32_t)nblocks;
+      P.nx = d->out_bf16_t ? (d->cols + 31) / 32 : 1u;
+      nblocks += d->out_bf16_t ? tiles : (total + 255) / 256;
+      if (nblocks > 0x7FFFFFFFull) return RT_ERR_INVALID_ARGUMENT;
+    } else if (d->out_bf16_t) {
+      k_adam_t<<<dim3((d->cols + 31) / 32, (d->rows + 31) / 32), dim3(32, 8), 0, (cudaStream_t)stream>>>(
+          d->param, d->grad, d->m, d->v, d->rows, d->cols, d->lr, d->beta1, d->beta2, d->eps, c1, c2, (__nv_bfloat16*)d->out_bf16,
+          d->ld_bf16, (__nv_bfloat16*)d->out_bf16_t, d->ld_bf16_t, gr);
+      note_launch();
+      RT_CHECK_LAUNCH();
+    } else {
+      const uint32_t blocks = (uint32_t)hmin<size_t>((total + 255) / 256, (size_t)num_sms() * 8);
+      k_adam<<<blocks, 256, 0, (cudaStream_t)stream>>>(d->param, d->grad, d->m, d->v, d->rows, d->cols, d->lr, d->beta1, d->beta2,
+                                                        d->eps, c1, c2, (__nv_bfloat16*)d->out_bf16, d->ld_bf16, nullptr, 0, gr);
+      note_launch();
+      RT_CHECK_LAUNCH();
+    }
+  }
+  if (B.count) {
+    k_adam_multi<<<(uint32_t)nblocks, 256, 0, (cudaStream_t)stream>>>(B);
+    note_launch();
+    RT_CHECK_LAUNCH();
+  }
   return RT_OK;
 }
+extern "C" rt_status rt_adam_step(const rt_adam_desc* d, rt_stream stream) { return rt_adam_step_multi(d, 1, stream); }

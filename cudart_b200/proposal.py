@@ -45,6 +45,17 @@ def gemm(a: torch.Tensor, b: torch.Tensor, bias=None, relu=False, mask=None, alp
     """C = alpha * a @ b.T (+ bias) (ReLU) (* (mask > 0)); a: bf16 (m, k), b: bf16 (n, k).
     groups > 1: a holds `groups` stacked (m, k) blocks and b stacked (n, k)
     blocks; block g of C is a_g @ b_g.T (out_t: stacked (n, m) transposes)."""
+    d = _gemm_desc(a, b, bias, relu, mask, alpha, out_f32, out_bf16, out_t, err, groups)
+    _check("rt_gemm_bf16", _abi.lib().rt_gemm_bf16(C.byref(d), _stream(stream)))
+
+
+def gemm_multi(products, stream=None):
+    """Independent products (keyword arguments of gemm() each) in one launch."""
+    ds = (_abi.GemmDesc * len(products))(*[_gemm_desc(**p) for p in products])
+    _check("rt_gemm_bf16_multi", _abi.lib().rt_gemm_bf16_multi(ds, len(products), _stream(stream)))
+
+
+def _gemm_desc(a, b, bias=None, relu=False, mask=None, alpha=1.0, out_f32=None, out_bf16=None, out_t=None, err=None, groups=1):
     m, k = a.shape[0] // groups, a.shape[1]
     n = b.shape[0] // groups
     if b.shape[1] != k:
@@ -67,7 +78,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, bias=None, relu=False, mask=None, alp
         d.ct_bf16, d.ldct = out_t.data_ptr(), out_t.stride(0)
     if err is not None:
         d.error_word = err.data_ptr()
-    _check("rt_gemm_bf16", _abi.lib().rt_gemm_bf16(C.byref(d), _stream(stream)))
+    return d
 
 
 def gemm_argmax(a: torch.Tensor, b: torch.Tensor, bias=None, out_index=None, out_value=None, out_margin=None, min_margin=0.0,
@@ -172,6 +183,14 @@ def colsum_grouped(x: torch.Tensor, groups: int, out: torch.Tensor, stream=None)
                                                                         _stream(stream)))
 
 
+def colsum_multi(sums, groups: int = 1, stream=None):
+    """Column sums (x, out) of each of `groups` stacked blocks, for every pair, in one launch."""
+    ds = (_abi.ColsumDesc * len(sums))()
+    for d, (x, out) in zip(ds, sums):
+        d.in_, d.out, d.groups, d.rows, d.cols, d.ld = x.data_ptr(), out.data_ptr(), groups, x.shape[0] // groups, x.shape[1], x.stride(0)
+    _check("rt_colsum_bf16_multi", _abi.lib().rt_colsum_bf16_multi(ds, len(sums), _stream(stream)))
+
+
 def gather_batch(orig, dir, labels, groups: int, group_stride: int, offset: int, batch: int, out: tuple, index=None, count=None,
                  hop: int = 1, stream=None):
     """Rows g * batch + b <- g * group_stride + q: q = k, or index[g][k] with an
@@ -259,27 +278,19 @@ class ProposalNet:
         gemm_xent(ws["H3"], W16[3], b[3], labels, 1.0 / B, ws["G"], ws["GT"], loss=ws["loss"], err=err, stream=stream)
         gW = self.grads[0::2]
         gb = self.grads[1::2]
-        # layer 4
-        gemm(ws["GT"], ws["H3T"], out_f32=gW[3], err=err, stream=stream)
-        colsum(ws["G"], gb[3], stream=stream)
         gemm(ws["G"], W16t[3], mask=ws["H3"], out_bf16=ws["D3"], out_t=ws["D3T"], err=err, stream=stream)
-        # layer 3
-        gemm(ws["D3T"], ws["H2T"], out_f32=gW[2], err=err, stream=stream)
-        colsum(ws["D3"], gb[2], stream=stream)
         gemm(ws["D3"], W16t[2], mask=ws["H2"], out_bf16=ws["D2"], out_t=ws["D2T"], err=err, stream=stream)
-        # layer 2
-        gemm(ws["D2T"], ws["H1T"], out_f32=gW[1], err=err, stream=stream)
-        colsum(ws["D2"], gb[1], stream=stream)
         gemm(ws["D2"], W16t[1], mask=ws["H1"], out_bf16=ws["D1"], out_t=ws["D1T"], err=err, stream=stream)
-        # layer 1
-        gemm(ws["D1T"], ws["XT"], out_f32=gW[0], err=err, stream=stream)
-        colsum(ws["D1"], gb[0], stream=stream)
+        # every layer's weight and bias gradients, which depend on the deltas alone: one launch each
+        gemm_multi([dict(a=ws[d], b=ws[x], out_f32=gW[i], err=err) for d, x, i in (("GT", "H3T", 3), ("D3T", "H2T", 2), ("D2T", "H1T", 1),
+                                                                                    ("D1T", "XT", 0))], stream=stream)
+        colsum_multi([(ws["G"], gb[3]), (ws["D3"], gb[2]), (ws["D2"], gb[1]), (ws["D1"], gb[0])], stream=stream)
         return ws["loss"].clone()  # the workspace is reused by the next step
 
     def adam(self, lr=1e-3, beta1=0.9, beta2=0.999, eps=1e-8, stream=None):
         self.step_count += 1
-        for i, (p, g, m, v) in enumerate(zip(self.params, self.grads, self.m, self.v)):
-            d = _abi.AdamDesc()
+        ds = (_abi.AdamDesc * len(self.params))()
+        for i, (d, p, g, m, v) in enumerate(zip(ds, self.params, self.grads, self.m, self.v)):
             d.param, d.grad, d.m, d.v = p.data_ptr(), g.data_ptr(), m.data_ptr(), v.data_ptr()
             if p.dim() == 2:
                 d.rows, d.cols = p.shape
@@ -289,7 +300,7 @@ class ProposalNet:
             else:
                 d.rows, d.cols = 1, p.shape[0]
             d.lr, d.beta1, d.beta2, d.eps, d.step = lr, beta1, beta2, eps, self.step_count
-            _check("rt_adam_step", _abi.lib().rt_adam_step(C.byref(d), _stream(stream)))
+        _check("rt_adam_step_multi", _abi.lib().rt_adam_step_multi(ds, len(self.params), _stream(stream)))
 
     def train_step(self, orig, dir, labels, box, lr=1e-3, stream=None):
         loss = self.forward_backward(orig, dir, labels, box, stream=stream)
@@ -414,23 +425,18 @@ class ProposalGroup:
         ws["loss"].zero_()
         gemm_xent(ws["H3"], W16[3], b[3], labels, 1.0 / B, ws["G"], ws["GT"], loss=ws["loss"], **kw)
         gW, gb = self.grads[0::2], self.grads[1::2]
-        gemm(ws["GT"], ws["H3T"], out_f32=gW[3], **kw)
-        colsum_grouped(ws["G"], G, gb[3], stream=stream)
         gemm(ws["G"], W16t[3], mask=ws["H3"], out_bf16=ws["D3"], out_t=ws["D3T"], **kw)
-        gemm(ws["D3T"], ws["H2T"], out_f32=gW[2], **kw)
-        colsum_grouped(ws["D3"], G, gb[2], stream=stream)
         gemm(ws["D3"], W16t[2], mask=ws["H2"], out_bf16=ws["D2"], out_t=ws["D2T"], **kw)
-        gemm(ws["D2T"], ws["H1T"], out_f32=gW[1], **kw)
-        colsum_grouped(ws["D2"], G, gb[1], stream=stream)
         gemm(ws["D2"], W16t[1], mask=ws["H1"], out_bf16=ws["D1"], out_t=ws["D1T"], **kw)
-        gemm(ws["D1T"], ws["XT"], out_f32=gW[0], **kw)
-        colsum_grouped(ws["D1"], G, gb[0], stream=stream)
+        gemm_multi([dict(a=ws[d], b=ws[x], out_f32=gW[i], err=err, groups=G)
+                    for d, x, i in (("GT", "H3T", 3), ("D3T", "H2T", 2), ("D2T", "H1T", 1), ("D1T", "XT", 0))], stream=stream)
+        colsum_multi([(ws["G"], gb[3]), (ws["D3"], gb[2]), (ws["D2"], gb[1]), (ws["D1"], gb[0])], groups=G, stream=stream)
         return ws["loss"]
 
     def adam(self, lr=1e-3, beta1=0.9, beta2=0.999, eps=1e-8, stream=None):
         self.step_count += 1
-        for i, (p, g, m, v) in enumerate(zip(self.params, self.grads, self.m, self.v)):
-            d = _abi.AdamDesc()
+        ds = (_abi.AdamDesc * len(self.params))()
+        for i, (d, p, g, m, v) in enumerate(zip(ds, self.params, self.grads, self.m, self.v)):
             d.param, d.grad, d.m, d.v = p.data_ptr(), g.data_ptr(), m.data_ptr(), v.data_ptr()
             if p.dim() == 2:
                 d.rows, d.cols = p.shape
@@ -441,7 +447,7 @@ class ProposalGroup:
             else:
                 d.rows, d.cols = 1, p.shape[0]
             d.lr, d.beta1, d.beta2, d.eps, d.step = lr, beta1, beta2, eps, self.step_count
-            _check("rt_adam_step", _abi.lib().rt_adam_step(C.byref(d), _stream(stream)))
+        _check("rt_adam_step_multi", _abi.lib().rt_adam_step_multi(ds, len(self.params), _stream(stream)))
 
     def train_step(self, orig, dir, labels, box, batch: int, lr=1e-3, stream=None):
         loss = self.forward_backward(orig, dir, labels, box, batch, stream=stream)

@@ -59,6 +59,9 @@ typedef struct rt_gemm_desc {
   uint32_t groups;      /* 0 or 1: one product */
 } rt_gemm_desc;
 rt_status rt_gemm_bf16(const rt_gemm_desc* d, rt_stream stream);
+/* The same for up to RT_MULTI_MAX independent products (no output of one is an input of another) in one launch. */
+#define RT_MULTI_MAX 8u
+rt_status rt_gemm_bf16_multi(const rt_gemm_desc* descs, uint32_t count, rt_stream stream);
 
 /* out_index[i] = argmax_j (A B^T + bias)[i][j] (lowest j among equal maxima),
  * out_value[i] = that maximum, out_margin[i] = maximum - second largest value;
@@ -186,6 +189,13 @@ rt_status rt_transpose_bf16_grouped(const void* in, uint32_t groups, uint32_t ro
                                     uint32_t ld_out, rt_stream stream);
 rt_status rt_colsum_bf16_grouped(const void* in, uint32_t groups, uint32_t rows, uint32_t cols, uint32_t ld, float* out,
                                  rt_stream stream);
+/* Up to RT_MULTI_MAX column sums (each as rt_colsum_bf16_grouped) in one launch. */
+typedef struct rt_colsum_desc {
+  const void* in;
+  float* out;
+  uint32_t groups, rows, cols, ld;
+} rt_colsum_desc;
+rt_status rt_colsum_bf16_multi(const rt_colsum_desc* descs, uint32_t count, rt_stream stream);
 
 /* Training batch of grouped networks. Row g batch + b of the outputs (origin,
  * direction, label) is input row g group_stride + q with
@@ -229,6 +239,8 @@ typedef struct rt_adam_desc {
   uint32_t groups; /* > 1: rows hold groups stacked matrices; out_bf16_t holds their transposes stacked (group g in rows g cols ..) */
 } rt_adam_desc;
 rt_status rt_adam_step(const rt_adam_desc* d, rt_stream stream);
+/* Up to RT_MULTI_MAX tensors in one launch. */
+rt_status rt_adam_step_multi(const rt_adam_desc* descs, uint32_t count, rt_stream stream);
 
 /* Slots of a built tree cut at `depth` (1..16): slot s follows the bits of s
  * (most significant first, 0 = left child) from the root for `depth` levels
