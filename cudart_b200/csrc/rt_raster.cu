@@ -4,9 +4,10 @@
 // The reference runs 2 x 2 blocks of 8 x 4 threads over the whole screen,
 // each block walking every face through a 192-face shared-memory cache. Here
 // the work is binned instead: one thread per face transforms its vertices,
-// drops faces off screen (and faces the barycentric test always rejects) and
-// computes the reference's zone rectangle; every face is appended to the list
-// of each zone of its rectangle (a counting sort: count, scan, fill); then one
+// drops faces off screen (and faces the barycentric test always rejects),
+// computes the reference's zone rectangle and counts the zones of it that the
+// face can touch (zone_touched); every face is appended to the lists of those
+// zones (a counting sort: count, scan, fill); then one
 // warp per 8 x 4 zone (lane = pixel, the reference's thread layout) walks its
 // zone's faces, keeping depth / id / (u, v) in registers and taking the
 // minimum (depth, face index). The per-pixel result is the reference's: the
@@ -48,24 +49,118 @@ struct Zones {
   float zsx, zsy;  // zone_scale = 0.5 * zone_count (:94-95)
 };
 
+// The pixel rectangle of a screen in device coordinates, as the zone pass computes them.
+struct Screen {
+  int zcx;
+  float w, h;
+};
+__device__ __forceinline__ float pixel_x(int x, const Screen& S) { return (float)x * 2.0f / S.w - 1.0f; }
+__device__ __forceinline__ float pixel_y(int y, const Screen& S) { return 1.0f - (float)y * 2.0f / S.h; }
+
+// Whether some pixel of a zone may pass the zone pass's test of a face: false only where u, v or u + v stay outside
+// [0, 1] at every pixel of the zone. The three are affine in the pixel (taken from the face's first vertex here), so
+// over a zone they stay within r of their value at its centre. `m` bounds what rounding changes, in the pixel's test and
+// in this one: a handful of roundings of 2^-24 on products below d^2, and pixel positions known to 2e-7, d being the
+// largest distance from the first vertex; with a factor of five to spare. NaN and infinities compare false: the pair is
+// kept. A rectangle starts on an even zone and a triangle fills half of it at the most: of the 2^20-face soup's 24M
+// (zone, face) pairs at 1080p under half are left, and the zone pass takes 0.75 ms instead of 1.50.
+struct ZoneTest {
+  float kx, ky, dx, dy;  // the zone's centre less the first vertex: kx + i dx, ky + j dy
+  float ux, uy, vx, vy;  // gradients
+  float ulo, uhi, vlo, shi;
+};
+__device__ __forceinline__ ZoneTest zone_test(const float4& a, const float4& b, const float4& c, const int4& r, const Screen& S) {
+  ZoneTest t;
+  const float sx = 2.0f / S.w, sy = 2.0f / S.h, hx = 3.5f * sx, hy = 1.5f * sy;
+  t.dx = 8.0f * sx;
+  t.dy = -4.0f * sy;
+  t.kx = (hx - 1.0f) - a.x;
+  t.ky = (1.0f - hy) - a.y;
+  const float bx = b.x - a.x, by = b.y - a.y, cx = c.x - a.x, cy = c.y - a.y, inv = a.w;
+  t.ux = cy * inv; t.uy = -cx * inv; t.vx = -by * inv; t.vy = bx * inv;
+  const float x0 = fabsf(t.kx + (float)r.x * t.dx) + hx, x1 = fabsf(t.kx + (float)r.z * t.dx) + hx;
+  const float y0 = fabsf(t.ky + (float)r.y * t.dy) + hy, y1 = fabsf(t.ky + (float)r.w * t.dy) + hy;
+  const float d = fmaxf(fmaxf(fmaxf(x0, x1), fmaxf(y0, y1)), fmaxf(fmaxf(fabsf(bx), fabsf(by)), fmaxf(fabsf(cx), fabsf(cy))));
+  const float m = (4e-6f * d + 2e-6f) * d * fabsf(inv) + 1e-5f;
+  const float ru = fabsf(t.ux) * hx + fabsf(t.uy) * hy, rv = fabsf(t.vx) * hx + fabsf(t.vy) * hy;
+  const float rs = fabsf(t.ux + t.vx) * hx + fabsf(t.uy + t.vy) * hy;
+  t.ulo = -m - ru; t.uhi = 1.0f + m + ru; t.vlo = -m - rv; t.shi = 1.0f + m + rs;
+  return t;
+}
+__device__ __forceinline__ bool zone_touched(const ZoneTest& t, int i, int j) {
+  const float x = __fmaf_rn((float)i, t.dx, t.kx), y = __fmaf_rn((float)j, t.dy, t.ky);
+  const float u = __fmaf_rn(x, t.ux, y * t.uy), v = __fmaf_rn(x, t.vx, y * t.vy);
+  return !(u < t.ulo || u > t.uhi || v < t.vlo || u + v > t.shi);
+}
+
+// Calls use(owner lane, zone) for every zone of the faces' rectangles that they may touch: a lane its own face's, or the
+// whole warp one lane's face after another where the rectangle has more than kOwnZones zones. Returns the number of
+// zones of the lane's own face.
+constexpr uint32_t kOwnZones = 64;
+template <class Use>
+__device__ __forceinline__ uint32_t for_touched_zones(bool have, const float4& a, const float4& b, const float4& c, const int4& r,
+                                                      const Screen& S, const Use& use) {
+  const uint32_t lane = lane_id();
+  const uint32_t n = have ? (uint32_t)(r.z - r.x + 1) * (uint32_t)(r.w - r.y + 1) : 0u;
+  uint32_t count = 0;
+  ZoneTest t = {};
+  if (n) t = zone_test(a, b, c, r, S);
+  if (n && n <= kOwnZones) {
+    for (int j = r.y; j <= r.w; ++j)
+      for (int i = r.x; i <= r.z; ++i)
+        if (zone_touched(t, i, j)) {
+          use(lane, (uint32_t)(j * S.zcx + i));
+          ++count;
+        }
+  }
+  for (uint32_t big = __ballot_sync(0xffffffffu, n > kOwnZones); big; big &= big - 1u) {
+    const int o = __ffs(big) - 1;
+    const uint32_t on = __shfl_sync(0xffffffffu, n, o);
+    const int x0 = __shfl_sync(0xffffffffu, r.x, o), y0 = __shfl_sync(0xffffffffu, r.y, o), x1 = __shfl_sync(0xffffffffu, r.z, o);
+    ZoneTest q;
+    const float* from = (const float*)&t;
+    float* to = (float*)&q;
+#pragma unroll
+    for (int k = 0; k < (int)(sizeof(ZoneTest) / 4); ++k) to[k] = __shfl_sync(0xffffffffu, from[k], o);
+    const uint32_t w = (uint32_t)(x1 - x0 + 1);
+    uint32_t mine = 0;
+    for (uint32_t k = lane; k < on; k += 32) {
+      const int i = x0 + (int)(k % w), j = y0 + (int)(k / w);
+      if (zone_touched(q, i, j)) {
+        use((uint32_t)o, (uint32_t)(j * S.zcx + i));
+        ++mine;
+      }
+    }
+    mine = __reduce_add_sync(0xffffffffu, mine);
+    if ((int)lane == o) count = mine;
+  }
+  return count;
+}
+
 // Per face: projected vertices, the zone rectangle (x0, y0, x1, y1) and the
-// number of zones it covers (0 when dropped). Faces naming a vertex past the
-// mesh are skipped with an error bit.
-__global__ __launch_bounds__(256) void k_raster_setup(const float4* __restrict__ verts, uint32_t vcount, const uint4* __restrict__ faces,
-                                                      uint32_t n, Mat4 M, Zones Z, float4* __restrict__ tri, int4* __restrict__ rect,
-                                                      uint32_t* __restrict__ cnt, uint32_t* __restrict__ block_sum, uint32_t* err) {
+// number of zones it may touch (0 when dropped); also every zone's count over
+// all faces (zcount), which serves if the pairs fit one chunk. Faces naming a
+// vertex past the mesh are skipped with an error bit.
+__global__ __launch_bounds__(kFacesPerBlock) void k_raster_setup(const float4* __restrict__ verts, uint32_t vcount,
+                                                                 const uint4* __restrict__ faces, uint32_t n, Mat4 M, Zones Z, Screen S,
+                                                                 float4* __restrict__ tri, int4* __restrict__ rect,
+                                                                 uint32_t* __restrict__ cnt, uint32_t* __restrict__ block_sum,
+                                                                 uint32_t* __restrict__ zcount, uint32_t* err) {
   __shared__ uint32_t s_sum;
   if (threadIdx.x == 0) s_sum = 0;
   __syncthreads();
   const uint32_t f = blockIdx.x * blockDim.x + threadIdx.x;
-  uint32_t c = 0;
+  bool have = false;
+  float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a, cc = a;
+  int4 r = make_int4(0, 0, -1, -1);
   if (f < n) {
     const uint4 fc = __ldg(faces + f);
     if (fc.x >= vcount || fc.y >= vcount || fc.z >= vcount) {
       atomicOr(err, (uint32_t)RT_DEVERR_NODE_CAPACITY);
     } else {
-      float4 a = project(M, __ldg(verts + fc.x));
-      const float4 b = project(M, __ldg(verts + fc.y)), cc = project(M, __ldg(verts + fc.z));
+      a = project(M, __ldg(verts + fc.x));
+      b = project(M, __ldg(verts + fc.y));
+      cc = project(M, __ldg(verts + fc.z));
       // the face's determinant (intersectTriPoint, :52-71, the same arithmetic as the
       // zone pass would do per pixel): a face the test always rejects gets no zone
       // pairs; otherwise its reciprocal rides in a.w
@@ -83,66 +178,73 @@ __global__ __launch_bounds__(256) void k_raster_setup(const float4* __restrict__
         const int y0 = max(__float2int_rz(Z.zsy * (1.0f - mxy)), 0) / 2 * 2;
         const int x1 = min(__float2int_rz(Z.zsx * (mxx + 1.0f)), Z.zcx - 1);
         const int y1 = min(__float2int_rz(Z.zsy * (1.0f - mny)), Z.zcy - 1);
-        rect[f] = make_int4(x0, y0, x1, y1);
-        if (x1 >= x0 && y1 >= y0) c = (uint32_t)(x1 - x0 + 1) * (uint32_t)(y1 - y0 + 1);
+        r = make_int4(x0, y0, x1, y1);
+        have = x1 >= x0 && y1 >= y0;
+        if (have) rect[f] = r;
       }
     }
-    cnt[f] = c;
   }
+  const uint32_t c = for_touched_zones(have, a, b, cc, r, S, [&](uint32_t, uint32_t z) { atomicAdd(zcount + z, 1u); });
+  if (f < n) cnt[f] = c;
   // per block of kFacesPerBlock faces (= blockDim) the pair count, for the host's chunking
   atomicAdd(&s_sum, c);
   __syncthreads();
   if (threadIdx.x == 0) block_sum[blockIdx.x] = s_sum;
 }
 
-// (zone, face) pairs of faces [f0, f1) at their offsets, in face order.
-// The (zone, face) pairs of faces [f0, f1) binned by zone without a sort:
-// k_raster_count counts each zone's faces, an exclusive scan turns the counts
-// into list starts, and k_raster_fill appends every face to its zones' lists.
-// The order inside a list is whatever the atomics give; the zone pass takes
-// the minimum (depth, face index), which is what visiting the faces in index
-// order with a strict depth test keeps.
-__global__ __launch_bounds__(256) void k_raster_count(const int4* __restrict__ rect, const uint32_t* __restrict__ cnt, uint32_t f0,
-                                                      uint32_t f1, int zcx, uint32_t* __restrict__ zcount) {
-  for (uint32_t f = f0 + blockIdx.x * blockDim.x + threadIdx.x; f < f1; f += gridDim.x * blockDim.x) {
-    if (!cnt[f]) continue;
-    const int4 r = rect[f];
-    for (int j = r.y; j <= r.w; ++j)
-      for (int i = r.x; i <= r.z; ++i) atomicAdd(zcount + (uint32_t)(j * zcx + i), 1u);
-  }
-}
-__global__ __launch_bounds__(256) void k_raster_fill(const int4* __restrict__ rect, const uint32_t* __restrict__ cnt, uint32_t f0,
-                                                     uint32_t f1, int zcx, const uint32_t* __restrict__ zoff, uint32_t* __restrict__ zfill,
-                                                     uint32_t* __restrict__ vals) {
-  for (uint32_t f = f0 + blockIdx.x * blockDim.x + threadIdx.x; f < f1; f += gridDim.x * blockDim.x) {
-    const uint32_t c = cnt[f];
-    if (!c) continue;
-    const int4 r = rect[f];
-    int i = r.x, j = r.y;
-    // four zones at a time: their atomics are in flight together before the stores
-    for (uint32_t q = 0; q < c; q += 4) {
-      uint32_t z[4], pos[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        z[k] = q + k < c ? (uint32_t)(j * zcx + i) : ~0u;
-        if (++i > r.z) { i = r.x; ++j; }
-      }
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-        if (z[k] != ~0u) pos[k] = zoff[z[k]] + atomicAdd(zfill + z[k], 1u);
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-        if (z[k] != ~0u) vals[pos[k]] = f;
+// The (zone, face) pairs of faces [f0, f1) binned by zone without a sort: the zones' counts (from k_raster_setup when
+// the chunk is the whole mesh, else from k_raster_bin<false>) are turned into list starts by an exclusive scan, and
+// k_raster_bin<true> appends every face to its zones' lists. The order inside a list is whatever the atomics give; the
+// zone pass takes the minimum (depth, face index), which is what visiting the faces in index order with a strict depth
+// test keeps.
+template <bool kFill>
+__global__ __launch_bounds__(256) void k_raster_bin(const float4* __restrict__ tri, const int4* __restrict__ rect,
+                                                    const uint32_t* __restrict__ cnt, uint32_t f0, uint32_t f1, Screen S,
+                                                    const uint32_t* __restrict__ zoff, uint32_t* __restrict__ zcount,
+                                                    uint32_t* __restrict__ vals) {
+  // whole warps step together: a face with many zones is shared by its warp
+  for (uint32_t base = f0 + blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < f1; base += gridDim.x * blockDim.x) {
+    const uint32_t f = base + lane_id();
+    const bool have = f < f1 && cnt[f] != 0u;
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a, c = a;
+    int4 r = make_int4(0, 0, -1, -1);
+    if (have) {
+      a = __ldg(tri + 3 * (size_t)f); b = __ldg(tri + 3 * (size_t)f + 1); c = __ldg(tri + 3 * (size_t)f + 2);
+      r = rect[f];
     }
+    // four zones at a time: their atomics are in flight together before the stores
+    uint32_t held = 0, hz[4], ho[4];
+    auto flush = [&]() {
+      uint32_t k[4];
+#pragma unroll
+      for (uint32_t q = 0; q < 4; ++q)
+        if (q < held) k[q] = zoff[hz[q]] + atomicAdd(zcount + hz[q], 1u);
+#pragma unroll
+      for (uint32_t q = 0; q < 4; ++q)
+        if (q < held) vals[k[q]] = base + ho[q];
+      held = 0;
+    };
+    for_touched_zones(have, a, b, c, r, S, [&](uint32_t owner, uint32_t z) {
+      if (!kFill) {
+        atomicAdd(zcount + z, 1u);
+      } else {
+#pragma unroll
+        for (uint32_t q = 0; q < 4; ++q)
+          if (q == held) { hz[q] = z; ho[q] = owner; }
+        if (++held == 4) flush();
+      }
+    });
+    if (kFill && held) flush();
   }
 }
 
 // One warp per zone; lane = pixel (x = lane % 8, y = lane / 8 inside the zone).
 __global__ __launch_bounds__(256) void k_raster_zones(const float4* __restrict__ tri, const uint32_t* __restrict__ vals,
                                                       const uint32_t* __restrict__ zs, const uint32_t* __restrict__ ze, uint32_t nz,
-                                                      int zcx, int width, int height, uint32_t id_mode, int32_t* __restrict__ fid,
+                                                      Screen S, int width, int height, uint32_t id_mode, int32_t* __restrict__ fid,
                                                       float2* __restrict__ uv, float* __restrict__ depth) {
   const uint32_t lane = threadIdx.x & 31u;
+  const int zcx = S.zcx;
   for (uint32_t z = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; z < nz; z += (gridDim.x * blockDim.x) >> 5) {
     const uint32_t s = zs[z], e = ze[z];
     if (s >= e) continue;
@@ -150,8 +252,7 @@ __global__ __launch_bounds__(256) void k_raster_zones(const float4* __restrict__
     const int y = (int)(z / (uint32_t)zcx) * 4 + (int)(lane >> 3);
     const bool inside = x >= 0 && x < width && y >= 0 && y < height;
     const size_t l = (size_t)y * (size_t)width + (size_t)x;
-    const float px = (float)x * 2.0f / (float)width - 1.0f;
-    const float py = 1.0f - (float)y * 2.0f / (float)height;
+    const float px = pixel_x(x, S), py = pixel_y(y, S);
     float best = inside ? depth[l] : 0.0f;
     int32_t bf = -1;
     float bu = 0.0f, bv = 0.0f;
@@ -256,9 +357,11 @@ extern "C" rt_status rt_rasterize(const rt_raster_desc* d, rt_stream stream) {
   memcpy(&M, d->matrix, 64);
   uint32_t* err = d->error_word ? d->error_word : L.err;
   if (!d->error_word && cudaMemsetAsync(L.err, 0, 4, st) != cudaSuccess) return RT_ERR_CUDA;
+  const Screen S{Z.zcx, (float)(int)d->width, (float)(int)d->height};
   const uint32_t nblocks = (n + kFacesPerBlock - 1) / kFacesPerBlock;
-  k_raster_setup<<<nblocks, kFacesPerBlock, 0, st>>>((const float4*)d->vertices, d->vertex_count, (const uint4*)d->faces, n, M, Z, L.tri,
-                                                      L.rect, L.cnt, L.block_sum, err);
+  if (cudaMemsetAsync(L.zoff, 0, ((size_t)nz + 1) * 4, st) != cudaSuccess) return RT_ERR_CUDA;
+  k_raster_setup<<<nblocks, kFacesPerBlock, 0, st>>>((const float4*)d->vertices, d->vertex_count, (const uint4*)d->faces, n, M, Z, S,
+                                                      L.tri, L.rect, L.cnt, L.block_sum, L.zoff, err);
   note_launch();
   RT_CHECK_LAUNCH();
   std::vector<uint32_t> bsum(nblocks);
@@ -277,17 +380,19 @@ extern "C" rt_status rt_rasterize(const rt_raster_desc* d, rt_stream stream) {
     b = e;
     if (P == 0) continue;
     const uint32_t fblocks = (uint32_t)hmin<uint64_t>((f1 - f0 + 255) / 256, (uint64_t)sms * 8);
-    if (cudaMemsetAsync(L.zoff, 0, ((size_t)nz + 1) * 4, st) != cudaSuccess || cudaMemsetAsync(L.zfill, 0, (size_t)nz * 4, st) != cudaSuccess)
-      return RT_ERR_CUDA;
-    k_raster_count<<<fblocks, 256, 0, st>>>(L.rect, L.cnt, f0, f1, Z.zcx, L.zoff);
-    note_launch();
-    RT_CHECK_LAUNCH();
+    if (cudaMemsetAsync(L.zfill, 0, (size_t)nz * 4, st) != cudaSuccess) return RT_ERR_CUDA;
+    if (f1 - f0 < n) {  // several chunks: this one's zone counts
+      if (cudaMemsetAsync(L.zoff, 0, ((size_t)nz + 1) * 4, st) != cudaSuccess) return RT_ERR_CUDA;
+      k_raster_bin<false><<<fblocks, 256, 0, st>>>(L.tri, L.rect, L.cnt, f0, f1, S, nullptr, L.zoff, nullptr);
+      note_launch();
+      RT_CHECK_LAUNCH();
+    }
     excl_scan(L.zoff, nz + 1, L.zsums, nullptr, st);
-    k_raster_fill<<<fblocks, 256, 0, st>>>(L.rect, L.cnt, f0, f1, Z.zcx, L.zoff, L.zfill, L.vals);
+    k_raster_bin<true><<<fblocks, 256, 0, st>>>(L.tri, L.rect, L.cnt, f0, f1, S, L.zoff, L.zfill, L.vals);
     note_launch();
     RT_CHECK_LAUNCH();
     k_raster_zones<<<(uint32_t)hmin<uint64_t>(((uint64_t)nz * 32 + 255) / 256, (uint64_t)sms * 16), 256, 0, st>>>(
-        L.tri, L.vals, L.zoff, L.zoff + 1, nz, Z.zcx, (int)d->width, (int)d->height, d->id_mode, d->face_id, (float2*)d->uv, d->depth);
+        L.tri, L.vals, L.zoff, L.zoff + 1, nz, S, (int)d->width, (int)d->height, d->id_mode, d->face_id, (float2*)d->uv, d->depth);
     note_launch();
     RT_CHECK_LAUNCH();
   }
