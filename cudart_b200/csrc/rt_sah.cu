@@ -29,7 +29,8 @@ constexpr float kTriCost = 0.125f;             // TRI_RAY_COST, :52
 constexpr float kBoxCost = 1.0f;               // BOX_RAY_COST, :53
 constexpr uint32_t kSahMinLeaf = 16;           // MIN_LEAF_SIZE, :55
 constexpr uint32_t kSahMaxLeaf = 224;          // MAX_LEAF_SIZE, :56
-constexpr uint32_t kBigNode = 4096;            // nodes above this many faces get a whole CTA
+constexpr uint32_t kBigNode = 512;             // nodes above this many faces get a whole CTA (a warp takes 32 faces at a time,
+                                               // three times over: at 4096 faces a level took 136 us, now 52 at the most)
 constexpr int kCta = 256;
 
 // Node of the build table (level order). info: bit 0 right child, bit 1 leaf,
@@ -185,7 +186,7 @@ __device__ Decision decide(const Bins& B, float3 pmn, float3 pmx, uint32_t count
 struct LevelArgs {
   SNode* table;
   uint32_t* table_count;  // [0] entries, [1] big entries of the next level, [2] no-split leaves
-  uint2* big_next;        // (table index, faces) of the next level's big nodes
+  uint4* big_next;        // (table index, faces, first) of the next level's big nodes
   const uint32_t* big_cur;  // table indices of this level's big nodes handled one CTA each
   uint32_t level_begin, level_end;
   const uint32_t* idx_in;
@@ -223,11 +224,50 @@ __device__ __forceinline__ void write_split(const LevelArgs& A, uint32_t e, cons
   R.id = kNone;
   A.table[c] = L;
   A.table[c + 1] = R;
-  if (L.count > kBigNode) A.big_next[atomicAdd(A.table_count + 1, 1u)] = make_uint2(c, L.count);
-  if (R.count > kBigNode) A.big_next[atomicAdd(A.table_count + 1, 1u)] = make_uint2(c + 1, R.count);
+  if (L.count > kBigNode) A.big_next[atomicAdd(A.table_count + 1, 1u)] = make_uint4(c, L.count, L.first, 0u);
+  if (R.count > kBigNode) A.big_next[atomicAdd(A.table_count + 1, 1u)] = make_uint4(c + 1, R.count, R.first, 0u);
   A.table[e].child = c;
   A.table[e].info = (nd.info & 1u) | ((uint32_t)sp.axis << 2);  // keep the right-child bit
   child_out = c;
+}
+
+// Stable partition of the positions [begin, end) by a whole CTA, kCta at a time in order: faces of bins <= m_min to lo,
+// lo + 1, ..., the others to ro, ro + 1, .... One barrier per step (two sets of counts), the next step's faces loaded
+// before it. (With a contiguous slice per thread, read twice at a stride, a level's partition took most of its time.)
+__device__ __forceinline__ void cta_partition(const LevelArgs& A, const Split& sp, int m_min, uint32_t begin, uint32_t end, uint32_t lo,
+                                              uint32_t ro) {
+  __shared__ uint32_t s_part[2][kCta / 32];
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+  uint32_t p = begin + threadIdx.x, set = 0;
+  Item it = {};
+  uint32_t id = 0;
+  if (p < end) { it = load_item(A.box_in + p); id = __ldg(A.idx_in + p); }
+  for (uint32_t base = begin; base < end; base += kCta, set ^= 1u) {
+    const bool valid = p < end;
+    const bool left = valid && bin_of(center_on(it, sp.axis), sp) <= m_min;
+    const uint32_t lb = __ballot_sync(0xffffffffu, left), vb = __ballot_sync(0xffffffffu, valid);
+    if (lane == 0) s_part[set][warp] = (uint32_t)__popc(lb) | (uint32_t)__popc(vb) << 16;
+    const Item cur = it;
+    const uint32_t cur_id = id;
+    p += kCta;
+    if (p < end) { it = load_item(A.box_in + p); id = __ldg(A.idx_in + p); }
+    __syncthreads();
+    uint32_t pre = 0, all = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < kCta / 32; ++w) {
+      const uint32_t x = s_part[set][w];
+      if (w < warp) pre += x;
+      all += x;
+    }
+    if (valid) {
+      const uint32_t dst = left ? lo + (pre & 0xffffu) + __popc(lb & below)
+                                : ro + (pre >> 16) - (pre & 0xffffu) + __popc(vb & ~lb & below);
+      A.idx_out[dst] = cur_id;
+      A.box_out[dst] = cur;
+    }
+    lo += all & 0xffffu;
+    ro += (all >> 16) - (all & 0xffffu);
+  }
 }
 
 // One warp per node of at most kBigNode faces (8 warps per CTA).
@@ -309,7 +349,6 @@ __global__ __launch_bounds__(kCta) void k_sah_small(LevelArgs A) {
 __global__ __launch_bounds__(kCta) void k_sah_big(LevelArgs A, uint32_t count_big) {
   __shared__ Bins B;
   __shared__ float s_red[6][kCta / 32];
-  __shared__ uint32_t s_scan[kCta / 32];
   __shared__ Decision s_d;
   __shared__ uint32_t s_child;
   if (blockIdx.x >= count_big) return;
@@ -317,6 +356,7 @@ __global__ __launch_bounds__(kCta) void k_sah_big(LevelArgs A, uint32_t count_bi
   const SNode nd = A.table[e];
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
   float3 cmn = make_float3(kHuge, kHuge, kHuge), cmx = make_float3(-kHuge, -kHuge, -kHuge);
+#pragma unroll 4
   for (uint32_t i = threadIdx.x; i < nd.count; i += kCta) {
     const Item it = load_item(A.box_in + nd.first + i);
     const float3 c = make_float3(0.5f * (it.mn.x + it.mx.x), 0.5f * (it.mn.y + it.mx.y), 0.5f * (it.mn.z + it.mx.z));
@@ -369,32 +409,18 @@ __global__ __launch_bounds__(kCta) void k_sah_big(LevelArgs A, uint32_t count_bi
     return;
   }
   if (s_child == kNone) return;
-  // stable partition: thread t owns the contiguous slice [t S, (t + 1) S) of
-  // the node; one block scan of the per-slice left counts places every slice
-  const uint32_t S = (nd.count + kCta - 1) / kCta;
-  const uint32_t a = min(nd.count, threadIdx.x * S), b = min(nd.count, a + S);
-  uint32_t my_left = 0;
-  for (uint32_t i = a; i < b; ++i) my_left += bin_of(center_on(load_item(A.box_in + nd.first + i), sp.axis), sp) <= d.m_min ? 1u : 0u;
-  uint32_t total_left;
-  const uint32_t lpre = block_excl_scan_nt<kCta>(my_left, s_scan, total_left);
-  uint32_t lo = nd.first + lpre, ro = nd.first + d.nl + (a - lpre);
-  for (uint32_t i = a; i < b; ++i) {
-    const Item it = load_item(A.box_in + nd.first + i);
-    const uint32_t id = A.idx_in[nd.first + i];
-    const uint32_t dst = bin_of(center_on(it, sp.axis), sp) <= d.m_min ? lo++ : ro++;
-    A.idx_out[dst] = id;
-    A.box_out[dst] = it;
-  }
+  cta_partition(A, sp, d.m_min, nd.first, nd.first + nd.count, nd.first, nd.first + d.nl);
 }
 
 // ---------------------------------------------------------------- huge nodes
 // Nodes of more than kHugeNode faces are cut into tiles of kTile faces that
 // separate CTAs process: bounds and bins meet in global order-key atomics, one
-// warp per node decides, a scan over the tiles' left counts places every
-// tile, and each tile scatters its faces stably (per-thread slices + a block
-// scan), so the result equals the single-owner kernels'.
-constexpr uint32_t kHugeNode = 32768;
-constexpr uint32_t kTile = 8192;
+// CTA per node decides and places every tile (the tiles keep their own bin
+// counts), and each tile scatters its faces stably, so the result equals the
+// single-owner kernels'.
+// 2^20 faces, a level of huge nodes: 50 us with 2048-face tiles (512 CTAs), 110 with 8192 (128).
+constexpr uint32_t kHugeNode = 8192;
+constexpr uint32_t kTile = 2048;
 
 struct HugeArgs {
   const uint32_t* node;   // [H] table index of huge node h
@@ -406,7 +432,8 @@ struct HugeArgs {
   Decision* dec;          // [H]
   Split* split;           // [H]
   uint32_t* child;        // [H] first child table index, kNone when a leaf
-  uint32_t* tleft;        // [tiles] left faces per tile, then its exclusive scan
+  uint32_t* tbins;        // [tiles][kBins] faces per tile and bin
+  uint32_t* tleft;        // [tiles] left faces in the node's earlier tiles
   uint32_t H, tiles;
 };
 
@@ -423,24 +450,25 @@ __global__ __launch_bounds__(kCta) void k_huge_bounds(LevelArgs A, HugeArgs G) {
   const SNode nd = A.table[G.node[h]];
   const uint32_t ts = G.tstart[t], te = min(nd.first + nd.count, ts + kTile);
   uint32_t k[6] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u};
+#pragma unroll 4
   for (uint32_t p = ts + threadIdx.x; p < te; p += kCta) {
     const Item it = load_item(A.box_in + p);
     const uint32_t cx = okey(0.5f * (it.mn.x + it.mx.x)), cy = okey(0.5f * (it.mn.y + it.mx.y)), cz = okey(0.5f * (it.mn.z + it.mx.z));
     k[0] = min(k[0], cx); k[1] = min(k[1], cy); k[2] = min(k[2], cz);
     k[3] = max(k[3], cx); k[4] = max(k[4], cy); k[5] = max(k[5], cz);
   }
+  // the CTA's bounds first: all tiles of a node meet in six words
+  __shared__ uint32_t s_k[6];
+  if (threadIdx.x < 6) s_k[threadIdx.x] = threadIdx.x < 3 ? 0xFFFFFFFFu : 0u;
+  __syncthreads();
 #pragma unroll
-  for (int o = 16; o; o >>= 1) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      k[c] = min(k[c], __shfl_xor_sync(0xffffffffu, k[c], o));
-      k[3 + c] = max(k[3 + c], __shfl_xor_sync(0xffffffffu, k[3 + c], o));
-    }
+  for (int c = 0; c < 3; ++c) {
+    const uint32_t mn = __reduce_min_sync(0xffffffffu, k[c]), mx = __reduce_max_sync(0xffffffffu, k[3 + c]);
+    if ((threadIdx.x & 31u) == 0) { atomicMin(s_k + c, mn); atomicMax(s_k + 3 + c, mx); }
   }
-  if ((threadIdx.x & 31u) == 0) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c) { atomicMin(G.keys + 8 * h + c, k[c]); atomicMax(G.keys + 8 * h + 3 + c, k[3 + c]); }
-  }
+  __syncthreads();
+  if (threadIdx.x < 3) atomicMin(G.keys + 8 * h + threadIdx.x, s_k[threadIdx.x]);
+  else if (threadIdx.x < 6) atomicMax(G.keys + 8 * h + threadIdx.x, s_k[threadIdx.x]);
 }
 
 __device__ __forceinline__ Split huge_split(const HugeArgs& G, uint32_t h) {
@@ -464,6 +492,7 @@ __global__ __launch_bounds__(kCta) void k_huge_bins(LevelArgs A, HugeArgs G) {
   __syncthreads();
   if (threadIdx.x < kBins) {
     const int m = (int)threadIdx.x;
+    G.tbins[kBins * (size_t)t + m] = B.cnt[m];
     if (B.cnt[m]) {
       Bins& g = G.bins[h];
       atomicAdd(&g.cnt[m], B.cnt[m]);
@@ -472,45 +501,52 @@ __global__ __launch_bounds__(kCta) void k_huge_bins(LevelArgs A, HugeArgs G) {
   }
 }
 
-// one warp per huge node
-__global__ __launch_bounds__(32) void k_huge_decide(LevelArgs A, HugeArgs G) {
+// One CTA per huge node: its first warp decides, then all place the node's tiles: a tile's left faces are those of its
+// bins up to the chosen boundary, so nothing is read again to count them.
+__global__ __launch_bounds__(kCta) void k_huge_decide(LevelArgs A, HugeArgs G) {
+  __shared__ uint32_t s_w[kCta / 32];
+  __shared__ int s_m;
   const uint32_t h = blockIdx.x;
-  const uint32_t e = G.node[h];
-  const SNode nd = A.table[e];
-  const Split sp = huge_split(G, h);
-  const Decision d = decide(G.bins[h], make_float3(nd.mn.x, nd.mn.y, nd.mn.z), make_float3(nd.mx.x, nd.mx.y, nd.mx.z), nd.count);
-  if (threadIdx.x == 0) {
-    uint32_t c = kNone;
-    if (d.m_min >= 0) {
-      write_split(A, e, nd, sp, d, c);
-    } else {
-      A.table[e].info = (nd.info & 1u) | 2u;
-      atomicAdd(A.table_count + 2, 1u);
+  if (threadIdx.x < 32) {
+    const uint32_t e = G.node[h];
+    const SNode nd = A.table[e];
+    const Split sp = huge_split(G, h);
+    const Decision d = decide(G.bins[h], make_float3(nd.mn.x, nd.mn.y, nd.mn.z), make_float3(nd.mx.x, nd.mx.y, nd.mx.z), nd.count);
+    if (threadIdx.x == 0) {
+      uint32_t c = kNone;
+      if (d.m_min >= 0) {
+        write_split(A, e, nd, sp, d, c);
+      } else {
+        A.table[e].info = (nd.info & 1u) | 2u;
+        atomicAdd(A.table_count + 2, 1u);
+      }
+      G.dec[h] = d;
+      G.split[h] = sp;
+      G.child[h] = c;
+      s_m = d.m_min;
     }
-    G.dec[h] = d;
-    G.split[h] = sp;
-    G.child[h] = c;
+  }
+  __syncthreads();
+  const int m_min = s_m;
+  if (m_min < 0) return;
+  const uint32_t t0 = G.tfirst[h], t1 = h + 1 < G.H ? G.tfirst[h + 1] : G.tiles;
+  uint32_t running = 0;
+  for (uint32_t base = t0; base < t1; base += kCta) {
+    const uint32_t t = base + threadIdx.x;
+    uint32_t left = 0;
+    if (t < t1) {
+      const uint32_t* b = G.tbins + kBins * (size_t)t;
+#pragma unroll
+      for (int m = 0; m < kBins; ++m) left += m <= m_min ? b[m] : 0u;
+    }
+    uint32_t total;
+    const uint32_t ex = block_excl_scan_nt<kCta>(left, s_w, total);
+    if (t < t1) G.tleft[t] = running + ex;
+    running += total;
   }
 }
 
-__global__ __launch_bounds__(kCta) void k_huge_count(LevelArgs A, HugeArgs G) {
-  __shared__ uint32_t s_w[kCta / 32];
-  const uint32_t t = blockIdx.x;
-  const uint32_t h = G.tnode[t];
-  const SNode nd = A.table[G.node[h]];
-  const uint32_t ts = G.tstart[t], te = min(nd.first + nd.count, ts + kTile);
-  const Decision& d = G.dec[h];
-  const Split sp = G.split[h];
-  uint32_t n = 0;
-  if (d.m_min >= 0)
-    for (uint32_t p = ts + threadIdx.x; p < te; p += kCta) n += bin_of(center_on(load_item(A.box_in + p), sp.axis), sp) <= d.m_min ? 1u : 0u;
-  uint32_t total;
-  block_excl_scan_nt<kCta>(n, s_w, total);
-  if (threadIdx.x == 0) G.tleft[t] = total;
-}
-
 __global__ __launch_bounds__(kCta) void k_huge_scatter(LevelArgs A, HugeArgs G) {
-  __shared__ uint32_t s_w[kCta / 32];
   const uint32_t t = blockIdx.x;
   const uint32_t h = G.tnode[t];
   const SNode nd = A.table[G.node[h]];
@@ -522,22 +558,8 @@ __global__ __launch_bounds__(kCta) void k_huge_scatter(LevelArgs A, HugeArgs G) 
   }
   if (G.child[h] == kNone) return;
   const Split sp = G.split[h];
-  const uint32_t left_before = G.tleft[t] - G.tleft[G.tfirst[h]];  // left faces in the node's earlier tiles
-  const uint32_t S = (te - ts + kCta - 1) / kCta;
-  const uint32_t a = min(te, ts + threadIdx.x * S), b = min(te, a + S);
-  uint32_t my_left = 0;
-  for (uint32_t p = a; p < b; ++p) my_left += bin_of(center_on(load_item(A.box_in + p), sp.axis), sp) <= d.m_min ? 1u : 0u;
-  uint32_t total;
-  const uint32_t lpre = block_excl_scan_nt<kCta>(my_left, s_w, total);
-  uint32_t lo = nd.first + left_before + lpre;
-  uint32_t ro = nd.first + d.nl + ((ts - nd.first) - left_before) + ((a - ts) - lpre);
-  for (uint32_t p = a; p < b; ++p) {
-    const Item it = load_item(A.box_in + p);
-    const uint32_t id = A.idx_in[p];
-    const uint32_t dst = bin_of(center_on(it, sp.axis), sp) <= d.m_min ? lo++ : ro++;
-    A.idx_out[dst] = id;
-    A.box_out[dst] = it;
-  }
+  const uint32_t left_before = G.tleft[t];
+  cta_partition(A, sp, d.m_min, ts, te, nd.first + left_before, nd.first + d.nl + ((ts - nd.first) - left_before));
 }
 
 // ---------------------------------------------------------------- setup
@@ -566,24 +588,25 @@ __global__ __launch_bounds__(256) void k_sah_init(const float4* __restrict__ box
 // keys[0..3] min xyzw (start 0xFFFFFFFF), keys[4..7] max xyzw (start 0).
 __global__ __launch_bounds__(256) void k_vertex_bounds(const float4* __restrict__ v, uint32_t n, uint32_t* keys) {
   uint32_t mn[4] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu}, mx[4] = {0u, 0u, 0u, 0u};
+#pragma unroll 4
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const float4 p = __ldg(v + i);
     const uint32_t k[4] = {okey(p.x), okey(p.y), okey(p.z), okey(p.w)};
 #pragma unroll
     for (int c = 0; c < 4; ++c) { mn[c] = min(mn[c], k[c]); mx[c] = max(mx[c], k[c]); }
   }
+  // the CTA's bounds first: thousands of warps in eight words took longer than the vertices (36 us for 3.1M)
+  __shared__ uint32_t s_k[8];
+  if (threadIdx.x < 8) s_k[threadIdx.x] = threadIdx.x < 4 ? 0xFFFFFFFFu : 0u;
+  __syncthreads();
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-      mn[c] = min(mn[c], __shfl_xor_sync(0xffffffffu, mn[c], o));
-      mx[c] = max(mx[c], __shfl_xor_sync(0xffffffffu, mx[c], o));
-    }
+    const uint32_t lo = __reduce_min_sync(0xffffffffu, mn[c]), hi = __reduce_max_sync(0xffffffffu, mx[c]);
+    if ((threadIdx.x & 31u) == 0) { atomicMin(s_k + c, lo); atomicMax(s_k + 4 + c, hi); }
   }
-  if ((threadIdx.x & 31u) == 0) {
-#pragma unroll
-    for (int c = 0; c < 4; ++c) { atomicMin(keys + c, mn[c]); atomicMax(keys + 4 + c, mx[c]); }
-  }
+  __syncthreads();
+  if (threadIdx.x < 4) atomicMin(keys + threadIdx.x, s_k[threadIdx.x]);
+  else if (threadIdx.x < 8) atomicMax(keys + threadIdx.x, s_k[threadIdx.x]);
 }
 __global__ void k_keys_to_box(const uint32_t* keys, float* hit) {
   const int c = threadIdx.x;
@@ -606,7 +629,7 @@ __global__ __launch_bounds__(256) void k_hyb_leaf_flags(const uint32_t* __restri
     flags_rev[m - 1 - k] = nodes[8 * (size_t)k] & 1u;
 }
 __global__ __launch_bounds__(256) void k_hyb_roots(const uint32_t* __restrict__ nodes, uint32_t m, const uint32_t* __restrict__ order_rev,
-                                                   SNode* table, uint2* big, uint32_t* counts) {
+                                                   SNode* table, uint4* big, uint32_t* counts) {
   for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < m; k += gridDim.x * blockDim.x) {
     const uint32_t* w = nodes + 8 * (size_t)k;
     if (!(w[0] & 1u)) continue;
@@ -616,7 +639,7 @@ __global__ __launch_bounds__(256) void k_hyb_roots(const uint32_t* __restrict__ 
     r.mx = make_float4(__uint_as_float(w[5]), __uint_as_float(w[6]), __uint_as_float(w[7]), 0.0f);
     r.first = w[1]; r.count = w[0] >> 1; r.parent = kNone; r.info = 0; r.child = kNone; r.sub = j; r.internal = 0; r.id = k;
     table[j] = r;
-    if (r.count > kBigNode) big[atomicAdd(counts + 1, 1u)] = make_uint2(j, r.count);
+    if (r.count > kBigNode) big[atomicAdd(counts + 1, 1u)] = make_uint4(j, r.count, r.first, 0u);
   }
 }
 
@@ -757,9 +780,9 @@ int sm_count() {
 }
 
 struct SahLayout {
-  uint32_t *idx_a, *idx_b, *big_list, *counts, *rank, *base, *marks, *sums, *scalars, *keys, *err, *leaf_lambda;
-  uint2 *big_a, *big_b;
-  uint32_t *h_node, *h_tnode, *h_tstart, *h_tfirst, *h_keys, *h_child, *h_tleft, *h_sums;
+  uint32_t *idx_a, *idx_b, *lists, *counts, *rank, *base, *marks, *sums, *scalars, *keys, *err, *leaf_lambda;
+  uint4 *big_a, *big_b;
+  uint32_t *h_keys, *h_child, *h_tbins, *h_tleft;
   Bins* h_bins;
   Decision* h_dec;
   Split* h_split;
@@ -780,22 +803,19 @@ size_t carve_sah(Carve& c, SahLayout& L, uint32_t n, uint32_t lbvh_depth, uint32
   L.idx_b = c.take<uint32_t>(n);
   L.box_a = c.take<Item>(n);
   L.box_b = c.take<Item>(n);
-  L.big_a = c.take<uint2>(n / kBigNode + 2);
-  L.big_b = c.take<uint2>(n / kBigNode + 2);
-  L.big_list = c.take<uint32_t>(n / kBigNode + 2);
+  L.big_a = c.take<uint4>(n / kBigNode + 2);
+  L.big_b = c.take<uint4>(n / kBigNode + 2);
   L.h_cap = n / kHugeNode + 2;
   L.t_cap = n / kTile + L.h_cap + 2;
-  L.h_node = c.take<uint32_t>(L.h_cap);
-  L.h_tfirst = c.take<uint32_t>(L.h_cap);
+  // a level's lists, uploaded together: the nodes of one CTA, the huge nodes and their first tiles, the tiles' nodes and starts
+  L.lists = c.take<uint32_t>((size_t)n / kBigNode + 2 + 2 * (size_t)L.h_cap + 2 * (size_t)L.t_cap);
   L.h_keys = c.take<uint32_t>(8 * (size_t)L.h_cap);
   L.h_child = c.take<uint32_t>(L.h_cap);
   L.h_bins = c.take<Bins>(L.h_cap);
   L.h_dec = c.take<Decision>(L.h_cap);
   L.h_split = c.take<Split>(L.h_cap);
-  L.h_tnode = c.take<uint32_t>(L.t_cap);
-  L.h_tstart = c.take<uint32_t>(L.t_cap);
-  L.h_tleft = c.take<uint32_t>(L.t_cap + 1);
-  L.h_sums = c.take<uint32_t>(L.t_cap / 1024 + 2);
+  L.h_tbins = c.take<uint32_t>((size_t)L.t_cap * kBins);
+  L.h_tleft = c.take<uint32_t>(L.t_cap);
   L.counts = c.take<uint32_t>(8);
   L.table = c.take<SNode>(L.table_cap);
   L.rank = c.take<uint32_t>(L.table_cap);
@@ -891,8 +911,8 @@ extern "C" rt_status rt_sah_build(const rt_sah_desc* d, rt_stream stream) {
     k_sah_init<<<grid, 256, 0, st>>>((const float4*)d->boxes, n, hit, L.idx_a, L.box_a, L.table, L.counts);
     note_launch();
     if (n > kBigNode) {
-      const uint2 root = make_uint2(0u, n);
-      if (cudaMemcpyAsync(L.big_a, &root, 8, cudaMemcpyHostToDevice, st) != cudaSuccess) return RT_ERR_CUDA;
+      const uint4 root = make_uint4(0u, n, 0u, 0u);
+      if (cudaMemcpyAsync(L.big_a, &root, 16, cudaMemcpyHostToDevice, st) != cudaSuccess) return RT_ERR_CUDA;
     }
   } else {
     rt_build_desc b = {};
@@ -931,81 +951,75 @@ extern "C" rt_status rt_sah_build(const rt_sah_desc* d, rt_stream stream) {
   uint32_t* idx_out = L.idx_b;
   Item* box_in = L.box_a;
   Item* box_out = L.box_b;
-  uint2* big_cur = L.big_a;
-  uint2* big_next = L.big_b;
-  std::vector<uint2> bigs;
+  uint4* big_cur = L.big_a;
+  uint4* big_next = L.big_b;
+  std::vector<uint4> bigs(nbig);
+  if (nbig && (cudaMemcpyAsync(bigs.data(), big_cur, (size_t)nbig * 16, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+               cudaStreamSynchronize(st) != cudaSuccess))
+    return RT_ERR_CUDA;
   std::vector<uint32_t> regular, h_node, h_tfirst, t_node, t_start;
   while (begin < end) {
     level_start.push_back(begin);
     // this level's big nodes: a CTA each, or tiles of several CTAs when huge
-    bigs.resize(nbig);
     regular.clear(); h_node.clear(); h_tfirst.clear(); t_node.clear(); t_start.clear();
-    if (nbig) {
-      if (cudaMemcpyAsync(bigs.data(), big_cur, (size_t)nbig * 8, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-          cudaStreamSynchronize(st) != cudaSuccess)
-        return RT_ERR_CUDA;
-    }
-    std::vector<SNode> firsts;  // first position of each huge node, read below
-    for (const uint2& bg : bigs) {
-      if (bg.y > kHugeNode && h_node.size() < L.h_cap) h_node.push_back(bg.x);
-      else regular.push_back(bg.x);
-    }
-    const uint32_t H = (uint32_t)h_node.size();
-    if (H) {
-      firsts.resize(H);
-      for (uint32_t h = 0; h < H; ++h)
-        if (cudaMemcpyAsync(&firsts[h], L.table + h_node[h], sizeof(SNode), cudaMemcpyDeviceToHost, st) != cudaSuccess) return RT_ERR_CUDA;
-      if (cudaStreamSynchronize(st) != cudaSuccess) return RT_ERR_CUDA;
-      for (uint32_t h = 0; h < H; ++h) {
+    for (const uint4& bg : bigs) {
+      if (bg.y > kHugeNode && h_node.size() < L.h_cap) {
         h_tfirst.push_back((uint32_t)t_node.size());
-        for (uint32_t o = 0; o < firsts[h].count; o += kTile) {
-          t_node.push_back(h);
-          t_start.push_back(firsts[h].first + o);
+        for (uint32_t o = 0; o < bg.y; o += kTile) {
+          t_node.push_back((uint32_t)h_node.size());
+          t_start.push_back(bg.z + o);
         }
+        h_node.push_back(bg.x);
+      } else {
+        regular.push_back(bg.x);
       }
     }
-    const uint32_t tiles = (uint32_t)t_node.size();
+    const uint32_t H = (uint32_t)h_node.size(), R = (uint32_t)regular.size(), tiles = (uint32_t)t_node.size();
     if (tiles > L.t_cap) return RT_ERR_CAPACITY;
-    const uint32_t zero = 0;
-    if (cudaMemcpyAsync(L.counts + 1, &zero, 4, cudaMemcpyHostToDevice, st) != cudaSuccess) return RT_ERR_CUDA;
-    if (!regular.empty() &&
-        cudaMemcpyAsync(L.big_list, regular.data(), regular.size() * 4, cudaMemcpyHostToDevice, st) != cudaSuccess)
-      return RT_ERR_CUDA;
+    if (cudaMemsetAsync(L.counts + 1, 0, 4, st) != cudaSuccess) return RT_ERR_CUDA;
+    if (!bigs.empty()) {  // one upload: [regular][h_node][h_tfirst][t_node][t_start]
+      regular.insert(regular.end(), h_node.begin(), h_node.end());
+      regular.insert(regular.end(), h_tfirst.begin(), h_tfirst.end());
+      regular.insert(regular.end(), t_node.begin(), t_node.end());
+      regular.insert(regular.end(), t_start.begin(), t_start.end());
+      if (cudaMemcpyAsync(L.lists, regular.data(), regular.size() * 4, cudaMemcpyHostToDevice, st) != cudaSuccess) return RT_ERR_CUDA;
+    }
     LevelArgs A;
-    A.table = L.table; A.table_count = L.counts; A.big_next = big_next; A.big_cur = L.big_list; A.level_begin = begin; A.level_end = end;
+    A.table = L.table; A.table_count = L.counts; A.big_next = big_next; A.big_cur = L.lists; A.level_begin = begin; A.level_end = end;
     A.idx_in = idx_in; A.box_in = box_in; A.idx_out = idx_out; A.box_out = box_out; A.final_idx = d->indices; A.err = L.err;
     A.table_cap = L.table_cap;
     if (H) {
-      if (cudaMemcpyAsync(L.h_node, h_node.data(), H * 4, cudaMemcpyHostToDevice, st) != cudaSuccess ||
-          cudaMemcpyAsync(L.h_tfirst, h_tfirst.data(), H * 4, cudaMemcpyHostToDevice, st) != cudaSuccess ||
-          cudaMemcpyAsync(L.h_tnode, t_node.data(), tiles * 4, cudaMemcpyHostToDevice, st) != cudaSuccess ||
-          cudaMemcpyAsync(L.h_tstart, t_start.data(), tiles * 4, cudaMemcpyHostToDevice, st) != cudaSuccess)
-        return RT_ERR_CUDA;
       HugeArgs G;
-      G.node = L.h_node; G.tnode = L.h_tnode; G.tstart = L.h_tstart; G.tfirst = L.h_tfirst; G.keys = L.h_keys; G.bins = L.h_bins;
-      G.dec = L.h_dec; G.split = L.h_split; G.child = L.h_child; G.tleft = L.h_tleft; G.H = H; G.tiles = tiles;
+      G.node = L.lists + R; G.tfirst = G.node + H; G.tnode = G.tfirst + H; G.tstart = G.tnode + tiles;
+      G.keys = L.h_keys; G.bins = L.h_bins;
+      G.dec = L.h_dec; G.split = L.h_split; G.child = L.h_child; G.tbins = L.h_tbins; G.tleft = L.h_tleft; G.H = H; G.tiles = tiles;
       k_huge_reset<<<H, 64, 0, st>>>(G);
       k_huge_bounds<<<tiles, kCta, 0, st>>>(A, G);
       k_huge_bins<<<tiles, kCta, 0, st>>>(A, G);
-      k_huge_decide<<<H, 32, 0, st>>>(A, G);
-      k_huge_count<<<tiles, kCta, 0, st>>>(A, G);
-      note_launch(5);
-      excl_scan(L.h_tleft, tiles, L.h_sums, nullptr, st);
+      k_huge_decide<<<H, kCta, 0, st>>>(A, G);
       k_huge_scatter<<<tiles, kCta, 0, st>>>(A, G);
+      note_launch(5);
+    }
+    if (R) {
+      k_sah_big<<<R, kCta, 0, st>>>(A, R);
       note_launch();
     }
-    if (!regular.empty()) {
-      k_sah_big<<<(uint32_t)regular.size(), kCta, 0, st>>>(A, (uint32_t)regular.size());
+    if (end - begin > (uint32_t)bigs.size()) {  // nodes of at most kBigNode faces
+      k_sah_small<<<(end - begin + 7) / 8, kCta, 0, st>>>(A);
       note_launch();
     }
-    k_sah_small<<<(end - begin + 7) / 8, kCta, 0, st>>>(A);
-    note_launch();
     RT_CHECK_LAUNCH();
-    if (cudaMemcpyAsync(host_counts, L.counts, 12, cudaMemcpyDeviceToHost, st) != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess)
+    // one wait per level: the counts, and the next level's big nodes (at most two per big node of this one)
+    const uint32_t most = (uint32_t)hmin<size_t>(2 * bigs.size(), n / kBigNode + 1);
+    bigs.resize(most);
+    if (cudaMemcpyAsync(host_counts, L.counts, 12, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        (most && cudaMemcpyAsync(bigs.data(), big_next, (size_t)most * 16, cudaMemcpyDeviceToHost, st) != cudaSuccess) ||
+        cudaStreamSynchronize(st) != cudaSuccess)
       return RT_ERR_CUDA;
     begin = end;
     end = host_counts[0] < L.table_cap ? host_counts[0] : L.table_cap;
-    nbig = host_counts[1];
+    if (host_counts[1] > most) return RT_ERR_CAPACITY;  // cannot happen
+    bigs.resize(host_counts[1]);
     std::swap(idx_in, idx_out);
     std::swap(box_in, box_out);
     std::swap(big_cur, big_next);
