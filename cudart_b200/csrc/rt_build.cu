@@ -16,7 +16,7 @@
 //   k_topo_morton    one CTA: the Morton levels of the tree, level by level,
 //                    with the reference's split-pointer semantics (see below);
 //                    leaf counts, pre-order ranks and node ids
-//   k_leaves         one warp per final leaf: expands median subtrees, writes
+//   k_leaves         32 final leaves at a time per warp: expands median subtrees, writes
 //                    node records, reorders faces, pre-gathers triangles
 //                    {v0, e1, e2}, reduces the leaf box and records the
 //                    parents of median nodes
@@ -353,7 +353,7 @@ __device__ __forceinline__ void topo_morton(const TopoArgs& A) {
 __global__ __launch_bounds__(kTopoThreads) void k_topo_morton(TopoArgs A) { topo_morton(A); }
 
 // ----------------------------------------------------------------------------
-// leaves: one warp per final leaf
+// leaves: a warp takes 32 consecutive leaves at a time
 // ----------------------------------------------------------------------------
 struct LeafArgs {
   const float4* verts;
@@ -382,122 +382,204 @@ struct LeafArgs {
 };
 
 constexpr int kMaxMedianDepth = 40;
-// One final leaf (leaf-order index g of its mesh), processed by one warp.
-// `hint` (lane 0's) is the Morton leaf of the warp's previous leaf of the same
-// mesh, or ~0u: a warp walking consecutive leaves then finds each one's Morton
-// leaf in a step or two instead of a binary search.
-__device__ __forceinline__ void leaf_body(const LeafArgs& A, const uint32_t g, uint32_t& hint) {
-  const uint32_t lane = lane_id();
-  const uint32_t mleaf_count = A.hdr[1];
-  {
-    uint32_t leaf_id = 0, first = 0, cnt = 0;
-    int plen = 0;  // median levels walked
-    if (lane == 0) {
-      // Morton leaf owning global leaf slot g: last k with ml_lambda[k] <= g
-      // (ml_lambda is non-decreasing)
-      uint32_t lo = 0;
-      if (hint < mleaf_count && A.ml_lambda[hint] <= g) {
-        lo = hint;
-        while (lo + 1 < mleaf_count && A.ml_lambda[lo + 1] <= g) ++lo;
-      } else {
-        uint32_t hi = mleaf_count - 1;
-        while (lo < hi) {
-          uint32_t mid = (lo + hi + 1) >> 1;
-          if (A.ml_lambda[mid] <= g) lo = mid; else hi = mid - 1;
-        }
-      }
-      hint = lo;
-      const uint4 rec = A.ml_rec[lo];
-      leaf_id = rec.x; first = rec.y; cnt = rec.z;  // first: absolute position
-      if (rec.w & 0x80000000u) {
-        uint32_t q = g - A.ml_lambda[lo];
-        uint32_t rank = A.ml_rank[lo];
-        uint32_t depth = rec.w & 0xFFFFu;
-        uint32_t nid = rec.x, size = rec.z, a = rec.y;
-        while (size >= A.max_leaf && plen < kMaxMedianDepth) {
-          const uint32_t left = size >> 1, right = size - left;
-          const uint32_t ll = median_leaves(left, A.max_leaf);
-          // the subtree's first leaf writes the internal record and its children's parent ids
-          if (q == 0 && nid < A.max_nodes) {
-            *(uint2*)(A.nodes + 8 * (size_t)nid) = make_uint2((depth % 3u) << 1, 2 * rank + 1);
-            if (2 * rank + 2 < A.parent_cap) {
-              A.parent_id[2 * rank + 1] = nid;
-              A.parent_id[2 * rank + 2] = nid;
-            }
-          }
-          ++plen;
-          if (q < ll) { nid = 2 * rank + 1; rank = rank + 1; size = left; }
-          else { q -= ll; nid = 2 * rank + 2; rank = rank + ll; a += left; size = right; }
-          ++depth;
-        }
-        leaf_id = nid; first = a; cnt = size;
-      }
-    }
-    leaf_id = __shfl_sync(0xffffffffu, leaf_id, 0);
-    first = __shfl_sync(0xffffffffu, first, 0);
-    cnt = __shfl_sync(0xffffffffu, cnt, 0);
 
+// What a lane knows of one final leaf: where its faces are, its node and its place in the blob.
+struct LeafMeta {
+  uint32_t first;   // absolute position of its first face
+  uint32_t cnt;
+  uint32_t node;    // its node, counted from the first mesh's root (~0: beyond the node array)
+  uint32_t group;   // its first group box, counted from the first mesh's
+  uint32_t vert_base, pos_base;  // its mesh's first vertex and first position
+};
+
+// Last k < n with v[k] <= x (v ascending, v[0] <= x), the same x for the whole warp: 32 places at a time.
+__device__ __forceinline__ uint32_t warp_last_le(const uint32_t* __restrict__ v, uint32_t n, uint32_t x) {
+  const uint32_t lane = lane_id();
+  uint32_t lo = 0, len = n;
+  while (len > 1) {
+    const uint32_t step = (len + 31) / 32, at = lane * step;
+    const uint32_t c = (uint32_t)__popc(__ballot_sync(0xffffffffu, at < len && v[lo + at] <= x)) - 1u;
+    lo += c * step;
+    len = min(step, len - c * step);
+  }
+  return lo;
+}
+// The Morton leaves of leaves g .. g + 31 of one mesh (lane l: leaf g + l), the first one's found by the whole warp.
+__device__ __forceinline__ uint32_t warp_morton_leaf(const LeafArgs& A, uint32_t g) {
+  const uint32_t lane = lane_id(), count = A.hdr[1];
+  const uint32_t first = warp_last_le(A.ml_lambda, count, g);
+  const uint32_t v = first + lane < count ? A.ml_lambda[first + lane] : ~0u;
+  uint32_t lo = 0;
+#pragma unroll
+  for (uint32_t step = 16; step; step >>= 1)
+    if (__shfl_sync(0xffffffffu, v, lo + step) <= g + lane) lo += step;
+  return first + lo;
+}
+
+// Leaf g (in its mesh's leaf order, in Morton leaf lo) of the mesh that A describes. Writes what does not need the faces: the nodes of a
+// median subtree whose first leaf this is, the blob's leaf entry.
+__device__ __forceinline__ LeafMeta leaf_meta(const LeafArgs& A, const uint32_t g, const uint32_t lo, uint32_t node_first,
+                                              uint32_t group_first) {
+  const uint4 rec = A.ml_rec[lo];
+  uint32_t nid = rec.x, first = rec.y, size = rec.z;  // first: absolute position
+  if (rec.w & 0x80000000u) {
+    uint32_t q = g - A.ml_lambda[lo], rank = A.ml_rank[lo], depth = rec.w & 0xFFFFu;
+    int plen = 0;  // median levels walked
+    while (size >= A.max_leaf && plen < kMaxMedianDepth) {
+      const uint32_t left = size >> 1, right = size - left;
+      const uint32_t ll = median_leaves(left, A.max_leaf);
+      // the subtree's first leaf writes the internal record and its children's parent ids
+      if (q == 0 && nid < A.max_nodes) {
+        *(uint2*)(A.nodes + 8 * (size_t)nid) = make_uint2((depth % 3u) << 1, 2 * rank + 1);
+        if (2 * rank + 2 < A.parent_cap) {
+          A.parent_id[2 * rank + 1] = nid;
+          A.parent_id[2 * rank + 2] = nid;
+        }
+      }
+      ++plen;
+      if (q < ll) { nid = 2 * rank + 1; rank = rank + 1; size = left; }
+      else { q -= ll; nid = 2 * rank + 2; rank = rank + ll; first += left; size = right; }
+      ++depth;
+    }
+  }
+  LeafMeta L;
+  L.first = first; L.cnt = size;
+  L.vert_base = A.vert_base; L.pos_base = A.pos_base;
+  const uint32_t lfirst = first - A.pos_base;   // position inside the mesh
+  const uint32_t gbase = (lfirst >> 3) + g;     // leaf g's groups: disjoint across leaves, no scan needed
+  L.group = group_first + gbase;
+  const bool fits = nid < A.max_nodes;
+  L.node = fits ? node_first + nid : kNone;
+  if (A.acc_leaves && fits) {
+    A.acc_leaves[g] = make_uint4(lfirst, size, gbase, nid);
+    A.leaf_lambda[nid] = g;
+  }
+  if (!fits) atomicOr(A.err, (uint32_t)RT_DEVERR_NODE_CAPACITY);
+  return L;
+}
+
+// The faces of up to 32 consecutive leaves, one leaf's metadata per lane (cnt 0: none), by one warp: per face the
+// reordered face, the triangle {v0, e1, e2} and (batched) the mesh-local index, per 8 faces of a leaf a padded group
+// box, per leaf its box and node words. The leaves' faces are taken 32 at a time as one sequence, cut back to whole
+// groups, so that short leaves share a step; the boxes are reduced inside the lanes of each group and then over a
+// leaf's groups, which are eight lanes apart, and a leaf that goes on past a step carries its box along. Boxes are
+// combined in position order with the selects of a sequential scan. The next step's indices and faces are loaded
+// while this one's vertices are on their way. (A warp per leaf with lane 0 finding it, one leaf and one dependent
+// load after another, took 1.29 ms for 2^24 faces of a soup and 1.31 ms for 9.9M in 1024 meshes; this takes 0.98 ms, bound by DRAM (5.8 TB/s
+// of scattered reads, 276 bytes per face), and 0.63.)
+// `out`: arrays of the whole build (nodes and group boxes of the first mesh).
+__device__ __forceinline__ void leaf_faces(const LeafArgs& out, const LeafMeta& L) {
+  const uint32_t lane = lane_id();
+  uint32_t incl = L.cnt;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= (uint32_t)o) incl += y;
+  }
+  const uint32_t off = incl - L.cnt, total = __shfl_sync(0xffffffffu, incl, 31);
+  struct Step {
+    uint32_t owner, rel, cnt, n;  // the lane's leaf, its place in it, the leaf's faces; faces of the step (lanes 0 .. n - 1)
+    uint32_t pos, idx;
+    uint4 f;
+  };
+  auto begin_step = [&](uint32_t w) {
+    Step s;
+    const uint32_t item = w + lane;
+    uint32_t lo = 0;
+#pragma unroll
+    for (uint32_t step = 16; step; step >>= 1) {  // last leaf that starts at or before the item
+      const uint32_t o = __shfl_sync(0xffffffffu, off, lo + step);
+      if (o <= item) lo += step;
+    }
+    // (empty leaves at the end start at `total`: items before it never reach them)
+    s.owner = lo;
+    s.rel = item - __shfl_sync(0xffffffffu, off, lo);
+    s.cnt = __shfl_sync(0xffffffffu, L.cnt, lo);
+    const bool whole = item < total && item - (s.rel & 7u) + min(8u, s.cnt - (s.rel & ~7u)) <= w + 32;
+    s.n = (uint32_t)__popc(__ballot_sync(0xffffffffu, whole));
+    s.pos = __shfl_sync(0xffffffffu, L.first, lo) + s.rel;
+    s.idx = 0;
+    s.f = make_uint4(0, 0, 0, 0);
+    if (lane < s.n) {
+      s.idx = __ldg(out.indices + s.pos);
+      s.f = ldg4(out.faces_in + s.idx);
+    }
+    return s;
+  };
+  float3 cmn = make_float3(kHuge, kHuge, kHuge), cmx = make_float3(-kHuge, -kHuge, -kHuge);  // box of a leaf that goes on
+  uint32_t w = 0;
+  if (total == 0) return;
+  Step s = begin_step(0);
+  while (w < total) {
+    const bool act = lane < s.n;
+    const uint32_t vb = __shfl_sync(0xffffffffu, L.vert_base, s.owner);
+    float4 v0 = make_float4(0.f, 0.f, 0.f, 0.f), v1 = v0, v2 = v0;
+    if (act) {
+      v0 = ldg4(out.verts + vb + s.f.x);
+      v1 = ldg4(out.verts + vb + s.f.y);
+      v2 = ldg4(out.verts + vb + s.f.z);
+    }
+    const Step c = s;
+    const uint32_t wn = w + c.n;
+    if (wn < total) s = begin_step(wn);
+    const uint32_t pb = __shfl_sync(0xffffffffu, L.pos_base, c.owner), group = __shfl_sync(0xffffffffu, L.group, c.owner);
+    const uint32_t node = __shfl_sync(0xffffffffu, L.node, c.owner), first = __shfl_sync(0xffffffffu, L.first, c.owner);
     float3 mn = make_float3(kHuge, kHuge, kHuge), mx = make_float3(-kHuge, -kHuge, -kHuge);
-    const uint32_t lfirst = first - A.pos_base;  // position inside the mesh
-    const uint32_t gbase = (lfirst >> 3) + g;      // leaf g's groups: disjoint across leaves, no scan needed
-    if (A.acc_leaves && lane == 0) {
-      A.acc_leaves[g] = make_uint4(lfirst, cnt, gbase, leaf_id);
-      A.leaf_lambda[leaf_id] = g;
-    }
-    for (uint32_t base = 0; base < cnt; base += 32) {
-      const uint32_t i = first + base + lane;
-      float3 tmn = make_float3(kHuge, kHuge, kHuge), tmx = make_float3(-kHuge, -kHuge, -kHuge);
-      if (base + lane < cnt) {
-        const uint32_t orig = A.indices[i];
-        const uint4 f = ldg4(A.faces_in + orig);
-        const float4 v0 = ldg4(A.verts + A.vert_base + f.x), v1 = ldg4(A.verts + A.vert_base + f.y), v2 = ldg4(A.verts + A.vert_base + f.z);
-        if (A.local_indices) A.local_indices[i] = orig - A.pos_base;
-        if (A.faces_out) A.faces_out[i] = f;
-        if (A.tris) {
-          float4 e1 = make_float4(v1.x - v0.x, v1.y - v0.y, v1.z - v0.z, 0.0f);
-          float4 e2 = make_float4(v2.x - v0.x, v2.y - v0.y, v2.z - v0.z, 0.0f);
-          A.tris[3 * (size_t)i + 0] = make_float4(v0.x, v0.y, v0.z, 0.0f);
-          A.tris[3 * (size_t)i + 1] = e1;
-          A.tris[3 * (size_t)i + 2] = e2;
-        }
-        tmn = make_float3(fmin_sel(fmin_sel(v0.x, v1.x), v2.x), fmin_sel(fmin_sel(v0.y, v1.y), v2.y), fmin_sel(fmin_sel(v0.z, v1.z), v2.z));
-        tmx = make_float3(fmax_sel(fmax_sel(v0.x, v1.x), v2.x), fmax_sel(fmax_sel(v0.y, v1.y), v2.y), fmax_sel(fmax_sel(v0.z, v1.z), v2.z));
+    if (act) {
+      if (out.local_indices) out.local_indices[c.pos] = c.idx - pb;
+      if (out.faces_out) out.faces_out[c.pos] = c.f;
+      if (out.tris) {
+        out.tris[3 * (size_t)c.pos + 0] = make_float4(v0.x, v0.y, v0.z, 0.0f);
+        out.tris[3 * (size_t)c.pos + 1] = make_float4(v1.x - v0.x, v1.y - v0.y, v1.z - v0.z, 0.0f);
+        out.tris[3 * (size_t)c.pos + 2] = make_float4(v2.x - v0.x, v2.y - v0.y, v2.z - v0.z, 0.0f);
       }
-      mn = make_float3(fmin_sel(mn.x, tmn.x), fmin_sel(mn.y, tmn.y), fmin_sel(mn.z, tmn.z));
-      mx = make_float3(fmax_sel(mx.x, tmx.x), fmax_sel(mx.y, tmx.y), fmax_sel(mx.z, tmx.z));
-      if (A.acc_groups) {
-#pragma unroll
-        for (int o = 1; o < 8; o <<= 1) {
-          tmn.x = fmin_sel(tmn.x, __shfl_xor_sync(0xffffffffu, tmn.x, o));
-          tmn.y = fmin_sel(tmn.y, __shfl_xor_sync(0xffffffffu, tmn.y, o));
-          tmn.z = fmin_sel(tmn.z, __shfl_xor_sync(0xffffffffu, tmn.z, o));
-          tmx.x = fmax_sel(tmx.x, __shfl_xor_sync(0xffffffffu, tmx.x, o));
-          tmx.y = fmax_sel(tmx.y, __shfl_xor_sync(0xffffffffu, tmx.y, o));
-          tmx.z = fmax_sel(tmx.z, __shfl_xor_sync(0xffffffffu, tmx.z, o));
-        }
-        if ((lane & 7u) == 0 && base + lane < cnt) {
-          pad_box(tmn, tmx);
-          const size_t gi = (size_t)gbase + ((base + lane) >> 3);
-          A.acc_groups[2 * gi] = make_float4(tmn.x, tmn.y, tmn.z, 0.0f);
-          A.acc_groups[2 * gi + 1] = make_float4(tmx.x, tmx.y, tmx.z, 0.0f);
-        }
+      mn = make_float3(fmin_sel(fmin_sel(v0.x, v1.x), v2.x), fmin_sel(fmin_sel(v0.y, v1.y), v2.y), fmin_sel(fmin_sel(v0.z, v1.z), v2.z));
+      mx = make_float3(fmax_sel(fmax_sel(v0.x, v1.x), v2.x), fmax_sel(fmax_sel(v0.y, v1.y), v2.y), fmax_sel(fmax_sel(v0.z, v1.z), v2.z));
+    }
+    // lanes past which the lane's group and leaf end (inside the step)
+    const uint32_t gend = lane - (c.rel & 7u) + min(8u, c.cnt - (c.rel & ~7u));
+    const uint32_t lend = min(c.n, lane + c.cnt - c.rel);
+    auto combine = [&](uint32_t o, uint32_t end) {
+      const float3 bn = make_float3(__shfl_down_sync(0xffffffffu, mn.x, o), __shfl_down_sync(0xffffffffu, mn.y, o),
+                                    __shfl_down_sync(0xffffffffu, mn.z, o));
+      const float3 bx = make_float3(__shfl_down_sync(0xffffffffu, mx.x, o), __shfl_down_sync(0xffffffffu, mx.y, o),
+                                    __shfl_down_sync(0xffffffffu, mx.z, o));
+      if (lane + o < end) {
+        mn = make_float3(fmin_sel(mn.x, bn.x), fmin_sel(mn.y, bn.y), fmin_sel(mn.z, bn.z));
+        mx = make_float3(fmax_sel(mx.x, bx.x), fmax_sel(mx.y, bx.y), fmax_sel(mx.z, bx.z));
       }
+    };
+    combine(1, gend);
+    combine(2, gend);
+    combine(4, gend);
+    if (act && (c.rel & 7u) == 0 && out.acc_groups) {
+      float3 pmn = mn, pmx = mx;
+      pad_box(pmn, pmx);
+      const size_t gi = (size_t)group + (c.rel >> 3);
+      out.acc_groups[2 * gi] = make_float4(pmn.x, pmn.y, pmn.z, 0.0f);
+      out.acc_groups[2 * gi + 1] = make_float4(pmx.x, pmx.y, pmx.z, 0.0f);
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      mn.x = fmin_sel(mn.x, __shfl_xor_sync(0xffffffffu, mn.x, o));
-      mn.y = fmin_sel(mn.y, __shfl_xor_sync(0xffffffffu, mn.y, o));
-      mn.z = fmin_sel(mn.z, __shfl_xor_sync(0xffffffffu, mn.z, o));
-      mx.x = fmax_sel(mx.x, __shfl_xor_sync(0xffffffffu, mx.x, o));
-      mx.y = fmax_sel(mx.y, __shfl_xor_sync(0xffffffffu, mx.y, o));
-      mx.z = fmax_sel(mx.z, __shfl_xor_sync(0xffffffffu, mx.z, o));
+    combine(8, lend);
+    combine(16, lend);
+    // a leaf's first lane of the step now holds the leaf's box over the step; lane 0 may hold the rest of a leaf
+    const bool head = act && (c.rel == 0 || lane == 0);
+    if (lane == 0 && c.rel != 0) {
+      mn = make_float3(fmin_sel(cmn.x, mn.x), fmin_sel(cmn.y, mn.y), fmin_sel(cmn.z, mn.z));
+      mx = make_float3(fmax_sel(cmx.x, mx.x), fmax_sel(cmx.y, mx.y), fmax_sel(cmx.z, mx.z));
     }
-    if (lane == 0) {
-      if (leaf_id >= A.max_nodes) { atomicOr(A.err, (uint32_t)RT_DEVERR_NODE_CAPACITY); return; }
-      uint32_t* nd = A.nodes + 8 * (size_t)leaf_id;
-      *(uint2*)nd = make_uint2(1u | (cnt << 1), lfirst);
+    const bool done = lane + c.cnt - c.rel <= c.n;  // the leaf ends inside the step
+    if (head && done && node != kNone) {
+      uint32_t* nd = out.nodes + 8 * (size_t)node;
+      *(uint2*)nd = make_uint2(1u | (c.cnt << 1), first - pb);
       write_box(nd, mn, mx);
     }
+    const uint32_t open = __ballot_sync(0xffffffffu, head && !done);  // at most the step's last leaf
+    if (open) {
+      const int o = __ffs(open) - 1;
+      cmn = make_float3(__shfl_sync(0xffffffffu, mn.x, o), __shfl_sync(0xffffffffu, mn.y, o), __shfl_sync(0xffffffffu, mn.z, o));
+      cmx = make_float3(__shfl_sync(0xffffffffu, mx.x, o), __shfl_sync(0xffffffffu, mx.y, o), __shfl_sync(0xffffffffu, mx.z, o));
+    }
+    w = wn;
   }
 }
 
@@ -544,16 +626,31 @@ __global__ __launch_bounds__(256) void k_propagate(uint32_t* __restrict__ nodes,
     if (nodes[8 * (size_t)p] & 1u) climb(nodes, parent_id, arrive, cap, p);
 }
 
-__global__ __launch_bounds__(256) void k_leaves(LeafArgs A) {
-  const uint32_t warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  const uint32_t leaf_count = A.hdr[0];
+// The next run of leaves of a warp, from a counter (zero at the start): runs of about 512 faces (fewer where that leaves
+// warps without one), at most 32 leaves, so that a warp with large leaves does not keep the launch waiting: runs dealt
+// out beforehand, by leaves alone, left half of the SM time idle on meshes of mixed sizes.
+__device__ __forceinline__ uint32_t leaf_run(uint32_t leaf_count, uint32_t faces) {
+  const unsigned long long want = max(64u, min(512u, faces / 8192u));
+  return (uint32_t)max(1ull, min(32ull, want * leaf_count / faces));
+}
+__device__ __forceinline__ uint32_t next_run(uint32_t* counter, uint32_t run) {
+  uint32_t g = 0;
+  if (lane_id() == 0) g = atomicAdd(counter, run);
+  return __shfl_sync(0xffffffffu, g, 0);
+}
+
+__global__ __launch_bounds__(256) void k_leaves(LeafArgs A, uint32_t faces, uint32_t* counter) {
+  const uint32_t leaf_count = A.hdr[0], lane = lane_id();
   if (A.hdr[8] & (RT_DEVERR_NODE_CAPACITY | RT_DEVERR_MORTON_CAPACITY)) return;
-  // a contiguous run of leaves per warp (the grid is one resident wave)
-  const uint32_t per = (leaf_count + nwarps - 1) / nwarps;
-  const uint32_t g0 = min(leaf_count, warp_global * per), g1 = min(leaf_count, g0 + per);
-  uint32_t hint = ~0u;
-  for (uint32_t g = g0; g < g1; ++g) leaf_body(A, g, hint);
+  const uint32_t run = leaf_run(leaf_count, faces);
+  for (;;) {
+    const uint32_t g = next_run(counter, run);
+    if (g >= leaf_count) break;
+    const uint32_t lo = warp_morton_leaf(A, g);
+    LeafMeta L = {};
+    if (lane < run && g + lane < leaf_count) L = leaf_meta(A, g + lane, lo, 0u, 0u);
+    leaf_faces(A, L);
+  }
 }
 
 // Two-child traversal records, indexed by pre-order rank (internal node p
@@ -606,7 +703,7 @@ struct BuildLayout {
   uint32_t* err;
   uint32_t* leaf_lambda;
   uint4* faces_tmp;
-  uint32_t* hit_done;  // the hit box's block counter
+  uint32_t* hit_done;  // the hit box's block counter, then the next leaf to hand out
   ClusterTemps ct;   // cluster tree build (RT_ACCEL_CLUSTERS only)
 };
 
@@ -649,7 +746,7 @@ size_t carve_build(Carve& c, BuildLayout& L, uint32_t n, uint32_t D, bool need_c
   L.err = c.take<uint32_t>(4);
   L.leaf_lambda = c.take<uint32_t>(L.max_nodes);
   L.faces_tmp = need_faces_tmp ? c.take<uint4>(n) : nullptr;
-  L.hit_done = c.take<uint32_t>(1);
+  L.hit_done = c.take<uint32_t>(2);
   L.ct = ClusterTemps{};
   if (clusters) carve_cluster_temps(c, L.ct, n, 1);
   return c.off + 256;
@@ -769,13 +866,13 @@ extern "C" rt_status rt_lbvh_build(const rt_build_desc* d, rt_stream stream_) {
   const int sms = sm_count();
 
   // 1. hit box
+  if (cudaMemsetAsync(L.hit_done, 0, 8, st) != cudaSuccess) return RT_ERR_CUDA;
   if (d->hitbox) {
     float4 mn = make_float4(d->hitbox[0], d->hitbox[1], d->hitbox[2], d->hitbox[3]);
     float4 mx = make_float4(d->hitbox[4], d->hitbox[5], d->hitbox[6], d->hitbox[7]);
     k_set_hitbox<<<1, 1, 0, st>>>(L.hit, mn, mx);
     note_launch();
   } else {
-    if (cudaMemsetAsync(L.hit_done, 0, 4, st) != cudaSuccess) return RT_ERR_CUDA;
     k_hitbox<<<kHitParts, 256, 0, st>>>((const float4*)d->vertices, d->vertex_count, L.partial, L.hit_done, L.hit);
     note_launch();
   }
@@ -828,7 +925,7 @@ extern "C" rt_status rt_lbvh_build(const rt_build_desc* d, rt_stream stream_) {
     A.local_indices = nullptr;
     A.parent_cap = count;
     static const int leaf_blocks = resident_blocks_of(k_leaves, 256);
-    k_leaves<<<sms * leaf_blocks, 256, 0, st>>>(A);
+    k_leaves<<<(uint32_t)hmin<uint64_t>((uint64_t)sms * leaf_blocks, (n + 255) / 256), 256, 0, st>>>(A, n, L.hit_done + 1);
     k_propagate<<<sms * 8, 256, 0, st>>>(d->nodes, L.parent_id, L.arrive, L.hdr, count);
     note_launch(2);
     RT_CHECK_LAUNCH();
@@ -921,7 +1018,8 @@ struct BatchArgs {
   uint32_t* hdr;          // [16 M]
   uint32_t* leaf_base;    // [M + 1]
   uint32_t* err;          // [4]
-  uint32_t* topo_done;    // finished topology CTAs
+  uint32_t* topo_done;    // finished topology CTAs, then the next leaf to hand out
+  uint32_t* leaf_next;
   // traversal blob
   uint32_t* acc_hdr;      // [64 M]
   float4* tnodes;         // [4 N]
@@ -1055,34 +1153,40 @@ __global__ __launch_bounds__(kTopoThreads) void k_batch_topo(BatchArgs B) {
 }
 
 __global__ __launch_bounds__(256) void k_batch_leaves(BatchArgs B) {
-  const uint32_t warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
   const uint32_t total = B.leaf_base[B.M];
-  // a contiguous run of leaves per warp (the grid is one resident wave): the
-  // mesh and the Morton-leaf search carry over from one leaf to the next
-  const uint32_t per = (total + nwarps - 1) / nwarps;
-  const uint32_t g0 = min(total, warp_global * per), g1 = min(total, g0 + per);
-  if (g0 >= g1) return;
-  uint32_t m = find_seg(B.leaf_base, B.M, g0), hint = ~0u;
-  LeafArgs A;
-  auto mesh_args = [&]() {
-    const uint32_t F = B.foff[m], n = B.foff[m + 1] - F;
-    const uint32_t bb = bfs_base(F, m), nb = node_base(F, m);
-    A.verts = B.verts; A.faces_in = B.faces_in; A.faces_out = B.faces_out; A.tris = B.tris; A.indices = B.idx;
+  const uint32_t lane = lane_id();
+  LeafArgs out = {};  // the whole build's arrays
+  out.verts = B.verts; out.faces_in = B.faces_in; out.faces_out = B.faces_out; out.tris = B.tris; out.indices = B.idx;
+  out.nodes = B.nodes; out.acc_groups = B.groups; out.local_indices = B.indices_out; out.err = B.err;
+  const uint32_t run = leaf_run(total, B.N);
+  for (;;) {
+    const uint32_t g = next_run(B.leaf_next, run);
+    if (g >= total) break;
+    const bool have = lane < run && g + lane < total;
+    const uint32_t m0 = warp_last_le(B.leaf_base, B.M, g);
+    uint32_t m = m0;
+    while (have && __ldg(B.leaf_base + m + 1) <= g + lane) ++m;
+    const uint32_t F = B.foff[m], n = B.foff[m + 1] - F, bb = bfs_base(F, m), nb = node_base(F, m);
+    LeafArgs A = {};
     A.ml_lambda = B.ml_lambda + bb; A.ml_rec = B.ml_rec + bb; A.ml_rank = B.ml_rank + bb;
-    A.parent_id = B.parent_id + nb; A.arrive = B.arrive + nb; A.nodes = B.nodes + 8 * (size_t)nb; A.max_nodes = 2 * n - 1;
+    A.parent_id = B.parent_id + nb; A.nodes = B.nodes + 8 * (size_t)nb; A.max_nodes = 2 * n - 1;
     A.max_leaf = B.q.max_leaf; A.hdr = B.hdr + 16 * m; A.err = B.err;
-    A.acc_leaves = B.acc_leaves + F; A.acc_groups = B.groups + 2 * (size_t)group_base(F, m); A.leaf_lambda = B.leaf_lambda + nb;
-    A.pos_base = F; A.vert_base = B.voff[m]; A.local_indices = B.indices_out; A.parent_cap = 2 * n - 1;
-  };
-  mesh_args();
-  for (uint32_t g = g0; g < g1; ++g) {
-    if (B.leaf_base[m + 1] <= g) {  // the next non-empty mesh
-      while (B.leaf_base[m + 1] <= g) ++m;
-      mesh_args();
-      hint = ~0u;
+    A.acc_leaves = B.acc_leaves + F; A.leaf_lambda = B.leaf_lambda + nb;
+    A.pos_base = F; A.vert_base = B.voff[m]; A.parent_cap = 2 * n - 1;
+    const uint32_t lg = g + lane - B.leaf_base[m];  // the leaf in its mesh
+    uint32_t lo = 0;
+    if (__all_sync(0xffffffffu, m == m0)) {
+      lo = warp_morton_leaf(A, g - B.leaf_base[m]);
+    } else if (have) {  // leaves of several meshes: each lane by itself
+      uint32_t hi = A.hdr[1] - 1;
+      while (lo < hi) {  // last k with ml_lambda[k] <= lg (non-decreasing)
+        const uint32_t mid = (lo + hi + 1) >> 1;
+        if (A.ml_lambda[mid] <= lg) lo = mid; else hi = mid - 1;
+      }
     }
-    leaf_body(A, g - B.leaf_base[m], hint);
+    LeafMeta L = {};
+    if (have) L = leaf_meta(A, lg, lo, nb, group_base(F, m));
+    leaf_faces(out, L);
   }
 }
 
@@ -1159,7 +1263,8 @@ size_t carve_batch(Carve& c, BatchArgs& B, uint32_t M, uint32_t N, bool clusters
   B.hdr = c.take<uint32_t>(16 * (size_t)M);
   B.leaf_base = c.take<uint32_t>((size_t)M + 1);
   B.err = c.take<uint32_t>(4);
-  B.topo_done = c.take<uint32_t>(1);
+  B.topo_done = c.take<uint32_t>(2);
+  B.leaf_next = B.topo_done ? B.topo_done + 1 : nullptr;
   B.ct = ClusterTemps{};
   if (clusters) carve_cluster_temps(c, B.ct, N, M);
   const size_t sort_bytes = batch_sort_bytes(N, M);
@@ -1222,7 +1327,7 @@ extern "C" rt_status rt_batch_build(const rt_batch_build_desc* d, rt_stream stre
   const int sms = sm_count();
   const uint32_t fblocks = (uint32_t)hmin<uint64_t>((N + 255) / 256, (uint64_t)sms * 16);
   if (cudaMemsetAsync(B.err, 0, 16, st) != cudaSuccess) return RT_ERR_CUDA;
-  if (cudaMemsetAsync(B.topo_done, 0, 4, st) != cudaSuccess) return RT_ERR_CUDA;
+  if (cudaMemsetAsync(B.topo_done, 0, 8, st) != cudaSuccess) return RT_ERR_CUDA;
   if (cudaMemsetAsync(B.hist, 0, (size_t)M * 64 * 4, st) != cudaSuccess) return RT_ERR_CUDA;
   if (cudaMemsetAsync(B.hitdone, 0, (size_t)M * 4, st) != cudaSuccess) return RT_ERR_CUDA;
   k_batch_hitbox<<<M * kHitSplit, 512, 0, st>>>(B);
@@ -1239,7 +1344,7 @@ extern "C" rt_status rt_batch_build(const rt_batch_build_desc* d, rt_stream stre
   RT_CHECK_LAUNCH();
   if (cudaMemsetAsync(B.arrive, 0, (2 * (size_t)N) * 4, st) != cudaSuccess) return RT_ERR_CUDA;
   static const int leaf_blocks = resident_blocks_of(k_batch_leaves, 256);
-  k_batch_leaves<<<sms * leaf_blocks, 256, 0, st>>>(B);
+  k_batch_leaves<<<(uint32_t)hmin<uint64_t>((uint64_t)sms * leaf_blocks, (N + 255) / 256), 256, 0, st>>>(B);
   note_launch();
   RT_CHECK_LAUNCH();
   // the node boxes and records (from the nodes) and the cluster trees (from the codes and triangles) are
