@@ -1098,20 +1098,34 @@ __device__ __forceinline__ void add2(float a0, float a1, float b0, float b1, flo
       : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
 }
 
+// Three-input maximum (one instruction on sm_100; a NaN operand is left out).
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
 // Top-1 sweep of 16 logits (TMEM columns col .. col + 15 of this row) plus
-// their biases into the four interleaved chains (chain j: columns = j mod 4).
-__device__ __forceinline__ void sweep16_top1(const uint32_t (&r)[16], const float* sb, uint32_t col, float (&bk)[4], int32_t (&ik)[4]) {
+// their biases: only their maximum is compared with the best so far, and a
+// larger one leaves all 16 in the thread's shared-memory slot (`save`, four
+// 16-byte pieces kFuseCompute apart), where its column is looked up once per
+// tile. 23 instructions instead of 56 for a compare and two selects per logit: 2M rays 3.48 -> 2.98 ms, now bound by the
+// chain of the three hidden layers and the logits' MMAs.
+__device__ __forceinline__ void sweep16_top1(const uint32_t (&r)[16], const float* sb, uint32_t col, float& best, int32_t& at, float4* save) {
   const float4* bp = (const float4*)(sb + col);
+  float x[16];
 #pragma unroll
-  for (int i4 = 0; i4 < 4; ++i4) {
-    const float4 b = bp[i4];
-    float x[4];
-    add2(__uint_as_float(r[4 * i4]), __uint_as_float(r[4 * i4 + 1]), b.x, b.y, x[0], x[1]);
-    add2(__uint_as_float(r[4 * i4 + 2]), __uint_as_float(r[4 * i4 + 3]), b.z, b.w, x[2], x[3]);
-    const int32_t base = (int32_t)(col + 4 * i4);
+  for (int i = 0; i < 4; ++i) {
+    const float4 b = bp[i];
+    add2(__uint_as_float(r[4 * i]), __uint_as_float(r[4 * i + 1]), b.x, b.y, x[4 * i], x[4 * i + 1]);
+    add2(__uint_as_float(r[4 * i + 2]), __uint_as_float(r[4 * i + 3]), b.z, b.w, x[4 * i + 2], x[4 * i + 3]);
+  }
+  const float m = fmaxf(max3(max3(x[0], x[1], x[2]), max3(x[3], x[4], x[5]), max3(x[6], x[7], x[8])),
+                        max3(max3(x[9], x[10], x[11]), max3(x[12], x[13], x[14]), x[15]));
+  if (m > best) {
+    best = m;
+    at = (int32_t)col;
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (x[j] > bk[j]) { bk[j] = x[j]; ik[j] = base; }
+    for (int i = 0; i < 4; ++i) save[i * kFuseCompute] = make_float4(x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3]);
   }
 }
 
@@ -1140,7 +1154,8 @@ __global__ void __launch_bounds__(kFuseThreads, 1)
   uint64_t* bias_full = part_free + 1;    // [2]
   uint64_t* bias_empty = bias_full + 2;   // [2]
   uint64_t* done = bias_empty + 2;
-  uint32_t* tmem_slot = (uint32_t*)(done + 1);
+  uint64_t* save_free = done + 1;
+  uint32_t* tmem_slot = (uint32_t*)(save_free + 1);
   volatile uint32_t* s_abort = tmem_slot + 1;
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
   if (threadIdx.x == 0) {
@@ -1160,6 +1175,7 @@ __global__ void __launch_bounds__(kFuseThreads, 1)
     mbar_init(part_ready, 3 * kBM);
     mbar_init(part_free, kBM);
     mbar_init(done, 1);
+    mbar_init(save_free, kFuseCompute);
     *s_abort = 0u;
     fence_mbar_init();
     prefetch_tmap(&t1);
@@ -1295,6 +1311,10 @@ __global__ void __launch_bounds__(kFuseThreads, 1)
         }
         continue;
       }
+      if (!kTop2 && k > 0) {  // the sweep's slots lie where the features go
+        ok = __all_sync(0xffffffffu, wait(save_free, (k - 1u) & 1u));
+        if (!ok) break;
+      }
       // features: (ray r, input i) pairs p = 128 i + r, i < 6
       for (uint32_t p = tid; p < 6u * kBM; p += kFuseCompute) {
         const uint32_t r = p & 127u, i = p >> 7, row = row0 + r;
@@ -1342,9 +1362,12 @@ __global__ void __launch_bounds__(kFuseThreads, 1)
         mbar_arrive(h_ready);
       }
       if (!ok) break;
-      // logits: running maximum (and runner-up) over four interleaved column
-      // chains of this quarter; chain j holds columns = j (mod 4), and ik[j]
-      // keeps the winner's column minus j
+      // logits: the running maximum with the 16 columns it came from (the first atoms of sA, which the third layer's
+      // MMAs have read, hold each thread's 16 values); or, with the runner-up, four interleaved column chains of this
+      // quarter, where chain j holds columns = j (mod 4) and ik[j] keeps the winner's column minus j
+      float best = -INFINITY;
+      int32_t at = -1;
+      float4* save = (float4*)sA + tid;
       float bk[4], sk[4];
       int32_t ik[4];
 #pragma unroll
@@ -1364,10 +1387,10 @@ __global__ void __launch_bounds__(kFuseThreads, 1)
 #pragma unroll
           for (uint32_t c = 0; c < kArgBN / 4; c += 32) {
             tmem_ld16_issue(tl + c + 16, rb);
-            sweep16_top1(ra, sb, col0 + c, bk, ik);
+            sweep16_top1(ra, sb, col0 + c, best, at, save);
             tmem_ld_wait(rb);
             if (c + 32 < kArgBN / 4) tmem_ld16_issue(tl + c + 32, ra);
-            sweep16_top1(rb, sb, col0 + c + 16, bk, ik);
+            sweep16_top1(rb, sb, col0 + c + 16, best, at, save);
             if (c + 32 < kArgBN / 4) tmem_ld_wait(ra);
           }
         } else if (ok) {
@@ -1399,8 +1422,23 @@ __global__ void __launch_bounds__(kFuseThreads, 1)
       mbar_arrive(bias_empty + bb);
       if (!ok) break;
       Top2 res = Top2{bk[0], sk[0], ik[0]};
+      if (kTop2) {
 #pragma unroll
-      for (int j = 1; j < 4; ++j) res = top2_merge(res, Top2{bk[j], sk[j], ik[j] + j});
+        for (int j = 1; j < 4; ++j) res = top2_merge(res, Top2{bk[j], sk[j], ik[j] + j});
+      } else {
+        res = Top2{best, -INFINITY, -1};
+        if (at >= 0) {  // the first of the 16 columns that holds the maximum
+#pragma unroll
+          for (int i = 3; i >= 0; --i) {
+            const float4 x = save[i * kFuseCompute];
+            if (x.w == best) res = Top2{x.w, -INFINITY, at + 4 * i + 3};
+            if (x.z == best) res = Top2{x.z, -INFINITY, at + 4 * i + 2};
+            if (x.y == best) res = Top2{x.y, -INFINITY, at + 4 * i + 1};
+            if (x.x == best) res = Top2{x.x, -INFINITY, at + 4 * i};
+          }
+        }
+        mbar_arrive(save_free);
+      }
       if (cq > 0) {
         if (k > 0) ok = __all_sync(0xffffffffu, wait(part_free, (k - 1u) & 1u));
         if (!ok) break;
