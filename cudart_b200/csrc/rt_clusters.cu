@@ -58,24 +58,36 @@ struct ClusterBuild {
   float4* crec;          // records, all meshes
 };
 
-__device__ __forceinline__ void mesh_of_chunk(const ClusterBuild& B, uint32_t b, uint32_t& m, uint32_t& F, uint32_t& n, uint32_t& j) {
+// Mesh m of chunk b (for which the warp's first chunk is `first`): its face offset, face count and b's index j among
+// its chunks. The warp finds the mesh of `first` together, 32 meshes at a step; a lane whose chunk is later goes on
+// from there (the lanes of a warp hold consecutive chunks).
+__device__ __forceinline__ void mesh_of_chunk(const ClusterBuild& B, uint32_t first, uint32_t b, uint32_t& m, uint32_t& F, uint32_t& n,
+                                              uint32_t& j) {
   if (!B.foff) {
     m = 0; F = 0; n = B.N; j = b;
     return;
   }
-  uint32_t lo = 0, hi = B.M - 1;  // largest m with cluster_chunk_base(F_m, m) <= b
-  while (lo < hi) {
-    const uint32_t mid = (lo + hi + 1) >> 1;
-    if (cluster_chunk_base(__ldg(B.foff + mid), mid) <= b) lo = mid; else hi = mid - 1;
+  uint32_t lo = 0, len = B.M;  // largest m with cluster_chunk_base(F_m, m) <= first
+  while (len > 1) {
+    const uint32_t step = (len + 31) / 32, at = lane_id() * step;
+    const uint32_t c = (uint32_t)__popc(__ballot_sync(0xffffffffu, at < len && cluster_chunk_base(__ldg(B.foff + lo + at), lo + at) <= first)) - 1u;
+    lo += c * step;
+    len = min(step, len - c * step);
   }
   m = lo;
+  while (m + 1 < B.M && cluster_chunk_base(__ldg(B.foff + m + 1), m + 1) <= b) ++m;
   F = __ldg(B.foff + m);
   n = __ldg(B.foff + m + 1) - F;
   j = b - cluster_chunk_base(F, m);
 }
 
-__device__ __forceinline__ unsigned long long key_xor(uint32_t c0, uint32_t c1, uint32_t b) {
-  return ((unsigned long long)(c0 ^ c1) << 32) | (b ^ (b + 1u));
+// The value of the boundary between positions pos - 1 and pos of a mesh's n codes, as its level: the number of leading
+// bits that the two keys share, -1 at the mesh's ends. The two boundaries that flank a node differ in it, since sorted
+// keys that agree up to a bit change there once, and the smaller value is the one with the higher level.
+__device__ __forceinline__ int level_before(const uint32_t* __restrict__ codes, uint32_t n, uint32_t pos) {
+  if (pos == 0 || pos >= n) return -1;
+  const uint32_t x = __ldg(codes + pos - 1) ^ __ldg(codes + pos);
+  return x ? __clz(x) : 32 + __clz((pos - 1) ^ pos);
 }
 
 __device__ __forceinline__ void tri_box(const float4* tr, float3& mn, float3& mx) {
@@ -87,58 +99,45 @@ __device__ __forceinline__ void tri_box(const float4* tr, float3& mn, float3& mx
   pad_box(mn, mx);
 }
 
-// Where a pass reads the child references and child boxes of completed nodes: shared memory for the chunk pass
-// (the chunk's positions and inner boundaries), global memory (through L2) for the record pass.
-struct SmemNodes {
-  const float (*lbox)[kClusterChunk];
-  const float (*ibox)[kClusterChunk];
-  const uint32_t* child;
-  uint32_t s;  // the chunk's first position
-  __device__ __forceinline__ void box(uint32_t ref, float3& mn, float3& mx) const {
-    const float(*b)[kClusterChunk] = (ref & kClusterLeaf) ? lbox : ibox;
-    const uint32_t k = (ref & ~kClusterLeaf) - s;
-    mn = make_float3(b[0][k], b[1][k], b[2][k]);
-    mx = make_float3(b[3][k], b[4][k], b[5][k]);
-  }
-  __device__ __forceinline__ uint32_t kid(uint32_t p, uint32_t side) const { return child[2 * (p - s) + side]; }
-  __device__ __forceinline__ void kid_box(uint32_t p, uint32_t side, float3& mn, float3& mx) const { box(kid(p, side), mn, mx); }
+// One slot pair of a completed internal node's 4-wide record: the child of positions lo .. hi with reference c, whose own
+// children (if any) are c0 and c1. A child that is a cluster (at most leaf_max positions) takes the first slot (the second
+// keeps NaN bounds), any other child one slot for each of its two children (c, its index, is its split). The slots' boxes are
+// the child's, or its children's.
+struct SlotPair {
+  uint32_t ref0, ref1;
 };
-struct GlobalNodes {
-  const ClusterTemps* T;
-  uint32_t F;
-  __device__ __forceinline__ uint32_t kid(uint32_t p, uint32_t side) const { return __ldcg(T->child + 2 * ((size_t)F + p) + side); }
-  __device__ __forceinline__ void kid_box(uint32_t p, uint32_t side, float3& mn, float3& mx) const {
-    const float4* q = T->cbox + 4 * ((size_t)F + p) + 2 * side;
-    const float4 a = __ldcg(q), b = __ldcg(q + 1);
-    mn = make_float3(a.x, a.y, a.z);
-    mx = make_float3(b.x, b.y, b.z);
-  }
-};
+__device__ __forceinline__ SlotPair slot_pair(uint32_t leaf_max, uint32_t lo, uint32_t hi, uint32_t c, uint32_t c0, uint32_t c1) {
+  if (hi - lo + 1 <= leaf_max) return SlotPair{cluster_leaf_ref(lo, hi - lo + 1), kNoChild};
+  return SlotPair{(c - lo + 1 <= leaf_max) ? cluster_leaf_ref(lo, c - lo + 1) : c0,
+                  (hi - c <= leaf_max) ? cluster_leaf_ref(c + 1, hi - c) : c1};
+}
 
-// The 4-wide record of a completed internal node p (positions l .. r, children l .. p and p + 1 .. r): child 0
-// fills slots 0 and 1, child 1 slots 2 and 3 -- a child that is a cluster (at most leaf_max positions) its first
-// slot (the second keeps NaN bounds), any other child one slot for each of its two children.
-template <class Nodes>
-__device__ __forceinline__ void write_record(const ClusterBuild& B, const Nodes& Nd, float4* rec, uint32_t p, uint32_t l, uint32_t r) {
+// The record of node p (positions l .. r) from the global child references and boxes.
+__device__ __forceinline__ void write_record(const ClusterBuild& B, uint32_t F, uint32_t p, uint32_t l, uint32_t r) {
   const float qnan = __int_as_float(0x7fffffff);
   float3 mn[4], mx[4];
   uint32_t ref[4];
-  auto child = [&](const int k, uint32_t lo, uint32_t hi) {
-    const uint32_t c = Nd.kid(p, (uint32_t)(k >> 1));
-    if (hi - lo + 1 <= B.leaf_max) {
-      Nd.kid_box(p, (uint32_t)(k >> 1), mn[k], mx[k]);
-      ref[k] = cluster_leaf_ref(lo, hi - lo + 1);
-      mn[k + 1] = mx[k + 1] = make_float3(qnan, qnan, qnan);
-      ref[k + 1] = kNoChild;
-    } else {  // an internal node (more than leaf_max >= 1 positions); its split is its own index
-      Nd.kid_box(c, 0, mn[k], mx[k]);
-      Nd.kid_box(c, 1, mn[k + 1], mx[k + 1]);
-      ref[k] = (c - lo + 1 <= B.leaf_max) ? cluster_leaf_ref(lo, c - lo + 1) : Nd.kid(c, 0);
-      ref[k + 1] = (hi - c <= B.leaf_max) ? cluster_leaf_ref(c + 1, hi - c) : Nd.kid(c, 1);
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const uint32_t lo = h ? p + 1 : l, hi = h ? r : p;
+    const uint32_t c = __ldcg(B.T.child + 2 * ((size_t)F + p) + h);
+    const bool leaf = hi - lo + 1 <= B.leaf_max;
+    const uint2 kid = leaf ? make_uint2(0, 0) : __ldcg((const uint2*)(B.T.child + 2 * ((size_t)F + c)));
+    const SlotPair S = slot_pair(B.leaf_max, lo, hi, c, kid.x, kid.y);
+    ref[2 * h] = S.ref0;
+    ref[2 * h + 1] = S.ref1;
+    const float4* q = B.T.cbox + 4 * ((size_t)F + (leaf ? p : c)) + (leaf ? 2 * h : 0);
+    const float4 a = __ldcg(q), b = __ldcg(q + 1);
+    mn[2 * h] = make_float3(a.x, a.y, a.z);
+    mx[2 * h] = make_float3(b.x, b.y, b.z);
+    mn[2 * h + 1] = mx[2 * h + 1] = make_float3(qnan, qnan, qnan);
+    if (!leaf) {
+      const float4 u = __ldcg(q + 2), v = __ldcg(q + 3);
+      mn[2 * h + 1] = make_float3(u.x, u.y, u.z);
+      mx[2 * h + 1] = make_float3(v.x, v.y, v.z);
     }
-  };
-  child(0, l, p);
-  child(2, p + 1, r);
+  }
+  float4* rec = B.crec + 8 * ((size_t)F + p);
   rec[0] = make_float4(mn[0].x, mn[1].x, mn[2].x, mn[3].x);
   rec[1] = make_float4(mn[0].y, mn[1].y, mn[2].y, mn[3].y);
   rec[2] = make_float4(mn[0].z, mn[1].z, mn[2].z, mn[3].z);
@@ -175,138 +174,181 @@ __device__ __forceinline__ void finish_root(const ClusterBuild& B, uint32_t m, u
   hdr[kHdrClusterValid] = 1u;
 }
 
+// A node moving up: reference, first and last position, box.
+struct ChunkNode {
+  uint32_t cur, l, r;
+  float3 mn, mx;
+};
+
+// Shared memory of the chunk pass. A box is two float4 (a node read is two 16-byte loads; six arrays of floats cost three
+// times the wavefronts), whose w words hold an inner node's first and last position (last 0: not complete).
+struct ChunkShared {
+  float4 box[2 * kClusterChunk][2];  // inner nodes (by boundary), then positions
+  uint2 child[kClusterChunk];
+  uint32_t other[kClusterChunk];     // arrival words
+  int level[kClusterChunk + 1];      // of boundaries s - 1 .. s + 511
+  alignas(16) uint32_t list[3][kClusterChunk];  // round r reads list r % 3 and fills list (r + 1) % 3
+  uint32_t count[3];
+  uint32_t records;
+
+  // index in box of node ref of the chunk that starts at position s
+  static __device__ __forceinline__ uint32_t at(uint32_t ref, uint32_t s) { return (ref & ~kClusterLeaf) - s + ((ref & kClusterLeaf) ? kClusterChunk : 0u); }
+  __device__ __forceinline__ ChunkNode node(uint32_t ref, uint32_t s) const {
+    const float4 a = box[at(ref, s)][0], b = box[at(ref, s)][1];
+    const bool leaf = (ref & kClusterLeaf) != 0;
+    const uint32_t pos = ref & ~kClusterLeaf;
+    return ChunkNode{ref, leaf ? pos : __float_as_uint(a.w), leaf ? pos : __float_as_uint(b.w), make_float3(a.x, a.y, a.z), make_float3(b.x, b.y, b.z)};
+  }
+};
+
+// One step of node c up: true if it arrived second at its parent, which is then complete and replaces it. False: the
+// sibling completes the parent, or the climb leaves the chunk (positions s .. e), or c is the root.
+__device__ __forceinline__ bool chunk_climb(const ClusterBuild& B, ChunkShared& S, uint32_t s, uint32_t e, uint32_t m, uint32_t F, uint32_t n,
+                                            ChunkNode& c) {
+  const int level_l = S.level[c.l - s], level_r = S.level[c.r + 1 - s];
+  if (max(level_l, level_r) < 0) {
+    finish_root(B, m, F, n, c.cur, c.mn, c.mx);
+    return false;
+  }
+  const bool left_child = level_r > level_l;
+  const uint32_t p = left_child ? c.r : c.l - 1;
+  if (p < s || p >= e) {  // the parent's boundary is not inside the chunk: the frontier pass goes on from here
+    B.T.frontier[2 * (size_t)blockIdx.x + (p < s ? 0 : 1)] = make_uint4(c.cur, c.l, c.r, 1u);
+    return false;
+  }
+  const uint32_t k = p - s;
+  (left_child ? S.child[k].x : S.child[k].y) = c.cur;
+  __threadfence_block();
+  const uint32_t old = atomicExch(S.other + k, (left_child ? c.l : c.r) + 1u);
+  if (old == 0) return false;
+  __threadfence_block();
+  if (left_child) c.r = old - 1u; else c.l = old - 1u;
+  const uint32_t sib = S.at(left_child ? S.child[k].y : S.child[k].x, s);
+  const float4 a = S.box[sib][0], b = S.box[sib][1];
+  c.mn = make_float3(fminf(c.mn.x, a.x), fminf(c.mn.y, a.y), fminf(c.mn.z, a.z));
+  c.mx = make_float3(fmaxf(c.mx.x, b.x), fmaxf(c.mx.y, b.y), fmaxf(c.mx.z, b.z));
+  c.cur = p;
+  S.box[k][0] = make_float4(c.mn.x, c.mn.y, c.mn.z, __uint_as_float(c.l));
+  S.box[k][1] = make_float4(c.mx.x, c.mx.y, c.mx.z, __uint_as_float(c.r));
+  return true;
+}
+
+// The slot pair of a record's child (positions lo .. hi, reference c) and its boxes' indices.
+constexpr uint32_t kNoBox = 0xffffu;
+__device__ __forceinline__ SlotPair chunk_pair(uint32_t leaf_max, const ChunkShared& S, uint32_t s, uint32_t lo, uint32_t hi, uint32_t c,
+                                               uint32_t& src) {
+  uint2 kid = make_uint2(0, 0);
+  if (hi - lo + 1 <= leaf_max) {
+    src = S.at(c, s) | kNoBox << 16;
+  } else {
+    kid = S.child[c - s];
+    src = S.at(kid.x, s) | S.at(kid.y, s) << 16;
+  }
+  return slot_pair(leaf_max, lo, hi, c, kid.x, kid.y);
+}
+
 // The chunk pass climbs in rounds: the nodes to move up (all positions first) sit in a compacted shared-memory
 // list; in a round every listed node arrives at its parent, and the second arrival at a parent completes it
 // (range and box, in shared memory) and lists it for the next round, so the threads of a warp work on listed
-// nodes side by side. After the last round the CTA writes, with coalesced stores, every position's box, every
-// inner boundary's child references, box and arrival word, and the records of the nodes completed here.
+// nodes side by side. Once a warp can hold what is listed, the first warp climbs on alone, a node per lane and without
+// barriers. Then the CTA writes every inner boundary's arrival word and the records of the nodes completed here: a thread
+// per record works out its references and which boxes it holds, then the threads take its six 16-byte parts of box
+// bounds one by one, so that neighbouring lanes store neighbouring bytes and read a box's neighbouring words. (A thread
+// per whole record stored 16 bytes in each of 32 lines at a time and, with every round between barriers, took
+// 87 us for 2^20 faces and 769 for 9.9M in 1024 meshes; now 63 and
+// 544, by issue slots and the latency of the rounds.)
 __global__ __launch_bounds__(kClusterChunk, 4) void k_cluster_chunk(ClusterBuild B) {
-  __shared__ uint32_t s_other[kClusterChunk];
-  __shared__ uint32_t s_child[2 * kClusterChunk];
-  __shared__ uint32_t s_range[2][kClusterChunk];  // first and last position of a node completed here (else last = 0)
-  __shared__ float s_ibox[6][kClusterChunk];
-  __shared__ float s_lbox[6][kClusterChunk];
-  __shared__ uint32_t s_code[kClusterChunk + 2];  // codes of positions s - 1 .. s + 512
-  __shared__ uint32_t s_list[3][kClusterChunk];   // round r reads list r % 3 and fills list (r + 1) % 3
-  __shared__ uint32_t s_count[3];
-  const uint32_t t = threadIdx.x;
+  __shared__ ChunkShared S;
+  const uint32_t t = threadIdx.x, lane = t & 31u;
   uint32_t m, F, n, j;
-  if (B.foff && B.M <= kClusterChunk) {
-    // the chunk's mesh in one step: the number of meshes whose first chunk is at or before this one, less one
-    const bool before = t < B.M && cluster_chunk_base(__ldg(B.foff + t), t) <= blockIdx.x;
-    m = (uint32_t)__syncthreads_count(before) - 1u;
-    F = __ldg(B.foff + m);
-    n = __ldg(B.foff + m + 1) - F;
-    j = blockIdx.x - cluster_chunk_base(F, m);
-  } else {
-    mesh_of_chunk(B, blockIdx.x, m, F, n, j);
-  }
+  mesh_of_chunk(B, blockIdx.x, blockIdx.x, m, F, n, j);
   const uint32_t s = j * kClusterChunk;
   if (t < 2) B.T.frontier[2 * (size_t)blockIdx.x + t] = make_uint4(0, 0, 0, 0);
   if (s >= n) return;  // a gap in the batched grid (the whole CTA)
   const uint32_t e = min(n, s + kClusterChunk) - 1;  // the chunk's last position; inner boundaries s .. e - 1
-  s_other[t] = 0;
-  s_range[1][t] = 0;
-  for (uint32_t q = t; q < kClusterChunk + 2; q += blockDim.x) {
-    const long long pos = (long long)s - 1 + q;
-    if (pos >= 0 && pos < (long long)n) s_code[q] = __ldg(B.codes + F + pos);
-  }
+  S.other[t] = 0;
+  S.box[t][1].w = 0.f;
   const uint32_t i = s + t;
+  S.level[t] = level_before(B.codes + F, n, i);
+  if (t == 0) S.level[kClusterChunk] = level_before(B.codes + F, n, s + kClusterChunk);
+  ChunkNode c;
   if (i <= e) {
-    float3 mn, mx;
-    tri_box(B.tris + 3 * ((size_t)F + i), mn, mx);
-    s_lbox[0][t] = mn.x; s_lbox[1][t] = mn.y; s_lbox[2][t] = mn.z; s_lbox[3][t] = mx.x; s_lbox[4][t] = mx.y; s_lbox[5][t] = mx.z;
-    s_list[0][t] = kClusterLeaf | i;
+    c.cur = kClusterLeaf | i;
+    c.l = c.r = i;
+    tri_box(B.tris + 3 * ((size_t)F + i), c.mn, c.mx);
+    S.box[kClusterChunk + t][0] = make_float4(c.mn.x, c.mn.y, c.mn.z, 0.f);
+    S.box[kClusterChunk + t][1] = make_float4(c.mx.x, c.mx.y, c.mx.z, 0.f);
   }
-  if (t == 0) {
-    s_count[0] = e - s + 1;
-    s_count[1] = 0;
-  }
+  if (t < 3) S.count[t] = 0;
+  if (t == 3) S.records = 0;
   __syncthreads();
-  const SmemNodes Nd{s_lbox, s_ibox, s_child, s};
-  for (uint32_t round = 0;; ++round) {
+  uint32_t count = e - s + 1, round = 0;
+  for (;; ++round) {
     // one barrier per round: the list after next (read two rounds ago) is emptied during this round
     const uint32_t cb = round % 3u, nb = (round + 1u) % 3u;
-    const uint32_t count = s_count[cb];
-    if (count == 0) break;
-    if (t < count) {
-      const uint32_t cur = s_list[cb][t];
-      uint32_t l, r;
-      if (cur & kClusterLeaf) {
-        l = r = cur & ~kClusterLeaf;
-      } else {
-        l = s_range[0][cur - s];
-        r = s_range[1][cur - s];
-      }
-      if (l == 0 && r == n - 1) {
-        float3 mn, mx;
-        Nd.box(cur, mn, mx);
-        finish_root(B, m, F, n, cur, mn, mx);
-      } else {
-        // boundary b's codes are s_code[b - s + 1] and s_code[b - s + 2] (b in s - 1 .. e)
-        const bool left_child = (l == 0) || (r != n - 1 && key_xor(s_code[r - s + 1], s_code[r - s + 2], r) <
-                                                             key_xor(s_code[l - s], s_code[l - s + 1], l - 1));
-        const uint32_t p = left_child ? r : l - 1;
-        if (p < s || p >= e) {  // the parent's boundary is not inside the chunk: the frontier pass goes on from here
-          B.T.frontier[2 * (size_t)blockIdx.x + (p < s ? 0 : 1)] = make_uint4(cur, l, r, 1u);
-        } else {
-          const uint32_t k = p - s;
-          s_child[2 * k + (left_child ? 0u : 1u)] = cur;
-          __threadfence_block();
-          const uint32_t old = atomicExch(s_other + k, (left_child ? l : r) + 1u);
-          if (old != 0) {  // second arrival: this thread completes the parent
-            __threadfence_block();
-            if (left_child) r = old - 1u; else l = old - 1u;
-            float3 amn, amx, bmn, bmx;
-            Nd.box(s_child[2 * k], amn, amx);
-            Nd.box(s_child[2 * k + 1], bmn, bmx);
-            s_ibox[0][k] = fminf(amn.x, bmn.x); s_ibox[1][k] = fminf(amn.y, bmn.y); s_ibox[2][k] = fminf(amn.z, bmn.z);
-            s_ibox[3][k] = fmaxf(amx.x, bmx.x); s_ibox[4][k] = fmaxf(amx.y, bmx.y); s_ibox[5][k] = fmaxf(amx.z, bmx.z);
-            s_range[0][k] = l;
-            s_range[1][k] = r;
-            // append to the next list, one shared-memory atomic per warp
-            const uint32_t am = __activemask();
-            const uint32_t lane = t & 31u, leader = __ffs(am) - 1u;
-            uint32_t base = 0;
-            if (lane == leader) base = atomicAdd(s_count + nb, (uint32_t)__popc(am));
-            base = __shfl_sync(am, base, leader);
-            s_list[nb][base + __popc(am & ((1u << lane) - 1u))] = p;
-          }
-        }
-      }
+    if (round) {
+      count = S.count[cb];
+      if (count <= 32) break;
+      if (t < count) c = S.node(S.list[cb][t], s);
     }
-    if (t == 0) s_count[(round + 2u) % 3u] = 0;
+    const bool up = t < count && chunk_climb(B, S, s, e, m, F, n, c);
+    // append to the next list, one shared-memory atomic per warp
+    const uint32_t who = __ballot_sync(0xffffffffu, up);
+    if (who) {
+      uint32_t base = 0;
+      if (lane == 0) base = atomicAdd(S.count + nb, (uint32_t)__popc(who));
+      base = __shfl_sync(0xffffffffu, base, 0);
+      if (up) S.list[nb][base + __popc(who & ((1u << lane) - 1u))] = c.cur;
+    }
+    if (t == 0) S.count[(round + 2u) % 3u] = 0;
     __syncthreads();
   }
+  if (t < 32) {
+    bool up = t < count;
+    if (up) c = S.node(S.list[round % 3u][t], s);
+    while (__any_sync(0xffffffffu, up)) {
+      if (up) up = chunk_climb(B, S, s, e, m, F, n, c);
+      __syncwarp();
+    }
+  }
+  __syncthreads();
   // Write-out. Every boundary's arrival word (coalesced; e's is zero: its children are never both inside one chunk),
   // the record of each node completed here with more than leaf_max positions, and
   // for the global pass and its records the nodes they read: the frontier nodes and the first child to arrive at
   // each parent still pending, each with its box and, when internal, its child references and their boxes.
   auto put_box = [&](float4* dst, uint32_t ref) {
-    float3 mn, mx;
-    Nd.box(ref, mn, mx);
-    dst[0] = make_float4(mn.x, mn.y, mn.z, 0.f);
-    dst[1] = make_float4(mx.x, mx.y, mx.z, 0.f);
+    const float4 a = S.box[S.at(ref, s)][0], b = S.box[S.at(ref, s)][1];
+    dst[0] = make_float4(a.x, a.y, a.z, 0.f);
+    dst[1] = make_float4(b.x, b.y, b.z, 0.f);
   };
   auto export_kids = [&](uint32_t ref) {
     if (ref & kClusterLeaf) return;
-    const uint32_t k0 = Nd.kid(ref, 0), k1 = Nd.kid(ref, 1);
-    *(uint2*)(B.T.child + 2 * ((size_t)F + ref)) = make_uint2(k0, k1);
-    put_box(B.T.cbox + 4 * ((size_t)F + ref), k0);
-    put_box(B.T.cbox + 4 * ((size_t)F + ref) + 2, k1);
+    const uint2 k = S.child[ref - s];
+    *(uint2*)(B.T.child + 2 * ((size_t)F + ref)) = k;
+    put_box(B.T.cbox + 4 * ((size_t)F + ref), k.x);
+    put_box(B.T.cbox + 4 * ((size_t)F + ref) + 2, k.y);
   };
+  bool record = false;
+  uint2 src;  // the record's four boxes (16-bit indices into box, kNoBox: none)
   if (i < e) {
-    const uint32_t word = s_other[t];
+    const uint32_t word = S.other[t];
     B.T.other[(size_t)F + i] = word;
-    const uint32_t l = s_range[0][t], r = s_range[1][t];
+    const uint32_t l = __float_as_uint(S.box[t][0].w), r = __float_as_uint(S.box[t][1].w);
     if (r != 0) {
-      if (r - l + 1 > B.leaf_max) write_record(B, Nd, B.crec + 8 * ((size_t)F + i), i, l, r);
+      record = r - l + 1 > B.leaf_max;
     } else if (word != 0) {  // one child arrived: a left child stored its first position (<= i), a right one its last
       const uint32_t side = (word - 1u <= i) ? 0u : 1u;
-      const uint32_t c = s_child[2 * t + side];
-      B.T.child[2 * ((size_t)F + i) + side] = c;
-      put_box(B.T.cbox + 4 * ((size_t)F + i) + 2 * side, c);
-      export_kids(c);
+      const uint32_t ch = side ? S.child[t].y : S.child[t].x;
+      B.T.child[2 * ((size_t)F + i) + side] = ch;
+      put_box(B.T.cbox + 4 * ((size_t)F + i) + 2 * side, ch);
+      export_kids(ch);
+    }
+    if (record) {  // the references and the zeros (the record's last 32 bytes)
+      float4* rec = B.crec + 8 * ((size_t)F + i);
+      const uint2 ch = S.child[t];
+      const SlotPair L = chunk_pair(B.leaf_max, S, s, l, i, ch.x, src.x), R = chunk_pair(B.leaf_max, S, s, i + 1, r, ch.y, src.y);
+      rec[6] = make_float4(__uint_as_float(L.ref0), __uint_as_float(L.ref1), __uint_as_float(R.ref0), __uint_as_float(R.ref1));
+      rec[7] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
   } else if (i == e && i + 1 < n) {
     B.T.other[(size_t)F + i] = 0u;
@@ -318,6 +360,28 @@ __global__ __launch_bounds__(kClusterChunk, 4) void k_cluster_chunk(ClusterBuild
       export_kids(fr.x);
     }
   }
+  const uint32_t who = __ballot_sync(0xffffffffu, record);
+  uint32_t base = 0;
+  if (lane == 0 && who) base = atomicAdd(&S.records, (uint32_t)__popc(who));
+  base = __shfl_sync(0xffffffffu, base, 0);
+  uint2* s_src = (uint2*)S.list[0];
+  if (record) {
+    const uint32_t q = base + __popc(who & ((1u << lane) - 1u));
+    s_src[q] = src;
+    S.list[2][q] = i;
+  }
+  __syncthreads();
+  const float* box = (const float*)S.box;
+  const float qnan = __int_as_float(0x7fffffff);
+  const uint32_t parts = 6 * S.records;
+  for (uint32_t q = t; q < parts; q += kClusterChunk) {
+    const uint32_t k = q / 6u, part = q - 6u * k;
+    const float* b = box + part + (part >= 3 ? 1u : 0u);
+    const uint2 x = s_src[k];
+    const uint32_t x1 = x.x >> 16, x3 = x.y >> 16;
+    B.crec[8 * ((size_t)F + S.list[2][k]) + part] = make_float4(b[8 * (x.x & 0xffffu)], x1 == kNoBox ? qnan : b[8 * x1], b[8 * (x.y & 0xffffu)],
+                                                                x3 == kNoBox ? qnan : b[8 * x3]);
+  }
 }
 
 // The rest of the climb, from the frontier nodes, through global memory. Each arriving child stores its
@@ -325,28 +389,29 @@ __global__ __launch_bounds__(kClusterChunk, 4) void k_cluster_chunk(ClusterBuild
 // acquire-release order at device scope; the second arrival reads the sibling's box, completes the parent and
 // marks it (its range) for k_cluster_records.
 __global__ __launch_bounds__(128) void k_cluster_frontier(ClusterBuild B) {
-  const uint32_t f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= 2 * cluster_chunks(B.N, B.M)) return;
-  const uint4 fr = B.T.frontier[f];
+  const uint32_t f = blockIdx.x * blockDim.x + threadIdx.x, nodes = 2 * cluster_chunks(B.N, B.M);
+  if ((f & ~31u) >= nodes) return;
+  uint4 fr = make_uint4(0, 0, 0, 0);
+  if (f < nodes) fr = B.T.frontier[f];
+  uint32_t m, F, n, j;
+  mesh_of_chunk(B, (f & ~31u) >> 1, f >> 1, m, F, n, j);
   if (fr.w == 0) {
-    B.T.chain[(size_t)f * (kClusterChain + 1) + kClusterChain] = 0;
+    if (f < nodes) B.T.chain[(size_t)f * (kClusterChain + 1) + kClusterChain] = 0;
     return;
   }
-  uint32_t m, F, n, j;
-  mesh_of_chunk(B, f >> 1, m, F, n, j);
   const uint32_t* codes = B.codes + F;
   uint32_t cur = fr.x, l = fr.y, r = fr.z;
   const float4 b0 = B.T.fbox[2 * (size_t)f], b1 = B.T.fbox[2 * (size_t)f + 1];
   float3 mn = make_float3(b0.x, b0.y, b0.z), mx = make_float3(b1.x, b1.y, b1.z);
   uint32_t* chain = B.T.chain + (size_t)f * (kClusterChain + 1);
   uint32_t done = 0;  // nodes completed by this climb (listed in chain for k_cluster_records)
+  int level_l = level_before(codes, n, l), level_r = level_before(codes, n, r + 1);
   for (;;) {
-    if (l == 0 && r == n - 1) {
+    if (max(level_l, level_r) < 0) {
       finish_root(B, m, F, n, cur, mn, mx);
       break;
     }
-    const bool left_child = (l == 0) || (r != n - 1 && key_xor(__ldg(codes + r), __ldg(codes + r + 1), r) <
-                                                         key_xor(__ldg(codes + l - 1), __ldg(codes + l), l - 1));
+    const bool left_child = level_r > level_l;
     const uint32_t p = left_child ? r : l - 1;
     const uint32_t side = left_child ? 0u : 1u;
     float4* slot = B.T.cbox + 4 * ((size_t)F + p);
@@ -356,13 +421,16 @@ __global__ __launch_bounds__(128) void k_cluster_frontier(ClusterBuild B) {
     cuda::atomic_ref<uint32_t, cuda::thread_scope_device> word(B.T.other[(size_t)F + p]);
     const uint32_t old = word.exchange((left_child ? l : r) + 1u, cuda::memory_order_acq_rel);
     if (old == 0) break;  // the sibling completes the parent
+    // the new flank's codes and the sibling's box come with one latency
     if (left_child) r = old - 1u; else l = old - 1u;
+    const int level = level_before(codes, n, left_child ? r + 1 : l);
     const float4 s0 = __ldcg(slot + 2 * (1 - side)), s1 = __ldcg(slot + 2 * (1 - side) + 1);
     mn = make_float3(fminf(mn.x, s0.x), fminf(mn.y, s0.y), fminf(mn.z, s0.z));
     mx = make_float3(fmaxf(mx.x, s1.x), fmaxf(mx.y, s1.y), fmaxf(mx.z, s1.z));
     B.T.prange[(size_t)F + p] = make_uint2(l, r + 1u);
     if (done < kClusterChain) chain[done++] = p;
     cur = p;
+    (left_child ? level_r : level_l) = level;
   }
   chain[kClusterChain] = done;
 }
@@ -375,12 +443,12 @@ __global__ __launch_bounds__(256) void k_cluster_records(ClusterBuild B) {
   const uint32_t done = chain[kClusterChain];
   if (done == 0) return;
   uint32_t m, F, n, j;
-  mesh_of_chunk(B, f >> 1, m, F, n, j);
+  mesh_of_chunk(B, f >> 1, f >> 1, m, F, n, j);
   for (uint32_t k = lane; k < done; k += 32) {
     const uint32_t p = chain[k];
     const uint2 pr = B.T.prange[(size_t)F + p];
     const uint32_t l = pr.x, r = pr.y - 1u;
-    if (r - l + 1 > B.leaf_max) write_record(B, GlobalNodes{&B.T, F}, B.crec + 8 * ((size_t)F + p), p, l, r);
+    if (r - l + 1 > B.leaf_max) write_record(B, F, p, l, r);
   }
 }
 
