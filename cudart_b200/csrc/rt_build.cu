@@ -44,8 +44,8 @@
 namespace rt {
 namespace {
 
-constexpr int kTopoThreads = 1024;
-constexpr int kTopoWarps = kTopoThreads / 32;
+constexpr int kTopoThreads = 1024;      // of the one CTA of a single build
+constexpr int kBatchTopoThreads = 512;  // of a mesh's CTA of a batched build
 
 // ----------------------------------------------------------------------------
 // hit box (when the caller gives none): min/max over all vertices
@@ -192,10 +192,190 @@ struct TopoArgs {
   uint32_t pos_base;            // first position of this mesh (0 for a single mesh)
 };
 
+// Morton levels whose nodes fit in shared memory: kTopoNodeBytes each, `cap` of them. False, with nothing written, if
+// there are more (topo_morton then does it in global memory). Level by level down, with the split lists' first cap / 2
+// entries beside the nodes; leaf counts up; ranks and the records down, where a node's counts make room for its rank.
+// One CTA, so all of it is latency: going down a level is one barrier and a binary search of a short list. (With every array
+// in global memory the same levels took 81 us for 2^20 faces (4096 cells), 62 for a terrain of 32k and 314 for 1024
+// meshes; now 38, 32 and 200.)
+constexpr uint32_t kTopoNodeBytes = 26;
+constexpr uint32_t kTopoNodes = 8192;        // of a single build: every tree of depth 12 or less fits
+constexpr uint32_t kBatchTopoNodes = 2560;   // of a batched build: 65 KB, three CTAs an SM
+template <int NT>
+__device__ __forceinline__ bool topo_shared(const TopoArgs& A, const uint32_t cap, char* smem) {
+  uint32_t* const ra = (uint32_t*)smem;
+  uint32_t* const rb = ra + cap;
+  uint32_t* const cnt = rb + cap;     // leaves of the subtree; going down, the pre-order rank
+  uint32_t* const lambda = cnt + cap;
+  uint32_t* const id = lambda + cap;
+  uint32_t* const C = id + cap;       // [cap / 2]
+  uint16_t* const child = (uint16_t*)(C + cap / 2);  // 0: none
+  uint16_t* const mcnt = child + cap;                // Morton leaves of the subtree; going down, the ordinal
+  __shared__ uint32_t s_start[34], s_last[32];   // per level: its list's start and last entry (0: empty, above no a)
+  __shared__ uint32_t s_vstar[34], s_made[33];   // per level: the a of its first visit at or after s_last; nodes made below it
+  __shared__ uint32_t s_level_lo[34];
+  __shared__ uint32_t s_over, s_overrun, s_nondet, s_past, s_err, s_depth, s_leaves, s_mleaves;
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, D = A.D;
+  if (tid < 32) {
+    const uint32_t v = A.level_hist ? A.level_hist[tid] : A.lev_count[tid];
+    uint32_t x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= (uint32_t)o) x += y;
+    }
+    const uint32_t start = (A.level_hist ? A.level_base : 0u) + x - v;
+    s_start[tid] = start;
+    s_last[tid] = v ? __ldg(A.C + start + v - 1) : 0u;
+    s_vstar[tid] = kNone;
+    s_made[tid] = 0;
+    if (tid == 31) s_start[32] = s_start[33] = start + v;
+    if (tid == 0) {
+      s_vstar[32] = s_vstar[33] = kNone;
+      s_made[32] = 0;
+      s_over = s_overrun = s_nondet = s_past = s_err = s_depth = 0;
+      ra[0] = A.pos_base;
+      rb[0] = A.pos_base + A.n;
+    }
+  }
+  __syncthreads();
+  const uint32_t first = s_start[0], S = s_start[32], held = min(S - first, cap / 2);
+  for (uint32_t i = tid; i < held; i += NT) C[i] = __ldg(A.C + first + i);
+  // a node of level L that is visited, at or after the level's last entry
+  auto note = [&](uint32_t L, uint32_t a, uint32_t b) {
+    if (L < 32 && b - a >= A.min_leaf && a >= s_last[L]) atomicMin(&s_vstar[L], a);
+  };
+  if (tid == 0) note(0, A.pos_base, A.pos_base + A.n);
+  __syncthreads();
+  // first index at or after level L's list whose entry s is above a (the lists are walked in order), S and kNone if none
+  auto scan = [&](uint32_t L, uint32_t a, uint32_t& s) {
+    for (uint32_t l = L; l < 32; ++l) {
+      if (s_last[l] <= a) continue;
+      uint32_t lo = s_start[l], hi = s_start[l + 1] - 1;
+      s = s_last[l];
+      while (lo < hi) {
+        const uint32_t mid = (lo + hi) >> 1, x = mid - first < held ? C[mid - first] : __ldg(A.C + mid);
+        if (x > a) { hi = mid; s = x; } else lo = mid + 1;
+      }
+      return lo;
+    }
+    s = kNone;
+    return S;
+  };
+  // A level's nodes stand in any order: a visit's place among the level's visits is its a. So children are handed their
+  // slots by a counter, and a level takes one barrier.
+  uint32_t lo = 0, hi = 1, L = 0;
+  for (; lo < hi; ++L) {
+    if (tid == 0) s_level_lo[L] = lo;
+    const bool visits = L < D && L < 32 && s_start[L] < s_start[L + 1];
+    const uint32_t vstar = visits ? s_vstar[L] : kNone;
+    // the pointer sticks at the next list's start if that entry, or the end, is what the first visit at or after s_last finds
+    bool stuck = false;
+    if (vstar != kNone) {
+      const uint32_t j = s_start[L + 1];
+      stuck = j == S || (j - first < held ? C[j - first] : __ldg(A.C + j)) > vstar;
+    }
+    for (uint32_t base = lo; base < hi; base += NT) {
+      const uint32_t i = base + tid;
+      bool internal = false;
+      uint32_t a = 0, b = 0, s = 0;
+      if (i < hi) {
+        a = ra[i]; b = rb[i];
+        if (visits && b - a >= A.min_leaf && !(stuck && a > vstar)) {
+          const uint32_t j = scan(L, a, s);
+          internal = s < b;
+          if (j >= s_start[L + 1]) atomicAdd(&s_overrun, 1u);
+          if (j < S && j >= s_start[min(D + 1, 32u)]) atomicAdd(&s_nondet, 1u);
+          if (j == S) atomicAdd(&s_past, 1u);
+        }
+      }
+      const uint32_t who = __ballot_sync(0xffffffffu, internal);
+      uint32_t c = 0;
+      if (who) {
+        if (lane == 0) c = atomicAdd(&s_made[L], 2u * (uint32_t)__popc(who));
+        c = hi + __shfl_sync(0xffffffffu, c, 0) + 2u * (uint32_t)__popc(who & ((1u << lane) - 1u));
+      }
+      if (internal) {
+        if (c + 2 > min(cap, A.cap_m)) {
+          s_over = 1;
+        } else {
+          ra[c] = a; rb[c] = s; ra[c + 1] = s; rb[c + 1] = b;
+          note(L + 1, a, s);
+          note(L + 1, s, b);
+        }
+      }
+      if (i < hi) child[i] = (uint16_t)(internal ? c : 0u);
+    }
+    __syncthreads();
+    if (s_over) return false;
+    lo = hi;
+    hi += s_made[L];
+  }
+  if (tid == 0) s_level_lo[L] = lo;
+  __syncthreads();
+  const uint32_t levels = L, maxl = A.max_leaf;
+  auto median = [&](uint32_t size) { return A.complete && size > maxl; };
+  for (int l = (int)levels - 1; l >= 0; --l) {
+    for (uint32_t i = s_level_lo[l] + tid; i < s_level_lo[l + 1]; i += NT) {
+      const uint32_t c = child[i], size = rb[i] - ra[i];
+      cnt[i] = c ? cnt[c] + cnt[c + 1] : median(size) ? median_leaves(size, maxl) : 1u;
+      mcnt[i] = c ? (uint16_t)(mcnt[c] + mcnt[c + 1]) : (uint16_t)1u;
+    }
+    __syncthreads();
+  }
+  if (tid == 0) {
+    s_leaves = cnt[0]; s_mleaves = mcnt[0];
+    cnt[0] = lambda[0] = id[0] = 0;
+    mcnt[0] = 0;
+    if (A.max_nodes) A.parent_id[0] = kNone;
+  }
+  __syncthreads();
+  uint32_t depth = 0, err = 0;
+  for (uint32_t l = 0; l < levels; ++l) {
+    for (uint32_t i = s_level_lo[l] + tid; i < s_level_lo[l + 1]; i += NT) {
+      const uint32_t c = child[i], nid = id[i], r = cnt[i], lam = lambda[i], o = mcnt[i];
+      const bool fits = nid < A.max_nodes;
+      if (!fits) err = RT_DEVERR_NODE_CAPACITY;
+      if (c) {
+        const uint32_t ll = cnt[c], ml = mcnt[c];
+        cnt[c] = r + 1; lambda[c] = lam; id[c] = 2 * r + 1; mcnt[c] = (uint16_t)o;
+        cnt[c + 1] = r + ll; lambda[c + 1] = lam + ll; id[c + 1] = 2 * r + 2; mcnt[c + 1] = (uint16_t)(o + ml);
+        if (2 * r + 1 < A.max_nodes) A.parent_id[2 * r + 1] = nid;
+        if (2 * r + 2 < A.max_nodes) A.parent_id[2 * r + 2] = nid;
+        if (fits) *(uint2*)(A.nodes + 8 * (size_t)nid) = make_uint2((l % 3u) << 1, 2 * r + 1);
+      } else if (fits) {
+        const uint32_t size = rb[i] - ra[i];
+        const bool med = median(size);
+        A.ml_lambda[o] = lam;
+        A.ml_rec[o] = make_uint4(nid, ra[i], size, l | (med ? 0x80000000u : 0u));
+        A.ml_rank[o] = r;
+        depth = max(depth, l + (med ? median_depth(size, maxl) : 0u) + 1u);
+      }
+    }
+    __syncthreads();
+  }
+  if (depth) atomicMax(&s_depth, depth);
+  if (err) atomicOr(&s_err, err);
+  __syncthreads();
+  if (tid == 0) {
+    A.hdr[0] = s_leaves;
+    A.hdr[1] = s_mleaves;
+    A.hdr[2] = 2 * s_leaves - 1;
+    A.hdr[3] = s_depth;
+    A.hdr[4] = S - first;
+    A.hdr[5] = s_overrun;
+    A.hdr[6] = s_nondet;
+    A.hdr[7] = s_past;
+    A.hdr[8] = s_err | ((2 * s_leaves - 1 > A.max_nodes) ? (uint32_t)RT_DEVERR_NODE_CAPACITY : 0u);
+  }
+  return true;
+}
+
+template <int NT>
 __device__ __forceinline__ void topo_morton(const TopoArgs& A) {
   __shared__ uint32_t s_start[34];
   __shared__ uint32_t s_level_lo[34];
-  __shared__ uint32_t s_warp[kTopoWarps];
+  __shared__ uint32_t s_warp[NT / 32];
   __shared__ uint32_t s_vstar, s_stuck, s_levels;
   __shared__ uint32_t s_overrun, s_nondet, s_past, s_err, s_depth;
   const uint32_t tid = threadIdx.x;
@@ -221,7 +401,7 @@ __device__ __forceinline__ void topo_morton(const TopoArgs& A) {
     const bool nonempty = L < 32 && s_start[L] < s_start[L + 1];
     const uint32_t lastL = nonempty ? __ldg(A.C + s_start[L + 1] - 1) : 0u;
     if (nonempty && L < D) {
-      for (uint32_t i = lo + tid; i < hi; i += kTopoThreads) {
+      for (uint32_t i = lo + tid; i < hi; i += NT) {
         uint32_t a = A.ra[i], b = A.rb[i];
         if (b - a >= A.min_leaf && a >= lastL) atomicMin(&s_vstar, i);
       }
@@ -233,7 +413,7 @@ __device__ __forceinline__ void topo_morton(const TopoArgs& A) {
     }
     __syncthreads();
     uint32_t running = hi;
-    for (uint32_t base = lo; base < hi; base += kTopoThreads) {
+    for (uint32_t base = lo; base < hi; base += NT) {
       const uint32_t i = base + tid;
       bool internal = false;
       uint32_t a = 0, b = 0, s = 0, inf = 0;
@@ -252,7 +432,7 @@ __device__ __forceinline__ void topo_morton(const TopoArgs& A) {
         inf = L | (internal ? 0x100u : 0u) | (median ? 0x200u : 0u);
       }
       uint32_t total;
-      uint32_t ex = block_excl_scan_nt<kTopoThreads>(internal ? 2u : 0u, s_warp, total);
+      uint32_t ex = block_excl_scan_nt<NT>(internal ? 2u : 0u, s_warp, total);
       if (i < hi) {
         uint32_t c = kNone;
         if (internal) {
@@ -284,7 +464,7 @@ __device__ __forceinline__ void topo_morton(const TopoArgs& A) {
 
   // bottom-up: leaves (final tree) and Morton leaves per subtree
   for (int l = (int)levels - 1; l >= 0; --l) {
-    for (uint32_t i = s_level_lo[l] + tid; i < s_level_lo[l + 1]; i += kTopoThreads) {
+    for (uint32_t i = s_level_lo[l] + tid; i < s_level_lo[l + 1]; i += NT) {
       uint32_t inf = A.info[i];
       if (inf & 0x100u) {
         uint32_t c = A.child[i];
@@ -302,7 +482,7 @@ __device__ __forceinline__ void topo_morton(const TopoArgs& A) {
   if (tid == 0) { A.rank[0] = 0; A.lambda[0] = 0; A.ord[0] = 0; A.id[0] = 0; }
   __syncthreads();
   for (uint32_t l = 0; l < levels; ++l) {
-    for (uint32_t i = s_level_lo[l] + tid; i < s_level_lo[l + 1]; i += kTopoThreads) {
+    for (uint32_t i = s_level_lo[l] + tid; i < s_level_lo[l + 1]; i += NT) {
       if (A.info[i] & 0x100u) {
         uint32_t c = A.child[i];
         uint32_t r = A.rank[i], lam = A.lambda[i], o = A.ord[i];
@@ -315,7 +495,7 @@ __device__ __forceinline__ void topo_morton(const TopoArgs& A) {
   }
   // emit Morton node records and the Morton-leaf table
   const uint32_t total_m = s_level_lo[levels];
-  for (uint32_t i = tid; i < total_m; i += kTopoThreads) {
+  for (uint32_t i = tid; i < total_m; i += NT) {
     const uint32_t inf = A.info[i];
     const uint32_t lvl = inf & 0xFFu;
     const uint32_t nid = A.id[i];
@@ -350,7 +530,13 @@ __device__ __forceinline__ void topo_morton(const TopoArgs& A) {
   }
 }
 
-__global__ __launch_bounds__(kTopoThreads) void k_topo_morton(TopoArgs A) { topo_morton(A); }
+__global__ __launch_bounds__(kTopoThreads) void k_topo_morton(TopoArgs A) {
+  extern __shared__ __align__(16) char topo_smem[];
+  if (!topo_shared<kTopoThreads>(A, kTopoNodes, topo_smem)) {
+    __syncthreads();
+    topo_morton<kTopoThreads>(A);
+  }
+}
 
 // ----------------------------------------------------------------------------
 // leaves: a warp takes 32 consecutive leaves at a time
@@ -777,6 +963,15 @@ int resident_blocks_of(K kernel, int threads) {
   return nb;
 }
 
+// Lets a topology kernel (one instance each) have the shared memory of `nodes` nodes; once per device.
+template <typename K>
+bool topo_smem_once(K kernel, uint32_t nodes) {
+  static PerDeviceOnce once;
+  return once.run([&] {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(nodes * kTopoNodeBytes)) == cudaSuccess;
+  });
+}
+
 }  // namespace
 
 SideStream* side_stream() {
@@ -901,7 +1096,8 @@ extern "C" rt_status rt_lbvh_build(const rt_build_desc* d, rt_stream stream_) {
     A.ml_lambda = L.ml_lambda; A.ml_rec = L.ml_rec; A.ml_rank = L.ml_rank; A.parent_id = L.parent_id;
     A.nodes = d->nodes; A.max_nodes = d->max_nodes; A.hdr = L.hdr;
     A.level_hist = nullptr; A.level_base = 0; A.pos_base = 0;
-    k_topo_morton<<<1, kTopoThreads, 0, st>>>(A);
+    if (!topo_smem_once(k_topo_morton, kTopoNodes)) return RT_ERR_CUDA;
+    k_topo_morton<<<1, kTopoThreads, kTopoNodes * kTopoNodeBytes, st>>>(A);
     note_launch();
     RT_CHECK_LAUNCH();
   }
@@ -1144,7 +1340,8 @@ __global__ __launch_bounds__(256) void k_batch_boxes_morton(BatchArgs B) {
   }
 }
 
-__global__ __launch_bounds__(kTopoThreads) void k_batch_topo(BatchArgs B) {
+__global__ __launch_bounds__(kBatchTopoThreads, 3) void k_batch_topo(BatchArgs B) {
+  extern __shared__ __align__(16) char topo_smem[];
   const uint32_t m = blockIdx.x;
   const uint32_t F = B.foff[m], n = B.foff[m + 1] - F;
   const uint32_t bb = bfs_base(F, m), nb = node_base(F, m);
@@ -1157,11 +1354,14 @@ __global__ __launch_bounds__(kTopoThreads) void k_batch_topo(BatchArgs B) {
   A.parent_id = B.parent_id + nb; A.nodes = B.nodes + 8 * (size_t)nb; A.max_nodes = 2 * n - 1; A.hdr = B.hdr + 16 * m;
   // the meshes before m hold F positions, so this mesh's level lists start at F
   A.level_hist = B.hist + 64 * m; A.level_base = F; A.pos_base = F;
-  topo_morton(A);
+  if (!topo_shared<kBatchTopoThreads>(A, kBatchTopoNodes, topo_smem)) {
+    __syncthreads();
+    topo_morton<kBatchTopoThreads>(A);
+  }
   // the CTA that finishes last (every other mesh's header is written) makes the leaf-order bases per mesh (an
   // exclusive scan of the leaf counts) and their total; nothing waits for it inside this kernel
   __shared__ uint32_t s_last;
-  __shared__ uint32_t s_warp2[kTopoWarps];
+  __shared__ uint32_t s_warp2[kBatchTopoThreads / 32];
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
@@ -1171,12 +1371,12 @@ __global__ __launch_bounds__(kTopoThreads) void k_batch_topo(BatchArgs B) {
   if (!s_last) return;
   __threadfence();
   uint32_t running = 0;
-  for (uint32_t c = 0; c < B.M; c += kTopoThreads) {
+  for (uint32_t c = 0; c < B.M; c += kBatchTopoThreads) {
     const uint32_t i = c + threadIdx.x;
     const uint32_t bad = i < B.M ? (__ldcg(B.hdr + 16 * i + 8) & (RT_DEVERR_NODE_CAPACITY | RT_DEVERR_MORTON_CAPACITY)) : 0u;
     const uint32_t v = (i < B.M && !bad) ? __ldcg(B.hdr + 16 * i) : 0u;
     uint32_t tot;
-    const uint32_t ex = block_excl_scan_nt<kTopoThreads>(v, s_warp2, tot);
+    const uint32_t ex = block_excl_scan_nt<kBatchTopoThreads>(v, s_warp2, tot);
     if (i < B.M) B.leaf_base[i] = running + ex;
     running += tot;
   }
@@ -1368,7 +1568,8 @@ extern "C" rt_status rt_batch_build(const rt_batch_build_desc* d, rt_stream stre
   if (s != RT_OK) return s;
   s = sort_split_levels(B.codes, N, B.C, B.hist, 64, sort_scratch, sort_bytes, st, B.foff, M);
   if (s != RT_OK) return s;
-  k_batch_topo<<<M, kTopoThreads, 0, st>>>(B);
+  if (!topo_smem_once(k_batch_topo, kBatchTopoNodes)) return RT_ERR_CUDA;
+  k_batch_topo<<<M, kBatchTopoThreads, kBatchTopoNodes * kTopoNodeBytes, st>>>(B);
   note_launch();
   RT_CHECK_LAUNCH();
   if (cudaMemsetAsync(B.arrive, 0, (2 * (size_t)N) * 4, st) != cudaSuccess) return RT_ERR_CUDA;
