@@ -189,6 +189,8 @@ struct LevelArgs {
   uint4* big_next;        // (table index, faces, first) of the next level's big nodes
   const uint32_t* big_cur;  // table indices of this level's big nodes handled one CTA each
   uint32_t level_begin, level_end;
+  uint32_t* range;        // a level of a run without waits: range[step], range[step + 1] instead of level_begin, level_end
+  uint32_t step;
   const uint32_t* idx_in;
   const Item* box_in;
   uint32_t* idx_out;
@@ -270,12 +272,8 @@ __device__ __forceinline__ void cta_partition(const LevelArgs& A, const Split& s
   }
 }
 
-// One warp per node of at most kBigNode faces (8 warps per CTA).
-__global__ __launch_bounds__(kCta) void k_sah_small(LevelArgs A) {
-  __shared__ Bins s_bins[kCta / 32];
-  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-  const uint32_t e = A.level_begin + blockIdx.x * (kCta / 32) + warp;
-  if (e >= A.level_end) return;
+// A node of at most kBigNode faces, by one warp.
+__device__ __forceinline__ void sah_small_node(const LevelArgs& A, const uint32_t e, Bins& B, const uint32_t lane) {
   const SNode nd = A.table[e];
   if (nd.count > kBigNode) return;
   if (nd.count <= kSahMinLeaf) {
@@ -299,7 +297,6 @@ __global__ __launch_bounds__(kCta) void k_sah_small(LevelArgs A) {
                       omax(cmx.z, __shfl_xor_sync(0xffffffffu, cmx.z, o)));
   }
   const Split sp = make_split(cmn, cmx);
-  Bins& B = s_bins[warp];
   bins_reset(B, (int)lane);
   __syncwarp();
   for (uint32_t i = lane; i < nd.count; i += 32) {
@@ -342,6 +339,28 @@ __global__ __launch_bounds__(kCta) void k_sah_small(LevelArgs A) {
     }
     lo += __popc(lb);
     ro += __popc(rb);
+  }
+}
+
+// A warp per node of at most kBigNode faces (8 warps per CTA). With A.range, one of kRunLevels launches that follow one
+// another without the host in between (no node above kBigNode is left): the CTA that finishes last writes where the
+// next but one level ends, which nothing in this launch reads.
+constexpr uint32_t kRunLevels = 6;
+constexpr uint32_t kRunDone = 16;  // range: kRunLevels + 2 bounds, then from here the launches' CTA counters
+__global__ __launch_bounds__(kCta) void k_sah_small(LevelArgs A) {
+  __shared__ Bins s_bins[kCta / 32];
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+  const uint32_t begin = A.range ? A.range[A.step] : A.level_begin, end = A.range ? A.range[A.step + 1] : A.level_end;
+  for (uint32_t e = begin + blockIdx.x * (kCta / 32) + warp; e < end; e += gridDim.x * (kCta / 32)) {
+    sah_small_node(A, e, s_bins[warp], lane);
+    __syncwarp();
+  }
+  if (!A.range) return;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(A.range + kRunDone + A.step, 1u) == gridDim.x - 1)
+      A.range[A.step + 2] = min(atomicAdd(A.table_count, 0u), A.table_cap);
   }
 }
 
@@ -644,29 +663,49 @@ __global__ __launch_bounds__(256) void k_hyb_roots(const uint32_t* __restrict__ 
 }
 
 // ---------------------------------------------------------------- numbering
+__device__ __forceinline__ void sah_internal(SNode* table, uint32_t i) {
+  SNode& x = table[i];
+  x.internal = ((x.info & 2u) || x.child == kNone) ? 0u : 1u + table[x.child].internal + table[x.child + 1].internal;
+}
 __global__ __launch_bounds__(256) void k_sah_internal(SNode* table, uint32_t b, uint32_t e) {
-  for (uint32_t i = b + blockIdx.x * blockDim.x + threadIdx.x; i < e; i += gridDim.x * blockDim.x) {
-    SNode& x = table[i];
-    x.internal = ((x.info & 2u) || x.child == kNone) ? 0u : 1u + table[x.child].internal + table[x.child + 1].internal;
-  }
+  for (uint32_t i = b + blockIdx.x * blockDim.x + threadIdx.x; i < e; i += gridDim.x * blockDim.x) sah_internal(table, i);
 }
 // subtree bases: base[j] = first + 2 * (splits of subtrees 0..j-1) (inclusive scan input 2 * internal)
 __global__ __launch_bounds__(256) void k_sah_base_in(const SNode* table, uint32_t roots, uint32_t* v) {
   for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < roots; j += gridDim.x * blockDim.x) v[j] = 2u * table[j].internal;
 }
+// The levels at the top of the tree (few nodes each), level after level in one CTA: a launch per level is mostly launch.
+constexpr uint32_t kTopLevels = 24;
+constexpr uint32_t kTopNodes = 4096;
+struct TopLevels {
+  uint32_t start[kTopLevels + 1], n;
+};
+__global__ __launch_bounds__(1024) void k_sah_internal_top(SNode* table, TopLevels T) {
+  for (uint32_t l = T.n; l-- > 0;) {
+    for (uint32_t i = T.start[l] + threadIdx.x; i < T.start[l + 1]; i += blockDim.x) sah_internal(table, i);
+    __syncthreads();
+  }
+}
 // top-down: rank = pre-order index of a split node among its subtree's splits
+__device__ __forceinline__ void sah_rank(SNode* table, uint32_t i, uint32_t* rank, const uint32_t* base, uint32_t first_base) {
+  SNode& x = table[i];
+  if (x.parent == kNone) {
+    rank[i] = 0;
+    return;
+  }
+  const SNode& p = table[x.parent];
+  const uint32_t rp = rank[x.parent];
+  rank[i] = (x.info & 1u) ? rp + 1u + table[p.child].internal : rp + 1u;
+  x.id = first_base + base[x.sub] + 2u * rp + (x.info & 1u);
+}
 __global__ __launch_bounds__(256) void k_sah_rank(SNode* table, uint32_t b, uint32_t e, uint32_t* rank, const uint32_t* base,
                                                   uint32_t first_base) {
-  for (uint32_t i = b + blockIdx.x * blockDim.x + threadIdx.x; i < e; i += gridDim.x * blockDim.x) {
-    SNode& x = table[i];
-    if (x.parent == kNone) {
-      rank[i] = 0;
-      continue;
-    }
-    const SNode& p = table[x.parent];
-    const uint32_t rp = rank[x.parent];
-    rank[i] = (x.info & 1u) ? rp + 1u + table[p.child].internal : rp + 1u;
-    x.id = first_base + base[x.sub] + 2u * rp + (x.info & 1u);
+  for (uint32_t i = b + blockIdx.x * blockDim.x + threadIdx.x; i < e; i += gridDim.x * blockDim.x) sah_rank(table, i, rank, base, first_base);
+}
+__global__ __launch_bounds__(1024) void k_sah_rank_top(SNode* table, TopLevels T, uint32_t* rank, const uint32_t* base, uint32_t first_base) {
+  for (uint32_t l = 0; l < T.n; ++l) {
+    for (uint32_t i = T.start[l] + threadIdx.x; i < T.start[l + 1]; i += blockDim.x) sah_rank(table, i, rank, base, first_base);
+    __syncthreads();
   }
 }
 __global__ __launch_bounds__(256) void k_sah_write(const SNode* table, uint32_t count, const uint32_t* rank, const uint32_t* base,
@@ -781,12 +820,14 @@ int sm_count() {
 
 struct SahLayout {
   uint32_t *idx_a, *idx_b, *lists, *counts, *rank, *base, *marks, *sums, *scalars, *keys, *err, *leaf_lambda;
-  uint4 *big_a, *big_b;
+  uint4* big;       // right behind counts
+  uint32_t* range;
   uint32_t *h_keys, *h_child, *h_tbins, *h_tleft;
   Bins* h_bins;
   Decision* h_dec;
   Split* h_split;
   uint32_t h_cap, t_cap;
+  size_t lists_cap;
   Item *box_a, *box_b;
   SNode* table;
   rt_build_info* lb_info;
@@ -803,12 +844,16 @@ size_t carve_sah(Carve& c, SahLayout& L, uint32_t n, uint32_t lbvh_depth, uint32
   L.idx_b = c.take<uint32_t>(n);
   L.box_a = c.take<Item>(n);
   L.box_b = c.take<Item>(n);
-  L.big_a = c.take<uint4>(n / kBigNode + 2);
-  L.big_b = c.take<uint4>(n / kBigNode + 2);
   L.h_cap = n / kHugeNode + 2;
   L.t_cap = n / kTile + L.h_cap + 2;
   // a level's lists, uploaded together: the nodes of one CTA, the huge nodes and their first tiles, the tiles' nodes and starts
-  L.lists = c.take<uint32_t>((size_t)n / kBigNode + 2 + 2 * (size_t)L.h_cap + 2 * (size_t)L.t_cap);
+  // right behind the lists' end the counts, so that a level's upload sets them, and then the level's new big nodes, so that
+  // one copy reads both
+  L.lists_cap = align_up((size_t)n / kBigNode + 2 + 2 * (size_t)L.h_cap + 2 * (size_t)L.t_cap, 4);
+  L.lists = c.take<uint32_t>(L.lists_cap + 4 * (1 + (size_t)n / kBigNode + 2));
+  L.counts = L.lists ? L.lists + L.lists_cap : nullptr;
+  L.big = (uint4*)(L.counts ? L.counts + 4 : nullptr);
+  L.range = c.take<uint32_t>(32);
   L.h_keys = c.take<uint32_t>(8 * (size_t)L.h_cap);
   L.h_child = c.take<uint32_t>(L.h_cap);
   L.h_bins = c.take<Bins>(L.h_cap);
@@ -816,7 +861,6 @@ size_t carve_sah(Carve& c, SahLayout& L, uint32_t n, uint32_t lbvh_depth, uint32
   L.h_split = c.take<Split>(L.h_cap);
   L.h_tbins = c.take<uint32_t>((size_t)L.t_cap * kBins);
   L.h_tleft = c.take<uint32_t>(L.t_cap);
-  L.counts = c.take<uint32_t>(8);
   L.table = c.take<SNode>(L.table_cap);
   L.rank = c.take<uint32_t>(L.table_cap);
   L.base = c.take<uint32_t>(n + 2);
@@ -891,7 +935,7 @@ extern "C" rt_status rt_sah_build(const rt_sah_desc* d, rt_stream stream) {
   const uint32_t grid = (uint32_t)hmin<uint64_t>((n + 255) / 256, (uint64_t)sms * 8);
   float* hit = (float*)L.scalars;  // 8 floats, then reused
   if (cudaMemsetAsync(L.err, 0, 4, st) != cudaSuccess) return RT_ERR_CUDA;
-  if (cudaMemsetAsync(L.counts, 0, 32, st) != cudaSuccess) return RT_ERR_CUDA;
+  if (cudaMemsetAsync(L.counts, 0, 16, st) != cudaSuccess) return RT_ERR_CUDA;
   uint32_t first_base = 1, roots = 1;
   if (d->lbvh_depth == 0) {
     rt_status s = rt_mesh_boxes(d->vertices, d->faces_in, n, d->boxes, d->indices, stream);
@@ -910,10 +954,6 @@ extern "C" rt_status rt_sah_build(const rt_sah_desc* d, rt_stream stream) {
     }
     k_sah_init<<<grid, 256, 0, st>>>((const float4*)d->boxes, n, hit, L.idx_a, L.box_a, L.table, L.counts);
     note_launch();
-    if (n > kBigNode) {
-      const uint4 root = make_uint4(0u, n, 0u, 0u);
-      if (cudaMemcpyAsync(L.big_a, &root, 16, cudaMemcpyHostToDevice, st) != cudaSuccess) return RT_ERR_CUDA;
-    }
   } else {
     rt_build_desc b = {};
     b.vertices = d->vertices; b.vertex_count = d->vertex_count; b.face_count = n; b.faces_in = d->faces_in;
@@ -935,7 +975,7 @@ extern "C" rt_status rt_sah_build(const rt_sah_desc* d, rt_stream stream) {
     excl_scan(L.marks, m, L.sums, nullptr, st);
     const uint32_t init[3] = {roots, 0, 0};
     if (cudaMemcpyAsync(L.counts, init, 12, cudaMemcpyHostToDevice, st) != cudaSuccess) return RT_ERR_CUDA;
-    k_hyb_roots<<<(m + 255) / 256, 256, 0, st>>>(d->nodes, m, L.marks, L.table, L.big_a, L.counts);
+    k_hyb_roots<<<(m + 255) / 256, 256, 0, st>>>(d->nodes, m, L.marks, L.table, L.big, L.counts);
     note_launch();
   }
   RT_CHECK_LAUNCH();
@@ -943,22 +983,54 @@ extern "C" rt_status rt_sah_build(const rt_sah_desc* d, rt_stream stream) {
   // levels
   std::vector<uint32_t> level_start;
   uint32_t begin = 0, end = roots;
-  uint32_t host_counts[3];
-  if (cudaMemcpyAsync(host_counts, L.counts, 12, cudaMemcpyDeviceToHost, st) != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess)
-    return RT_ERR_CUDA;
-  uint32_t nbig = host_counts[1];
   uint32_t* idx_in = L.idx_a;
   uint32_t* idx_out = L.idx_b;
   Item* box_in = L.box_a;
   Item* box_out = L.box_b;
-  uint4* big_cur = L.big_a;
-  uint4* big_next = L.big_b;
-  std::vector<uint4> bigs(nbig);
-  if (nbig && (cudaMemcpyAsync(bigs.data(), big_cur, (size_t)nbig * 16, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-               cudaStreamSynchronize(st) != cudaSuccess))
+  // `back`: the counts, then the level's big nodes, read together
+  std::vector<uint4> bigs, back;
+  auto read_back = [&](size_t most) {
+    back.resize(1 + most);
+    if (cudaMemcpyAsync(back.data(), L.counts, back.size() * 16, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        cudaStreamSynchronize(st) != cudaSuccess || back[0].y > most)
+      return false;
+    bigs.assign(back.begin() + 1, back.begin() + 1 + back[0].y);
+    return true;
+  };
+  if (!d->lbvh_depth) {
+    back.push_back(make_uint4(1u, 0u, 0u, 0u));
+    if (n > kBigNode) bigs.push_back(make_uint4(0u, n, 0u, 0u));
+  } else if (!read_back(n / kBigNode + 1)) {
     return RT_ERR_CUDA;
+  }
   std::vector<uint32_t> regular, h_node, h_tfirst, t_node, t_start;
   while (begin < end) {
+    if (bigs.empty()) {
+      // only nodes of at most kBigNode faces are left, and so below: kRunLevels levels with one wait at their end (a
+      // wait and the copies around it take 25 us). A level that has nothing to do costs its launch.
+      uint32_t run[32] = {begin, end};
+      if (cudaMemcpyAsync(L.range, run, sizeof(run), cudaMemcpyHostToDevice, st) != cudaSuccess) return RT_ERR_CUDA;
+      LevelArgs A = {};
+      A.table = L.table; A.table_count = L.counts; A.big_next = L.big; A.range = L.range; A.final_idx = d->indices; A.err = L.err;
+      A.table_cap = L.table_cap;
+      uint64_t most = end - begin;
+      for (A.step = 0; A.step < kRunLevels; ++A.step) {
+        A.idx_in = idx_in; A.box_in = box_in; A.idx_out = idx_out; A.box_out = box_out;
+        k_sah_small<<<(uint32_t)hmin<uint64_t>((most + 7) / 8, (uint64_t)sms * 8), kCta, 0, st>>>(A);
+        most = hmin<uint64_t>(2 * most, L.table_cap);
+        std::swap(idx_in, idx_out);
+        std::swap(box_in, box_out);
+      }
+      note_launch(kRunLevels);
+      RT_CHECK_LAUNCH();
+      if (cudaMemcpyAsync(run, L.range, (kRunLevels + 2) * 4, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+          cudaStreamSynchronize(st) != cudaSuccess)
+        return RT_ERR_CUDA;
+      for (uint32_t l = 0; l < kRunLevels && run[l] < run[l + 1]; ++l) level_start.push_back(run[l]);
+      begin = run[kRunLevels];
+      end = run[kRunLevels + 1];
+      continue;
+    }
     level_start.push_back(begin);
     // this level's big nodes: a CTA each, or tiles of several CTAs when huge
     regular.clear(); h_node.clear(); h_tfirst.clear(); t_node.clear(); t_start.clear();
@@ -976,21 +1048,23 @@ extern "C" rt_status rt_sah_build(const rt_sah_desc* d, rt_stream stream) {
     }
     const uint32_t H = (uint32_t)h_node.size(), R = (uint32_t)regular.size(), tiles = (uint32_t)t_node.size();
     if (tiles > L.t_cap) return RT_ERR_CAPACITY;
-    if (cudaMemsetAsync(L.counts + 1, 0, 4, st) != cudaSuccess) return RT_ERR_CUDA;
-    if (!bigs.empty()) {  // one upload: [regular][h_node][h_tfirst][t_node][t_start]
-      regular.insert(regular.end(), h_node.begin(), h_node.end());
-      regular.insert(regular.end(), h_tfirst.begin(), h_tfirst.end());
-      regular.insert(regular.end(), t_node.begin(), t_node.end());
-      regular.insert(regular.end(), t_start.begin(), t_start.end());
-      if (cudaMemcpyAsync(L.lists, regular.data(), regular.size() * 4, cudaMemcpyHostToDevice, st) != cudaSuccess) return RT_ERR_CUDA;
-    }
-    LevelArgs A;
-    A.table = L.table; A.table_count = L.counts; A.big_next = big_next; A.big_cur = L.lists; A.level_begin = begin; A.level_end = end;
+    // one upload: [regular][h_node][h_tfirst][t_node][t_start] and the counts, of which the big nodes' starts again
+    regular.insert(regular.end(), h_node.begin(), h_node.end());
+    regular.insert(regular.end(), h_tfirst.begin(), h_tfirst.end());
+    regular.insert(regular.end(), t_node.begin(), t_node.end());
+    regular.insert(regular.end(), t_start.begin(), t_start.end());
+    if (regular.size() > L.lists_cap) return RT_ERR_CAPACITY;  // cannot happen
+    uint32_t* const lists = L.counts - regular.size();
+    const uint32_t counts[4] = {back[0].x, 0u, back[0].z, 0u};
+    regular.insert(regular.end(), counts, counts + 4);
+    if (cudaMemcpyAsync(lists, regular.data(), regular.size() * 4, cudaMemcpyHostToDevice, st) != cudaSuccess) return RT_ERR_CUDA;
+    LevelArgs A = {};
+    A.table = L.table; A.table_count = L.counts; A.big_next = L.big; A.big_cur = lists; A.level_begin = begin; A.level_end = end;
     A.idx_in = idx_in; A.box_in = box_in; A.idx_out = idx_out; A.box_out = box_out; A.final_idx = d->indices; A.err = L.err;
     A.table_cap = L.table_cap;
     if (H) {
       HugeArgs G;
-      G.node = L.lists + R; G.tfirst = G.node + H; G.tnode = G.tfirst + H; G.tstart = G.tnode + tiles;
+      G.node = lists + R; G.tfirst = G.node + H; G.tnode = G.tfirst + H; G.tstart = G.tnode + tiles;
       G.keys = L.h_keys; G.bins = L.h_bins;
       G.dec = L.h_dec; G.split = L.h_split; G.child = L.h_child; G.tbins = L.h_tbins; G.tleft = L.h_tleft; G.H = H; G.tiles = tiles;
       k_huge_reset<<<H, 64, 0, st>>>(G);
@@ -1010,38 +1084,35 @@ extern "C" rt_status rt_sah_build(const rt_sah_desc* d, rt_stream stream) {
     }
     RT_CHECK_LAUNCH();
     // one wait per level: the counts, and the next level's big nodes (at most two per big node of this one)
-    const uint32_t most = (uint32_t)hmin<size_t>(2 * bigs.size(), n / kBigNode + 1);
-    bigs.resize(most);
-    if (cudaMemcpyAsync(host_counts, L.counts, 12, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-        (most && cudaMemcpyAsync(bigs.data(), big_next, (size_t)most * 16, cudaMemcpyDeviceToHost, st) != cudaSuccess) ||
-        cudaStreamSynchronize(st) != cudaSuccess)
-      return RT_ERR_CUDA;
+    if (!read_back(hmin<size_t>(2 * bigs.size(), n / kBigNode + 1))) return RT_ERR_CUDA;
     begin = end;
-    end = host_counts[0] < L.table_cap ? host_counts[0] : L.table_cap;
-    if (host_counts[1] > most) return RT_ERR_CAPACITY;  // cannot happen
-    bigs.resize(host_counts[1]);
+    end = back[0].x < L.table_cap ? back[0].x : L.table_cap;
     std::swap(idx_in, idx_out);
     std::swap(box_in, box_out);
-    std::swap(big_cur, big_next);
   }
   const uint32_t total = end;
   const uint32_t levels = (uint32_t)level_start.size();
   level_start.push_back(total);
 
   // numbering: split counts bottom-up, subtree bases, ranks top-down
-  for (int l = (int)levels - 1; l >= 0; --l) {
+  TopLevels T = {};
+  while (T.n < levels && T.n < kTopLevels && level_start[T.n + 1] - level_start[T.n] <= kTopNodes) ++T.n;
+  for (uint32_t l = 0; l <= T.n; ++l) T.start[l] = level_start[l];
+  for (int l = (int)levels - 1; l >= (int)T.n; --l) {
     const uint32_t b = level_start[l], e = level_start[l + 1];
     k_sah_internal<<<(uint32_t)hmin<uint64_t>((e - b + 255) / 256, (uint64_t)sms * 8), 256, 0, st>>>(L.table, b, e);
   }
-  note_launch(levels);
+  if (T.n) k_sah_internal_top<<<1, 1024, 0, st>>>(L.table, T);
+  note_launch(levels - T.n + (T.n ? 1 : 0));
   k_sah_base_in<<<(roots + 255) / 256, 256, 0, st>>>(L.table, roots, L.base);
   note_launch();
   excl_scan(L.base, roots, L.sums, L.scalars + 4, st);
-  for (uint32_t l = 0; l < levels; ++l) {
+  if (T.n) k_sah_rank_top<<<1, 1024, 0, st>>>(L.table, T, L.rank, L.base, first_base);
+  for (uint32_t l = T.n; l < levels; ++l) {
     const uint32_t b = level_start[l], e = level_start[l + 1];
     k_sah_rank<<<(uint32_t)hmin<uint64_t>((e - b + 255) / 256, (uint64_t)sms * 8), 256, 0, st>>>(L.table, b, e, L.rank, L.base, first_base);
   }
-  note_launch(levels);
+  note_launch(levels - T.n + (T.n ? 1 : 0));
   // node count = first_base + 2 * (all splits) = first_base + scan total
   uint32_t splits2 = 0;
   if (cudaMemcpyAsync(&splits2, L.scalars + 4, 4, cudaMemcpyDeviceToHost, st) != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess)
