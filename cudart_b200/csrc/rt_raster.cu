@@ -167,6 +167,9 @@ __global__ __launch_bounds__(kFacesPerBlock) void k_raster_setup(const float4* _
       const float det = (b.x - a.x) * (cc.y - a.y) - (cc.x - a.x) * (b.y - a.y);
       const bool degenerate = det > -kRasterEps && det < kRasterEps;
       a.w = degenerate ? 0.0f : 1.0f / det;
+      // a depth that no point of the face lies below, as the zone pass computes them: its weights are within 2^-22 of
+      // convex and its sum rounds five times, together less than half of 2^-20 of the largest depth
+      cc.w = fminf(fminf(a.z, b.z), cc.z) - 9.5367431640625e-7f * fmaxf(fmaxf(fabsf(a.z), fabsf(b.z)), fabsf(cc.z));
       tri[3 * (size_t)f] = a;
       tri[3 * (size_t)f + 1] = b;
       tri[3 * (size_t)f + 2] = cc;
@@ -238,7 +241,10 @@ __global__ __launch_bounds__(256) void k_raster_bin(const float4* __restrict__ t
   }
 }
 
-// One warp per zone; lane = pixel (x = lane % 8, y = lane / 8 inside the zone).
+// One warp per zone; lane = pixel (x = lane % 8, y = lane / 8 inside the zone). The zone's faces are taken 32 at a time,
+// one per lane, and those whose nearest depth lies behind the zone's farthest pixel so far go at once; the others are
+// tested by the whole warp. 2^20 faces of a soup at 1920 x 1080: 754 us with a test of every face, now 556, by issue
+// slots (74%) and the loads' wavefronts. (Taking the nearest of the 32 first: 620.)
 __global__ __launch_bounds__(256) void k_raster_zones(const float4* __restrict__ tri, const uint32_t* __restrict__ vals,
                                                       const uint32_t* __restrict__ zs, const uint32_t* __restrict__ ze, uint32_t nz,
                                                       Screen S, int width, int height, uint32_t id_mode, int32_t* __restrict__ fid,
@@ -256,24 +262,49 @@ __global__ __launch_bounds__(256) void k_raster_zones(const float4* __restrict__
     float best = inside ? depth[l] : 0.0f;
     int32_t bf = -1;
     float bu = 0.0f, bv = 0.0f;
-    for (uint32_t p = s; p < e; ++p) {
-      const uint32_t f = __ldg(vals + p);
-      const float4 a = __ldg(tri + 3 * (size_t)f), b = __ldg(tri + 3 * (size_t)f + 1), c = __ldg(tri + 3 * (size_t)f + 2);
-      // intersectTriPoint (:52-71); the face setup pass computed 1 / det (a.w) and
-      // emitted no pairs for faces with |det| below the threshold
-      const float inv_det = a.w;
-      const float u = ((c.x - px) * (a.y - py) - (a.x - px) * (c.y - py)) * inv_det;
-      if (u < 0.0f || u > 1.0f) continue;
-      const float v = ((a.x - px) * (b.y - py) - (b.x - px) * (a.y - py)) * inv_det;
-      if (v < 0.0f || u + v > 1.0f) continue;
-      const float t = (1.0f - u - v) * a.z + u * b.z + v * c.z;
-      // the earliest face wins a depth tie: faces arrive in any order, and the
-      // depth of an earlier chunk (bf < 0) is only beaten by a strictly nearer face
-      if (inside && t > 0 && (t < best || (t == best && bf >= 0 && (int32_t)f < bf))) {
-        best = t;
-        bf = (int32_t)f;
-        bu = u;
-        bv = v;
+    // the zone's farthest depth so far; as integers, since a pixel whose depth is not positive takes no face at all
+    float far = 0.0f;
+    auto farthest = [&] { far = __int_as_float(__reduce_max_sync(0xffffffffu, inside ? __float_as_int(best) : (int)0x80000000)); };
+    farthest();
+    uint32_t f32 = 0;
+    float lo32 = 0.0f;
+    auto load32 = [&](uint32_t p) {  // a face per lane, and its nearest depth (c.w)
+      if (p >= e) return;
+      f32 = __ldg(vals + p);
+      lo32 = __ldg(&tri[3 * (size_t)f32 + 2].w);
+    };
+    load32(s + lane);
+    for (uint32_t p = s; p < e; p += 32) {
+      const uint32_t mine = f32;
+      const float lo = lo32;
+      uint32_t todo = __ballot_sync(0xffffffffu, p + lane < e && !(lo > far));
+      load32(p + 32 + lane);
+      while (todo) {
+        const uint32_t f = __shfl_sync(0xffffffffu, mine, __ffs((int)todo) - 1);
+        todo &= todo - 1u;
+        const float4 a = __ldg(tri + 3 * (size_t)f), b = __ldg(tri + 3 * (size_t)f + 1), c = __ldg(tri + 3 * (size_t)f + 2);
+        // intersectTriPoint (:52-71); the face setup pass computed 1 / det (a.w) and
+        // emitted no pairs for faces with |det| below the threshold
+        const float inv_det = a.w;
+        const float u = ((c.x - px) * (a.y - py) - (a.x - px) * (c.y - py)) * inv_det;
+        const float v = ((a.x - px) * (b.y - py) - (b.x - px) * (a.y - py)) * inv_det;
+        bool won = false;
+        if (!(u < 0.0f || u > 1.0f) && !(v < 0.0f || u + v > 1.0f)) {
+          const float t = (1.0f - u - v) * a.z + u * b.z + v * c.z;
+          // the earliest face wins a depth tie: faces arrive in any order, and the
+          // depth of an earlier chunk (bf < 0) is only beaten by a strictly nearer face
+          if (inside && t > 0 && (t < best || (t == best && bf >= 0 && (int32_t)f < bf))) {
+            best = t;
+            bf = (int32_t)f;
+            bu = u;
+            bv = v;
+            won = true;
+          }
+        }
+        if (__any_sync(0xffffffffu, won)) {
+          farthest();
+          todo &= __ballot_sync(0xffffffffu, !(lo > far));
+        }
       }
     }
     if (bf >= 0) {

@@ -44,3 +44,27 @@ def test_zone_lists_change_nothing(oracle, kind, w, h):
         assert np.array_equal(got["uv"].cpu().numpy().view(np.uint32), uo.view(np.uint32))
         hit = do != oracle.HUGE
         assert np.array_equal(got["id"].cpu().numpy()[hit].view(np.uint32), fo[hit].astype(np.uint32))
+
+
+@pytest.mark.parametrize("depths", ["equal", "ulps apart", "steep", "wide", "negative", "infinite"])
+def test_faces_behind_a_zone_change_nothing(oracle, depths):
+    """Many faces over few zones, where the walk leaves out faces behind a zone's farthest depth: ties and near ties by
+    index, planes steep enough for their rounding to matter, depths of every magnitude and sign."""
+    import torch
+    from cudart_b200 import core
+    w, h, n = 40, 22, 3000
+    rng = np.random.default_rng(len(depths))
+    v, f = _faces("corners", n, w, h, rng)
+    z = {"equal": lambda: np.full(3 * n, 0.5), "ulps apart": lambda: np.repeat(0.5 + rng.integers(-3, 4, n) * 2.0 ** -24, 3),
+         "steep": lambda: np.where(rng.random(3 * n) < 0.3, 1e4, 1.0) * rng.uniform(0.999, 1.001, 3 * n),
+         "wide": lambda: 10.0 ** rng.uniform(-30, 30, 3 * n), "negative": lambda: rng.uniform(-1, 0.2, 3 * n),
+         "infinite": lambda: np.where(rng.random(3 * n) < 0.01, np.inf, rng.uniform(0.1, 2.0, 3 * n))}[depths]()
+    v[:, 2] = z
+    m = np.eye(4, dtype=np.float32).ravel()
+    with np.errstate(all="ignore"):
+        fo, uo, do = oracle.rasterize(v, f, m, w, h)
+    for cap in (0, 1):
+        got = core.rasterize(torch.from_numpy(v).cuda(), torch.from_numpy(f.view(np.int32)).cuda(), m, w, h, pair_capacity=cap)
+        assert np.array_equal(got["id"].cpu().numpy().ravel(), fo.ravel())
+        assert np.array_equal(got["depth"].cpu().numpy().ravel().view(np.uint32), do.ravel().view(np.uint32))
+        assert np.array_equal(got["uv"].cpu().numpy().ravel().view(np.uint32), uo.ravel().view(np.uint32))
