@@ -13,8 +13,8 @@
 //   level sort       split positions by split level (clz of the xor of adjacent
 //                    codes, computed as the pass reads them): the per-level
 //                    ascending split lists the recursion walks
-//   k_topo_morton    one CTA: the Morton levels of the tree, level by level,
-//                    with the reference's split-pointer semantics (see below);
+//   k_topo_morton    one CTA: the Morton levels of the tree, level by level in
+//                    shared memory, with the reference's split-pointer semantics (see below);
 //                    leaf counts, pre-order ranks and node ids
 //   k_leaves         32 final leaves at a time per warp: expands median subtrees, writes
 //                    node records, reorders faces, pre-gathers triangles

@@ -15,7 +15,6 @@
 // left first: the k-th split of a subtree rooted when the counter stood at B
 // gets B + 2k, B + 2k + 1) are assigned afterwards from the tree's shape:
 // subtree split counts bottom-up, pre-order ranks top-down.
-#include <utility>
 #include <vector>
 
 #include "../../include/rt_sah.h"
@@ -187,9 +186,9 @@ struct LevelArgs {
   SNode* table;
   uint32_t* table_count;  // [0] entries, [1] big entries of the next level, [2] no-split leaves
   uint4* big_next;        // (table index, faces, first) of the next level's big nodes
-  const uint32_t* big_cur;  // table indices of this level's big nodes handled one CTA each
-  uint32_t level_begin, level_end;
-  uint32_t* range;        // a level of a run without waits: range[step], range[step + 1] instead of level_begin, level_end
+  uint32_t* regular;      // table indices of this level's big nodes handled one CTA each
+  uint32_t* head;         // [0] of those, [1] huge nodes, [2] their tiles
+  uint32_t* range;        // level `step` of a run: table entries range[step] .. range[step + 1] - 1
   uint32_t step;
   const uint32_t* idx_in;
   const Item* box_in;
@@ -342,36 +341,25 @@ __device__ __forceinline__ void sah_small_node(const LevelArgs& A, const uint32_
   }
 }
 
-// A warp per node of at most kBigNode faces (8 warps per CTA). With A.range, one of kRunLevels launches that follow one
-// another without the host in between (no node above kBigNode is left): the CTA that finishes last writes where the
-// next but one level ends, which nothing in this launch reads.
-constexpr uint32_t kRunLevels = 6;
-constexpr uint32_t kRunDone = 16;  // range: kRunLevels + 2 bounds, then from here the launches' CTA counters
+// A warp per node of at most kBigNode faces (8 warps per CTA).
 __global__ __launch_bounds__(kCta) void k_sah_small(LevelArgs A) {
   __shared__ Bins s_bins[kCta / 32];
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-  const uint32_t begin = A.range ? A.range[A.step] : A.level_begin, end = A.range ? A.range[A.step + 1] : A.level_end;
+  const uint32_t begin = A.range[A.step], end = A.range[A.step + 1];
   for (uint32_t e = begin + blockIdx.x * (kCta / 32) + warp; e < end; e += gridDim.x * (kCta / 32)) {
     sah_small_node(A, e, s_bins[warp], lane);
     __syncwarp();
   }
-  if (!A.range) return;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    if (atomicAdd(A.range + kRunDone + A.step, 1u) == gridDim.x - 1)
-      A.range[A.step + 2] = min(atomicAdd(A.table_count, 0u), A.table_cap);
-  }
 }
 
 // One CTA per node of more than kBigNode faces.
-__global__ __launch_bounds__(kCta) void k_sah_big(LevelArgs A, uint32_t count_big) {
+__global__ __launch_bounds__(kCta) void k_sah_big(LevelArgs A) {
   __shared__ Bins B;
   __shared__ float s_red[6][kCta / 32];
   __shared__ Decision s_d;
   __shared__ uint32_t s_child;
-  if (blockIdx.x >= count_big) return;
-  const uint32_t e = A.big_cur[blockIdx.x];
+  if (blockIdx.x >= A.head[0]) return;
+  const uint32_t e = A.regular[blockIdx.x];
   const SNode nd = A.table[e];
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
   float3 cmn = make_float3(kHuge, kHuge, kHuge), cmx = make_float3(-kHuge, -kHuge, -kHuge);
@@ -440,12 +428,14 @@ __global__ __launch_bounds__(kCta) void k_sah_big(LevelArgs A, uint32_t count_bi
 // 2^20 faces, a level of huge nodes: 50 us with 2048-face tiles (512 CTAs), 110 with 8192 (128).
 constexpr uint32_t kHugeNode = 8192;
 constexpr uint32_t kTile = 2048;
+constexpr uint32_t kRunLevels = 5;             // levels between two reads by the host (a read and its wait 30 us, a level's
+                                               // launches with nothing to do 5 to 20)
 
 struct HugeArgs {
-  const uint32_t* node;   // [H] table index of huge node h
-  const uint32_t* tnode;  // [tiles] huge slot of tile t
-  const uint32_t* tstart; // [tiles] first face (position) of tile t
-  const uint32_t* tfirst; // [H] first tile of node h
+  uint32_t* node;         // [H] table index of huge node h
+  uint32_t* tnode;        // [tiles] huge slot of tile t
+  uint32_t* tstart;       // [tiles] first face (position) of tile t
+  uint32_t* tfirst;       // [H] first tile of node h
   uint32_t* keys;         // [H][8] centroid bounds as order keys (min xyz, max xyz)
   Bins* bins;             // [H]
   Decision* dec;          // [H]
@@ -453,18 +443,13 @@ struct HugeArgs {
   uint32_t* child;        // [H] first child table index, kNone when a leaf
   uint32_t* tbins;        // [tiles][kBins] faces per tile and bin
   uint32_t* tleft;        // [tiles] left faces in the node's earlier tiles
-  uint32_t H, tiles;
+  uint32_t cap;           // of H
+  const uint32_t* head;   // LevelArgs::head
 };
-
-__global__ __launch_bounds__(256) void k_huge_reset(HugeArgs G) {
-  const uint32_t h = blockIdx.x;
-  if (h >= G.H) return;
-  if (threadIdx.x < 3) { G.keys[8 * h + threadIdx.x] = 0xFFFFFFFFu; G.keys[8 * h + 3 + threadIdx.x] = 0u; }
-  if (threadIdx.x < kBins) bins_reset(G.bins[h], (int)threadIdx.x);
-}
 
 __global__ __launch_bounds__(kCta) void k_huge_bounds(LevelArgs A, HugeArgs G) {
   const uint32_t t = blockIdx.x;
+  if (t >= G.head[2]) return;
   const uint32_t h = G.tnode[t];
   const SNode nd = A.table[G.node[h]];
   const uint32_t ts = G.tstart[t], te = min(nd.first + nd.count, ts + kTile);
@@ -498,6 +483,7 @@ __device__ __forceinline__ Split huge_split(const HugeArgs& G, uint32_t h) {
 __global__ __launch_bounds__(kCta) void k_huge_bins(LevelArgs A, HugeArgs G) {
   __shared__ Bins B;
   const uint32_t t = blockIdx.x;
+  if (t >= G.head[2]) return;
   const uint32_t h = G.tnode[t];
   const SNode nd = A.table[G.node[h]];
   const uint32_t ts = G.tstart[t], te = min(nd.first + nd.count, ts + kTile);
@@ -526,6 +512,7 @@ __global__ __launch_bounds__(kCta) void k_huge_decide(LevelArgs A, HugeArgs G) {
   __shared__ uint32_t s_w[kCta / 32];
   __shared__ int s_m;
   const uint32_t h = blockIdx.x;
+  if (h >= G.head[1]) return;
   if (threadIdx.x < 32) {
     const uint32_t e = G.node[h];
     const SNode nd = A.table[e];
@@ -548,7 +535,7 @@ __global__ __launch_bounds__(kCta) void k_huge_decide(LevelArgs A, HugeArgs G) {
   __syncthreads();
   const int m_min = s_m;
   if (m_min < 0) return;
-  const uint32_t t0 = G.tfirst[h], t1 = h + 1 < G.H ? G.tfirst[h + 1] : G.tiles;
+  const uint32_t t0 = G.tfirst[h], t1 = h + 1 < G.head[1] ? G.tfirst[h + 1] : G.head[2];
   uint32_t running = 0;
   for (uint32_t base = t0; base < t1; base += kCta) {
     const uint32_t t = base + threadIdx.x;
@@ -567,6 +554,7 @@ __global__ __launch_bounds__(kCta) void k_huge_decide(LevelArgs A, HugeArgs G) {
 
 __global__ __launch_bounds__(kCta) void k_huge_scatter(LevelArgs A, HugeArgs G) {
   const uint32_t t = blockIdx.x;
+  if (t >= G.head[2]) return;
   const uint32_t h = G.tnode[t];
   const SNode nd = A.table[G.node[h]];
   const uint32_t ts = G.tstart[t], te = min(nd.first + nd.count, ts + kTile);
@@ -584,7 +572,7 @@ __global__ __launch_bounds__(kCta) void k_huge_scatter(LevelArgs A, HugeArgs G) 
 // ---------------------------------------------------------------- setup
 // SAH: positions start as the faces in order, the root's box is the mesh box.
 __global__ __launch_bounds__(256) void k_sah_init(const float4* __restrict__ boxes, uint32_t n, const float* __restrict__ hit,
-                                                  uint32_t* idx, Item* items, SNode* table, uint32_t* counts) {
+                                                  uint32_t* idx, Item* items, SNode* table, uint4* big, uint32_t* counts) {
   for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
     idx[p] = p;
     items[p].mn = boxes[2 * (size_t)p];
@@ -599,7 +587,10 @@ __global__ __launch_bounds__(256) void k_sah_init(const float4* __restrict__ box
     counts[0] = 1;
     counts[1] = 0;
     counts[2] = 0;
-    if (n > kBigNode) { counts[1] = 1; }
+    if (n > kBigNode) {
+      counts[1] = 1;
+      big[0] = make_uint4(0u, n, 0u, 0u);
+    }
   }
 }
 
@@ -659,6 +650,51 @@ __global__ __launch_bounds__(256) void k_hyb_roots(const uint32_t* __restrict__ 
     r.first = w[1]; r.count = w[0] >> 1; r.parent = kNone; r.info = 0; r.child = kNone; r.sub = j; r.internal = 0; r.id = k;
     table[j] = r;
     if (r.count > kBigNode) big[atomicAdd(counts + 1, 1u)] = make_uint4(j, r.count, r.first, 0u);
+  }
+}
+
+// A level's lists from the big nodes that the level before it left: the nodes of one CTA, the huge ones and their tiles;
+// and the level's table entries. One CTA (at most n / kBigNode nodes), so that the host need not wait between levels.
+__global__ __launch_bounds__(1024) void k_sah_lists(LevelArgs A, HugeArgs G, uint32_t begin) {
+  __shared__ uint32_t s_warp[32];
+  const uint32_t count = A.table_count[1];
+  uint32_t regular = 0, huge = 0, tiles = 0;
+  for (uint32_t c = 0; c < count; c += 1024) {
+    const uint32_t i = c + threadIdx.x;
+    const uint4 node = i < count ? A.big_next[i] : make_uint4(0, 0, 0, 0);
+    bool is_huge = node.y > kHugeNode;
+    uint32_t total;
+    const uint32_t h = huge + block_excl_scan_nt<1024>(is_huge ? 1u : 0u, s_warp, total);
+    huge = min(huge + total, G.cap);
+    is_huge = is_huge && h < G.cap;
+    const uint32_t t = tiles + block_excl_scan_nt<1024>(is_huge ? (node.y + kTile - 1) / kTile : 0u, s_warp, total);
+    tiles += total;
+    const uint32_t r = regular + block_excl_scan_nt<1024>(i < count && !is_huge ? 1u : 0u, s_warp, total);
+    regular += total;
+    if (is_huge) {
+      G.node[h] = node.x;
+      G.tfirst[h] = t;
+    } else if (i < count) {
+      A.regular[r] = node.x;
+    }
+  }
+  __syncthreads();
+  const uint32_t lane = threadIdx.x & 31u;
+  for (uint32_t h = threadIdx.x >> 5; h < huge; h += 32) {  // a huge node's tiles, and its bounds and bins empty
+    const SNode& node = A.table[G.node[h]];
+    const uint32_t t = G.tfirst[h];
+    for (uint32_t o = lane; o * kTile < node.count; o += 32) {
+      G.tnode[t + o] = h;
+      G.tstart[t + o] = node.first + o * kTile;
+    }
+    if (lane < 3) { G.keys[8 * h + lane] = 0xFFFFFFFFu; G.keys[8 * h + 3 + lane] = 0u; }
+    bins_reset(G.bins[h], (int)lane);
+  }
+  if (threadIdx.x == 0) {
+    A.head[0] = regular; A.head[1] = huge; A.head[2] = tiles;
+    A.table_count[1] = 0;
+    if (A.step == 0) A.range[0] = begin;
+    A.range[A.step + 1] = min(A.table_count[0], A.table_cap);
   }
 }
 
@@ -819,15 +855,14 @@ int sm_count() {
 }
 
 struct SahLayout {
-  uint32_t *idx_a, *idx_b, *lists, *counts, *rank, *base, *marks, *sums, *scalars, *keys, *err, *leaf_lambda;
-  uint4* big;       // right behind counts
-  uint32_t* range;
+  uint32_t *idx_a, *idx_b, *counts, *rank, *base, *marks, *sums, *scalars, *keys, *err, *leaf_lambda;
+  uint4* big;
+  uint32_t *regular, *h_node, *h_tfirst, *t_node, *t_start;
   uint32_t *h_keys, *h_child, *h_tbins, *h_tleft;
   Bins* h_bins;
   Decision* h_dec;
   Split* h_split;
   uint32_t h_cap, t_cap;
-  size_t lists_cap;
   Item *box_a, *box_b;
   SNode* table;
   rt_build_info* lb_info;
@@ -846,14 +881,14 @@ size_t carve_sah(Carve& c, SahLayout& L, uint32_t n, uint32_t lbvh_depth, uint32
   L.box_b = c.take<Item>(n);
   L.h_cap = n / kHugeNode + 2;
   L.t_cap = n / kTile + L.h_cap + 2;
-  // a level's lists, uploaded together: the nodes of one CTA, the huge nodes and their first tiles, the tiles' nodes and starts
-  // right behind the lists' end the counts, so that a level's upload sets them, and then the level's new big nodes, so that
-  // one copy reads both
-  L.lists_cap = align_up((size_t)n / kBigNode + 2 + 2 * (size_t)L.h_cap + 2 * (size_t)L.t_cap, 4);
-  L.lists = c.take<uint32_t>(L.lists_cap + 4 * (1 + (size_t)n / kBigNode + 2));
-  L.counts = L.lists ? L.lists + L.lists_cap : nullptr;
-  L.big = (uint4*)(L.counts ? L.counts + 4 : nullptr);
-  L.range = c.take<uint32_t>(32);
+  L.regular = c.take<uint32_t>(n / kBigNode + 2);
+  L.h_node = c.take<uint32_t>(L.h_cap);
+  L.h_tfirst = c.take<uint32_t>(L.h_cap);
+  L.t_node = c.take<uint32_t>(L.t_cap);
+  L.t_start = c.take<uint32_t>(L.t_cap);
+  L.big = c.take<uint4>(n / kBigNode + 2);
+  // what the host reads of a run of levels: counts [4], head [4], range [kRunLevels + 1]
+  L.counts = c.take<uint32_t>(8 + kRunLevels + 1);
   L.h_keys = c.take<uint32_t>(8 * (size_t)L.h_cap);
   L.h_child = c.take<uint32_t>(L.h_cap);
   L.h_bins = c.take<Bins>(L.h_cap);
@@ -952,7 +987,7 @@ extern "C" rt_status rt_sah_build(const rt_sah_desc* d, rt_stream stream) {
       k_keys_to_box<<<1, 32, 0, st>>>(L.keys, hit);
       note_launch(2);
     }
-    k_sah_init<<<grid, 256, 0, st>>>((const float4*)d->boxes, n, hit, L.idx_a, L.box_a, L.table, L.counts);
+    k_sah_init<<<grid, 256, 0, st>>>((const float4*)d->boxes, n, hit, L.idx_a, L.box_a, L.table, L.big, L.counts);
     note_launch();
   } else {
     rt_build_desc b = {};
@@ -983,112 +1018,52 @@ extern "C" rt_status rt_sah_build(const rt_sah_desc* d, rt_stream stream) {
   // levels
   std::vector<uint32_t> level_start;
   uint32_t begin = 0, end = roots;
-  uint32_t* idx_in = L.idx_a;
-  uint32_t* idx_out = L.idx_b;
-  Item* box_in = L.box_a;
-  Item* box_out = L.box_b;
-  // `back`: the counts, then the level's big nodes, read together
-  std::vector<uint4> bigs, back;
-  auto read_back = [&](size_t most) {
-    back.resize(1 + most);
-    if (cudaMemcpyAsync(back.data(), L.counts, back.size() * 16, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-        cudaStreamSynchronize(st) != cudaSuccess || back[0].y > most)
-      return false;
-    bigs.assign(back.begin() + 1, back.begin() + 1 + back[0].y);
-    return true;
-  };
-  if (!d->lbvh_depth) {
-    back.push_back(make_uint4(1u, 0u, 0u, 0u));
-    if (n > kBigNode) bigs.push_back(make_uint4(0u, n, 0u, 0u));
-  } else if (!read_back(n / kBigNode + 1)) {
-    return RT_ERR_CUDA;
-  }
-  std::vector<uint32_t> regular, h_node, h_tfirst, t_node, t_start;
+  LevelArgs A = {};
+  A.table = L.table; A.table_count = L.counts; A.big_next = L.big; A.regular = L.regular; A.head = L.counts + 4; A.range = L.counts + 8;
+  A.final_idx = d->indices; A.err = L.err; A.table_cap = L.table_cap;
+  A.idx_in = L.idx_a; A.box_in = L.box_a; A.idx_out = L.idx_b; A.box_out = L.box_b;
+  HugeArgs G;
+  G.node = L.h_node; G.tfirst = L.h_tfirst; G.tnode = L.t_node; G.tstart = L.t_start; G.keys = L.h_keys; G.bins = L.h_bins;
+  G.dec = L.h_dec; G.split = L.h_split; G.child = L.h_child; G.tbins = L.h_tbins; G.tleft = L.h_tleft; G.cap = L.h_cap; G.head = A.head;
+  // kRunLevels levels at a time, their grids by what can be there at most: `nodes` in the level, `bigs` of them above
+  // kBigNode faces (their ranges are disjoint)
+  bool huge = n > kHugeNode, big = n > kBigNode;
+  uint64_t nodes = roots, bigs = roots;
   while (begin < end) {
-    if (bigs.empty()) {
-      // only nodes of at most kBigNode faces are left, and so below: kRunLevels levels with one wait at their end (a
-      // wait and the copies around it take 25 us). A level that has nothing to do costs its launch.
-      uint32_t run[32] = {begin, end};
-      if (cudaMemcpyAsync(L.range, run, sizeof(run), cudaMemcpyHostToDevice, st) != cudaSuccess) return RT_ERR_CUDA;
-      LevelArgs A = {};
-      A.table = L.table; A.table_count = L.counts; A.big_next = L.big; A.range = L.range; A.final_idx = d->indices; A.err = L.err;
-      A.table_cap = L.table_cap;
-      uint64_t most = end - begin;
-      for (A.step = 0; A.step < kRunLevels; ++A.step) {
-        A.idx_in = idx_in; A.box_in = box_in; A.idx_out = idx_out; A.box_out = box_out;
-        k_sah_small<<<(uint32_t)hmin<uint64_t>((most + 7) / 8, (uint64_t)sms * 8), kCta, 0, st>>>(A);
-        most = hmin<uint64_t>(2 * most, L.table_cap);
-        std::swap(idx_in, idx_out);
-        std::swap(box_in, box_out);
+    for (A.step = 0; A.step < kRunLevels; ++A.step) {
+      k_sah_lists<<<1, 1024, 0, st>>>(A, G, begin);
+      if (huge) {
+        const uint32_t H = (uint32_t)hmin<uint64_t>(bigs, n / (kHugeNode + 1)), tiles = n / kTile + H;
+        k_huge_bounds<<<tiles, kCta, 0, st>>>(A, G);
+        k_huge_bins<<<tiles, kCta, 0, st>>>(A, G);
+        k_huge_decide<<<H, kCta, 0, st>>>(A, G);
+        k_huge_scatter<<<tiles, kCta, 0, st>>>(A, G);
+        note_launch(4);
       }
-      note_launch(kRunLevels);
-      RT_CHECK_LAUNCH();
-      if (cudaMemcpyAsync(run, L.range, (kRunLevels + 2) * 4, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-          cudaStreamSynchronize(st) != cudaSuccess)
-        return RT_ERR_CUDA;
-      for (uint32_t l = 0; l < kRunLevels && run[l] < run[l + 1]; ++l) level_start.push_back(run[l]);
-      begin = run[kRunLevels];
-      end = run[kRunLevels + 1];
-      continue;
-    }
-    level_start.push_back(begin);
-    // this level's big nodes: a CTA each, or tiles of several CTAs when huge
-    regular.clear(); h_node.clear(); h_tfirst.clear(); t_node.clear(); t_start.clear();
-    for (const uint4& bg : bigs) {
-      if (bg.y > kHugeNode && h_node.size() < L.h_cap) {
-        h_tfirst.push_back((uint32_t)t_node.size());
-        for (uint32_t o = 0; o < bg.y; o += kTile) {
-          t_node.push_back((uint32_t)h_node.size());
-          t_start.push_back(bg.z + o);
-        }
-        h_node.push_back(bg.x);
-      } else {
-        regular.push_back(bg.x);
+      if (big) {
+        k_sah_big<<<(uint32_t)hmin<uint64_t>(bigs, n / (kBigNode + 1)), kCta, 0, st>>>(A);
+        note_launch();
       }
-    }
-    const uint32_t H = (uint32_t)h_node.size(), R = (uint32_t)regular.size(), tiles = (uint32_t)t_node.size();
-    if (tiles > L.t_cap) return RT_ERR_CAPACITY;
-    // one upload: [regular][h_node][h_tfirst][t_node][t_start] and the counts, of which the big nodes' starts again
-    regular.insert(regular.end(), h_node.begin(), h_node.end());
-    regular.insert(regular.end(), h_tfirst.begin(), h_tfirst.end());
-    regular.insert(regular.end(), t_node.begin(), t_node.end());
-    regular.insert(regular.end(), t_start.begin(), t_start.end());
-    if (regular.size() > L.lists_cap) return RT_ERR_CAPACITY;  // cannot happen
-    uint32_t* const lists = L.counts - regular.size();
-    const uint32_t counts[4] = {back[0].x, 0u, back[0].z, 0u};
-    regular.insert(regular.end(), counts, counts + 4);
-    if (cudaMemcpyAsync(lists, regular.data(), regular.size() * 4, cudaMemcpyHostToDevice, st) != cudaSuccess) return RT_ERR_CUDA;
-    LevelArgs A = {};
-    A.table = L.table; A.table_count = L.counts; A.big_next = L.big; A.big_cur = lists; A.level_begin = begin; A.level_end = end;
-    A.idx_in = idx_in; A.box_in = box_in; A.idx_out = idx_out; A.box_out = box_out; A.final_idx = d->indices; A.err = L.err;
-    A.table_cap = L.table_cap;
-    if (H) {
-      HugeArgs G;
-      G.node = lists + R; G.tfirst = G.node + H; G.tnode = G.tfirst + H; G.tstart = G.tnode + tiles;
-      G.keys = L.h_keys; G.bins = L.h_bins;
-      G.dec = L.h_dec; G.split = L.h_split; G.child = L.h_child; G.tbins = L.h_tbins; G.tleft = L.h_tleft; G.H = H; G.tiles = tiles;
-      k_huge_reset<<<H, 64, 0, st>>>(G);
-      k_huge_bounds<<<tiles, kCta, 0, st>>>(A, G);
-      k_huge_bins<<<tiles, kCta, 0, st>>>(A, G);
-      k_huge_decide<<<H, kCta, 0, st>>>(A, G);
-      k_huge_scatter<<<tiles, kCta, 0, st>>>(A, G);
-      note_launch(5);
-    }
-    if (R) {
-      k_sah_big<<<R, kCta, 0, st>>>(A, R);
-      note_launch();
-    }
-    if (end - begin > (uint32_t)bigs.size()) {  // nodes of at most kBigNode faces
-      k_sah_small<<<(end - begin + 7) / 8, kCta, 0, st>>>(A);
-      note_launch();
+      k_sah_small<<<(uint32_t)hmin<uint64_t>((nodes + 7) / 8, (uint64_t)sms * 8), kCta, 0, st>>>(A);
+      note_launch(2);
+      nodes = hmin<uint64_t>(2 * nodes, L.table_cap);
+      bigs = hmin<uint64_t>(2 * bigs, n);
+      const uint32_t* idx = A.idx_in;
+      const Item* box = A.box_in;
+      A.idx_in = A.idx_out; A.box_in = A.box_out;
+      A.idx_out = (uint32_t*)idx; A.box_out = (Item*)box;
     }
     RT_CHECK_LAUNCH();
-    // one wait per level: the counts, and the next level's big nodes (at most two per big node of this one)
-    if (!read_back(hmin<size_t>(2 * bigs.size(), n / kBigNode + 1))) return RT_ERR_CUDA;
-    begin = end;
-    end = back[0].x < L.table_cap ? back[0].x : L.table_cap;
-    std::swap(idx_in, idx_out);
-    std::swap(box_in, box_out);
+    uint32_t run[8 + kRunLevels + 1];
+    if (cudaMemcpyAsync(run, L.counts, sizeof(run), cudaMemcpyDeviceToHost, st) != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess)
+      return RT_ERR_CUDA;
+    const uint32_t* range = run + 8;
+    for (uint32_t l = 0; l < kRunLevels && range[l] < range[l + 1]; ++l) level_start.push_back(range[l]);
+    begin = range[kRunLevels];
+    end = run[0] < L.table_cap ? run[0] : L.table_cap;
+    huge = huge && run[5] > 0;  // none in the run's last level: none below it
+    big = big && run[4] + run[5] > 0;
+    nodes = end - begin;
   }
   const uint32_t total = end;
   const uint32_t levels = (uint32_t)level_start.size();
@@ -1106,18 +1081,15 @@ extern "C" rt_status rt_sah_build(const rt_sah_desc* d, rt_stream stream) {
   note_launch(levels - T.n + (T.n ? 1 : 0));
   k_sah_base_in<<<(roots + 255) / 256, 256, 0, st>>>(L.table, roots, L.base);
   note_launch();
-  excl_scan(L.base, roots, L.sums, L.scalars + 4, st);
+  excl_scan(L.base, roots, L.sums, nullptr, st);
   if (T.n) k_sah_rank_top<<<1, 1024, 0, st>>>(L.table, T, L.rank, L.base, first_base);
   for (uint32_t l = T.n; l < levels; ++l) {
     const uint32_t b = level_start[l], e = level_start[l + 1];
     k_sah_rank<<<(uint32_t)hmin<uint64_t>((e - b + 255) / 256, (uint64_t)sms * 8), 256, 0, st>>>(L.table, b, e, L.rank, L.base, first_base);
   }
   note_launch(levels - T.n + (T.n ? 1 : 0));
-  // node count = first_base + 2 * (all splits) = first_base + scan total
-  uint32_t splits2 = 0;
-  if (cudaMemcpyAsync(&splits2, L.scalars + 4, 4, cudaMemcpyDeviceToHost, st) != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess)
-    return RT_ERR_CUDA;
-  const uint32_t node_count = first_base + splits2;
+  // every split made two table entries: the node and leaf counts without waiting for the scans
+  const uint32_t splits2 = total - roots, node_count = first_base + splits2, leaf_total = roots + splits2 / 2;
   if (cudaMemsetAsync(L.marks, 0, (size_t)n * 4 + 4, st) != cudaSuccess) return RT_ERR_CUDA;
   k_sah_write<<<(uint32_t)hmin<uint64_t>((total + 255) / 256, (uint64_t)sms * 8), 256, 0, st>>>(L.table, total, L.rank, L.base, first_base,
                                                                                               d->nodes, d->max_nodes, L.marks, L.err);
@@ -1133,9 +1105,6 @@ extern "C" rt_status rt_sah_build(const rt_sah_desc* d, rt_stream stream) {
       d->nodes, node_count, L.marks, d->indices, (const uint4*)d->faces_in, (const float4*)d->vertices, (uint4*)d->faces_out,
       (float4*)d->tris, AL.leaves, AL.groups, L.leaf_lambda, n, L.err);
   note_launch();
-  uint32_t leaf_total = 0;
-  if (cudaMemcpyAsync(&leaf_total, L.scalars + 5, 4, cudaMemcpyDeviceToHost, st) != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess)
-    return RT_ERR_CUDA;
   if (d->accel) {
     k_sah_accel<<<(uint32_t)hmin<uint64_t>((node_count + 255) / 256, (uint64_t)sms * 8), 256, 0, st>>>(d->nodes, node_count, leaf_total,
                                                                                                         L.leaf_lambda, AL.tnodes, AL.hdr);

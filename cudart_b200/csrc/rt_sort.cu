@@ -1,5 +1,5 @@
 // rt_sort.cu -- stable LSD radix sort of 32-bit keys with optional 32-bit
-// values, 8-bit digits, one launch per digit pass (onesweep).
+// values, 8-bit digits, a count and a scatter launch per digit pass.
 //
 // Replaces the reference's sort family (CUDA_radixSortGeneral, CUDA_radixSort,
 // CUDA_bitonicSort*, CUDA_bubbleSort512; kernels/CUDA_radixSortGeneral.cu:397-482

@@ -8,17 +8,17 @@ once more; a profiler capturing the last launch of the named kernel sees a
 steady-state launch. Cases (kernel of interest in brackets):
 
   bench_step     three steps of the main workload (build, primary, bounce)     [launch list]
-  build_16m      LBVH build of a 2^24-face soup, twice                            [k_radix_scatter, k_leaves, k_boxes_morton]
+  build_16m      LBVH build of a 2^24-face soup, twice                            [k_sort_scatter, k_leaves, k_boxes_morton]
   batch_build    batched build of 1024 meshes (9.9M faces), twice                 [launch list]
   trace_primary  2^20-face soup, 1920x1080 primary rays, tuned tile schedule   [k_trace_accel]
   trace_bounce   the same scene's diffuse bounces, cooperative schedule          [k_trace_coop]
   mlp_propose    proposal network inference on 2^18 rays (4096 slots)            [k_mlp_propose_tc]
   mlp_train      one training step, batch 8192                                   [k_gemm_xent_tc, k_gemm_tc]
   sah_build      SAH build of the 2^20-face soup                                 [k_sah_small, k_huge_bins, k_sah_big]
-  raster         rasteriser, 2^20-face soup, 1920x1080                           [k_raster_zones, k_raster_emit]
-  mlp_grouped    64 grouped networks: 3 training steps of 1024 rays each,        [k_gemm_tc, k_softmax_xent, ...]
+  raster         rasteriser, 2^20-face soup, 1920x1080                           [k_raster_zones, k_raster_bin]
+  mlp_grouped    64 grouped networks: 3 training steps of 1024 rays each,        [k_gemm_tc, k_gemm_xent_tc, ...]
                  then proposals for 64 x 518,400 rays
-  sort_16m       2^24 random (key, value) pairs, 32-bit keys, sorted twice         [k_onesweep, k_sort_hist]
+  sort_16m       2^24 random (key, value) pairs, 32-bit keys, sorted twice         [k_sort_scatter, k_sort_count]
   trace_clusters 2^20-face soup with its cluster tree: packet primaries, per-lane [k_trace_clusters*]
                  bounces, twice each
   c4_frame [M]   M (default 64) deformed instances of the 1/16-size learned       [launch list, k_batch_trace_clusters*]
