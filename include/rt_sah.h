@@ -50,8 +50,9 @@ typedef struct rt_sah_desc {
 
 /* Scratch bytes and node capacity for a build of face_count faces. */
 rt_status rt_sah_sizes(uint32_t face_count, uint32_t lbvh_depth, size_t* scratch_bytes, uint32_t* max_nodes);
-/* Builds the tree. The call waits for the stream once per tree level (it reads
- * the level's node count), so it cannot be captured in a CUDA graph. */
+/* Builds the tree. The call waits for the stream once per few tree levels (it
+ * reads their node counts), so it cannot be captured in a CUDA graph; the last
+ * kernels are still running when it returns. */
 rt_status rt_sah_build(const rt_sah_desc* d, rt_stream stream);
 
 #ifdef __cplusplus
