@@ -765,7 +765,8 @@ __global__ __launch_bounds__(256) void k_transpose_bf16(const __nv_bfloat16* __r
 // so the results are the same bits. Needs even cols and ld. Several inputs can
 // share a launch, their column blocks side by side. Bound by latency (256
 // threads per 64 columns): four rows in flight took 85 us for 8192 rows, once
-// for each of a step's four inputs; the four together now take 61.
+// for each of a step's four inputs; the four together took 61 with 32, and 34
+// with the next 32 on their way (kDeep) and 32 columns a CTA.
 struct ColsumProblem {
   const __nv_bfloat16* in;
   float* out;
@@ -775,28 +776,47 @@ struct ColsumBatch {
   ColsumProblem p[kMulti];
   uint32_t count;
 };
-__global__ __launch_bounds__(256) void k_colsum2_bf16(const __grid_constant__ ColsumBatch B) {
+template <uint32_t kLanes, bool kDeep>
+__global__ __launch_bounds__(8 * kLanes) void k_colsum2_bf16(const __grid_constant__ ColsumBatch B) {
   constexpr int kAhead = 32;
-  __shared__ float2 part[8][33];
+  __shared__ float2 part[8][kLanes + 1];
   uint32_t i = 0;
   while (i + 1 < B.count && blockIdx.x >= B.p[i + 1].first) ++i;
   const uint32_t rows = B.p[i].rows, cols = B.p[i].cols, ld2 = B.p[i].ld / 2;
   float* out = B.p[i].out;
-  const uint32_t t = blockIdx.x - B.p[i].first, c = (t % B.p[i].nx * 32 + threadIdx.x) * 2, g = t / B.p[i].nx;
+  const uint32_t t = blockIdx.x - B.p[i].first, c = (t % B.p[i].nx * kLanes + threadIdx.x) * 2, g = t / B.p[i].nx;
   const __nv_bfloat162* p = (const __nv_bfloat162*)(B.p[i].in + (size_t)g * rows * B.p[i].ld + c);
   float s0 = 0.0f, s1 = 0.0f;
   if (c < cols) {
     uint32_t r = threadIdx.y;
-    for (; r + 8 * (kAhead - 1) < rows; r += 8 * kAhead) {
-      __nv_bfloat162 h[kAhead];
+    __nv_bfloat162 h[kDeep ? 2 : 1][kAhead];  // deep: one half is added up while the other is on its way
+    auto load = [&](__nv_bfloat162 (&x)[kAhead], uint32_t first) {
 #pragma unroll
-      for (int k = 0; k < kAhead; ++k) h[k] = p[(size_t)(r + 8 * k) * ld2];
+      for (int k = 0; k < kAhead; ++k) x[k] = p[(size_t)(first + 8 * k) * ld2];
+    };
+    auto add = [&](const __nv_bfloat162 (&x)[kAhead]) {
 #pragma unroll
       for (int k = 0; k < kAhead; ++k) {
-        s0 += __low2float(h[k]);
-        s1 += __high2float(h[k]);
+        s0 += __low2float(x[k]);
+        s1 += __high2float(x[k]);
+      }
+    };
+    const uint32_t steps = rows > r ? (rows - r + 7) / 8 / kAhead : 0;
+    if constexpr (kDeep) {
+      if (steps) load(h[0], r);
+      for (uint32_t k = 0; k < steps; k += 2, r += 16 * kAhead) {
+        if (k + 1 < steps) load(h[1], r + 8 * kAhead);
+        add(h[0]);
+        if (k + 2 < steps) load(h[0], r + 16 * kAhead);
+        if (k + 1 < steps) add(h[1]);
+      }
+    } else {
+      for (uint32_t k = 0; k < steps; ++k, r += 8 * kAhead) {
+        load(h[0], r);
+        add(h[0]);
       }
     }
+    r = threadIdx.y + steps * 8 * kAhead;
     for (; r < rows; r += 8) {
       const __nv_bfloat162 h = p[(size_t)r * ld2];
       s0 += __low2float(h);
@@ -1794,6 +1814,12 @@ extern "C" rt_status rt_colsum_bf16_multi(const rt_colsum_desc* d, uint32_t coun
   if (rt_device_check() != RT_OK) return RT_ERR_NO_DEVICE;
   ColsumBatch B = {};
   uint64_t blocks = 0;
+  for (uint32_t i = 0; i < count; ++i) blocks += colsum_by_two(d + i) ? (uint64_t)((d[i].cols + 63) / 64) * d[i].groups : 0u;
+  // few CTAs: latency bounds them, so narrow ones with twice the rows in flight (128 registers); with more than two per
+  // SM the wide ones win by their occupancy (64 groups of 1024 x 4096: 93 us against 103)
+  const bool deep = blocks <= 2u * (uint64_t)num_sms();
+  const uint32_t width = deep ? 32u : 64u;
+  blocks = 0;
   for (uint32_t i = 0; i < count; ++i) {
     if (d[i].cols == 0) continue;
     if (!colsum_by_two(d + i)) {
@@ -1805,12 +1831,13 @@ extern "C" rt_status rt_colsum_bf16_multi(const rt_colsum_desc* d, uint32_t coun
     }
     ColsumProblem& P = B.p[B.count++];
     P.in = (const __nv_bfloat16*)d[i].in; P.out = d[i].out; P.rows = d[i].rows; P.cols = d[i].cols; P.ld = d[i].ld;
-    P.nx = (d[i].cols + 63) / 64; P.first = (uint32_t)blocks;
+    P.nx = (d[i].cols + width - 1) / width; P.first = (uint32_t)blocks;
     blocks += (uint64_t)P.nx * d[i].groups;
     if (blocks > 0x7FFFFFFFull) return RT_ERR_INVALID_ARGUMENT;
   }
   if (B.count) {
-    k_colsum2_bf16<<<(uint32_t)blocks, dim3(32, 8), 0, (cudaStream_t)stream>>>(B);
+    if (deep) k_colsum2_bf16<16, true><<<(uint32_t)blocks, dim3(16, 8), 0, (cudaStream_t)stream>>>(B);
+    else k_colsum2_bf16<32, false><<<(uint32_t)blocks, dim3(32, 8), 0, (cudaStream_t)stream>>>(B);
     note_launch();
     RT_CHECK_LAUNCH();
   }

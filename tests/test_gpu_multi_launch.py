@@ -63,3 +63,22 @@ def test_adam_multi_equals_single_steps():
     for a, b in zip(nets[0].params + nets[0].m + nets[0].v + nets[0].W16 + nets[0].W16t,
                     nets[1].params + nets[1].m + nets[1].v + nets[1].W16 + nets[1].W16t):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("rows", [1, 7, 8, 9, 255, 256, 257, 511, 512, 513, 770, 8192, 10001])
+@pytest.mark.parametrize("cols,groups", [(32, 1), (34, 3), (4096, 1), (130, 400)])
+def test_colsum_order(rows, cols, groups):
+    """Wide and narrow column sums (many and few blocks) add in the order of the one-column kernel, which an odd leading
+    dimension takes: the same bits."""
+    import torch
+    from cudart_b200 import proposal
+    if rows * groups > 500000:
+        rows = 500000 // groups
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    x = torch.randn((groups * rows, cols), device="cuda", generator=g).to(torch.bfloat16)
+    odd = torch.zeros((groups * rows, cols + 1), device="cuda", dtype=torch.bfloat16)
+    odd[:, :cols] = x
+    a, b = torch.empty(groups * cols, device="cuda"), torch.empty(groups * cols, device="cuda")
+    proposal.colsum_multi([(x, a)], groups=groups)
+    proposal.colsum_multi([(odd[:, :cols], b)], groups=groups)
+    assert torch.equal(a.view(torch.int32), b.view(torch.int32))
