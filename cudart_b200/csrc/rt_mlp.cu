@@ -496,7 +496,9 @@ __global__ void __launch_bounds__(kXentThreads, 1)
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   const int32_t m0 = (int32_t)(grp * X.gm + blockIdx.x * kBM);
-  const uint32_t ntiles = n / kArgBN, total_tiles = 2 * ntiles;
+  // pass 1 takes every tile, pass 2 this CTA's share of them (gridDim.z shares)
+  const uint32_t ntiles = n / kArgBN, share = ntiles / gridDim.z, total_tiles = ntiles + share;
+  auto tile_of = [&](uint32_t t2) { return t2 < ntiles ? t2 : blockIdx.z * share + (t2 - ntiles); };
 
   if (warp == 16) {
     if (lane == 0) {
@@ -507,7 +509,7 @@ __global__ void __launch_bounds__(kXentThreads, 1)
       for (; q < total; ++q) {
         const uint32_t s = q % kStages;
         if (q >= kStages && !mbar_wait(empty + s, ((q / kStages) - 1u) & 1u, X.err)) break;
-        const uint32_t t = (q / num_k) % ntiles, kc = q % num_k;
+        const uint32_t t = tile_of(q / num_k), kc = q % num_k;
         mbar_arrive_expect_tx(full + s, kArgTileB);
         tma_load_2d(sB + s * kArgTileB, &tb, (int32_t)(kc * kBK), (int32_t)(grp * n + t * kArgBN), full + s);
       }
@@ -549,7 +551,7 @@ __global__ void __launch_bounds__(kXentThreads, 1)
     float mx = -INFINITY, sum = 0.0f, xl = 0.0f, inv = 0.0f;
     bool ok = true;
     for (uint32_t t2 = 0; t2 < total_tiles; ++t2) {
-      const uint32_t buf = t2 & 1u, pass = t2 / ntiles, t = t2 - pass * ntiles;
+      const uint32_t buf = t2 & 1u, pass = t2 >= ntiles ? 1u : 0u, t = tile_of(t2);
       if (t2 == ntiles && ok) {
         // merge the four column quarters of each row (quarter 0 merges 1, 2, 3 in that order) and share the result
         if (cq > 0) {
@@ -571,7 +573,7 @@ __global__ void __launch_bounds__(kXentThreads, 1)
           // every partial has been read above: slot 0 now carries the merged row
           s_x[trow] = make_float4(mx, sum, 0.0f, 0.0f);
           mbar_arrive(xch_b);
-          if (X.loss_sum) {  // one addition per warp: 8192 rows added one by one were off by 1.6e-6
+          if (X.loss_sum && blockIdx.z == 0) {  // one addition per warp: 8192 rows added one by one were off by 1.6e-6
             float l = valid ? (logf(sum) + mx - xl) * X.scale : 0.0f;
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
@@ -1710,7 +1712,12 @@ extern "C" rt_status rt_gemm_xent_bf16(const rt_gemm_xent_desc* d, rt_stream str
                cudaSuccess;
       }))
     return RT_ERR_CUDA;
-  k_gemm_xent_tc<<<dim3(d->m / kBM, G), kXentThreads, xent_smem(num_k, d->n), (cudaStream_t)stream>>>(ta, tb, X, num_k);
+  // few rows: several CTAs repeat pass 1 for the same 128 rows (in the same order, so with the same bits) and share out
+  // pass 2's tiles, as long as they all run at once (8192 rows, 64 CTAs: 121 us, 128: 87)
+  const uint32_t rows128 = d->m / kBM * G, ntiles = d->n / kArgBN;
+  uint32_t split = 1;
+  while (2 * split * rows128 <= (uint32_t)num_sms() && ntiles % (2 * split) == 0) split *= 2;
+  k_gemm_xent_tc<<<dim3(d->m / kBM, G, split), kXentThreads, xent_smem(num_k, d->n), (cudaStream_t)stream>>>(ta, tb, X, num_k);
   note_launch();
   RT_CHECK_LAUNCH();
   return RT_OK;

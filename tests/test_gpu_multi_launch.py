@@ -82,3 +82,32 @@ def test_colsum_order(rows, cols, groups):
     proposal.colsum_multi([(x, a)], groups=groups)
     proposal.colsum_multi([(odd[:, :cols], b)], groups=groups)
     assert torch.equal(a.view(torch.int32), b.view(torch.int32))
+
+
+@pytest.mark.parametrize("rows,classes,groups", [(128, 256, 1), (128, 4096, 1), (384, 1024, 2), (2432, 512, 1), (9472, 512, 1), (9600, 512, 1)])
+def test_xent_shares(rows, classes, groups):
+    """The gradient's tiles shared out among the CTAs of a row block (few rows: up to 16 shares) against the same rows
+    padded to a batch that leaves one share: the same bits, and the loss once."""
+    import torch
+    from cudart_b200 import proposal
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    pad = 128 * 160  # more row blocks than SMs: one share
+    a = torch.randn((groups, pad, 128), device="cuda", generator=g).to(torch.bfloat16)
+    b = torch.randn((groups * classes, 128), device="cuda", generator=g).to(torch.bfloat16)
+    bias = torch.randn(groups * classes, device="cuda", generator=g)
+    lab = torch.randint(0, classes, (groups, pad), dtype=torch.int32, device="cuda", generator=g)
+    got = {}
+    for m in (rows, pad):
+        x, y = a[:, :m].reshape(groups * m, 128).contiguous(), lab[:, :m].reshape(-1).contiguous()
+        out = torch.empty((groups * m, classes), device="cuda", dtype=torch.bfloat16)
+        out_t = torch.empty((groups * classes, m), device="cuda", dtype=torch.bfloat16)
+        loss, err = torch.zeros(1, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+        proposal.gemm_xent(x, b, bias, y, 1.0 / rows, out, out_t, loss=loss, err=err, groups=groups)
+        assert int(err.item()) == 0
+        got[m] = out.view(groups, m, classes)[:, :rows], out_t.view(groups, classes, m)[:, :, :rows], loss
+    assert torch.equal(got[rows][0].view(torch.int16), got[pad][0].view(torch.int16))
+    assert torch.equal(got[rows][1].view(torch.int16), got[pad][1].view(torch.int16))
+    logits = (a[:, :rows].double() @ b.view(groups, classes, 128).transpose(1, 2).double()) + bias.view(groups, 1, classes)
+    want = torch.nn.functional.cross_entropy(logits.reshape(-1, classes), lab[:, :rows].reshape(-1).long(), reduction="sum") / rows
+    # a row's loss holds a handful of float32 roundings and __expf errors of up to 2^-21: 1e-5 of the sum is wide of both
+    assert abs(float(got[rows][2]) - float(want)) <= 1e-5 * float(want) + 1e-6
