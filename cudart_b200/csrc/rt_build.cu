@@ -893,7 +893,7 @@ struct BuildLayout {
 };
 
 constexpr uint32_t kHitParts = 1184;  // 8 blocks per SM on 148 SMs
-constexpr uint32_t kHitSplit = 8;     // CTAs per mesh of the batched hit box
+constexpr uint32_t kHitSplit = 8;     // CTAs per mesh of the batched hit box, at most
 
 __host__ __device__ uint32_t morton_cap_dev(uint32_t n, uint32_t D) {
   uint64_t a = (D >= 31) ? (1ull << 32) : ((1ull << (D + 1)) - 1);
@@ -1215,6 +1215,7 @@ struct BatchArgs {
   // scratch
   float4* hits;           // [2M]
   float4* hitpart;        // [2 M kHitSplit]: the hit box shares of k_batch_hitbox
+  uint32_t hit_split;     // shares per mesh, at most kHitSplit
   uint32_t* hitdone;      // [M]: finished shares per mesh
   uint32_t* idx;          // [N] global face index in sorted order
   uint32_t* C;            // [N] split positions
@@ -1245,9 +1246,10 @@ struct BatchArgs {
 // Per-mesh hitbox: one 512-thread block per mesh, four loads in flight per
 // thread (the largest meshes bound the launch).
 __global__ __launch_bounds__(512) void k_batch_hitbox(BatchArgs B) {
-  // kHitSplit CTAs per mesh, each over its share of the mesh's vertices; the last of them combines the shares
-  const uint32_t m = blockIdx.x / kHitSplit, part = blockIdx.x % kHitSplit;
-  const uint32_t w0 = B.voff[m], w1 = B.voff[m + 1], share = (w1 - w0 + kHitSplit - 1) / kHitSplit;
+  // `split` CTAs per mesh, each over its share of the mesh's vertices; the last of them combines the shares
+  const uint32_t split = B.hit_split;
+  const uint32_t m = blockIdx.x / split, part = blockIdx.x % split;
+  const uint32_t w0 = B.voff[m], w1 = B.voff[m + 1], share = (w1 - w0 + split - 1) / split;
   const uint32_t v0 = min(w1, w0 + part * share), v1 = min(w1, v0 + share);
   if (part == 0 && threadIdx.x == 0) {
     B.acc_hdr[64 * (size_t)m + kHdrClusterValid] = 0;  // set again by the cluster build, if any
@@ -1278,28 +1280,39 @@ __global__ __launch_bounds__(512) void k_batch_hitbox(BatchArgs B) {
   s_mn[threadIdx.x] = f4min(f4min(mn[0], mn[1]), f4min(mn[2], mn[3]));
   s_mx[threadIdx.x] = f4max(f4max(mx[0], mx[1]), f4max(mx[2], mx[3]));
   __syncthreads();
-  for (int o = 256; o > 0; o >>= 1) {
-    if (threadIdx.x < o) {
-      s_mn[threadIdx.x] = f4min(s_mn[threadIdx.x], s_mn[threadIdx.x + o]);
-      s_mx[threadIdx.x] = f4max(s_mx[threadIdx.x], s_mx[threadIdx.x + o]);
-    }
-    __syncthreads();
+  if (threadIdx.x >= 32) return;  // (a barrier per step of the tree and eight CTAs a mesh: 118 us for 1024 meshes, now 73)
+  // the first warp pairs the threads 256, 128, .. 1 apart: 16 values per lane, then the lanes
+  float4 a[16], c[16];
+#pragma unroll
+  for (int w = 0; w < 16; ++w) { a[w] = s_mn[32 * w + threadIdx.x]; c[w] = s_mx[32 * w + threadIdx.x]; }
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+    for (int w = 0; w < o; ++w) { a[w] = f4min(a[w], a[w + o]); c[w] = f4max(c[w], c[w + o]); }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    auto down = [&](const float4& v) {
+      return make_float4(__shfl_down_sync(0xffffffffu, v.x, o), __shfl_down_sync(0xffffffffu, v.y, o), __shfl_down_sync(0xffffffffu, v.z, o),
+                         __shfl_down_sync(0xffffffffu, v.w, o));
+    };
+    a[0] = f4min(a[0], down(a[0]));
+    c[0] = f4max(c[0], down(c[0]));
   }
   if (threadIdx.x == 0) {
-    B.hitpart[2 * (size_t)blockIdx.x] = s_mn[0];
-    B.hitpart[2 * (size_t)blockIdx.x + 1] = s_mx[0];
+    B.hitpart[2 * (size_t)blockIdx.x] = a[0];
+    B.hitpart[2 * (size_t)blockIdx.x + 1] = c[0];
     __threadfence();
-    // the mesh's last share to finish combines its kHitSplit shares in share order (an empty share holds +-huge
+    // the mesh's last share to finish combines its shares in share order (an empty share holds +-huge
     // and changes nothing); nothing waits for it inside the launch
-    if (atomicAdd(B.hitdone + m, 1u) == kHitSplit - 1) {
+    if (atomicAdd(B.hitdone + m, 1u) == split - 1) {
       __threadfence();
-      float4 a = __ldcg(B.hitpart + 2 * (size_t)m * kHitSplit), b = __ldcg(B.hitpart + 2 * (size_t)m * kHitSplit + 1);
-      for (uint32_t p = 1; p < kHitSplit; ++p) {
-        a = f4min(a, __ldcg(B.hitpart + 2 * ((size_t)m * kHitSplit + p)));
-        b = f4max(b, __ldcg(B.hitpart + 2 * ((size_t)m * kHitSplit + p) + 1));
+      float4 lo = __ldcg(B.hitpart + 2 * (size_t)m * split), hi = __ldcg(B.hitpart + 2 * (size_t)m * split + 1);
+      for (uint32_t p = 1; p < split; ++p) {
+        lo = f4min(lo, __ldcg(B.hitpart + 2 * ((size_t)m * split + p)));
+        hi = f4max(hi, __ldcg(B.hitpart + 2 * ((size_t)m * split + p) + 1));
       }
-      B.hits[2 * m] = a;
-      B.hits[2 * m + 1] = b;
+      B.hits[2 * m] = lo;
+      B.hits[2 * m + 1] = hi;
     }
   }
 }
@@ -1559,7 +1572,10 @@ extern "C" rt_status rt_batch_build(const rt_batch_build_desc* d, rt_stream stre
   if (cudaMemsetAsync(B.topo_done, 0, 8, st) != cudaSuccess) return RT_ERR_CUDA;
   if (cudaMemsetAsync(B.hist, 0, (size_t)M * 64 * 4, st) != cudaSuccess) return RT_ERR_CUDA;
   if (cudaMemsetAsync(B.hitdone, 0, (size_t)M * 4, st) != cudaSuccess) return RT_ERR_CUDA;
-  k_batch_hitbox<<<M * kHitSplit, 512, 0, st>>>(B);
+  // eight shares of few meshes fill the chip (64 meshes: 106 us at four or eight, 132 at two); of many they are launches of
+  // CTAs with little to do (1024 meshes: 100 us at eight, 73 at four)
+  B.hit_split = M > 512 ? kHitSplit / 2 : kHitSplit;
+  k_batch_hitbox<<<M * B.hit_split, 512, 0, st>>>(B);
   k_batch_boxes_morton<<<fblocks, 256, 0, st>>>(B);
   note_launch(2);
   RT_CHECK_LAUNCH();

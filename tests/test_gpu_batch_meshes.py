@@ -31,3 +31,17 @@ def test_uneven_meshes(sizes, clusters):
         s = slice(int(ro[m]), int(ro[m + 1]))
         h = core.trace(one, O[s], D[s], schedule=dict(clusters=True) if clusters else None)
         assert torch.equal(h["id"], hits["id"][s]) and torch.equal(h["t"], hits["t"][s])
+
+
+@pytest.mark.parametrize("count", [511, 513])
+def test_hit_box_shares(count):
+    """The batched hit box in eight shares per mesh and in four (many meshes), down to fewer vertices than shares: the
+    codes of every mesh against its own build."""
+    import torch
+    from cudart_b200 import core
+    meshes = [scenes.soup(1 + (i * 37) % 29, seed=i) for i in range(count - 1)] + [scenes.soup(9001, seed=7)]
+    verts, faces, fo, vo = scenes.concat_batch(meshes)
+    t = core.batch_build(torch.from_numpy(verts).cuda(), torch.from_numpy(faces.view(np.int32)).cuda(), fo, vo)
+    for m in list(range(0, count - 1, 17)) + [count - 1]:
+        one = core.build_lbvh(torch.from_numpy(meshes[m].vertices).cuda(), torch.from_numpy(meshes[m].faces.view(np.int32)).cuda())
+        assert torch.equal(t.codes[fo[m]:fo[m + 1]], one.codes) and torch.equal(t.indices[fo[m]:fo[m + 1]], one.indices)
