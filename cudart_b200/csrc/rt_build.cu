@@ -214,7 +214,7 @@ __device__ __forceinline__ bool topo_shared(const TopoArgs& A, const uint32_t ca
   __shared__ uint32_t s_start[34], s_last[32];   // per level: its list's start and last entry (0: empty, above no a)
   __shared__ uint32_t s_vstar[34], s_made[33];   // per level: the a of its first visit at or after s_last; nodes made below it
   __shared__ uint32_t s_level_lo[34];
-  __shared__ uint32_t s_over, s_overrun, s_nondet, s_past, s_err, s_depth, s_leaves, s_mleaves;
+  __shared__ uint32_t s_overrun, s_nondet, s_past, s_err, s_depth, s_leaves, s_mleaves;
   const uint32_t tid = threadIdx.x, lane = tid & 31u, D = A.D;
   if (tid < 32) {
     const uint32_t v = A.level_hist ? A.level_hist[tid] : A.lev_count[tid];
@@ -233,7 +233,7 @@ __device__ __forceinline__ bool topo_shared(const TopoArgs& A, const uint32_t ca
     if (tid == 0) {
       s_vstar[32] = s_vstar[33] = kNone;
       s_made[32] = 0;
-      s_over = s_overrun = s_nondet = s_past = s_err = s_depth = 0;
+      s_overrun = s_nondet = s_past = s_err = s_depth = 0;
       ra[0] = A.pos_base;
       rb[0] = A.pos_base + A.n;
     }
@@ -263,7 +263,10 @@ __device__ __forceinline__ bool topo_shared(const TopoArgs& A, const uint32_t ca
     return S;
   };
   // A level's nodes stand in any order: a visit's place among the level's visits is its a. So children are handed their
-  // slots by a counter, and a level takes one barrier.
+  // slots by a counter, and a level takes one barrier. The same counter says whether they fit: nothing adds to it after
+  // the level's barrier, so every thread leaves at the same level (a flag shared by the levels would not do: the next
+  // level may set it before a slow warp has read it for this one).
+  const uint32_t room = min(cap, A.cap_m);
   uint32_t lo = 0, hi = 1, L = 0;
   for (; lo < hi; ++L) {
     if (tid == 0) s_level_lo[L] = lo;
@@ -296,9 +299,7 @@ __device__ __forceinline__ bool topo_shared(const TopoArgs& A, const uint32_t ca
         c = hi + __shfl_sync(0xffffffffu, c, 0) + 2u * (uint32_t)__popc(who & ((1u << lane) - 1u));
       }
       if (internal) {
-        if (c + 2 > min(cap, A.cap_m)) {
-          s_over = 1;
-        } else {
+        if (c + 2 <= room) {
           ra[c] = a; rb[c] = s; ra[c + 1] = s; rb[c + 1] = b;
           note(L + 1, a, s);
           note(L + 1, s, b);
@@ -307,9 +308,10 @@ __device__ __forceinline__ bool topo_shared(const TopoArgs& A, const uint32_t ca
       if (i < hi) child[i] = (uint16_t)(internal ? c : 0u);
     }
     __syncthreads();
-    if (s_over) return false;
+    const uint32_t made = s_made[L];
+    if (hi + made > room) return false;
     lo = hi;
-    hi += s_made[L];
+    hi += made;
   }
   if (tid == 0) s_level_lo[L] = lo;
   __syncthreads();
