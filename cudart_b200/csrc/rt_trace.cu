@@ -1111,7 +1111,7 @@ __device__ __forceinline__ void trace_warp_packet_clusters(const uint32_t r, con
             // every lane takes the warp's stack and its own slots of this record, nearest on top
             for (int i = 0; i < sp; ++i) {
               l_ref[i] = stack[i].x;
-              l_t[i] = __uint_as_float(stack[i].y);
+              l_t[i] = __uint_as_float(stack[i].y & ~3u);  // without the slot number: never above the entry distance
             }
             cswap_tr(t, k, 0, 1);
             cswap_tr(t, k, 2, 3);
