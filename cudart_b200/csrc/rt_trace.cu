@@ -1239,23 +1239,25 @@ __device__ __forceinline__ void trace_warp_packet_clusters(const uint32_t r, con
 // of shared memory per warp) holds active rays only: the warp takes 32 slots
 // at a time with one atomic, reads their tmax together, writes the inactive
 // ones (tmax <= 0) as misses at once and appends the others in slot order.
-// The warp steps in rounds of one kind: a lane that reaches a cluster holds it
-// until kHoldLanes lanes hold one (or no lane is at a record any more), and
-// then those lanes test their triangles together; until then the lanes at
-// records step on. About a quarter of the steps are clusters, and they cost
-// more than records do, so with both kinds in every step (a record for some
-// lanes, then a cluster for the others) few lanes were active in the longer
-// half: 10.6 of 32 on average, 14.2 in rounds. Bounce launch of the instanced
-// frame 8.03 -> 6.6 ms, 59.6M scattered rays over 1024 meshes 19.5 -> 16.1 ms;
-// kHoldLanes 10 / 14 / 16 / 20 there: 16.5 / 16.1 / 16.1 / 17+ ms. Each ray's
-// own sequence of steps is the one it would take alone. What bounds it now:
-// the latency of the dependent loads (46% of the stalls) and the L1 data pipe
-// (63% of its wavefronts). A round that tests one triangle per lane instead
-// of the whole cluster waits for memory once per triangle: 17.9 ms.
+// The warp steps in rounds of one kind: either the lanes at clusters test their
+// triangles together or the lanes at records step on, the clusters' turn coming
+// when at least half of the busy lanes hold one. About a quarter of the steps
+// are clusters, and they cost more than records do, so with both kinds in every
+// step (a record for some lanes, then a cluster for the others) few lanes were
+// active in the longer half: 10.6 of 32 on average. Bounce launch of the
+// instanced frame 8.03 -> 6.6 ms, 59.6M scattered rays over 1024 meshes
+// 19.5 -> 16.1 ms. A fixed number of held clusters (16) gave the same there, but
+// kept coherent lanes, which reach their clusters together, waiting until they
+// had drifted apart: camera rays at 1920 x 1080 on a terrain of 4.2M triangles
+// 1.08 ms with both kinds in every step, 1.72 with 16 held, 1.05 with half; a
+// third instead of half 1.03, and the scattered rays 2% slower. Each ray's own
+// sequence of steps is the one it would take alone. What bounds it now: the
+// latency of the dependent loads (46% of the stalls) and the L1 data pipe (63%
+// of its wavefronts). A round that tests one triangle per lane instead of the
+// whole cluster waits for memory once per triangle: 17.9 ms.
 // `slot_ray` maps a slot to a ray (false for a slot without one); `mesh_args`
 // sets the cluster-tree arguments of an active ray's mesh.
 constexpr uint32_t kRefillQueue = 64;
-constexpr uint32_t kHoldLanes = 16;
 template <bool kCount, class SlotRay, class MeshArgs>
 __device__ __forceinline__ void refill_walks(const TraceArgs& A, uint32_t* counter, const uint32_t slots, const uint32_t threshold,
                                              uint32_t* q_ray, float* q_tmax, const SlotRay& slot_ray, const MeshArgs& mesh_args) {
@@ -1350,7 +1352,7 @@ __device__ __forceinline__ void refill_walks(const TraceArgs& A, uint32_t* count
     // one round: either every lane at a record tests it, or every lane at a cluster tests its triangles
     const uint32_t held = __ballot_sync(0xffffffffu, busy && (ref & kClusterLeaf) != 0);
     const uint32_t walking = __ballot_sync(0xffffffffu, busy);
-    const bool tri_round = (uint32_t)__popc(held) >= kHoldLanes || held == walking;
+    const bool tri_round = 2 * __popc(held) >= __popc(walking);
     if (!busy || tri_round != ((ref & kClusterLeaf) != 0)) continue;
     if (!cluster_ref_ok(ref, C.n, steps)) {
       if (A.err) atomicOr(A.err, (uint32_t)RT_DEVERR_ACCEL_MISSING);
@@ -1387,7 +1389,6 @@ __device__ __forceinline__ void refill_walks(const TraceArgs& A, uint32_t* count
         float th, u, v;
         if (mt_test(o, d, zu, zv, v0, e1, e2, th, u, v) && (th < bt || (best >= 0 && th == bt && (int32_t)pos < best))) {
           best = (int32_t)pos; bt = th; bu = u; bv = v;
-
         }
       };
       float4 a0 = ldg4(tp), a1 = ldg4(tp + 1), a2 = ldg4(tp + 2);
