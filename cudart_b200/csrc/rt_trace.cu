@@ -1052,11 +1052,14 @@ __device__ __forceinline__ void trace_warp_packet_clusters(const uint32_t r, con
     int sp = 0;                                    // the same for every lane, as ref is
     uint32_t steps = 0;
     bool alone = false;  // this warp left the packet walk
-    float cur_t = 0.0f;  // counters only: the warp's entry distance of the node at hand
+    // counters only: this ray's own entry distance of the node at hand (+inf: not entered) and of the stacked ones. A ray
+    // counts the records and clusters that it enters itself within its reach, whatever the warp visits.
+    float cur_t = 0.0f, own[kCount ? kStack : 1];
     uint32_t l_ref[kAlone ? kStack : 1];
     float l_t[kAlone ? kStack : 1];
     auto test_cluster = [&]() {
       const uint32_t p0 = ref & kClusterFirstMask, p1 = p0 + ((ref >> 28) & 7u) + 1u;
+      if (kCount && cur_t != INFINITY && cur_t <= reach) tests += p1 - p0;
       for (uint32_t pos = p0; pos < p1; ++pos) {
         const float4 v0 = ldg4(tris + 3 * (size_t)pos);
         const float4 e1 = ldg4(tris + 3 * (size_t)pos + 1);
@@ -1068,7 +1071,6 @@ __device__ __forceinline__ void trace_warp_packet_clusters(const uint32_t r, con
         }
       }
       if (live) reach = bt * kCullSlack;
-      if (kCount && live && cur_t <= reach) tests += p1 - p0;
     };
     for (;;) {
       if (!cluster_ref_ok(ref, C.n, steps)) {
@@ -1095,7 +1097,7 @@ __device__ __forceinline__ void trace_warp_packet_clusters(const uint32_t r, con
             k[q] = u4c(wr, q);
           }
         }
-        if (kCount && live && cur_t <= reach) visits += 4;
+        if (kCount && cur_t != INFINITY && cur_t <= reach) visits += 4;
         // the warp's smallest entry distance of each slot (not below 0), the slot number in its two lowest bits: rounded
         // down by at most three units in the last place, so a stacked slot is never skipped too early
         bool mine = false;
@@ -1148,12 +1150,17 @@ __device__ __forceinline__ void trace_warp_packet_clusters(const uint32_t r, con
           const uint32_t lo = (kk & 1u) ? k[1] : k[0], hi = (kk & 1u) ? k[3] : k[2];
           return (kk & 2u) ? hi : lo;
         };
+        auto slot_t = [&](uint32_t kk) {
+          const float lo = (kk & 1u) ? t[1] : t[0], hi = (kk & 1u) ? t[3] : t[2];
+          return (kk & 2u) ? hi : lo;
+        };
         if (key[0] < kPacketMiss) {
 #pragma unroll
           for (int q = 3; q >= 1; --q) {
             if (key[q] < kPacketMiss) {
               if (sp < kStack) {
                 stack[sp] = make_uint2(slot_ref(key[q]), key[q]);
+                if (kCount) own[sp] = slot_t(key[q]);
                 ++sp;
               } else if (A.err) {
                 atomicOr(A.err, (uint32_t)RT_DEVERR_STACK_OVERFLOW);
@@ -1161,7 +1168,7 @@ __device__ __forceinline__ void trace_warp_packet_clusters(const uint32_t r, con
             }
           }
           ref = slot_ref(key[0]);
-          if (kCount) cur_t = __uint_as_float(key[0]);
+          if (kCount) cur_t = slot_t(key[0]);
           __syncwarp();
           continue;
         }
@@ -1174,7 +1181,7 @@ __device__ __forceinline__ void trace_warp_packet_clusters(const uint32_t r, con
         const uint2 top = stack[--sp];
         if (__any_sync(0xffffffffu, __uint_as_float(top.y & ~3u) <= reach)) {
           ref = top.x;
-          if (kCount) cur_t = __uint_as_float(top.y & ~3u);
+          if (kCount) cur_t = own[sp];
           more = true;
           break;
         }

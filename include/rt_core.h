@@ -295,7 +295,8 @@ typedef struct rt_trace_desc {
   float* hit_t;             /* out: t of the hit, or tmax on a miss (may alias tmax, as CUDABuffer depths do) */
   float* hit_uv;            /* out: float2 (u, v); (0, 0) on a miss */
   uint32_t* ray_visits;     /* optional out: nodes popped per ray */
-  uint32_t* ray_tests;      /* optional out: triangles tested per ray */
+  uint32_t* ray_tests;      /* optional out: triangles tested per ray. (RT_TRACE_COOP and RT_TRACE_PACKET, where a warp works
+                               for all its rays: a ray's counts are the boxes and triangles that it wants itself) */
   uint32_t* error_word;     /* optional device word: RT_DEVERR_* bits are OR-ed in */
   const void* accel;        /* optional traversal blob from rt_lbvh_build (with tris): faster, same results */
   uint32_t face_count_hint; /* the face count the blob was built for (required with accel) */
@@ -307,8 +308,8 @@ typedef struct rt_trace_desc {
   const uint32_t* ray_order; /* optional permutation from rt_ray_order: threads take rays in this order */
   uint32_t treelet_depth;   /* persistent 4-wide walks: levels of 4-wide records below the root (0..4, at most 85
                                records, 10.9 KB) that each CTA copies to shared memory and reads from there (0: none) */
-  uint32_t lane_threshold;  /* RT_TRACE_PACKET: a warp leaves the packet walk for per-lane walks (from the same stacks)
-                               once fewer than this many lanes still want the node it is at (0: never);
+  uint32_t lane_threshold;  /* RT_TRACE_PACKET: a warp leaves the packet walk for per-lane walks (from the same stack) at a
+                               record of whose slots fewer than this many lanes enter any (0: never);
                                RT_TRACE_REFILL: a warp fetches new rays for its idle lanes once this many are idle */
 } rt_trace_desc;
 
