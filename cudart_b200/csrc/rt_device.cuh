@@ -328,6 +328,10 @@ static __global__ __launch_bounds__(256) void k_wide_nodes(const float4* __restr
 }
 
 constexpr int kStack = 64;
+// Stack of the walks of 4-wide node records. Such a record takes two levels of the tree and pushes up to three entries
+// where the two-child walk pushes two, so 96 take every tree that 64 take there (with 64, a tree of 45 levels whose boxes
+// all hold the ray lost the farthest subtrees).
+constexpr int kWideStack = 96;
 constexpr float kBoxPad = 1.220703125e-4f;      // 2^-13
 constexpr float kCullSlack = 1.0001220703125f;  // 1 + 2^-13
 

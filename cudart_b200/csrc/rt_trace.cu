@@ -276,8 +276,9 @@ __device__ __forceinline__ void trace_ray_accel(const uint32_t r, const TraceArg
     const float ix = 1.0f / fix_dir(d.x), iy = 1.0f / fix_dir(d.y), iz = 1.0f / fix_dir(d.z);
     const float4 oi = scaled_origin(o, ix, iy, iz);
     const float zu = o.w * 0.0f, zv = d.w * 0.0f;
-    uint32_t st_ref[kStack];
-    float st_t[kStack];
+    constexpr int kDepth = kWide ? kWideStack : kStack;
+    uint32_t st_ref[kDepth];
+    float st_t[kDepth];
     int sp = 0;
     const uint32_t root = C.stage ? kStagedBit : __ldg(C.hdr);
     uint32_t ref = root, skip = kNoSkip;
@@ -315,7 +316,7 @@ __device__ __forceinline__ void trace_ray_accel(const uint32_t r, const TraceArg
 #pragma unroll
             for (int k = 3; k >= 1; --k) {
               if (wt[k] != INFINITY) {
-                if (sp < kStack) {
+                if (sp < kDepth) {
                   st_ref[sp] = wr[k];
                   st_t[sp] = wt[k];
                   ++sp;
@@ -342,7 +343,7 @@ __device__ __forceinline__ void trace_ray_accel(const uint32_t r, const TraceArg
         }
         if (ha && hb) {
           const bool a_first = ta <= tb;
-          if (sp < kStack) {
+          if (sp < kDepth) {
             st_ref[sp] = a_first ? rb : ra;
             st_t[sp] = a_first ? tb : ta;
             ++sp;
@@ -523,8 +524,9 @@ __device__ __forceinline__ void trace_warp_coop(const uint32_t r, const bool val
   const float ix = 1.0f / fix_dir(d.x), iy = 1.0f / fix_dir(d.y), iz = 1.0f / fix_dir(d.z);
   const float4 oi = scaled_origin(o, ix, iy, iz);
   const float zu = o.w * 0.0f, zv = d.w * 0.0f;
-  uint32_t st_ref[kStack];
-  float st_t[kStack];
+  constexpr int kDepth = kWide ? kWideStack : kStack;
+  uint32_t st_ref[kDepth];
+  float st_t[kDepth];
   int sp = 0;
   const uint32_t root = C.stage ? kStagedBit : __ldg(C.hdr);
   uint32_t ref = root, skip = kNoSkip;
@@ -564,7 +566,7 @@ __device__ __forceinline__ void trace_warp_coop(const uint32_t r, const bool val
 #pragma unroll
             for (int k = 3; k >= 1; --k) {
               if (wt[k] != INFINITY) {
-                if (sp < kStack) {
+                if (sp < kDepth) {
                   st_ref[sp] = wr[k];
                   st_t[sp] = wt[k];
                   ++sp;
@@ -591,7 +593,7 @@ __device__ __forceinline__ void trace_warp_coop(const uint32_t r, const bool val
         }
         if (ha && hb) {
           const bool a_first = ta <= tb;
-          if (sp < kStack) {
+          if (sp < kDepth) {
             st_ref[sp] = a_first ? rb : ra;
             st_t[sp] = a_first ? tb : ta;
             ++sp;
