@@ -28,6 +28,7 @@ TRACE_WIDE = 0x4
 TRACE_CLUSTERS = 0x8
 TRACE_PACKET = 0x10
 TRACE_REFILL = 0x20
+TRACE_PER_LANE = 0x40
 ACCEL_CLUSTERS = 0x2
 MAX_RAYS = 0x7FFFFFFF  # RT_MAX_RAYS: the most rays one trace call takes
 

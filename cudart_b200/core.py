@@ -322,7 +322,8 @@ def trace_desc(tree: Tree, orig, dir, tmax=None, id_mode: int = 0, counters: boo
             d.lane_threshold = int(sch.get("lane_threshold", 0))  # packet walks: fall back to per-lane walks
         d.schedule = ((_abi.TRACE_WHILE_WHILE if sch.get("while_while", False) else 0) | (_abi.TRACE_COOP if sch.get("coop", False) else 0)
                       | (_abi.TRACE_WIDE if sch.get("wide", False) else 0) | (_abi.TRACE_CLUSTERS if sch.get("clusters", False) else 0)
-                      | (_abi.TRACE_PACKET if sch.get("packet", False) else 0) | (_abi.TRACE_REFILL if sch.get("refill", False) else 0))
+                      | (_abi.TRACE_PACKET if sch.get("packet", False) else 0) | (_abi.TRACE_REFILL if sch.get("refill", False) else 0)
+                      | (_abi.TRACE_PER_LANE if sch.get("per_lane", False) else 0))
         if sch.get("sorted", False):
             order = ray_order(orig, dir, tmax, tree_box(tree), ray_count=R, stream=stream)
             out["_order"] = order  # keep it alive until the trace has run

@@ -639,13 +639,35 @@ __device__ __forceinline__ void trace_warp_coop(const uint32_t r, const bool val
       // leaves of more than 256 triangles (tree_complete = 0) keep the groups
       // past 32 to this lane: they are tested below by the owner alone
     }
-    // 3. spread the warp's (ray, group) items over the lanes
-    // (t bits, position) of the best hit so far; with no hit yet, (tmax bits, 0),
-    // which no accepted hit equals (t < tmax is required)
-    const unsigned long long key0 = ((unsigned long long)__float_as_uint(bt + 0.0f) << 32) | (uint32_t)(best >= 0 ? best : 0);
-    coop_items<8>(lane, mask, first, cnt, C.F, o, d, zu, zv, A.tris, key0, bt, bu, bv, s_key, s_uvt);
-    // 4. read back the merged best and move on
-    if (has_leaf) {
+    // 3. the groups' triangles. The lanes of coherent rays want much the same groups of the same leaf: each tests its own,
+    // a load serving the whole warp, if the groups that any lane wants would be shared by two lanes or more of 32 on
+    // average (counting up to 16 items as one step). Else the warp's (ray, group) items are spread over the lanes. Camera
+    // rays of the 2^20-triangle soup at 1920 x 1080 with items only, then with both: 2.51 -> 1.80 ms in rows, 2.42 -> 1.39
+    // in pixel tiles; their bounces 2.81 -> 2.74; terrains are within 2%. Deciding for the
+    // lanes' own groups twice as readily loses 5% on soups, four times as readily 20 to 50% on bounces and terrains.
+    const uint32_t any = __reduce_or_sync(0xffffffffu, mask), items = __reduce_add_sync(0xffffffffu, (uint32_t)__popc(mask));
+    if (16u * ((uint32_t)__popc(any) - 1u) < items) {
+      for (uint32_t gs = any; gs; gs &= gs - 1u) {
+        const uint32_t g = (uint32_t)__ffs((int)gs) - 1u;
+        if (!(mask >> g & 1u)) continue;
+        const uint32_t kend = min(cnt, g * 8 + 8);
+        for (uint32_t k = g * 8; k < kend; ++k) {
+          const uint32_t pos = first + k;
+          const float4* tp = A.tris + 3 * ((size_t)C.F + pos);
+          const float4 v0 = ldg4(tp), e1 = ldg4(tp + 1), e2 = ldg4(tp + 2);
+          float t, u, v;
+          if (!mt_test(o, d, zu, zv, v0, e1, e2, t, u, v)) continue;
+          if (t < bt || (best >= 0 && t == bt && (int32_t)pos < best)) {
+            best = (int32_t)pos; bt = t; bu = u; bv = v;
+            best_phase = phase;
+          }
+        }
+      }
+    } else if (items) {
+      // (t bits, position) of the best hit so far; with no hit yet, (tmax bits, 0),
+      // which no accepted hit equals (t < tmax is required)
+      const unsigned long long key0 = ((unsigned long long)__float_as_uint(bt + 0.0f) << 32) | (uint32_t)(best >= 0 ? best : 0);
+      coop_items<8>(lane, mask, first, cnt, C.F, o, d, zu, zv, A.tris, key0, bt, bu, bv, s_key, s_uvt);
       const unsigned long long k = s_key[lane];
       if (k < key0) {
         best = (int32_t)(k & 0xFFFFFFFFu);
@@ -653,6 +675,9 @@ __device__ __forceinline__ void trace_warp_coop(const uint32_t r, const bool val
         bu = uvt.x; bv = uvt.y; bt = uvt.z;
         best_phase = phase;
       }
+    }
+    // 4. move on
+    if (has_leaf) {
       // groups beyond the first 32 (leaves of more than 256 triangles): this lane alone
       for (uint32_t g = 32; g * 8 < cnt; ++g) {
         const uint32_t gbase = __ldg(C.leaves + (C.F + ~ref)).z;
@@ -2068,12 +2093,20 @@ rt_status launch_clusters(const rt_trace_desc* d, const TraceArgs& A, cudaStream
   return RT_OK;
 }
 
-// A call that asks for no schedule (and no counters) gets the warp-cooperative walk of the 4-wide records too: node
-// trees stop at leaves of up to 223 triangles, and a lane alone with such a leaf keeps 31 others waiting. Camera
-// rays and bounces together, per-lane walk -> this one: 128 x 128 terrain at 512 x 512 0.82 -> 0.32 ms, 2^14-triangle
-// soup at 400 x 300 0.78 -> 0.56 ms, 2^17 at 1000 x 700 3.15 -> 1.95 ms, 2^20 at 1920 x 1080 7.32 -> 5.51 ms (there
-// its camera rays alone lose, 2.29 -> 2.58 ms: neighbouring rays read the same leaves together).
-bool no_schedule(const rt_trace_desc* d) { return d->schedule == 0 && !d->work_counter && !d->ray_visits && !d->ray_tests; }
+// A call that asks for no schedule (and no counters) gets the warp-cooperative walk of the 4-wide records: node trees
+// stop at leaves of up to 223 triangles, and a lane alone with such a leaf keeps 31 others waiting. Camera rays in rows
+// at 1920 x 1080, per-lane two-child walk -> this one: 128 x 128 terrain 445 -> 193 us, 512 x 512 1.83 -> 0.60 ms, soups
+// of 2^14 / 2^16 / 2^18 / 2^20 triangles 1.22 -> 1.17, 1.86 -> 1.68, 1.78 -> 1.41, 2.26 -> 1.80 ms; their bounces 3.19 ->
+// 2.50, 4.79 -> 3.10, 4.22 -> 2.24, 4.70 -> 2.74. Where hundreds of rays share a triangle the lanes agree in nearly
+// everything and the sharing is only work: 4096 triangles at 3840 x 2160 (2025 rays each) 1.67 -> 1.92 ms in rows, at
+// 1920 x 1080 (506) 567 -> 579 us; in pixel tiles 16384 at 1920 x 1080 (127) 826 -> 906. So rays without a tmax of their own,
+// as camera rays are, keep the per-lane walk from 400 rays a triangle in rows and 96 in tiles (terrains gain
+// there still: 7938 triangles in tiles, 261 rays each, 194 us per lane and 134 shared; 3042, 682, 110 and 92).
+bool default_coop(const rt_trace_desc* d) {
+  if (d->schedule || d->work_counter || d->ray_visits || d->ray_tests) return false;
+  const bool tiles = d->image_width && !d->ray_order && d->ray_count % d->image_width == 0;
+  return d->tmax || d->ray_count < (tiles ? 96ull : 400ull) * d->face_count_hint;
+}
 
 // Blob traversal launch for every schedule of rt_trace_desc.
 template <bool kSeed, bool kWide>
@@ -2096,7 +2129,7 @@ rt_status launch_accel_w(const rt_trace_desc* d, const TraceArgs& A, const SeedA
   const uint32_t pblocks = (uint32_t)sms() * (d->persistent_blocks_per_sm ? d->persistent_blocks_per_sm : 8u);
   const uint32_t sblocks = (M.slots + 127) / 128;
   if (d->work_counter && cudaMemsetAsync(d->work_counter, 0, 4, st) != cudaSuccess) return RT_ERR_CUDA;
-  if ((d->schedule & RT_TRACE_COOP) || (!kSeed && no_schedule(d))) {
+  if ((d->schedule & RT_TRACE_COOP) || (!kSeed && default_coop(d))) {
     if (d->work_counter) {
       if (count) k_trace_coop_persistent<true, kSeed, kWide><<<pblocks, 128, stage_smem, st>>>(A, C, M, d->work_counter, S);
       else k_trace_coop_persistent<false, kSeed, kWide><<<pblocks, 128, stage_smem, st>>>(A, C, M, d->work_counter, S);
@@ -2124,7 +2157,7 @@ rt_status launch_accel_w(const rt_trace_desc* d, const TraceArgs& A, const SeedA
 template <bool kSeed>
 rt_status launch_accel(const rt_trace_desc* d, const TraceArgs& A, const SeedArgs& S, cudaStream_t st) {
   if (d->schedule & RT_TRACE_CLUSTERS) return kSeed ? RT_ERR_UNSUPPORTED : launch_clusters(d, A, st);
-  if ((d->schedule & RT_TRACE_WIDE) || (!kSeed && no_schedule(d))) return launch_accel_w<kSeed, true>(d, A, S, st);
+  if ((d->schedule & RT_TRACE_WIDE) || (!kSeed && default_coop(d))) return launch_accel_w<kSeed, true>(d, A, S, st);
   return launch_accel_w<kSeed, false>(d, A, S, st);
 }
 

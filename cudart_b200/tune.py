@@ -31,11 +31,11 @@ def candidates(image_width: int):
     widths = [0, image_width] if image_width else [0]
     out = []
     for w, ww in itertools.product(widths, (False, True)):
-        out.append({"image_width": w, "persistent": False, "blocks_per_sm": 0, "while_while": ww, "sorted": False})
+        out.append({"image_width": w, "persistent": False, "blocks_per_sm": 0, "while_while": ww, "sorted": False, "per_lane": True})
         for bps in (8, 16):
             out.append({"image_width": w, "persistent": True, "blocks_per_sm": bps, "while_while": ww, "sorted": False})
     for ww, (p, bps) in itertools.product((False, True), ((False, 0), (True, 16))):
-        out.append({"image_width": 0, "persistent": p, "blocks_per_sm": bps, "while_while": ww, "sorted": True})
+        out.append({"image_width": 0, "persistent": p, "blocks_per_sm": bps, "while_while": ww, "sorted": True, "per_lane": True})
     # warp-cooperative leaf tests (always while-while)
     for w, srt, (p, bps) in itertools.product(widths, (False, True), ((False, 0), (True, 8), (True, 16))):
         if srt and w:

@@ -304,7 +304,9 @@ typedef struct rt_trace_desc {
   uint32_t image_width;     /* > 0 and dividing ray_count: rays are a row-major image; a warp takes an 8x4 pixel tile */
   uint32_t* work_counter;   /* optional device word: persistent warps fetch rays through it (the call zeroes it) */
   uint32_t persistent_blocks_per_sm; /* with work_counter: CTAs of 128 threads per SM (0 = 8) */
-  uint32_t schedule;        /* RT_TRACE_* bits */
+  uint32_t schedule;        /* RT_TRACE_* bits. 0 without a work_counter: the library chooses, by the ray and face counts and
+                               whether tmax is given, between the per-lane two-child walk (RT_TRACE_PER_LANE; always, with
+                               ray_visits or ray_tests) and RT_TRACE_COOP | RT_TRACE_WIDE */
   const uint32_t* ray_order; /* optional permutation from rt_ray_order: threads take rays in this order */
   uint32_t treelet_depth;   /* persistent 4-wide walks: levels of 4-wide records below the root (0..4, at most 85
                                records, 10.9 KB) that each CTA copies to shared memory and reads from there (0: none) */
@@ -329,6 +331,7 @@ typedef struct rt_trace_desc {
                                   it claims 32 slots per atomic, writes the inactive ones (tmax <= 0) as misses at once and
                                   queues the active ones for its lanes; a round of the warp steps lanes at records or lanes at
                                   clusters, never both (WHILE_WHILE is ignored) */
+#define RT_TRACE_PER_LANE 0x40u /* each lane walks a ray of its own: asks for that where no other bit is given (rt_trace_closest) */
 
 /* A tracing order for incoherent rays: ray indices sorted by direction octant,
  * then by the Morton code of the origin inside box (min xyz, max xyz, HOST);
