@@ -1082,11 +1082,9 @@ extern "C" rt_status rt_lbvh_build(const rt_build_desc* d, rt_stream stream_) {
     RT_CHECK_LAUNCH();
   }
   // 3. sort (code, index)
-  if (cudaMemsetAsync(L.err, 0, 16, st) != cudaSuccess) return RT_ERR_CUDA;
-  rt_status s = radix_sort_pairs(codes, d->indices, n, 0, 32, 1, L.sort_scratch, L.sort_bytes, st);
-  if (s != RT_OK) return s;
   // 4. per-level split lists
-  s = sort_split_levels(codes, n, L.C, L.lev_count, 256, L.sort_scratch, L.sort_bytes, st);
+  if (cudaMemsetAsync(L.err, 0, 16, st) != cudaSuccess) return RT_ERR_CUDA;
+  rt_status s = sort_codes_and_levels(codes, d->indices, n, L.C, L.lev_count, 256, L.sort_scratch, L.sort_bytes, st);
   if (s != RT_OK) return s;
   // 5. Morton top tree
   {
@@ -1582,9 +1580,7 @@ extern "C" rt_status rt_batch_build(const rt_batch_build_desc* d, rt_stream stre
   note_launch(2);
   RT_CHECK_LAUNCH();
   // every mesh's faces in Morton order (a mesh is a segment of the sort), then its split positions in level order
-  rt_status s = radix_sort_pairs(B.codes, B.idx, N, 0, 32, 1, sort_scratch, sort_bytes, st, B.foff, M);
-  if (s != RT_OK) return s;
-  s = sort_split_levels(B.codes, N, B.C, B.hist, 64, sort_scratch, sort_bytes, st, B.foff, M);
+  rt_status s = sort_codes_and_levels(B.codes, B.idx, N, B.C, B.hist, 64, sort_scratch, sort_bytes, st, B.foff, M);
   if (s != RT_OK) return s;
   if (!topo_smem_once(k_batch_topo, kBatchTopoNodes)) return RT_ERR_CUDA;
   k_batch_topo<<<M, kBatchTopoThreads, kBatchTopoNodes * kTopoNodeBytes, st>>>(B);

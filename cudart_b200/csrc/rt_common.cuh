@@ -133,20 +133,18 @@ constexpr size_t radix_scratch_bytes_of(uint32_t n) {
   return 2 * a + 4 * (4 * tiles * 256 + 4 * 64 + 4 * 256) + 256;
 }
 size_t radix_scratch_bytes(uint32_t n);
-// Scratch of a sort in M segments, any n (radix_scratch_bytes covers M = 1 with more than 4096 keys).
+// Scratch of a build's sorts in M segments, any n.
 size_t segment_sort_scratch_bytes(uint32_t n, uint32_t M);
 // Stable sort of (key, value) pairs by bits [begin_bit, end_bit) of the key; init_vals: the values are the keys' input
-// positions. With M > 1 segments (seg_off: DEVICE, M + 1 ascending offsets from 0 to n) each segment is sorted by itself.
+// positions.
 rt_status radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_t begin_bit, uint32_t end_bit, int init_vals,
-                           void* scratch, size_t scratch_bytes, cudaStream_t stream, const uint32_t* seg_off = nullptr, uint32_t M = 1);
-// The split positions of sorted Morton codes in level order, per segment: position i + 1 at level clz(code[i] ^ code[i + 1]),
-// ascending inside a level; positions without a split (equal codes, and a segment's last) at level 32, after the others.
-// splits: n words, a segment's in its own places; level_counts[m * count_stride + l]: positions of level l (l < 64 and
-// below count_stride) of a segment that is not empty.
-rt_status sort_split_levels(const uint32_t* codes, uint32_t n, uint32_t* splits, uint32_t* level_counts, uint32_t count_stride,
-                            void* scratch, size_t scratch_bytes, cudaStream_t stream, const uint32_t* seg_off = nullptr,
-                            uint32_t M = 1);
-// First chunk of segment m, whose keys start at F, in a sort with chunks of per_chunk keys (chunks never span segments).
-__host__ __device__ __forceinline__ uint32_t sort_chunk_base(uint32_t F, uint32_t m, uint32_t per_chunk) { return F / per_chunk + m; }
+                           void* scratch, size_t scratch_bytes, cudaStream_t stream);
+// The sorts of a build, each segment by itself (M > 1: seg_off, DEVICE, M + 1 ascending offsets from 0 to n). The codes
+// with their input positions (into idx), stably; then the split positions of the sorted codes in level order: position
+// i + 1 at level clz(code[i] ^ code[i + 1]), ascending inside a level; positions without a split (equal codes, and a
+// segment's last) at level 32, after the others. splits: n words, a segment's in its own places;
+// level_counts[m * count_stride + l]: positions of level l (l < 64 and below count_stride) of a segment that is not empty.
+rt_status sort_codes_and_levels(uint32_t* codes, uint32_t* idx, uint32_t n, uint32_t* splits, uint32_t* level_counts, uint32_t count_stride,
+                                void* scratch, size_t scratch_bytes, cudaStream_t stream, const uint32_t* seg_off = nullptr, uint32_t M = 1);
 
 }  // namespace rt

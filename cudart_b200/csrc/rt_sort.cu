@@ -16,7 +16,10 @@
 //     while the next tile's keys are on their way. No CTA waits for another.
 //   * segments (the meshes of a batched build) are sorted side by side: every
 //     chunk belongs to one segment, and counts are added up inside it, so the
-//     segment number is never a sort key.
+//     segment number is not a sort key of those passes. Where segments are short
+//     on average, the short ones go several to a CTA, which does every pass of
+//     both of a build's sorts in shared memory (k_sort_segments); so does a
+//     whole build of at most 4096 faces.
 //   * n <= 4096, one segment: a single CTA does every pass in shared memory
 //     (one launch).
 // Traffic per pass: keys (and values) read once and written once, and the keys
@@ -93,6 +96,14 @@ __device__ __forceinline__ uint32_t match_digit(uint32_t d) {
   return m;
 }
 
+// First chunk of segment m, whose keys start at F, among chunks of per_chunk keys (chunks never span segments). Where
+// short segments have no chunks, a segment has more than kSegWindow keys, and the windows before it serve as well as the
+// segments before it to keep one segment's chunks apart from the next one's, however many segments there are.
+constexpr uint32_t kSegWindow = 2048;
+__host__ __device__ __forceinline__ uint32_t chunk_base(uint32_t F, uint32_t m, uint32_t per_chunk, uint32_t short_segs) {
+  return F / per_chunk + (short_segs ? F / kSegWindow : m);
+}
+
 // One pass over chunked keys. kMode 0: keys_in are the keys; 1: the key of position i is the split level of the sorted
 // Morton codes in keys_in, clz(code[i] ^ code[i + 1]) (32 for equal codes and for a segment's last position).
 struct PassArgs {
@@ -104,6 +115,7 @@ struct PassArgs {
   uint32_t per_chunk;        // keys of a whole chunk
   const uint32_t* seg_off;   // null: one segment, 0 .. n
   const uint32_t* chunk_seg; // segment of each chunk (~0: no chunk); with seg_off
+  uint32_t short_segs;       // segments of at most kSegWindow keys have no chunks
   uint32_t* rows;            // [chunks][256]
   uint32_t* groups;          // [chunks / kGroup + 1][256], zero before the pass
   uint32_t* totals;          // optional: [segments][totals_stride] digit counts
@@ -123,7 +135,7 @@ __device__ __forceinline__ bool chunk_of(const PassArgs& P, uint32_t c, Chunk& C
     if (C.seg == ~0u) return false;
     C.seg_begin = __ldg(P.seg_off + C.seg);
     C.seg_end = __ldg(P.seg_off + C.seg + 1);
-    C.first_chunk = sort_chunk_base(C.seg_begin, C.seg, P.per_chunk);
+    C.first_chunk = chunk_base(C.seg_begin, C.seg, P.per_chunk, P.short_segs);
   }
   C.n_chunks = (C.seg_end - C.seg_begin + P.per_chunk - 1) / P.per_chunk;
   C.begin = C.seg_begin + (c - C.first_chunk) * P.per_chunk;
@@ -360,17 +372,178 @@ __global__ __launch_bounds__(kScThreads, kItems == 16 ? 2 : 3) void k_sort_scatt
 }
 
 // The segment of every chunk (~0 for a gap of the chunk numbering).
-__global__ __launch_bounds__(256) void k_chunk_segs(const uint32_t* __restrict__ off, uint32_t M, uint32_t per_chunk, uint32_t chunks,
-                                                    uint32_t* __restrict__ chunk_seg) {
+__global__ __launch_bounds__(256) void k_chunk_segs(const uint32_t* __restrict__ off, uint32_t M, uint32_t per_chunk, uint32_t short_segs,
+                                                    uint32_t chunks, uint32_t* __restrict__ chunk_seg) {
   const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= chunks) return;
-  uint32_t lo = 0, hi = M - 1;  // largest m with sort_chunk_base(off[m], m) <= c
+  uint32_t lo = 0, hi = M - 1;  // largest m with chunk_base(off[m], m) <= c
   while (lo < hi) {
     const uint32_t mid = (lo + hi + 1) >> 1;
-    if (sort_chunk_base(__ldg(off + mid), mid, per_chunk) <= c) lo = mid; else hi = mid - 1;
+    if (chunk_base(__ldg(off + mid), mid, per_chunk, short_segs) <= c) lo = mid; else hi = mid - 1;
   }
-  const uint32_t F = __ldg(off + lo), j = c - sort_chunk_base(F, lo, per_chunk);
-  chunk_seg[c] = (uint64_t)j * per_chunk < __ldg(off + lo + 1) - F ? lo : ~0u;
+  const uint32_t F = __ldg(off + lo), n = __ldg(off + lo + 1) - F, j = c - chunk_base(F, lo, per_chunk, short_segs);
+  const bool has = (uint64_t)j * per_chunk < n && !(short_segs && n <= kSegWindow);
+  chunk_seg[c] = has ? lo : ~0u;
+}
+
+// Both sorts of a build for short segments: a CTA takes the segments of at most `window` keys that start in its window of
+// so many positions (a longer one is the window's last, and left out), at most 4096 keys in all, and does every pass in
+// shared memory: by code (four digits), by segment where there are several; then the split levels by level and by
+// segment. The threads' rows of a pass are as many as the keys need. Bound by the latency of its eight to ten passes. What
+// it replaces at these sizes is a chain of eleven launches, with a CTA of its own for every segment in ten of them; whole
+// builds of 65,536 meshes of 10 faces 8.65 -> 3.06 ms, 20,000 of 100 3.92 -> 1.54, 1024 of 200 284 -> 216 us, 16 of 64
+// 128 -> 81, one mesh of 4096 124 -> 106, of 17 75 -> 56.
+constexpr int kSegThreads = 512;
+constexpr int kSegWarps = kSegThreads / 32;
+constexpr int kSegItems = kTile / kSegThreads;
+constexpr size_t kSegSmem = kTile * (2 * 4 + 3 * 2);
+__global__ __launch_bounds__(kSegThreads) void k_sort_segments(uint32_t* __restrict__ keys, uint32_t* __restrict__ vals, uint32_t n,
+                                                               const uint32_t* __restrict__ off, uint32_t M, uint32_t window,
+                                                               uint32_t* __restrict__ splits, uint32_t* __restrict__ level_counts,
+                                                               uint32_t stride) {
+  extern __shared__ uint32_t dyn[];
+  uint32_t *k0 = dyn, *k1 = dyn + kTile;  // keys, and where the pass puts them
+  uint16_t *v0 = (uint16_t*)(dyn + 2 * kTile), *v1 = v0 + kTile;
+  uint16_t* const seg = v0 + 2 * kTile;  // segment of each input position, counted from the CTA's first
+  __shared__ __align__(16) uint16_t s_cnt[kSegWarps][kRadix];
+  __shared__ uint32_t s_start[kRadix];
+  __shared__ uint32_t s_warp[kRadix / 32];
+  __shared__ uint32_t s_m[2];
+  const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, lt = lanemask_lt();
+  uint32_t m0 = 0, m1 = 1, a = 0, e = n;
+  if (off) {
+    if (warp < 2) {  // the segments that start before the window (warp 0) and before its end (warp 1), 32 places at a time
+      const uint64_t x = (uint64_t)(blockIdx.x + warp) * window;
+      uint32_t lo = 0, len = M;  // the answer is in lo .. lo + len
+      while (len > 0) {
+        const uint32_t step = (len + 31) / 32, at = lane * step;
+        const uint32_t c = (uint32_t)__popc(__ballot_sync(0xffffffffu, at < len && __ldg(off + lo + at) < x));
+        if (c == 0) break;
+        lo += (c - 1) * step + 1;
+        len = min(step, len - (c - 1) * step) - 1;
+      }
+      if (lane == 0) s_m[warp] = lo;
+    }
+    __syncthreads();
+    m0 = s_m[0];
+    m1 = s_m[1];
+    if (m0 >= m1) return;
+    a = __ldg(off + m0);
+    e = __ldg(off + m1);
+    const uint32_t last = __ldg(off + m1 - 1);
+    if (e - last > window) { e = last; --m1; }
+  }
+  const uint32_t count = e - a, segs = m1 - m0, items = (count + kSegThreads - 1) / kSegThreads;
+  if (count == 0 || items > (uint32_t)kSegItems) return;
+  for (uint32_t i = tid; i < count; i += kSegThreads) {
+    k0[i] = __ldg(keys + a + i);
+    v0[i] = (uint16_t)i;
+    uint32_t lo = 0, hi = segs - 1;
+    while (lo < hi) {
+      const uint32_t mid = (lo + hi + 1) >> 1;
+      if (__ldg(off + m0 + mid) <= a + i) lo = mid; else hi = mid - 1;
+    }
+    seg[i] = (uint16_t)lo;
+  }
+  for (uint32_t i = tid; i < segs * 64u; i += kSegThreads)
+    if ((i & 63u) < stride) level_counts[(size_t)(m0 + (i >> 6)) * stride + (i & 63u)] = 0;
+
+  // one stable pass by eight bits of the keys, or of the values' segments
+  auto pass = [&](uint32_t shift, bool by_seg) {
+    *reinterpret_cast<uint4*>(&s_cnt[warp][8 * lane]) = make_uint4(0, 0, 0, 0);
+    __syncthreads();
+    uint32_t place[kSegItems], digit[kSegItems];
+#pragma unroll
+    for (int r = 0; r < kSegItems; ++r) {
+      if ((uint32_t)r >= items) break;
+      const uint32_t p = (warp * items + r) * 32 + lane;
+      const bool valid = p < count;
+      const uint32_t w = !valid ? 0u : by_seg ? seg[v0[p]] : k0[p], d = (w >> shift) & 255u;
+      uint32_t peers = __ballot_sync(0xffffffffu, valid);
+#pragma unroll
+      for (int b = 0; b < 8; ++b) {
+        const bool bit = (d >> b) & 1u;
+        const uint32_t v = __ballot_sync(0xffffffffu, bit);
+        peers &= bit ? v : ~v;
+      }
+      const uint32_t pre = s_cnt[warp][d];
+      digit[r] = d;
+      place[r] = pre + __popc(peers & lt);
+      __syncwarp();
+      if (valid && (peers & lt) == 0) s_cnt[warp][d] = (uint16_t)(pre + __popc(peers));
+      __syncwarp();
+    }
+    __syncthreads();
+    uint32_t x = 0, total = 0;
+    if (tid < kRadix) {
+#pragma unroll
+      for (int w = 0; w < kSegWarps; ++w) {
+        const uint32_t c = s_cnt[w][tid];
+        s_cnt[w][tid] = (uint16_t)total;
+        total += c;
+      }
+      x = total;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= (uint32_t)o) x += y;
+      }
+      if (lane == 31) s_warp[warp] = x;
+    }
+    __syncthreads();
+    if (tid < kRadix) {
+      uint32_t start = x - total;
+      for (uint32_t w = 0; w < warp; ++w) start += s_warp[w];
+      s_start[tid] = start;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kSegItems; ++r) {
+      if ((uint32_t)r >= items) break;
+      const uint32_t p = (warp * items + r) * 32 + lane;
+      if (p < count) {
+        const uint32_t to = s_start[digit[r]] + s_cnt[warp][digit[r]] + place[r];
+        k1[to] = k0[p];
+        v1[to] = v0[p];
+      }
+    }
+    __syncthreads();
+    uint32_t* const k = k0; k0 = k1; k1 = k;
+    uint16_t* const v = v0; v0 = v1; v1 = v;
+  };
+  __syncthreads();
+  for (uint32_t shift = 0; shift < 32; shift += 8) pass(shift, false);
+  if (segs > 1) pass(0, true);
+  if (segs > 256) pass(8, true);
+  for (uint32_t i = tid; i < count; i += kSegThreads) {
+    const uint32_t code = k0[i], s = seg[v0[i]];
+    keys[a + i] = code;
+    vals[a + i] = a + v0[i];
+    uint32_t level = 32;
+    if (i + 1 < count && seg[v0[i + 1]] == s) {
+      const uint32_t x = code ^ k0[i + 1];
+      if (x) level = (uint32_t)__clz(x);
+    }
+    k1[i] = s << 8 | level;
+    v1[i] = (uint16_t)i;
+  }
+  __syncthreads();
+  uint32_t* const k = k0; k0 = k1; k1 = k;
+  uint16_t* const v = v0; v0 = v1; v1 = v;
+  pass(0, false);
+  if (segs > 1) pass(8, false);
+  if (segs > 256) pass(16, false);
+  for (uint32_t base = warp * 32; base < count; base += kSegThreads) {
+    const uint32_t i = base + lane;
+    const bool valid = i < count;
+    const uint32_t key = valid ? k0[i] : ~0u, before = __shfl_up_sync(0xffffffffu, key, 1);
+    if (valid) splits[a + i] = a + v0[i] + 1;
+    // the first lane of a run of one segment and level counts it
+    const bool head = lane == 0 || key != before;
+    const uint32_t heads = __ballot_sync(0xffffffffu, head) & ~(lt | 1u << lane);
+    if (valid && head && (key & 255u) < stride)
+      atomicAdd(level_counts + (size_t)(m0 + (key >> 8)) * stride + (key & 255u), (heads ? (uint32_t)__ffs((int)heads) - 1u : 32u) - lane);
+  }
 }
 
 // n <= kTile: every pass in shared memory, one CTA. Dynamic shared memory:
@@ -461,6 +634,7 @@ bool small_smem_ready() {
 // 2^24 pairs: 8192-key tiles take 461 us, 6144 about 480, 4096 (three CTAs per SM) 610.
 struct SortPlan {
   uint32_t items, per_chunk, chunks;
+  uint32_t short_segs;  // segments of at most kSegWindow keys go to k_sort_segments
 };
 SortPlan sort_plan(uint32_t n, uint32_t M) {
   constexpr uint32_t kSms = 148;
@@ -469,7 +643,12 @@ SortPlan sort_plan(uint32_t n, uint32_t M) {
   const uint32_t T = kScThreads * P.items, tiles = (uint32_t)(((uint64_t)n + T - 1) / T);
   const uint32_t per = P.items == 16 ? (tiles + 2 * kSms - 1) / (2 * kSms) : 1;
   P.per_chunk = per * T;
-  P.chunks = M > 1 ? n / P.per_chunk + M : (tiles + per - 1) / per;
+  // With fewer than kSegWindow keys a segment on average, a chunk of its own for each would be mostly set-up (and 1 KB of
+  // counts each: 90 MB for 65,536 meshes of 10 faces, now 6): the short ones go to k_sort_segments, one CTA for every
+  // kSegWindow keys. 4096 meshes of 2000 faces: whole build 2.03 -> 1.81 ms; with more faces a mesh on average most
+  // segments are longer than a window anyway.
+  P.short_segs = M > 1 && M > n / kSegWindow ? 1u : 0u;
+  P.chunks = M > 1 ? chunk_base(n, M, P.per_chunk, P.short_segs) + P.short_segs : (tiles + per - 1) / per;
   return P;
 }
 // Scratch regions, in carve order: the other key and value buffers, the chunks' digit counts, the groups' (zeroed, one
@@ -513,10 +692,42 @@ rt_status launch_pass(const PassArgs& P, const SortPlan& S, cudaStream_t st) {
   return launch_pass_of<kVals, 16, kBits, kMode>(P, S.chunks, st);
 }
 
-rt_status make_chunk_segs(const SortLayout& L, const SortPlan& S, const uint32_t* seg_off, uint32_t M, cudaStream_t st) {
-  k_chunk_segs<<<(S.chunks + 255) / 256, 256, 0, st>>>(seg_off, M, S.per_chunk, S.chunks, L.chunk_seg);
+// k_sort_segments over windows of `window` positions; fails where its shared memory is refused.
+rt_status launch_segments(uint32_t* codes, uint32_t* idx, uint32_t n, uint32_t* splits, uint32_t* level_counts, uint32_t count_stride,
+                          const uint32_t* seg_off, uint32_t M, uint32_t window, cudaStream_t st) {
+  static PerDeviceOnce once;
+  if (!once.run([] {
+        return cudaFuncSetAttribute(k_sort_segments, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSegSmem) == cudaSuccess;
+      }))
+    return RT_ERR_CUDA;
+  k_sort_segments<<<(n - 1) / window + 1, kSegThreads, kSegSmem, st>>>(codes, idx, n, seg_off, M, window, splits, level_counts, count_stride);
   note_launch();
   RT_CHECK_LAUNCH();
+  return RT_OK;
+}
+
+// The digit passes over chunked keys [0, 8 * passes) from begin_bit; the result is in keys and vals.
+rt_status chunked_passes(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_t begin_bit, uint32_t passes, int init_vals, const SortPlan& S,
+                         const SortLayout& L, const uint32_t* seg_off, cudaStream_t stream) {
+  if (cudaMemsetAsync(L.groups, 0, passes * L.group_words * 4, stream) != cudaSuccess) return RT_ERR_CUDA;
+  uint32_t *ks = keys, *vs = vals, *kd = L.kalt, *vd = L.valt;
+  for (uint32_t p = 0; p < passes; ++p) {
+    PassArgs P = {};
+    P.keys_in = ks; P.keys_out = kd;
+    P.vals_in = (p == 0 && init_vals) ? nullptr : vs; P.vals_out = vd;
+    P.n = n; P.shift = begin_bit + 8 * p; P.per_chunk = S.per_chunk; P.short_segs = S.short_segs;
+    if (L.chunk_seg) { P.seg_off = seg_off; P.chunk_seg = L.chunk_seg; }
+    P.rows = L.rows; P.groups = L.groups + p * L.group_words;
+    const rt_status s = vals ? launch_pass<true, 8, 0>(P, S, stream) : launch_pass<false, 8, 0>(P, S, stream);
+    if (s != RT_OK) return s;
+    uint32_t* t;
+    t = ks; ks = kd; kd = t;
+    t = vs; vs = vd; vd = t;
+  }
+  if (ks != keys) {
+    if (cudaMemcpyAsync(keys, ks, (size_t)n * 4, cudaMemcpyDeviceToDevice, stream) != cudaSuccess) return RT_ERR_CUDA;
+    if (vals && cudaMemcpyAsync(vals, vs, (size_t)n * 4, cudaMemcpyDeviceToDevice, stream) != cudaSuccess) return RT_ERR_CUDA;
+  }
   return RT_OK;
 }
 
@@ -534,12 +745,12 @@ size_t segment_sort_scratch_bytes(uint32_t n, uint32_t M) {
 }
 
 rt_status radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_t begin_bit, uint32_t end_bit, int init_vals,
-                           void* scratch, size_t scratch_bytes, cudaStream_t stream, const uint32_t* seg_off, uint32_t M) {
+                           void* scratch, size_t scratch_bytes, cudaStream_t stream) {
   if (n == 0) return RT_OK;
   if (end_bit <= begin_bit || end_bit > 32) return RT_ERR_INVALID_ARGUMENT;
   if (n > kMaxKeys) return RT_ERR_INVALID_ARGUMENT;
   const uint32_t passes = (end_bit - begin_bit + 7) / 8;
-  if (M <= 1 && n <= (uint32_t)kTile) {
+  if (n <= (uint32_t)kTile) {
     if (!small_smem_ready()) return RT_ERR_CUDA;
     if (vals) k_radix_small<true><<<1, kThreads, kSmallSmem, stream>>>(keys, vals, n, begin_bit, passes, init_vals);
     else k_radix_small<false><<<1, kThreads, kSmallSmem, stream>>>(keys, nullptr, n, begin_bit, passes, 0);
@@ -548,55 +759,41 @@ rt_status radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_t 
     return RT_OK;
   }
   if (!scratch) return RT_ERR_SCRATCH_TOO_SMALL;
-  const SortPlan S = sort_plan(n, M);
+  const SortPlan S = sort_plan(n, 1);
   Carve c(scratch, scratch_bytes);
-  const SortLayout L = carve_sort(c, n, M, S);
+  const SortLayout L = carve_sort(c, n, 1, S);
   if (!c.ok()) return RT_ERR_SCRATCH_TOO_SMALL;
-  if (cudaMemsetAsync(L.groups, 0, passes * L.group_words * 4, stream) != cudaSuccess) return RT_ERR_CUDA;
-  if (M > 1) {
-    const rt_status s = make_chunk_segs(L, S, seg_off, M, stream);
-    if (s != RT_OK) return s;
-  }
-  uint32_t *ks = keys, *vs = vals, *kd = L.kalt, *vd = L.valt;
-  for (uint32_t p = 0; p < passes; ++p) {
-    PassArgs P = {};
-    P.keys_in = ks; P.keys_out = kd;
-    P.vals_in = (p == 0 && init_vals) ? nullptr : vs; P.vals_out = vd;
-    P.n = n; P.shift = begin_bit + 8 * p; P.per_chunk = S.per_chunk;
-    if (M > 1) { P.seg_off = seg_off; P.chunk_seg = L.chunk_seg; }
-    P.rows = L.rows; P.groups = L.groups + p * L.group_words;
-    const rt_status s = vals ? launch_pass<true, 8, 0>(P, S, stream) : launch_pass<false, 8, 0>(P, S, stream);
-    if (s != RT_OK) return s;
-    uint32_t* t;
-    t = ks; ks = kd; kd = t;
-    t = vs; vs = vd; vd = t;
-  }
-  if (ks != keys) {
-    if (cudaMemcpyAsync(keys, ks, (size_t)n * 4, cudaMemcpyDeviceToDevice, stream) != cudaSuccess) return RT_ERR_CUDA;
-    if (vals && cudaMemcpyAsync(vals, vs, (size_t)n * 4, cudaMemcpyDeviceToDevice, stream) != cudaSuccess) return RT_ERR_CUDA;
-  }
-  return RT_OK;
+  return chunked_passes(keys, vals, n, begin_bit, passes, init_vals, S, L, nullptr, stream);
 }
 
-rt_status sort_split_levels(const uint32_t* codes, uint32_t n, uint32_t* splits, uint32_t* level_counts, uint32_t count_stride,
-                            void* scratch, size_t scratch_bytes, cudaStream_t stream, const uint32_t* seg_off, uint32_t M) {
+rt_status sort_codes_and_levels(uint32_t* codes, uint32_t* idx, uint32_t n, uint32_t* splits, uint32_t* level_counts, uint32_t count_stride,
+                                void* scratch, size_t scratch_bytes, cudaStream_t stream, const uint32_t* seg_off, uint32_t M) {
   if (n == 0) return RT_OK;
-  if (!scratch || n > kMaxKeys) return RT_ERR_INVALID_ARGUMENT;
+  if (n > kMaxKeys) return RT_ERR_INVALID_ARGUMENT;
+  if (M <= 1) seg_off = nullptr;
+  if (n <= (uint32_t)kTile) return launch_segments(codes, idx, n, splits, level_counts, count_stride, seg_off, M, kTile, stream);
+  if (!scratch) return RT_ERR_INVALID_ARGUMENT;
   const SortPlan S = sort_plan(n, M);
   Carve c(scratch, scratch_bytes);
   const SortLayout L = carve_sort(c, n, M, S);
   if (!c.ok()) return RT_ERR_SCRATCH_TOO_SMALL;
-  if (cudaMemsetAsync(L.groups, 0, L.group_words * 4, stream) != cudaSuccess) return RT_ERR_CUDA;
-  if (M > 1) {
-    const rt_status s = make_chunk_segs(L, S, seg_off, M, stream);
-    if (s != RT_OK) return s;
+  if (L.chunk_seg) {
+    k_chunk_segs<<<(S.chunks + 255) / 256, 256, 0, stream>>>(seg_off, M, S.per_chunk, S.short_segs, S.chunks, L.chunk_seg);
+    note_launch();
+    RT_CHECK_LAUNCH();
   }
+  rt_status s = chunked_passes(codes, idx, n, 0, 32 / 8, 1, S, L, seg_off, stream);
+  if (s != RT_OK) return s;
+  // the split levels, from the sorted codes
+  if (cudaMemsetAsync(L.groups, 0, L.group_words * 4, stream) != cudaSuccess) return RT_ERR_CUDA;
   PassArgs P = {};
   P.keys_in = codes; P.vals_out = splits; P.val_base = 1;
-  P.n = n; P.per_chunk = S.per_chunk;
-  if (M > 1) { P.seg_off = seg_off; P.chunk_seg = L.chunk_seg; }
+  P.n = n; P.per_chunk = S.per_chunk; P.short_segs = S.short_segs;
+  if (L.chunk_seg) { P.seg_off = seg_off; P.chunk_seg = L.chunk_seg; }
   P.rows = L.rows; P.groups = L.groups; P.totals = level_counts; P.totals_stride = count_stride;
-  return launch_pass<true, 6, 1>(P, S, stream);
+  s = launch_pass<true, 6, 1>(P, S, stream);
+  if (s != RT_OK || !S.short_segs) return s;
+  return launch_segments(codes, idx, n, splits, level_counts, count_stride, seg_off, M, kSegWindow, stream);
 }
 
 }  // namespace rt
