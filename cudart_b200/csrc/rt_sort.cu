@@ -9,7 +9,8 @@
 //     pass is two launches. k_sort_count reads its chunk's keys and writes the
 //     chunk's 256 digit counts (and adds them to a sum per 16 chunks);
 //     k_sort_scatter adds up the counts before its chunk, then takes the
-//     chunk's tiles one after another: ranks the keys stably (the lanes of
+//     chunk's tiles one after another (with few chunks it counts the keys
+//     itself, and the pass is one launch): ranks the keys stably (the lanes of
 //     equal digit, plus per-warp counters),
 //     stages the tile in shared memory in sorted order and writes it out so
 //     that consecutive threads write consecutive addresses of each digit run,
@@ -116,7 +117,7 @@ struct PassArgs {
   const uint32_t* seg_off;   // null: one segment, 0 .. n
   const uint32_t* chunk_seg; // segment of each chunk (~0: no chunk); with seg_off
   uint32_t short_segs;       // segments of at most kSegWindow keys have no chunks
-  uint32_t* rows;            // [chunks][256]
+  uint32_t* rows;            // [chunks][256]; null: few chunks of one segment, whose CTAs count the keys themselves
   uint32_t* groups;          // [chunks / kGroup + 1][256], zero before the pass
   uint32_t* totals;          // optional: [segments][totals_stride] digit counts
   uint32_t totals_stride;
@@ -239,7 +240,30 @@ __global__ __launch_bounds__(kScThreads, kItems == 16 ? 2 : 3) void k_sort_scatt
     const uint32_t c = blockIdx.x, cs = C.first_chunk, ce = cs + C.n_chunks, d = tid & 255u;
     const uint32_t g0 = (cs + kGroup - 1) / kGroup, g1 = max(g0, ce / kGroup);  // whole groups of the segment
     uint32_t all = 0, part = 0;
-    if (d < D) {
+    if (!P.rows) {
+      uint32_t* const s_own = s_dyn;  // keys before the chunk, then the others: four counters per digit each, picked by lane
+      for (uint32_t i = tid; i < 8 * D; i += kScThreads) s_own[i] = 0;
+      __syncthreads();
+      for (uint32_t i0 = tid; i0 < P.n; i0 += 8 * kScThreads) {
+        uint32_t k[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) k[q] = i0 + q * kScThreads < P.n ? load_key<kMode>(P, C, i0 + q * kScThreads) : 0u;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const uint32_t i = i0 + q * kScThreads;
+          if (i < P.n) atomicAdd(&s_own[(i < C.begin ? 0u : 4u * D) + ((k[q] >> P.shift) & (D - 1u)) * 4u + (lane & 3u)], 1u);
+        }
+      }
+      __syncthreads();
+      if (tid < (int)D) {
+#pragma unroll
+        for (uint32_t q = 0; q < 4; ++q) {
+          part += s_own[4 * d + q];
+          all += s_own[4 * (D + d) + q];
+        }
+        all += part;
+      }
+    } else if (d < D) {
       if (tid < kRadix) {
         sum_rows(P.groups, d, g0, g1, c / kGroup, all, part);
       } else {
@@ -679,9 +703,9 @@ rt_status launch_pass_of(const PassArgs& P, uint32_t chunks, cudaStream_t st) {
         }))
       return RT_ERR_CUDA;
   }
-  k_sort_count<kBits, kMode><<<chunks, kCountThreads, 0, st>>>(P);
+  if (P.rows) k_sort_count<kBits, kMode><<<chunks, kCountThreads, 0, st>>>(P);
   k_sort_scatter<kVals, kItems, kBits, kMode><<<chunks, kScThreads, smem, st>>>(P);
-  note_launch(2);
+  note_launch(P.rows ? 2 : 1);
   RT_CHECK_LAUNCH();
   return RT_OK;
 }
@@ -706,10 +730,17 @@ rt_status launch_segments(uint32_t* codes, uint32_t* idx, uint32_t n, uint32_t* 
   return RT_OK;
 }
 
+// Few chunks of one segment: each CTA of a scatter launch counts all the keys for itself, and the count launch and its
+// zeroed sums go. 32-bit keys alone: 8192 45.2 -> 26.7 us, 16,384 45.3 -> 35.0, 30,000 45.8 -> 43.6, 40,000 46.1 -> 47.3
+// (one launch per pass with a look-back took 45.9, 47.8, 47.8, 49.8). The split levels read two codes per key: builds of
+// 16,384 faces 153 -> 147 us, of 30,000 163 -> 172 with both.
+constexpr uint32_t kSelfCount = 16, kSelfCountLevels = 8;
+
 // The digit passes over chunked keys [0, 8 * passes) from begin_bit; the result is in keys and vals.
 rt_status chunked_passes(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_t begin_bit, uint32_t passes, int init_vals, const SortPlan& S,
                          const SortLayout& L, const uint32_t* seg_off, cudaStream_t stream) {
-  if (cudaMemsetAsync(L.groups, 0, passes * L.group_words * 4, stream) != cudaSuccess) return RT_ERR_CUDA;
+  const bool self_count = !L.chunk_seg && S.chunks <= kSelfCount;
+  if (!self_count && cudaMemsetAsync(L.groups, 0, passes * L.group_words * 4, stream) != cudaSuccess) return RT_ERR_CUDA;
   uint32_t *ks = keys, *vs = vals, *kd = L.kalt, *vd = L.valt;
   for (uint32_t p = 0; p < passes; ++p) {
     PassArgs P = {};
@@ -717,7 +748,7 @@ rt_status chunked_passes(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_t be
     P.vals_in = (p == 0 && init_vals) ? nullptr : vs; P.vals_out = vd;
     P.n = n; P.shift = begin_bit + 8 * p; P.per_chunk = S.per_chunk; P.short_segs = S.short_segs;
     if (L.chunk_seg) { P.seg_off = seg_off; P.chunk_seg = L.chunk_seg; }
-    P.rows = L.rows; P.groups = L.groups + p * L.group_words;
+    P.rows = self_count ? nullptr : L.rows; P.groups = L.groups + p * L.group_words;
     const rt_status s = vals ? launch_pass<true, 8, 0>(P, S, stream) : launch_pass<false, 8, 0>(P, S, stream);
     if (s != RT_OK) return s;
     uint32_t* t;
@@ -785,12 +816,13 @@ rt_status sort_codes_and_levels(uint32_t* codes, uint32_t* idx, uint32_t n, uint
   rt_status s = chunked_passes(codes, idx, n, 0, 32 / 8, 1, S, L, seg_off, stream);
   if (s != RT_OK) return s;
   // the split levels, from the sorted codes
-  if (cudaMemsetAsync(L.groups, 0, L.group_words * 4, stream) != cudaSuccess) return RT_ERR_CUDA;
+  const bool self_count = !L.chunk_seg && S.chunks <= kSelfCountLevels;
+  if (!self_count && cudaMemsetAsync(L.groups, 0, L.group_words * 4, stream) != cudaSuccess) return RT_ERR_CUDA;
   PassArgs P = {};
   P.keys_in = codes; P.vals_out = splits; P.val_base = 1;
   P.n = n; P.per_chunk = S.per_chunk; P.short_segs = S.short_segs;
   if (L.chunk_seg) { P.seg_off = seg_off; P.chunk_seg = L.chunk_seg; }
-  P.rows = L.rows; P.groups = L.groups; P.totals = level_counts; P.totals_stride = count_stride;
+  P.rows = self_count ? nullptr : L.rows; P.groups = L.groups; P.totals = level_counts; P.totals_stride = count_stride;
   s = launch_pass<true, 6, 1>(P, S, stream);
   if (s != RT_OK || !S.short_segs) return s;
   return launch_segments(codes, idx, n, splits, level_counts, count_stride, seg_off, M, kSegWindow, stream);
