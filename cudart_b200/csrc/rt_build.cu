@@ -1563,9 +1563,14 @@ extern "C" rt_status rt_batch_build(const rt_batch_build_desc* d, rt_stream stre
   if (cudaMemsetAsync(B.topo_done, 0, 8, st) != cudaSuccess) return RT_ERR_CUDA;
   if (cudaMemsetAsync(B.hist, 0, (size_t)M * 64 * 4, st) != cudaSuccess) return RT_ERR_CUDA;
   if (cudaMemsetAsync(B.hitdone, 0, (size_t)M * 4, st) != cudaSuccess) return RT_ERR_CUDA;
-  // eight shares of few meshes fill the chip (64 meshes: 106 us at four or eight, 132 at two); of many they are launches of
-  // CTAs with little to do (1024 meshes: 100 us at eight, 73 at four)
-  B.hit_split = M > 512 ? kHitSplit / 2 : kHitSplit;
+  // shares of the hit box: while the CTAs fit the chip at once (four an SM) a share of 1024 vertices is worth a CTA, beyond
+  // that one of 8192 (on average: the largest meshes want more). By shares 1 / 2 / 4 / 8: 64 meshes of 1000 faces 5.6 / 5.1 /
+  // 5.7 / 8.2 us, of 10,000 32 / 19 / 13 / 13, of 62,000 183 / 103 / 66 / 52; 256 of 1000 7 / 9 / 13 / 21, of 8000 41 / 34 /
+  // 34 / 40, of 30,000 118 / 93 / 84 / 82; 1024 of 200 14 / 20 / 36 / 64, of 9000 98 / 92 / 102 / 135; 65,536 of 10
+  // 0.67 / 1.16 / 2.19 / 4.16 ms.
+  const uint64_t share = M * kHitSplit <= 4u * (uint32_t)sms ? 1024 : 8192;
+  B.hit_split = 1;
+  while (B.hit_split < kHitSplit && (uint64_t)d->vertex_count >= 2 * B.hit_split * share * M) B.hit_split *= 2;
   k_batch_hitbox<<<M * B.hit_split, 512, 0, st>>>(B);
   k_batch_boxes_morton<<<fblocks, 256, 0, st>>>(B);
   note_launch(2);
