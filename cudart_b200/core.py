@@ -225,6 +225,7 @@ def build_sah(vertices: torch.Tensor, faces: torch.Tensor, hitbox=None, lbvh_dep
     d.info = out.info.data_ptr()
     d.scratch, d.scratch_bytes = scratch.data_ptr(), scratch.numel()
     _abi.check("rt_sah_build", _abi.lib().rt_sah_build(C.byref(d), _stream(stream)))
+    out.clusters = False
     return out
 
 

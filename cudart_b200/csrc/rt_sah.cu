@@ -831,6 +831,7 @@ __global__ __launch_bounds__(256) void k_sah_accel(const uint32_t* __restrict__ 
     acc_hdr[0] = (nodes[0] & 1u) ? ~leaf_lambda[0] : 0u;
     acc_hdr[1] = leaf_count;
     acc_hdr[2] = node_count;
+    acc_hdr[kHdrClusterValid] = 0;  // an LBVH build may have left its cluster tree in the blob
   }
   for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < node_count; p += gridDim.x * blockDim.x)
     accel_node(nodes, leaf_lambda, tnodes, p);
