@@ -976,7 +976,7 @@ bool topo_smem_once(K kernel, uint32_t nodes) {
 
 }  // namespace
 
-SideStream* side_stream() {
+SideStream* side_stream(cudaStream_t st) {
   // one per host thread and device (a stream takes part in one capture at a time, and a thread's calls are
   // ordered, so the fork and join events of two calls never interleave); kept until the process exits
   constexpr int kMaxDevices = 64;
@@ -995,7 +995,18 @@ SideStream* side_stream() {
     if (!ok) cudaGetLastError();
     state[dev] = ok ? 1 : -1;
   }
-  return state[dev] == 1 ? &per_device[dev] : nullptr;
+  if (state[dev] != 1) return nullptr;
+  // an earlier call of this thread may have taken the side stream into a capture that has not ended: only that capture's
+  // calls can use it until then
+  cudaStreamCaptureStatus side = cudaStreamCaptureStatusNone, own = cudaStreamCaptureStatusNone;
+  unsigned long long side_id = 0, own_id = 0;
+  if (cudaStreamGetCaptureInfo(per_device[dev].s, &side, &side_id) != cudaSuccess ||
+      (side != cudaStreamCaptureStatusNone && cudaStreamGetCaptureInfo(st, &own, &own_id) != cudaSuccess)) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  if (side != cudaStreamCaptureStatusNone && (own == cudaStreamCaptureStatusNone || own_id != side_id)) return nullptr;
+  return &per_device[dev];
 }
 
 }  // namespace rt
@@ -1128,7 +1139,7 @@ extern "C" rt_status rt_lbvh_build(const rt_build_desc* d, rt_stream stream_) {
     // cluster tree sets, is cleared before they part.
     const bool cluster_tree = accel && clusters;
     if (accel && cudaMemsetAsync(AL.hdr + kHdrClusterValid, 0, 4, st) != cudaSuccess) return RT_ERR_CUDA;
-    SideStream* side = cluster_tree ? side_stream() : nullptr;
+    SideStream* side = cluster_tree ? side_stream(st) : nullptr;
     cudaStream_t ns = st;
     if (side) {
       if (cudaEventRecord(side->fork, st) != cudaSuccess || cudaStreamWaitEvent(side->s, side->fork, 0) != cudaSuccess)
@@ -1589,7 +1600,7 @@ extern "C" rt_status rt_batch_build(const rt_batch_build_desc* d, rt_stream stre
   RT_CHECK_LAUNCH();
   // the node boxes and records (from the nodes) and the cluster trees (from the codes and triangles) are
   // independent: with cluster trees, the node half runs on a side stream beside them
-  SideStream* side = clusters ? side_stream() : nullptr;
+  SideStream* side = clusters ? side_stream(st) : nullptr;
   cudaStream_t ns = st;
   if (side) {
     if (cudaEventRecord(side->fork, st) != cudaSuccess || cudaStreamWaitEvent(side->s, side->fork, 0) != cudaSuccess)

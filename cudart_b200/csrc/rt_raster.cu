@@ -430,7 +430,7 @@ extern "C" rt_status rt_rasterize(const rt_raster_desc* d, rt_stream stream) {
   // Most frames fit the pair buffer: the whole frame is launched as one chunk that does nothing if it does not fit, and
   // the pair count is read beside it on a side stream, so that the host's wait for it is no gap on the device (2^20
   // faces 1020 -> 965 us, of 2394 before this file's other changes).
-  SideStream* side = side_stream();
+  SideStream* side = side_stream(st);
   cudaStream_t rs = side ? side->s : st;
   if (side && (cudaEventRecord(side->fork, st) != cudaSuccess || cudaStreamWaitEvent(side->s, side->fork, 0) != cudaSuccess)) return RT_ERR_CUDA;
   rt_status s = chunk(0, n, PairLimit{L.total, L.cap});
