@@ -429,11 +429,32 @@ constexpr int kCoopWarps = 4;  // 128-thread CTAs
 // current best, and its t (a -0 keeps its sign, which the key drops), are
 // written by the lane whose key is the minimum right after its merge. key0 is this lane's best so far (t bits, position); on return
 // s_key[lane] / s_uvt[lane] hold the merged best of this lane's ray.
-template <uint32_t kGroup>
+//
+// A lane's best (u, v, t) in shared memory: in one word of 16 bytes, or (the two-child walk, 3 to 5% faster so) in two.
+template <bool kOne>
+struct CoopUvt {
+  float4 x[32];
+  __device__ __forceinline__ void put(uint32_t i, float u, float v, float t) { x[i] = make_float4(u, v, t, 0.0f); }
+  __device__ __forceinline__ void get(uint32_t i, float& u, float& v, float& t) const {
+    const float4 a = x[i];
+    u = a.x; v = a.y; t = a.z;
+  }
+};
+template <>
+struct CoopUvt<false> {
+  float2 x[32];
+  float y[32];
+  __device__ __forceinline__ void put(uint32_t i, float u, float v, float t) { x[i] = make_float2(u, v); y[i] = t; }
+  __device__ __forceinline__ void get(uint32_t i, float& u, float& v, float& t) const {
+    const float2 a = x[i];
+    u = a.x; v = a.y; t = y[i];
+  }
+};
+template <uint32_t kGroup, class Uvt>
 __device__ __forceinline__ void coop_items(const uint32_t lane, const uint32_t mask, const uint32_t first, const uint32_t cnt,
                                            const uint32_t F, const float4& o, const float4& d, const float zu, const float zv,
                                            const float4* __restrict__ tris, const unsigned long long key0, const float bt,
-                                           const float bu, const float bv, unsigned long long* s_key, float4* s_uvt) {
+                                           const float bu, const float bv, unsigned long long* s_key, Uvt& s_uvt) {
   const uint32_t my_items = __popc(mask);
   uint32_t incl = my_items;
 #pragma unroll
@@ -450,7 +471,7 @@ __device__ __forceinline__ void coop_items(const uint32_t lane, const uint32_t m
   const uint32_t split = groups <= 4 ? 3u : groups <= 8 ? 2u : groups <= 16 ? 1u : 0u;
   const uint32_t total = groups << split;
   s_key[lane] = key0;
-  s_uvt[lane] = make_float4(bu, bv, bt, 0.0f);
+  s_uvt.put(lane, bu, bv, bt);
   __syncwarp();
   for (uint32_t base = 0; base < total; base += 32) {
     const bool have = base + lane < total;
@@ -500,14 +521,14 @@ __device__ __forceinline__ void coop_items(const uint32_t lane, const uint32_t m
     }
     __syncwarp();
     // (u, v, t) of the owner's minimum, written by the one lane holding that key
-    if (have && cand != ~0ull && s_key[owner] == cand) s_uvt[owner] = make_float4(cu, cv, ct, 0.0f);
+    if (have && cand != ~0ull && s_key[owner] == cand) s_uvt.put(owner, cu, cv, ct);
     __syncwarp();
   }
 }
 
 template <bool kCount, bool kSeed = false, bool kWide = false>
 __device__ __forceinline__ void trace_warp_coop(const uint32_t r, const bool valid, const TraceArgs& A, const AccelArgs& C,
-                                                unsigned long long* s_key, float4* s_uvt, const SeedArgs& S = SeedArgs{}) {
+                                                unsigned long long* s_key, CoopUvt<kWide>& s_uvt, const SeedArgs& S = SeedArgs{}) {
   const uint32_t lane = lane_id();
   float4 o = make_float4(0.f, 0.f, 0.f, 0.f), d = make_float4(0.f, 0.f, 1.f, 0.f);
   float tmax0 = -1.0f;
@@ -645,8 +666,13 @@ __device__ __forceinline__ void trace_warp_coop(const uint32_t r, const bool val
     // rays of the 2^20-triangle soup at 1920 x 1080 with items only, then with both: 2.51 -> 1.80 ms in rows, 2.42 -> 1.39
     // in pixel tiles; their bounces 2.81 -> 2.74; terrains are within 2%. Deciding for the
     // lanes' own groups twice as readily loses 5% on soups, four times as readily 20 to 50% on bounces and terrains.
-    const uint32_t any = __reduce_or_sync(0xffffffffu, mask), items = __reduce_add_sync(0xffffffffu, (uint32_t)__popc(mask));
-    if (16u * ((uint32_t)__popc(any) - 1u) < items) {
+    // (The two-child walk spreads them always: deciding costs it 3 to 10% on terrains.)
+    uint32_t any = 0, items = 1;
+    if constexpr (kWide) {
+      any = __reduce_or_sync(0xffffffffu, mask);
+      items = __reduce_add_sync(0xffffffffu, (uint32_t)__popc(mask));
+    }
+    if (kWide && 16u * ((uint32_t)__popc(any) - 1u) < items) {
       for (uint32_t gs = any; gs; gs &= gs - 1u) {
         const uint32_t g = (uint32_t)__ffs((int)gs) - 1u;
         if (!(mask >> g & 1u)) continue;
@@ -671,8 +697,7 @@ __device__ __forceinline__ void trace_warp_coop(const uint32_t r, const bool val
       const unsigned long long k = s_key[lane];
       if (k < key0) {
         best = (int32_t)(k & 0xFFFFFFFFu);
-        const float4 uvt = s_uvt[lane];
-        bu = uvt.x; bv = uvt.y; bt = uvt.z;
+        s_uvt.get(lane, bu, bv, bt);
         best_phase = phase;
       }
     }
@@ -940,7 +965,7 @@ __device__ __forceinline__ void trace_ray_clusters(const uint32_t r, const Trace
 // lane) are tested by the whole warp (coop_items), and every lane moves on.
 template <bool kCount>
 __device__ __forceinline__ void trace_warp_coop_clusters(const uint32_t r, const bool valid, const TraceArgs& A, const ClusterArgs& C,
-                                                         unsigned long long* s_key, float4* s_uvt) {
+                                                         unsigned long long* s_key, CoopUvt<true>& s_uvt) {
   const uint32_t lane = lane_id();
   float4 o = make_float4(0.f, 0.f, 0.f, 0.f), d = make_float4(0.f, 0.f, 1.f, 0.f);
   float tmax0 = -1.0f;
@@ -1013,8 +1038,7 @@ __device__ __forceinline__ void trace_warp_coop_clusters(const uint32_t r, const
       const unsigned long long key = s_key[lane];
       if (key < key0) {
         best = (int32_t)(key & 0xFFFFFFFFu);
-        const float4 uvt = s_uvt[lane];
-        bu = uvt.x; bv = uvt.y; bt = uvt.z;
+        s_uvt.get(lane, bu, bv, bt);
       }
       if (!pop_within(st_ref, st_t, sp, bt, ref)) alive = false;
     }
@@ -1477,7 +1501,7 @@ __global__ __launch_bounds__(128) void k_trace_accel(TraceArgs A, AccelArgs C, S
 template <bool kCount, bool kSeed, bool kWide>
 __global__ __launch_bounds__(128, kSeed ? 6 : (kCount ? 0 : 7)) void k_trace_coop(TraceArgs A, AccelArgs C, SlotMap M, SeedArgs S) {
   __shared__ unsigned long long s_key[kCoopWarps][32];
-  __shared__ float4 s_uvt[kCoopWarps][32];
+  __shared__ CoopUvt<kWide> s_uvt[kCoopWarps];
   const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
   uint32_t r = 0;
   const bool valid = s < M.slots && M.ray_of(s, r);
@@ -1490,7 +1514,7 @@ template <bool kCount, bool kSeed, bool kWide>
 __global__ __launch_bounds__(128, kSeed ? 6 : (kCount ? 0 : 7)) void k_trace_coop_persistent(TraceArgs A, AccelArgs C, SlotMap M, uint32_t* counter,
                                                                           SeedArgs S) {
   __shared__ unsigned long long s_key[kCoopWarps][32];
-  __shared__ float4 s_uvt[kCoopWarps][32];
+  __shared__ CoopUvt<kWide> s_uvt[kCoopWarps];
   __shared__ uint32_t s_rec[kMaxStaged];
   extern __shared__ float4 s_tree[];
   C.F = C.G = 0;
@@ -1594,7 +1618,7 @@ template <bool kCount, bool kSeed, bool kWide>
 __global__ __launch_bounds__(128, kSeed ? 6 : (kCount ? 0 : 7)) void k_batch_trace_coop(TraceArgs A, BatchTraceArgs B, SeedArgs S,
                                                                                       uint32_t* counter) {
   __shared__ unsigned long long s_key[kCoopWarps][32];
-  __shared__ float4 s_uvt[kCoopWarps][32];
+  __shared__ CoopUvt<kWide> s_uvt[kCoopWarps];
   const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
   for (;;) {
     uint32_t base = 0;
@@ -1652,7 +1676,7 @@ __global__ __launch_bounds__(128) void k_trace_clusters_persistent(TraceArgs A, 
 template <bool kCount>
 __global__ __launch_bounds__(128) void k_trace_clusters_coop(TraceArgs A, ClusterArgs C, SlotMap M, uint32_t* counter) {
   __shared__ unsigned long long s_key[kCoopWarps][32];
-  __shared__ float4 s_uvt[kCoopWarps][32];
+  __shared__ CoopUvt<true> s_uvt[kCoopWarps];
   const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
   C.F = 0;
   for (;;) {
@@ -1789,7 +1813,7 @@ __global__ __launch_bounds__(128, 8) void k_batch_trace_clusters_packet(TraceArg
 template <bool kCount>
 __global__ __launch_bounds__(128) void k_batch_trace_clusters_coop(TraceArgs A, BatchTraceArgs B, uint32_t* counter) {
   __shared__ unsigned long long s_key[kCoopWarps][32];
-  __shared__ float4 s_uvt[kCoopWarps][32];
+  __shared__ CoopUvt<true> s_uvt[kCoopWarps];
   const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
   for (;;) {
     uint32_t base = 0;
