@@ -48,7 +48,8 @@ RASTER_EXPORTS = ("rt_camera_view_dir", "rt_raster_matrix", "rt_raster_scratch_b
 PROPOSE_EXPORTS = (
     "rt_propose_abi_version", "rt_gemm_bf16", "rt_gemm_argmax_bf16", "rt_ray_features", "rt_softmax_xent", "rt_transpose_bf16",
     "rt_colsum_bf16", "rt_adam_step", "rt_subtree_slots", "rt_hit_labels", "rt_trace_closest_seeded", "rt_transpose_bf16_grouped",
-    "rt_gemm_bf16_multi", "rt_colsum_bf16_multi", "rt_adam_step_multi", "rt_colsum_bf16_grouped", "rt_gather_batch", "rt_batch_subtree_slots", "rt_batch_hit_labels", "rt_batch_trace_seeded",
+    "rt_gemm_bf16_multi", "rt_colsum_bf16_multi", "rt_adam_step_multi", "rt_colsum_bf16_grouped", "rt_gather_batch",
+    "rt_batch_subtree_slots", "rt_batch_hit_labels", "rt_batch_trace_seeded",
     "rt_group_select", "rt_mlp_propose", "rt_gemm_xent_bf16", "rt_tc_wait_selftest",
 )
 

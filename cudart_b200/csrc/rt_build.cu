@@ -652,9 +652,9 @@ __device__ __forceinline__ LeafMeta leaf_meta(const LeafArgs& A, const uint32_t 
 // groups, so that short leaves share a step; the boxes are reduced inside the lanes of each group and then over a
 // leaf's groups, which are eight lanes apart, and a leaf that goes on past a step carries its box along. Boxes are
 // combined in position order with the selects of a sequential scan. The next step's indices and faces are loaded
-// while this one's vertices are on their way. (A warp per leaf with lane 0 finding it, one leaf and one dependent
-// load after another, took 1.29 ms for 2^24 faces of a soup and 1.31 ms for 9.9M in 1024 meshes; this takes 0.98 ms, bound by DRAM (5.8 TB/s
-// of scattered reads, 276 bytes per face), and 0.63.)
+// while this one's vertices are on their way. (A warp per leaf with lane 0 finding it, one leaf and one dependent load
+// after another, took 1.29 ms for 2^24 faces of a soup and 1.31 ms for 9.9M in 1024 meshes; this takes 0.98 ms, bound by
+// DRAM (5.8 TB/s of scattered reads, 276 bytes per face), and 0.63.)
 // `out`: arrays of the whole build (nodes and group boxes of the first mesh).
 __device__ __forceinline__ void leaf_faces(const LeafArgs& out, const LeafMeta& L) {
   const uint32_t lane = lane_id();

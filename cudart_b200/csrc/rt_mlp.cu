@@ -1130,8 +1130,9 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
 // their biases: only their maximum is compared with the best so far, and a
 // larger one leaves all 16 in the thread's shared-memory slot (`save`, four
 // 16-byte pieces kFuseCompute apart), where its column is looked up once per
-// tile. 23 instructions instead of 56 for a compare and two selects per logit: 2M rays 3.48 -> 2.98 ms, now bound by the
-// chain of the three hidden layers and the logits' MMAs.
+// tile. 23 instructions instead of 56 for a compare and two selects per logit:
+// 2M rays 3.48 -> 2.98 ms, now bound by the chain of the three hidden layers
+// and the logits' MMAs.
 __device__ __forceinline__ void sweep16_top1(const uint32_t (&r)[16], const float* sb, uint32_t col, float& best, int32_t& at, float4* save) {
   const float4* bp = (const float4*)(sb + col);
   float x[16];

@@ -655,7 +655,9 @@ bool small_smem_ready() {
 // Tiles and chunks of an n-key sort with M segments. Tiles of 2048, 4096 or 8192 keys (4, 8 or 16 per thread): the
 // smallest that leaves every SM's two (three for 4096) resident CTAs at most one tile each, so that small sorts
 // spread over the chip and large ones have long digit runs; chunks of as many whole tiles as give two CTAs per SM.
-// 2^24 pairs: 8192-key tiles take 461 us, 6144 about 480, 4096 (three CTAs per SM) 610.
+// 2^24 pairs: 8192-key tiles take 461 us, 6144 about 480, 4096 (three CTAs per SM) 610. The plan takes 148 SMs whatever the
+// device has: the scratch that a caller sized by it must not depend on the device that is current then and later (with
+// fewer SMs the chunks run in more than one wave, with the same results).
 struct SortPlan {
   uint32_t items, per_chunk, chunks;
   uint32_t short_segs;  // segments of at most kSegWindow keys go to k_sort_segments
@@ -663,7 +665,7 @@ struct SortPlan {
 SortPlan sort_plan(uint32_t n, uint32_t M) {
   constexpr uint32_t kSms = 148;
   SortPlan P;
-    P.items = n <= 2 * kSms * kScThreads * 4 ? 4 : (n <= 3 * kSms * kScThreads * 8 ? 8 : 16);
+  P.items = n <= 2 * kSms * kScThreads * 4 ? 4 : (n <= 3 * kSms * kScThreads * 8 ? 8 : 16);
   const uint32_t T = kScThreads * P.items, tiles = (uint32_t)(((uint64_t)n + T - 1) / T);
   const uint32_t per = P.items == 16 ? (tiles + 2 * kSms - 1) / (2 * kSms) : 1;
   P.per_chunk = per * T;
@@ -731,10 +733,10 @@ rt_status launch_segments(uint32_t* codes, uint32_t* idx, uint32_t n, uint32_t* 
 }
 
 // Few chunks of one segment: each CTA of a scatter launch counts all the keys for itself, and the count launch and its
-// zeroed sums go. 32-bit keys alone: 8192 45.2 -> 26.7 us, 16,384 45.3 -> 35.0, 30,000 45.8 -> 43.6, 40,000 46.1 -> 47.3
-// (one launch per pass with a look-back took 45.9, 47.8, 47.8, 49.8). The split levels read two codes per key: builds of
+// zeroed sums go. 32-bit keys alone: 4097 30.6 -> 19.8 us, 16,384 31.0 -> 24.8, 20,481 32.0 -> 26.7, 30,000 34.1 -> 36.0 (one
+// launch per pass with a look-back took 31.2, 33.3, 33.6 and 35.1). The split levels read two codes per key: builds of
 // 16,384 faces 153 -> 147 us, of 30,000 163 -> 172 with both.
-constexpr uint32_t kSelfCount = 16, kSelfCountLevels = 8;
+constexpr uint32_t kSelfCount = 12, kSelfCountLevels = 8;
 
 // The digit passes over chunked keys [0, 8 * passes) from begin_bit; the result is in keys and vals.
 rt_status chunked_passes(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_t begin_bit, uint32_t passes, int init_vals, const SortPlan& S,

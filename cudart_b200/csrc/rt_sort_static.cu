@@ -17,10 +17,11 @@
 //
 // Sharing: all calls (all streams, all threads) use the same array, which keeps
 // whatever the previous call left in it. Each sort first zeroes the part that
-// must start at zero (the sums of the chunks' digit counts) and writes every other word before reading it (the ping-pong key and
-// value buffers), so a call never sees the previous call's contents. Two calls that overlap
-// on the GPU (different streams, or host threads without ordering) race on the
-// array and corrupt each other's results; callers must serialize them.
+// must start at zero (the sums of the chunks' digit counts) and writes every
+// other word before reading it (the ping-pong key and value buffers), so a call
+// never sees the previous call's contents. Two calls that overlap on the GPU
+// (different streams, or host threads without ordering) race on the array and
+// corrupt each other's results; callers must serialize them.
 #include <mutex>
 
 #include "rt_common.cuh"

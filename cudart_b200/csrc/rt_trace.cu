@@ -418,18 +418,6 @@ __device__ __forceinline__ void trace_ray_accel(const uint32_t r, const TraceArg
 // are written by the lane whose key is the minimum right after its merge.
 constexpr int kCoopWarps = 4;  // 128-thread CTAs
 
-// The triangle tests of one warp-cooperative step. Each lane holds `mask`:
-// bit g set = group g of its leaf is to be tested, i.e. positions
-// first + kGroup g .. min(cnt, kGroup (g + 1)) - 1 + first of its mesh (whose
-// positions start at F in the triangle stream). The (ray, group) items of the
-// whole warp are spread over the 32 lanes: a lane tests one group against the
-// ray of the item's owner (fetched by shuffles) and merges its best hit into
-// the owner's slot with a 64-bit shared-memory atomicMin on (t bits, position),
-// the same (t, position) rule as the other schedules. The (u, v) of the
-// current best, and its t (a -0 keeps its sign, which the key drops), are
-// written by the lane whose key is the minimum right after its merge. key0 is this lane's best so far (t bits, position); on return
-// s_key[lane] / s_uvt[lane] hold the merged best of this lane's ray.
-//
 // A lane's best (u, v, t) in shared memory: in one word of 16 bytes, or (the two-child walk, 3 to 5% faster so) in two.
 template <bool kOne>
 struct CoopUvt {
@@ -450,6 +438,19 @@ struct CoopUvt<false> {
     u = a.x; v = a.y; t = y[i];
   }
 };
+
+// The triangle tests of one warp-cooperative step. Each lane holds `mask`:
+// bit g set = group g of its leaf is to be tested, i.e. positions
+// first + kGroup g .. min(cnt, kGroup (g + 1)) - 1 + first of its mesh (whose
+// positions start at F in the triangle stream). The (ray, group) items of the
+// whole warp are spread over the 32 lanes: a lane tests one group against the
+// ray of the item's owner (fetched by shuffles) and merges its best hit into
+// the owner's slot with a 64-bit shared-memory atomicMin on (t bits, position),
+// the same (t, position) rule as the other schedules. The (u, v) of the
+// current best, and its t (a -0 keeps its sign, which the key drops), are
+// written by the lane whose key is the minimum right after its merge. key0 is
+// this lane's best so far (t bits, position); on return s_key[lane] and
+// s_uvt[lane] hold the merged best of this lane's ray.
 template <uint32_t kGroup, class Uvt>
 __device__ __forceinline__ void coop_items(const uint32_t lane, const uint32_t mask, const uint32_t first, const uint32_t cnt,
                                            const uint32_t F, const float4& o, const float4& d, const float zu, const float zv,

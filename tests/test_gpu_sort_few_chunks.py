@@ -6,7 +6,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [4097, 6143, 6145, 16383, 16384, 16385, 32767, 32768, 32769])
+@pytest.mark.parametrize("n", [4097, 6143, 6145, 16383, 16384, 16385, 24575, 24576, 24577, 32769])
 @pytest.mark.parametrize("values", ["random", "equal", "few", "descending"])
 def test_against_torch(n, values):
     import torch
@@ -29,7 +29,7 @@ def test_against_torch(n, values):
         assert np.array_equal(a.cpu().numpy().view(np.uint32), k[order])
 
 
-@pytest.mark.parametrize("n", [4097, 16384, 16385, 32769])
+@pytest.mark.parametrize("n", [4097, 16384, 16385, 24576, 24577])
 def test_builds(oracle, n):
     import torch
     from cudart_b200 import core, scenes
