@@ -460,7 +460,7 @@ __global__ __launch_bounds__(kSegThreads) void k_sort_segments(uint32_t* __restr
   const uint32_t count = e - a, segs = m1 - m0, items = (count + kSegThreads - 1) / kSegThreads;
   if (count == 0 || items > (uint32_t)kSegItems) return;
   for (uint32_t i = tid; i < count; i += kSegThreads) {
-    k0[i] = __ldg(keys + a + i);
+    k0[i] = keys[a + i];
     v0[i] = (uint16_t)i;
     uint32_t lo = 0, hi = segs - 1;
     while (lo < hi) {
